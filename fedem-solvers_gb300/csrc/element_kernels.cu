@@ -97,14 +97,6 @@ __device__ inline void seedBackward(const BackwardSeed& b, int i) {
     const int base = atomicAdd(ctr + 1, nr);
     for (int k = 0; k < nr; ++k) queue[base + k] = b.roots[r0 + k];
     atomicAdd(ctr + 2, b.slotCnt[i]);
-    if (b.strideL > 0) {  // the large roots into the large-front queue
-      const int l0 = b.rootOffL[i], nl = b.rootOffL[i + 1] - l0;
-      int* ctrL = b.ctrL + 4 * q;
-      int* queueL = b.queueL + (size_t)q * b.strideL;
-      const int baseL = atomicAdd(ctrL + 1, nl);
-      for (int k = 0; k < nl; ++k) queueL[baseL + k] = b.rootsL[l0 + k];
-      atomicAdd(ctrL + 2, b.slotCntL[i]);
-    }
   }
 }
 

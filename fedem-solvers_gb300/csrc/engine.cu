@@ -892,7 +892,6 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
     // the block-per-front kernels; the warp kernels size their shared memory by
     // the small fronts only
     std::vector<unsigned char> large(nfr, 0);
-    std::vector<int> nLargeChild(nfr, 0);
     for (int f = 0; f < nfr; ++f) {
       if (nrow[f] > kLargeFrontRows) large[f] = 1;
       if (large[f] && parent[f] >= 0) large[parent[f]] = 1;  // parents follow their children
@@ -902,7 +901,6 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
       if (large[f]) {
         maxRowLarge = std::max(maxRowLarge, nrow[f]);
         ++nLargeFronts;
-        if (parent[f] >= 0) ++nLargeChild[parent[f]];
       } else {
         maxRowAll = std::max(maxRowAll, nrow[f]);
       }
@@ -913,10 +911,8 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
     }
     if (maxRowLarge >= 1024) { err = "front of 1024 rows or more"; return -905; }
     UPV(d_.fLarge, uint8_t, large);
-    UPV(d_.fNlarge, int, nLargeChild);
     pplan_.fLarge = d_.fLarge;
-    pplan_.fNlarge = d_.fNlarge;
-    pplan_.maxRowLarge = maxRowLarge;
+    pplan_.nLarge = nLargeFronts;
     // leaf-to-root path lengths: parents follow their children in each model's order
     std::vector<int> pathLen(nfr, 1);
     for (int f = nfr - 1; f >= 0; --f) {
@@ -925,19 +921,10 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
     }
     // tasks with the longest paths first: the cascades' critical paths (the
     // deep trees of the large models) start in the first wave of warps
-    std::vector<int> leaves, largeTasks;
-    for (int f = 0; f < nfr; ++f) {
+    std::vector<int> leaves;
+    for (int f = 0; f < nfr; ++f)
       if (nchild[f] == 0 && !large[f]) leaves.push_back(f);
-      if (large[f] && nLargeChild[f] == 0) largeTasks.push_back(f);
-    }
     std::stable_sort(leaves.begin(), leaves.end(), [&](int a, int b) { return pathLen[a] > pathLen[b]; });
-    std::stable_sort(largeTasks.begin(), largeTasks.end(), [&](int a, int b) { return pathLen[a] > pathLen[b]; });
-    if (!largeTasks.empty()) {
-      int* dLT = nullptr;
-      UPV(dLT, int, largeTasks);
-      pplan_.largeTasks = dLT;
-    }
-    pplan_.nLargeTasks = (int)largeTasks.size();
     int* dLeaves = nullptr;
     UPV(dLeaves, int, leaves);
     pplan_.leaves = dLeaves;
@@ -993,24 +980,13 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
       bwInline[f] = all ? 1 : 0;
     }
     // the warp queue starts at the tops of the small subtrees (roots, or fronts
-    // under a large parent); the large-front queue at the large roots, its
-    // chains ending at large fronts without large children
+    // under a large parent)
     auto smallTop = [&](int f) { return !large[f] && (parent[f] < 0 || large[parent[f]]); };
     std::vector<int> rootOff(nm + 1, 0), roots, leafCnt(nm, 0);
-    std::vector<int> rootOffL(nm + 1, 0), rootsL, chainL(nm, 0);
     for (int f = 0; f < nfr; ++f) {
       if (smallTop(f)) ++rootOff[fmodel[f] + 1];
       if (!large[f] && (bwInline[f] || (nchild[f] == 0 && !(parent[f] >= 0 && bwInline[parent[f]]))))
         ++leafCnt[fmodel[f]];
-      if (large[f] && parent[f] < 0) ++rootOffL[fmodel[f] + 1];
-      if (large[f] && nLargeChild[f] == 0) ++chainL[fmodel[f]];
-    }
-    for (int m = 0; m < nm; ++m) rootOffL[m + 1] += rootOffL[m];
-    rootsL.resize(rootOffL[nm]);
-    {
-      std::vector<int> fill(rootOffL.begin(), rootOffL.end() - 1);
-      for (int f = 0; f < nfr; ++f)
-        if (large[f] && parent[f] < 0) rootsL[fill[fmodel[f]]++] = f;
     }
     {
       unsigned char* dInline = nullptr;
@@ -1033,9 +1009,8 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
     // counters (4 per solve), the factorisation's per-front counters and one set
     // per refinement forward elimination (each + its leaf counter)
     const int nq = std::max(1, opt_.fp32Factor ? opt_.refineSweeps : 1);
-    // with large fronts: their queue counters (4 per solve) and per-front counters
-    // (factor + one set per refinement forward elimination) follow
-    const size_t largeInts = nLargeFronts > 0 ? 4 * (size_t)nq + (size_t)nq * (nfr + 1) : 0;
+    // with large fronts: their signals and barriers (PersistentPlan::cntLarge) follow
+    const size_t largeInts = (size_t)nLargeFronts * (2 + 3 * (size_t)nq);
     ctrInts_ = 4 + 4 * (size_t)nq + (size_t)nq * (nfr + 1) + largeInts;
     ctrBlock_ = alloc<int>(ctrInts_);
     if (!ctrBlock_) { err = "out of device memory (counters)"; return -906; }
@@ -1044,26 +1019,9 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
     pplan_.bwCtr = ctrBlock_ + 4;
     pplan_.cntFactor = ctrBlock_ + 4 + 4 * nq;
     pplan_.cntForward = pplan_.cntFactor + (nfr + 1);
+    pplan_.cntLarge = pplan_.cntFactor + (size_t)nq * (nfr + 1);
     pplan_.bwQueue = alloc<int>((size_t)nq * std::max<size_t>(leaves.size(), 1));
     queueInts_ = (size_t)nq * std::max<size_t>(leaves.size(), 1);
-    if (nLargeFronts > 0) {
-      pplan_.bwLCtr = pplan_.cntFactor + (size_t)nq * (nfr + 1);
-      pplan_.cntLargeFactor = pplan_.bwLCtr + 4 * nq;
-      pplan_.cntLargeForward = pplan_.cntLargeFactor + (nfr + 1);
-      pplan_.largeStride = std::max<int>((int)largeTasks.size(), 1);
-      pplan_.bwLQueue = alloc<int>((size_t)nq * pplan_.largeStride);
-      largeQueueInts_ = (size_t)nq * pplan_.largeStride;
-      int *dRootOffL = nullptr, *dRootsL = nullptr, *dChainL = nullptr;
-      UPV(dRootOffL, int, rootOffL);
-      UPV(dRootsL, int, rootsL);
-      UPV(dChainL, int, chainL);
-      seed_.strideL = pplan_.largeStride;
-      seed_.rootOffL = dRootOffL;
-      seed_.rootsL = dRootsL;
-      seed_.slotCntL = dChainL;
-      seed_.queueL = pplan_.bwLQueue;
-      seed_.ctrL = pplan_.bwLCtr;
-    }
     seed_.nq = nq;
     seed_.stride = (int)std::max<size_t>(leaves.size(), 1);
     seed_.rootOff = dRootOff;
@@ -1073,6 +1031,127 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
     seed_.ctr = pplan_.bwCtr;
     pplan_.errFlag = alloc<int>(1);
     d_.errFlag = pplan_.errFlag;
+    if (nLargeFronts > 0) {
+      // ---- large fronts: ordinals, maps, waves (front_large.cu) -----------------
+      const size_t elemB = opt_.fp32Factor ? 4 : 8;
+      std::vector<int> ordinal(nfr, -1), lf, lparent, level;
+      for (int f = 0; f < nfr; ++f)
+        if (large[f]) {
+          ordinal[f] = (int)lf.size();
+          lf.push_back(f);
+        }
+      const int nL = nLargeFronts;
+      lparent.assign(nL, -1);
+      level.assign(nL, 0);
+      std::vector<int64_t> invOff(nL);
+      std::vector<int> inv, asmCol, asmColOff(nL), diagAsm, diagOff(nL);
+      for (int li = 0; li < nL; ++li) {  // children precede their parents
+        const int f = lf[li];
+        if (parent[f] >= 0) {
+          lparent[li] = ordinal[parent[f]];
+          level[lparent[li]] = std::max(level[lparent[li]], level[li] + 1);
+        }
+        invOff[li] = (int64_t)inv.size();
+        for (int c = 0; c < nchild[f]; ++c) {
+          const int ch = childList[childOffV[f] + c];
+          const size_t base = inv.size();
+          inv.resize(base + nrow[f], -1);
+          for (int a = 0; a < nrow[ch] - npiv[ch]; ++a) inv[base + relIndex[relOffV[ch] + a]] = a;
+        }
+        // the original entries lie column by column
+        asmColOff[li] = (int)asmCol.size();
+        diagOff[li] = (int)diagAsm.size();
+        int k = 0;
+        for (int j = 0; j < npiv[f]; ++j) {
+          asmCol.push_back(k);
+          int diag = -1;
+          for (; k < nasmv[f] && asmPos[asmOffV[f] + k] / nrow[f] == j; ++k)
+            if (asmPos[asmOffV[f] + k] == j + nrow[f] * j) diag = (int)(asmOffV[f] + k);
+          if (diag < 0) { err = "front without a diagonal entry"; return -911; }
+          diagAsm.push_back(diag);
+        }
+        asmCol.push_back(k);
+        if (k != nasmv[f]) { err = "original entries not in column order"; return -911; }
+      }
+      LargePlan base;
+      base.err = pplan_.errFlag;
+      base.maxRow = (maxRowLarge + 3) & ~3;
+      {
+        int *dp = nullptr, *di = nullptr, *da = nullptr, *dao = nullptr, *dd = nullptr, *ddo = nullptr;
+        int64_t* dio = nullptr;
+        UPV(dp, int, lparent); UPV(di, int, inv); UPV(dio, int64_t, invOff); UPV(da, int, asmCol);
+        UPV(dao, int, asmColOff); UPV(dd, int, diagAsm); UPV(ddo, int, diagOff);
+        base.parent = dp; base.inv = di; base.invOff = dio; base.asmCol = da; base.asmColOff = dao;
+        base.diagAsm = dd; base.diagOff = ddo;
+      }
+      int sms = 0;
+      FG_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
+      const int levels = 1 + *std::max_element(level.begin(), level.end());
+      std::vector<std::vector<int>> byLevel(levels);
+      for (int li = 0; li < nL; ++li) byLevel[level[li]].push_back(li);
+      for (int shape = 0; shape < 5; ++shape) {
+        const bool solve = shape == 4;
+        const int cap = std::max(1, solve ? sms : sms * (2 << shape) / 16);
+        // blocks a front can use: factorisation, four trailing blocks of the first
+        // panel per thread block (one per sub-core); solves, 64 rows below the
+        // pivots per thread block, at most 8
+        auto wanted = [&](int li) {
+          const int f = lf[li], nr = nrow[f], np = npiv[f];
+          if (solve) return std::min(8, std::max(1, (nr - np + 63) / 64));
+          const int nb = (nr - std::min(32, np) + 15) / 16, tasks = nb * (nb + 1) / 2 * (opt_.fp32Factor ? 1 : 2);
+          return std::max(1, std::min(cap, (tasks + 3) / 4));
+        };
+        std::vector<LargeTask> tasks;
+        std::vector<int> expect(nL, 0);
+        int width = 1;
+        std::vector<std::vector<std::pair<int, int>>> waves;  // (ordinal, blocks)
+        for (int l = 0; l < levels; ++l) {
+          std::vector<int> order = byLevel[l];
+          std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return wanted(a) > wanted(b); });
+          for (size_t i0 = 0; i0 < order.size(); i0 += (size_t)cap) {
+            const size_t i1 = std::min(order.size(), i0 + (size_t)cap);
+            long long sum = 0;
+            for (size_t i = i0; i < i1; ++i) sum += wanted(order[i]);
+            std::vector<std::pair<int, int>> w;
+            int used = 0;
+            for (size_t i = i0; i < i1; ++i) {
+              // every front gets a block; the rest in proportion to what it can use
+              long long g = wanted(order[i]);
+              const int rest = cap - used - (int)(i1 - i - 1);
+              if (sum > cap) g = std::max<long long>(1, g * cap / sum);
+              g = std::min<long long>(g, rest);
+              w.push_back({order[i], (int)g});
+              used += (int)g;
+            }
+            width = std::max(width, used);
+            waves.push_back(w);
+          }
+        }
+        tasks.assign(waves.size() * (size_t)width, LargeTask{-1, 0, 0, 1});
+        for (size_t w = 0; w < waves.size(); ++w) {
+          int b = 0;
+          for (const auto& q : waves[w])
+            for (int r = 0; r < q.second; ++r) {
+              tasks[w * width + b++] = LargeTask{lf[q.first], q.first, r, q.second};
+              if (lparent[q.first] >= 0) ++expect[lparent[q.first]];
+              if (solve)
+                pplan_.large[4].stageCap =
+                    std::max(pplan_.large[4].stageCap,
+                             largeSolveStage(nrow[lf[q.first]], npiv[lf[q.first]], q.second, elemB));
+            }
+        }
+        const int64_t stageCap = pplan_.large[4].stageCap;
+        LargeTask* dt = nullptr;
+        int* de = nullptr;
+        UPV(dt, LargeTask, tasks); UPV(de, int, expect);
+        pplan_.large[shape] = base;
+        pplan_.large[shape].tasks = dt;
+        pplan_.large[shape].expect = de;
+        pplan_.large[shape].nWaves = (int)waves.size();
+        pplan_.large[shape].grid = width;
+        pplan_.large[shape].stageCap = stageCap;
+      }
+    }
   }
 #undef UPV
   trace.mark("queues and counters", stream_);
@@ -1251,7 +1330,8 @@ int Engine::timeFactor(int reps, double* msPerLaunch, double* bytes) {
   const size_t cntBytes = sizeof(int) * ((size_t)d_.nfrontTot + 1);
   auto clear = [&]() {
     cudaMemsetAsync(pplan_.cntFactor, 0, cntBytes, stream_);
-    if (pplan_.cntLargeFactor) cudaMemsetAsync(pplan_.cntLargeFactor, 0, cntBytes, stream_);
+    if (pplan_.nLarge > 0)  // the factorisation's and the first forward elimination's
+      cudaMemsetAsync(pplan_.cntLarge, 0, sizeof(int) * 3 * (size_t)pplan_.nLarge, stream_);
   };
   clear();
   enqueueFactor(stream_);  // warm-up
@@ -1321,7 +1401,8 @@ void Engine::ensureTuned() {
   if (iterated_ || d_.nfrontTot <= 0) return;
   if (autotune() != 0) {  // keep the defaults
     pplan_.factorPanel = 0;
-    pplan_.forwardWarps = pplan_.backwardWarps = pplan_.largeCluster = 8;
+    pplan_.forwardWarps = pplan_.backwardWarps = 8;
+    pplan_.largeCluster = 16;
   }
 }
 
@@ -1329,9 +1410,9 @@ int Engine::autotune() {
   const auto t0 = std::chrono::steady_clock::now();
   char key[256];
   snprintf(key, sizeof key, "dev%d f%d s%d r%d p%d L%d n%d l%d t%d", device_, opt_.fp32Factor ? 1 : 0,
-           opt_.refineSweeps, pplan_.maxRow, pplan_.maxNpiv, pplan_.maxRowLarge,
+           opt_.refineSweeps, pplan_.maxRow, pplan_.maxNpiv, pplan_.nLarge > 0 ? pplan_.large[4].maxRow : 0,
            (int)std::lround(std::log2((double)d_.nfrontTot + 1.0)), (int)std::lround(std::log2(pplan_.nLeaves + 1.0)),
-           pplan_.nLargeTasks > 0 ? (int)std::lround(std::log2(pplan_.nLargeTasks + 1.0)) : -1);
+           pplan_.nLarge > 0 ? (int)std::lround(std::log2(pplan_.nLarge + 1.0)) : -1);
   {
     std::lock_guard<std::mutex> lk(g_shapeMutex);
     auto it = g_shapeCache.find(key);
@@ -1386,19 +1467,18 @@ int Engine::autotune() {
     }
     pplan_.factorPanel = pick;
   }
-  // 2. large fronts: cluster size (the small cascade runs first, untimed)
-  if (ok && pplan_.nLargeTasks > 0) {
+  // 2. large fronts: share of the GPU (the small cascade runs first, untimed)
+  if (ok && pplan_.nLarge > 0) {
     float best = -1.f;
-    int pick = 8;
-    for (int c : {8, 4, 2, 16}) {
-      if (c > 8 && largeClusterCapacity(pplan_, f32, c) < 1) continue;  // not on this device
+    int pick = 16;
+    for (int c : {16, 8, 4, 2}) {
       pplan_.largeCluster = c;
       const float t = timeIt(
           [&] {
             resetIterationCounters(stream_);
             launchFactorForwardCascade(d_, pplan_, f32, rhs, stream_);
           },
-          [&] { launchLargeFactorForward(d_, pplan_, f32, rhs, stream_); });
+          [&] { launchLargeFactor(d_, pplan_, f32, stream_); });
       if (t < 0.f) ok = false;
       if (t >= 0.f && (best < 0.f || t < best)) best = t, pick = c;
     }
@@ -1475,7 +1555,8 @@ void Engine::enqueueFactor(cudaStream_t s, bool withBackward) {
   // factorisation and the first forward elimination in one cascade (small
   // fronts by warps, then the large fronts above them by thread blocks)
   launchFactorForwardCascade(d_, pplan_, opt_.fp32Factor, d_.del, s, withBackward, opt_.refineSweeps <= 1);
-  launchLargeFactorForward(d_, pplan_, opt_.fp32Factor, d_.del, s);
+  launchLargeFactor(d_, pplan_, opt_.fp32Factor, s);
+  launchLargeForward(d_, pplan_, opt_.fp32Factor, d_.del, 0, s);
 }
 
 // phase-timing events: external event nodes inside a captured graph, plain
@@ -1520,7 +1601,6 @@ void Engine::enqueueSolve(cudaStream_t s, bool timedForward, bool backwardDone) 
 void Engine::resetIterationCounters(cudaStream_t s) {
   cudaMemsetAsync(ctrBlock_, 0, sizeof(int) * ctrInts_, s);
   if (queueInts_) cudaMemsetAsync(pplan_.bwQueue, 0xff, sizeof(int) * queueInts_, s);
-  if (largeQueueInts_) cudaMemsetAsync(pplan_.bwLQueue, 0xff, sizeof(int) * largeQueueInts_, s);
 }
 
 // first half of a Newton iteration: step start (predictor) or the corrector's
@@ -1909,16 +1989,16 @@ int Engine::parkModels(const std::vector<int>& ms) {
 void Engine::enqueueIteration(cudaStream_t s) {
   enqueueAssembly(s);
   enqueueSolveUpdate(s);
-  const int nl = 1, sw = opt_.refineSweeps;
+  const int sw = opt_.refineSweeps;
   // kernels per batched iteration: 12 fixed (begin step, predict, elements x2, residual,
   // element Newton build + rotate (one fused kernel for compressed beams), CSR gather,
   // increment, norms partial + control, step end) + the factorisation with the first
   // forward elimination + per further solve a refinement residual and a forward
   // elimination + a back substitution per solve (the first solve's inside the
-  // factorisation's launch when fused)
-  const int solveLaunches = (2 * sw - 1 + (sw - 1)) * (pplan_.nLargeTasks > 0 ? 2 : 1) -
-                            (fuseBackward_ ? 1 : 0);
-  launchesPerIter_ = (d_.beamSparse ? 11 : 12) + nl * (pplan_.nLargeTasks > 0 ? 2 : 1) + solveLaunches +
+  // factorisation's launch when fused) + for large fronts their factorisation and a
+  // forward elimination and a back substitution per solve
+  launchesPerIter_ = (d_.beamSparse ? 11 : 12) + 1 + 2 * (sw - 1) + sw - (fuseBackward_ ? 1 : 0) +
+                     (pplan_.nLarge > 0 ? 1 + 2 * sw : 0) +
                      (d_.urQs ? 1 : 0) +
                      (d_.nmotTot > 0 ? 1 : 0) + (d_.nmrTot > 0 ? 1 : 0) + (d_.naxTot > 0 ? 3 : 0) +
                      (d_.nldTot > 0 ? 1 : 0) + (d_.njointTot > 0 ? 2 : 0) + (d_.ncxTot > 0 ? 3 : 0) +

@@ -92,9 +92,7 @@ struct DevData {
   int64_t *fRowOff, *fLOff, *fUOff, *fWOff, *fChildOff, *fRelOff, *fAsmOff;  // fUOff: the front's packed
                                                                             // update matrix in its parent's segment
   int *frontRows, *childList, *relIndex;
-  // large fronts (one thread block each) and every front's number of large children
-  uint8_t* fLarge;
-  int* fNlarge;
+  uint8_t* fLarge;  // large fronts (front_large.cu)
   // children's update rows of each front, in child order: W index and
   // (child ordinal << 16 | destination row), cgOff[f]..cgOff[f+1]
   int *cgOff, *cgSrc, *cgDst;

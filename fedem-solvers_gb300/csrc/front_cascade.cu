@@ -913,7 +913,7 @@ int stagingCapacity(const PersistentPlan& p, size_t elemBytes) {
 }
 
 bool fusableBackward(const PersistentPlan& p, bool fp32) {
-  return p.nLeaves > 0 && p.nLargeTasks == 0 &&
+  return p.nLeaves > 0 && p.nLarge == 0 &&
          (long long)stagingCapacity(p, fp32 ? sizeof(float) : sizeof(double)) >= (long long)p.maxRow * p.maxNpiv;
 }
 

@@ -3,48 +3,53 @@
 //
 // Large fronts are marked upward-closed on the host (every ancestor of a large
 // front is large), so the warp kernels of front_cascade.cu finish every small
-// subtree first and these kernels take the tops of the assembly trees:
-//   factor + forward: a cascade over the large fronts (clusters of blocks start
-//     at large fronts whose children are all small, a parent's counter
-//     completes on its last large child, the completing cluster climbs to it;
-//     nothing waits on another cluster);
-//   forward (refinement sweeps): the same cascade without the factorisation,
-//     one block per front;
-//   backward: a top-down work queue of large fronts seeded with the large roots
-//     (a block waits only for a slot that a running block fills), before the
-//     warp queue takes the small fronts below them.
+// subtree first and these kernels take the tops of the assembly trees.  Each
+// of the three passes (factorisation, forward elimination, back substitution)
+// is one cooperative launch of at most one block per SM.  The host lays the
+// fronts out in waves (fronts of one tree level, their blocks shared out by
+// work); a block walks its column of that table, so it always knows its next
+// front, its rank and the number of blocks working on it (LargeTask).  A front
+// starts when its large children (its parent, in the back substitution) have
+// signalled, and its blocks meet at barriers of their own; all blocks are
+// resident (cooperative launch), each wait is bounded and sets errFlag when it
+// runs out, after which every block runs to its end without waiting.
+//
+// Why whole-GPU fronts: a GB300 SM sub-core issues one FP64 instruction per 64
+// cycles whatever its active lanes, so one front's update on one cluster sets
+// the pace (space-frame tower, 15 fronts deep, FP64: 4.3 ms on clusters of 16
+// blocks that factored each panel redundantly; the split here is by entry, so
+// every sub-core of the GPU takes an equal share of a panel's update).
+//
 // A large front is factored in place in its outputs: its pivot columns in its
 // L block (nrow x npiv, column-major) and its trailing lower triangle in its
 // packed update matrix (column by column, inside the parent's segment), so no
-// workspace is needed.  Blocked right-looking LDL^T in panels of up to 32
-// pivots: each panel is factored in shared memory (its diagonal block by one
-// warp, the rows below it one per thread, no barrier inside), then the
-// trailing lower triangle is updated with it, C -= L_p D_p L_p^T, in 64 x 64
-// tiles (FP32 fronts: mma.sync TF32 products on the tensor cores in the 3xTF32
-// split; FP64 fronts: 4 x 4 register blocks), the tiles shared out over the blocks of a
-// thread-block cluster (GB300's FP64 units are thin: one front's update on one
-// SM would set the pace).  Semantics as the warp kernels and the reference's
-// SPRFC1/SPRFS1/SPRBS1 seam (solExtensionModule.f90:153-505): no pivoting, a
-// pivot is singular when |d_k| <= tolFactorize |a_kk|, negative pivots counted,
-// children's update matrices added in child order (fixed summation order).
-// Front data written by other threads or blocks are read through L2 (__ldcg).
-
-#include <cooperative_groups.h>
+// workspace is needed.  Blocked right-looking LDL^T in panels of 32 pivots:
+//   every block factors the panel's diagonal block itself (the same arithmetic,
+//     so the same values; cheaper than a broadcast);
+//   the rows below it are shared out, one warp per row, one lane per column;
+//   after a barrier the trailing triangle is updated, C -= L_p D_p L_p^T, in
+//     16 x 16 blocks, a warp each (FP32 fronts: mma.sync TF32 products on the
+//     tensor cores in the 3xTF32 split) or a warp per half (FP64 fronts).
+// Every entry's arithmetic is the same whichever block or warp does it, so the
+// result does not depend on the number of blocks.  Semantics as the warp
+// kernels and the reference's SPRFC1/SPRFS1/SPRBS1 seam
+// (solExtensionModule.f90:153-505): no pivoting, a pivot is singular when
+// |d_k| <= tolFactorize |a_kk|, negative pivots counted, children's update
+// matrices added in child order (fixed summation order).
+// Front data written in the same launch are read through L2 (__ldcg).
 
 #include <algorithm>
-#include <type_traits>
-
 #include <atomic>
+#include <type_traits>
 
 #include "kernels.h"
 
 namespace fgpu {
 namespace {
 
-namespace cg = cooperative_groups;
-
-constexpr int kLT = 256;         // threads per large-front block
-constexpr int kTile = 64;        // trailing-update tile (rows and columns)
+constexpr int kLT = 256;  // threads per block
+constexpr int kLW = kLT / 32;
+constexpr int kPanel = 32;  // pivots per panel
 
 // lower-triangle entry (ii >= jj) of an nu x nu matrix packed column by column
 __device__ inline int64_t packedAt(int ii, int jj, int nu) {
@@ -73,21 +78,55 @@ __device__ inline void st(T* p, T v) {
   __stcg(p, v);
 }
 
-// a barrier of all threads of the cluster, their global writes visible to
-// every thread of the cluster afterwards (each thread fences first)
-__device__ inline void clusterBarrier() {
-  __threadfence();
-  cg::this_cluster().sync();
+// ---- waits ------------------------------------------------------------------
+// Waits until *c >= target, bounded; every thread of the block calls it and
+// afterwards sees what the signalling blocks wrote (through L2).  Once a wait
+// has run out (here or in another block) it returns at once: `dead` stays set.
+struct WaitState {
+  int* err;
+  long long limit;
+  bool dead;
+};
+__device__ inline int acquireCount(const int* c) {
+  int v;
+  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];\n" : "=r"(v) : "l"(c) : "memory");
+  return v;
+}
+__device__ inline void signalCount(int* c) {
+  asm volatile("red.release.gpu.global.add.s32 [%0], 1;\n" ::"l"(c) : "memory");
+}
+__device__ inline void waitCount(const int* c, int target, WaitState& ws) {
+  bool out = false;
+  if (threadIdx.x == 0 && !ws.dead) {
+    long long spins = 0;
+    while (acquireCount(c) < target) {
+      ++spins;
+      if (spins > 256) __nanosleep(32);
+      if (spins > ws.limit || ((spins & 1023) == 0 && *(volatile const int*)ws.err)) {
+        atomicOr(ws.err, 1);
+        out = true;
+        break;
+      }
+    }
+  }
+  if (__syncthreads_or(out)) ws.dead = true;
+}
+// barrier of the G blocks of one front (phase: 1, 2, ... per front)
+__device__ inline void groupBarrier(int* bar, int G, int phase, WaitState& ws) {
+  if (G == 1) {
+    __syncthreads();
+    return;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) signalCount(bar);
+  waitCount(bar, G * phase, ws);
 }
 
-// ---- FP32 trailing tiles on the tensor cores --------------------------------
-// C(64 x 64 tile) -= A B with A(m, k) = P(r0 + m, k) and B(k, n) = P(c0 + n, k) d_k
-// (k < kb <= 32, zero beyond kb), as mma.sync m16n8k8 TF32 products with FP32
-// accumulation in the 3xTF32 split (x = hi + lo, both TF32; a b = hi hi + hi lo
-// + lo hi), which keeps the FP32 accuracy of the update.  Warp w takes rows
-// 16 (w & 3) .. +15 and columns 32 (w >> 2) .. +31 of the tile (four 16 x 8
-// products); fragment layouts of m16n8k8.row.col: lane = 4 g + t holds
-// A(g, t), A(g + 8, t), A(g, t + 4), A(g + 8, t + 4); B(t, g), B(t + 4, g);
+// ---- FP32 trailing blocks on the tensor cores ---------------------------------
+// mma.sync m16n8k8 TF32 products with FP32 accumulation in the 3xTF32 split
+// (x = hi + lo, both TF32; a b = hi hi + hi lo + lo hi), which keeps the FP32
+// accuracy of the update.  Fragment layouts of m16n8k8.row.col: lane = 4 g + t
+// holds A(g, t), A(g + 8, t), A(g, t + 4), A(g + 8, t + 4); B(t, g), B(t + 4, g);
 // C(g, 2t), C(g, 2t + 1), C(g + 8, 2t), C(g + 8, 2t + 1).
 __device__ inline uint32_t tf32Of(float x) {
   uint32_t r;
@@ -108,648 +147,702 @@ __device__ inline void mmaTf32(float* c, const uint32_t* a, const uint32_t* b) {
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
-// acc[j][q]: this thread's C fragment of the warp's j-th 16 x 8 product
-__device__ inline void tileUpdateMma(const float* P, int ldp, const float* dpan, int kb, int pr, int r0, int c0,
-                                     float acc[4][4]) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int g = lane >> 2, t = lane & 3;
-  const int rb = r0 + 16 * (w & 3), cb = c0 + 32 * (w >> 2);
+// shared memory of the factorisation: the panel's factored diagonal block
+// (Lt[k][i] = l_ik), its pivots, their reciprocals and the original diagonal,
+// the elimination's column buffers, and per warp the staged operand rows of one
+// trailing block (k-major: 16 rows, and 16 or 8 columns)
+template <typename T>
+struct FactorShared {
+  T Lt[kPanel][kPanel];
+  T d[kPanel], dinv[kPanel], diag0[kPanel];
+  T ubuf[2][kPanel];
+  T A[kLW][kPanel][16 + (sizeof(T) == 4 ? 4 : 0)];
+  T B[kLW][kPanel][std::is_same<T, float>::value ? 20 : 8];
+};
+
+// Partial LDL^T of the kb x kb diagonal block (lower triangle in s.Lt[col][row],
+// unscaled) by warps 0 to 3: columns c = 4 q + w in the registers of warp w, one
+// row per lane.  Each step publishes its column through shared memory; the four
+// warps then scale it and update their own columns, the next pivot's first.
+// The chain per pivot is one reciprocal, a product and a multiply-subtract (about
+// 0.3 us in FP64), so a second warp per sub-core would only queue behind it.
+template <typename T>
+__device__ void factorDiagonal(FactorShared<T>& s, int kb, double tolFact, int& neg, bool& sing) {
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (w < 4) {
+    T a[8];
 #pragma unroll
-  for (int j = 0; j < 4; ++j)
+    for (int q = 0; q < 8; ++q) {
+      const int c = 4 * q + w;
+      a[q] = (c < kb && lane < kb && lane >= c) ? s.Lt[c][lane] : T(0);
+    }
+    if (w == 0) s.ubuf[0][lane] = a[0];
+#pragma unroll
+    for (int k = 0; k < kPanel; ++k) {
+      if (k >= kb) break;
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      const T u = s.ubuf[k & 1][lane];
+      const T dk = s.ubuf[k & 1][k];
+      const bool bad = singularPivot(dk, s.diag0[k], tolFact);
+      const T inv = bad ? T(0) : T(1) / dk;
+      if (dk < T(0)) ++neg;
+      sing |= bad;
+      const T l = u * inv;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int c = 4 * q + w;
+        if (4 * q + 3 > k && c > k && c < kb) {
+          a[q] -= l * s.ubuf[k & 1][c];  // rows above the column hold unused values
+          if (c == k + 1) s.ubuf[(k + 1) & 1][lane] = a[q];
+        }
+      }
+      if ((k & 3) == w) {
+        s.Lt[k][lane] = lane > k ? l : T(0);
+        if (lane == 0) {
+          s.d[k] = dk;
+          s.dinv[k] = inv;
+        }
+      }
+    }
+  }
+  __syncthreads();
+}
+
+// one warp's 16 x 8 half of the trailing block (rows r0.., columns c0..; front
+// indices), FP64: lane = 8 lc + lr has rows lr, lr + 8 and columns lc, lc + 4
+__device__ inline void trailingBlock(const Front<double>& F, FactorShared<double>& s, int k0, int kb, int r0, int c0) {
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nr = F.nr;
+  double va[16], vb[8];
+#pragma unroll
+  for (int t = 0; t < 16; ++t) {
+    const int r = r0 + (lane & 15), k = 2 * t + (lane >> 4);
+    va[t] = (r < nr && k < kb) ? ld(F.L + r + (int64_t)nr * (k0 + k)) : 0.0;
+  }
+#pragma unroll
+  for (int t = 0; t < 8; ++t) {
+    const int c = c0 + (lane & 7), k = 4 * t + (lane >> 3);
+    vb[t] = (c < nr && k < kb) ? ld(F.L + c + (int64_t)nr * (k0 + k)) : 0.0;
+  }
+  const int lr = lane & 7, lc = lane >> 3;
+  double* dst[2][2];
+  double cur[2][2];
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      const int r = r0 + lr + 8 * a, c = c0 + lc + 4 * b;
+      dst[a][b] = (r < nr && r >= c) ? F.at(r, c) : nullptr;
+      cur[a][b] = dst[a][b] ? ld(dst[a][b]) : 0.0;
+    }
+  __syncwarp();
+#pragma unroll
+  for (int t = 0; t < 16; ++t) s.A[w][2 * t + (lane >> 4)][lane & 15] = va[t];
+#pragma unroll
+  for (int t = 0; t < 8; ++t) {
+    const int k = 4 * t + (lane >> 3);
+    s.B[w][k][lane & 7] = k < kb ? vb[t] * s.d[k] : 0.0;
+  }
+  __syncwarp();
+  double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+#pragma unroll 8
+  for (int k = 0; k < kb; ++k) {
+    const double a0 = s.A[w][k][lr], a1 = s.A[w][k][lr + 8], b0 = s.B[w][k][lc], b1 = s.B[w][k][lc + 4];
+    acc[0][0] += a0 * b0;
+    acc[0][1] += a0 * b1;
+    acc[1][0] += a1 * b0;
+    acc[1][1] += a1 * b1;
+  }
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+      if (dst[a][b]) st(dst[a][b], cur[a][b] - acc[a][b]);
+}
+
+// one warp's 16 x 16 trailing block, FP32 on the tensor cores
+__device__ inline void trailingBlock(const Front<float>& F, FactorShared<float>& s, int k0, int kb, int r0, int c0) {
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nr = F.nr;
+  float va[16], vb[16];
+#pragma unroll
+  for (int t = 0; t < 16; ++t) {
+    const int r = r0 + (lane & 15), c = c0 + (lane & 15), k = 2 * t + (lane >> 4);
+    va[t] = (r < nr && k < kb) ? ld(F.L + r + (int64_t)nr * (k0 + k)) : 0.0f;
+    vb[t] = (c < nr && k < kb) ? ld(F.L + c + (int64_t)nr * (k0 + k)) : 0.0f;
+  }
+  const int g = lane >> 2, t4 = lane & 3;
+  float* dst[2][4];
+  float cur[2][4];
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int r = r0 + g + 8 * (q >> 1), c = c0 + 8 * j + 2 * t4 + (q & 1);
+      dst[j][q] = (r < nr && c < nr && r >= c) ? F.at(r, c) : nullptr;
+      cur[j][q] = dst[j][q] ? ld(dst[j][q]) : 0.0f;
+    }
+  __syncwarp();
+#pragma unroll
+  for (int t = 0; t < 16; ++t) {
+    const int k = 2 * t + (lane >> 4);
+    s.A[w][k][lane & 15] = va[t];
+    s.B[w][k][lane & 15] = k < kb ? vb[t] * s.d[k] : 0.0f;
+  }
+  __syncwarp();
+  float acc[2][4];
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
 #pragma unroll
     for (int q = 0; q < 4; ++q) acc[j][q] = 0.0f;
-  for (int k0 = 0; k0 < kb; k0 += 8) {
-    const int ka = k0 + t, kc = k0 + t + 4;
-    auto av = [&](int r, int k) { return (r < pr && k < kb) ? P[k * ldp + r] : 0.0f; };
-    uint32_t ah[4], al[4];
-    split3(av(rb + g, ka), ah[0], al[0]);
-    split3(av(rb + g + 8, ka), ah[1], al[1]);
-    split3(av(rb + g, kc), ah[2], al[2]);
-    split3(av(rb + g + 8, kc), ah[3], al[3]);
-    const float da = ka < kb ? dpan[ka] : 0.0f, dc = kc < kb ? dpan[kc] : 0.0f;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int c = cb + 8 * j + g;
+  for (int kk = 0; kk < kPanel; kk += 8) {
+    if (kk >= kb) break;
+    uint32_t ah[4], al[4];
+    split3(s.A[w][kk + t4][g], ah[0], al[0]);
+    split3(s.A[w][kk + t4][g + 8], ah[1], al[1]);
+    split3(s.A[w][kk + t4 + 4][g], ah[2], al[2]);
+    split3(s.A[w][kk + t4 + 4][g + 8], ah[3], al[3]);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
       uint32_t bh[2], bl[2];
-      split3(av(c, ka) * da, bh[0], bl[0]);
-      split3(av(c, kc) * dc, bh[1], bl[1]);
+      split3(s.B[w][kk + t4][8 * j + g], bh[0], bl[0]);
+      split3(s.B[w][kk + t4 + 4][8 * j + g], bh[1], bl[1]);
       mmaTf32(acc[j], al, bh);
       mmaTf32(acc[j], ah, bl);
       mmaTf32(acc[j], ah, bh);
     }
   }
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (dst[j][q]) st(dst[j][q], cur[j][q] - acc[j][q]);
 }
 
-// Assembly (original entries, then the children's update matrices in child
-// order) and the blocked partial LDL^T of large front f by the blocks of a
-// cluster (crank of csize): the assembly is split over all their threads,
-// every block factors each panel itself (the same arithmetic, so the same
-// values) and takes its share of the trailing tiles; block 0 writes the panel
-// back and reports the pivots.  Shared memory: the panel P (kb <= 32 columns of
-// ldp rows, column-major: the panel's rows k0 .. nr-1), diag0 (np), dpan (kb).
+// Assembly of front f: entry (i, j) = the children's contributions in child
+// order, then the original entry.  Pulled by target through the children's
+// inverse row maps, so nothing waits between children: a warp takes 128 rows
+// of one column at a time.
 template <typename T>
-__device__ void factorLarge(const DevData& d, int f, const T* asmVal, T* Lbase, T* Ubase, double tolFact, T* P,
-                            int ldp, int kbMax, T* diag0, T* dpan, int crank, int csize) {
-  const int tid = threadIdx.x;
-  const int gtid = crank * kLT + tid, gstride = csize * kLT;
-  Front<T> F{Lbase + d.fLOff[f], Ubase + d.fUOff[f], d.fNrow[f], d.fNpiv[f], d.fNrow[f] - d.fNpiv[f]};
-  const int nr = F.nr, np = F.np, nu = F.nu;
-  const int64_t nL = (int64_t)nr * np, nU = (int64_t)nu * (nu + 1) / 2;
-  clusterBarrier();
-  for (int64_t k = gtid; k < nL; k += gstride) st(F.L + k, T(0));
-  for (int64_t k = gtid; k < nU; k += gstride) st(F.U + k, T(0));
-  clusterBarrier();
-  const int64_t ao = d.fAsmOff[f];
-  const int na = d.fNasm[f];
-  for (int k = gtid; k < na; k += gstride) {  // original entries: pivot columns only, distinct positions
-    const int p = __ldg(d.asmPos + ao + k);
-    st(F.L + p, __ldg(asmVal + ao + k));
-  }
-  clusterBarrier();
-  for (int k = tid; k < np; k += kLT) diag0[k] = ld(F.L + k + (int64_t)nr * k);
-  // extend-add, child by child (positions are distinct within one child)
-  const T* seg = Ubase + d.fSegOff[f];
-  const int* spos = d.segPos + d.fSegOff[f];
+__device__ void assembleLarge(const DevData& d, const LargePlan& lp, const LargeTask& t, const Front<T>& F,
+                              const T* asmVal, const T* Ubase) {
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nr = F.nr, np = F.np, f = t.f;
   const int nch = d.fNchild[f];
-  const int64_t co = d.fChildOff[f];
-  int64_t off = 0;
-  for (int c = 0; c < nch; ++c) {
-    const int ch = d.childList[co + c];
-    const int cu = d.fNrow[ch] - d.fNpiv[ch];
-    const int64_t len = (int64_t)cu * (cu + 1) / 2;
-    if (c > 0) clusterBarrier();
-    // four entries per thread at a time, every load issued before the stores
-    // (positions are distinct within one child)
-    for (int64_t k0 = gtid; k0 < len; k0 += 4 * (int64_t)gstride) {
-      T* q[4];
-      T sv[4], cur[4];
+  const int* chl = d.childList + d.fChildOff[f];
+  const int* inv = lp.inv + lp.invOff[t.li];
+  const int64_t ao = d.fAsmOff[f];
+  const int* colPtr = lp.asmCol + lp.asmColOff[t.li];
+  const int nrb = (nr + 127) >> 7;
+  for (int u = t.rank + t.G * w; u < nr * nrb; u += t.G * kLW) {
+    const int j = u / nrb, i0 = (u - j * nrb) << 7;
+    if (i0 + 127 < j) continue;
+    T v[4] = {T(0), T(0), T(0), T(0)};
+    for (int c = 0; c < nch; ++c) {
+      const int* ic = inv + (int64_t)c * nr;
+      const int b = __ldg(ic + j);
+      if (b < 0) continue;
+      const int ch = __ldg(chl + c);
+      const int cu = __ldg(d.fNrow + ch) - __ldg(d.fNpiv + ch);
+      const T* U = Ubase + __ldg(d.fUOff + ch) + ((int64_t)b * cu - (int64_t)b * (b - 1) / 2 - b);
+      int a[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int64_t k = k0 + (int64_t)u * gstride;
-        const int p = k < len ? (__ldg(spos + off + k) & 0xfffff) : -1;
-        q[u] = p >= 0 ? F.at(p % nr, p / nr) : nullptr;
-        sv[u] = p >= 0 ? ld(seg + off + k) : T(0);
+      for (int q = 0; q < 4; ++q) {
+        const int i = i0 + 32 * q + lane;
+        a[q] = (i < nr && i >= j) ? __ldg(ic + i) : -1;
       }
+      T x[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) cur[u] = q[u] ? ld(q[u]) : T(0);
+      for (int q = 0; q < 4; ++q) x[q] = a[q] >= 0 ? ld(U + a[q]) : T(0);
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (q[u]) st(q[u], cur[u] + sv[u]);
+      for (int q = 0; q < 4; ++q) v[q] += x[q];
     }
-    off += len;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int i = i0 + 32 * q + lane;
+      if (i < nr && i >= j) st(F.at(i, j), v[q]);
+    }
+    if (j < np) {
+      __syncwarp();
+      const int k1 = __ldg(colPtr + j + 1);
+      for (int k = __ldg(colPtr + j) + lane; k < k1; k += 32) {
+        const int i = __ldg(d.asmPos + ao + k) - nr * j;
+        if (i >= i0 && i < i0 + 128) {
+          T* q = F.L + i + (int64_t)nr * j;
+          st(q, ld(q) + ld(asmVal + ao + k));
+        }
+      }
+    }
   }
-  int neg = 0;
+}
+
+// Assembly and blocked partial LDL^T of large front t.f by its G blocks
+template <typename T>
+__device__ void factorLarge(const DevData& d, const LargePlan& lp, const LargeTask& t, const T* asmVal, T* Lbase,
+                            T* Ubase, double tolFact, FactorShared<T>& s, WaitState& ws) {
+  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+  const int f = t.f, G = t.G;
+  const Front<T> F{Lbase + d.fLOff[f], Ubase + d.fUOff[f], d.fNrow[f], d.fNpiv[f], d.fNrow[f] - d.fNpiv[f]};
+  const int nr = F.nr, np = F.np;
+  int* bar = lp.bar + t.li;
+  const int gw = t.rank + G * w, nw = G * kLW;  // warps numbered across the blocks first: one per sub-core
+  assembleLarge<T>(d, lp, t, F, asmVal, Ubase);
+  int phase = 0, neg = 0;
   bool sing = false;
-  for (int k0 = 0; k0 < np; k0 += kbMax) {
-    clusterBarrier();  // the panel's columns complete (assembly, earlier trailing updates)
-    const int kb = min(kbMax, np - k0), pr = nr - k0;  // panel columns and rows
-    for (int kk = 0; kk < kb; ++kk)
-      for (int r = tid; r < pr; r += kLT) P[kk * ldp + r] = ld(F.L + (k0 + r) + (int64_t)nr * (k0 + kk));
-    __syncthreads();
-    // the panel's kb x kb diagonal block, right-looking, by warp 0 alone: lane
-    // r owns row r; the unscaled value of each scaled entry (row r, column k) is
-    // kept in the unused upper triangle (row k, column r)
-    if (tid < 32) {
-      const int r = tid;
-      for (int kk = 0; kk < kb; ++kk) {
-        const T dk = P[kk * ldp + kk];
-        const bool bad = singularPivot(dk, diag0[k0 + kk], tolFact);
-        if (r == 0) {
-          sing |= bad;
-          if (dk < T(0)) ++neg;
-          dpan[kk] = dk;
-        }
-        const T inv = bad ? T(0) : T(1) / dk;
-        T l = T(0);
-        if (r > kk && r < kb) {
-          const T u = P[kk * ldp + r];
-          P[r * ldp + kk] = u;
-          l = u * inv;
-          P[kk * ldp + r] = l;
-        }
-        __syncwarp();
-        if (r > kk && r < kb)
-          for (int j = kk + 1; j <= r; ++j) P[j * ldp + r] -= l * P[j * ldp + kk];
-        __syncwarp();
-      }
+  for (int k0 = 0; k0 < np; k0 += kPanel) {
+    groupBarrier(bar, G, ++phase, ws);  // the panel's columns complete (assembly, earlier trailing updates)
+    const int kb = min(kPanel, np - k0);
+    for (int q = tid; q < kPanel * kPanel; q += kLT) {
+      const int c = q >> 5, r = q & 31;
+      if (c < kb && r < kb && r >= c) s.Lt[c][r] = ld(F.L + (k0 + r) + (int64_t)nr * (k0 + c));
     }
+    if (tid < kb) s.diag0[tid] = ld(asmVal + lp.diagAsm[lp.diagOff[t.li] + k0 + tid]);
+    // this warp's first row below the block, loaded beside the block's factorisation
+    const int rBelow = k0 + kb;
+    T a0 = T(0);
+    if (rBelow + gw < nr && lane < kb) a0 = ld(F.L + (rBelow + gw) + (int64_t)nr * (k0 + lane));
     __syncthreads();
-    // the panel's rows below the block, each on its own: for k in order,
-    // a = P(r, k) - sum_{j < k} l_rj u_kj, l_rk = a / d_k (the right-looking
-    // updates of the row, in the same order)
-    for (int r = kb + tid; r < pr; r += kLT) {
-      T lr[32];
-#pragma unroll
-      for (int kk = 0; kk < 32; ++kk) {
-        if (kk >= kb) break;
-        T a = P[kk * ldp + r];
-#pragma unroll
-        for (int j = 0; j < kk; ++j) a -= lr[j] * P[kk * ldp + j];
-        const bool bad = singularPivot(dpan[kk], diag0[k0 + kk], tolFact);
-        lr[kk] = a * (bad ? T(0) : T(1) / dpan[kk]);
+    factorDiagonal<T>(s, kb, tolFact, neg, sing);
+    // rows below the block: lane j holds column j; for k in order a_j -= a_k l_jk, then l_j = a_j / d_j
+    const T di = lane < kb ? s.dinv[lane] : T(0);
+    for (int r = rBelow + gw; r < nr; r += nw) {
+      T a = a0;
+      if (r + nw < nr && lane < kb) a0 = ld(F.L + (r + nw) + (int64_t)nr * (k0 + lane));
+      for (int k = 0; k < kb - 1; ++k) {
+        const T x = __shfl_sync(0xffffffffu, a, k);
+        a -= x * s.Lt[k][lane];  // zero at and above the diagonal
       }
-#pragma unroll
-      for (int kk = 0; kk < 32; ++kk) {
-        if (kk >= kb) break;
-        P[kk * ldp + r] = lr[kk];
-      }
+      if (lane < kb) st(F.L + r + (int64_t)nr * (k0 + lane), a * di);
     }
-    __syncthreads();
-    if (crank == 0)
-      for (int kk = 0; kk < kb; ++kk)
-        for (int r = kk + tid; r < pr; r += kLT) st(F.L + (k0 + r) + (int64_t)nr * (k0 + kk), P[kk * ldp + r]);
-    // trailing lower triangle, rows and columns k0 + kb .. nr-1 (panel-local
-    // kb .. pr-1): C(i, j) -= sum_k P(i, k) d_k P(j, k), tile by tile; a
-    // thread's 4 x 4 block is rows lr + 16 a and columns lc + 16 b of the tile
-    const int nt = pr - kb;
-    const int ntiles = (nt + kTile - 1) / kTile;
-    const int lr = tid & 15, lc = tid >> 4;
-    int tcount = 0;
-    for (int tj = 0; tj < ntiles; ++tj)
-      for (int ti = tj; ti < ntiles; ++ti) {
-        if (tcount++ % csize != crank) continue;  // this block's share of the tiles
-        const int r0 = kb + ti * kTile, c0 = kb + tj * kTile;
-        if constexpr (std::is_same<T, float>::value) {
-          // FP32 fronts: the tile's product on the tensor cores (3xTF32)
-          float acc[4][4];
-          tileUpdateMma(P, ldp, dpan, kb, pr, r0, c0, acc);
-          const int lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
-          // the tile's sixteen entries of this thread: every load before the stores
-          T* dst[4][4];
-          T cur[4][4];
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              const int r = r0 + 16 * (w & 3) + g + 8 * (q >> 1), c = c0 + 32 * (w >> 2) + 8 * j + 2 * t + (q & 1);
-              dst[j][q] = (r < pr && c < pr && r >= c) ? F.at(k0 + r, k0 + c) : nullptr;
-              cur[j][q] = dst[j][q] ? ld(dst[j][q]) : T(0);
-            }
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-              if (dst[j][q]) st(dst[j][q], cur[j][q] - acc[j][q]);
-        } else {
-          // FP64 fronts: 4 x 4 register blocks on the FP64 units
-          T acc[4][4];
-#pragma unroll
-          for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int b = 0; b < 4; ++b) acc[a][b] = T(0);
-          for (int kk = 0; kk < kb; ++kk) {
-            const T* Pk = P + kk * ldp;
-            const T dk = dpan[kk];
-            T av[4], bv[4];
-#pragma unroll
-            for (int a = 0; a < 4; ++a) {
-              const int r = r0 + lr + 16 * a;
-              av[a] = r < pr ? Pk[r] : T(0);
-            }
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-              const int c = c0 + lc + 16 * b;
-              bv[b] = c < pr ? Pk[c] * dk : T(0);
-            }
-#pragma unroll
-            for (int a = 0; a < 4; ++a)
-#pragma unroll
-              for (int b = 0; b < 4; ++b) acc[a][b] += av[a] * bv[b];
-          }
-          T* dst[4][4];
-          T cur[4][4];
-#pragma unroll
-          for (int b = 0; b < 4; ++b) {
-            const int c = c0 + lc + 16 * b;
-#pragma unroll
-            for (int a = 0; a < 4; ++a) {
-              const int r = r0 + lr + 16 * a;
-              dst[a][b] = (r < pr && c < pr && r >= c) ? F.at(k0 + r, k0 + c) : nullptr;
-              cur[a][b] = dst[a][b] ? ld(dst[a][b]) : T(0);
-            }
-          }
-#pragma unroll
-          for (int b = 0; b < 4; ++b)
-#pragma unroll
-            for (int a = 0; a < 4; ++a)
-              if (dst[a][b]) st(dst[a][b], cur[a][b] - acc[a][b]);
-        }
+    groupBarrier(bar, G, ++phase, ws);  // the panel's rows complete
+    // every block has read the unfactored diagonal block by now
+    if (t.rank == 0)
+      for (int q = tid; q < kPanel * kPanel; q += kLT) {
+        const int c = q >> 5, r = q & 31;
+        if (c < kb && r < kb && r >= c) st(F.L + (k0 + r) + (int64_t)nr * (k0 + c), r == c ? s.d[c] : s.Lt[c][r]);
       }
+    const int nt = nr - rBelow;
+    if (nt <= 0) break;
+    // trailing lower triangle in 16 x 16 blocks (row block rb >= column block cb)
+    constexpr int kHalves = std::is_same<T, float>::value ? 1 : 2;
+    const int nb = (nt + 15) >> 4, ntask = kHalves * (nb * (nb + 1) / 2);
+    for (int task = gw; task < ntask; task += nw) {
+      const int blk = task / kHalves, half = task % kHalves;
+      int rb = (int)((sqrtf(8.0f * (float)blk + 1.0f) - 1.0f) * 0.5f);
+      while ((rb + 1) * (rb + 2) / 2 <= blk) ++rb;
+      while (rb * (rb + 1) / 2 > blk) --rb;
+      const int cb = blk - rb * (rb + 1) / 2;
+      const int c0 = rBelow + 16 * cb + 8 * half;
+      if (c0 < nr) trailingBlock(F, s, k0, kb, rBelow + 16 * rb, c0);
+    }
   }
-  if (tid == 0 && crank == 0) {
+  if (tid == 0 && t.rank == 0) {
     const int m = d.fModel[f];
     if (neg) atomicAdd(&d.m.negPiv[m], neg);
     if (sing) atomicOr(&d.m.status[m], SS_SINGULAR);
   }
-  clusterBarrier();  // L block and update matrix complete
 }
 
-// forward elimination of large front f (v: nr values in shared memory), in
-// blocks of 32 pivots: warp 0 eliminates the block's unit lower triangle with
-// shuffles, then every thread updates its rows below the block with it
+// The waves of this block whose front's model has all of `want` in its flags,
+// as a mask in shared memory (kLT waves from `base`): one round of loads, so
+// that an iteration with nothing to do passes its waves at once.
+__device__ inline void scanWaves(const DevData& d, const LargePlan& lp, int base, int want, unsigned char* todo) {
+  const int wv = base + threadIdx.x;
+  bool on = false;
+  if (wv < lp.nWaves) {
+    const int f = lp.tasks[(int64_t)wv * gridDim.x + blockIdx.x].f;
+    on = f >= 0 && (d.m.flags[d.fModel[f]] & want) == want;
+  }
+  todo[threadIdx.x] = on ? 1 : 0;
+  __syncthreads();
+}
+
 template <typename T>
-__device__ void forwardLarge(const DevData& d, int f, const T* Lbase, const double* rhs, T* X, T* W, T* v,
-                             T* Ltri) {
-  const int tid = threadIdx.x, lane = tid & 31;
-  const int nr = d.fNrow[f], np = d.fNpiv[f], nu = nr - np;
+__global__ void __launch_bounds__(kLT) kLargeFactor(DevData d, LargePlan lp, const T* asmVal, T* Lbase, T* Ubase,
+                                                     double tolFact) {
+  pdlEntry();
+  extern __shared__ __align__(16) unsigned char smraw[];
+  FactorShared<T>& s = *reinterpret_cast<FactorShared<T>*>(smraw);
+  WaitState ws{lp.err, lp.spinLimit, false};
+  __shared__ unsigned char todo[kLT];
+  for (int wv = 0; wv < lp.nWaves; ++wv) {
+    if (wv % kLT == 0) scanWaves(d, lp, wv, FL_ACTIVE | FL_TANGENT, todo);
+    if (!todo[wv % kLT]) {
+      if (wv % kLT == kLT - 1) __syncthreads();
+      continue;
+    }
+    const LargeTask t = lp.tasks[(int64_t)wv * gridDim.x + blockIdx.x];
+    const int need = lp.expect[t.li];
+    if (need > 0) waitCount(lp.done + t.li, need, ws);
+    factorLarge<T>(d, lp, t, asmVal, Lbase, Ubase, tolFact, s, ws);
+    __syncthreads();
+    const int par = lp.parent[t.li];
+    if (threadIdx.x == 0 && par >= 0) signalCount(lp.done + par);
+  }
+}
+
+// ---- solves -----------------------------------------------------------------
+// asynchronous global -> shared copies of single elements
+template <typename T>
+__device__ inline void copyAsync(T* dstShared, const T* srcGlobal) {
+  const unsigned dst = (unsigned)__cvta_generic_to_shared(dstShared);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(dst), "l"(srcGlobal), "n"(sizeof(T)));
+}
+__device__ inline void copyAsyncWait() {
+  asm volatile("cp.async.commit_group;\n" ::);
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+}
+
+// values of L a block of the solves stages in shared memory: the pivot block
+// (np columns, an odd number of rows apart so that the back substitution's
+// reads across columns hit different banks) and its share of the rows below
+// (forward) or of the columns (backward)
+__host__ __device__ inline int64_t forwardStage(int nr, int np, int G) {
+  return (int64_t)np * (np | 1) + (int64_t)((nr - np + G - 1) / G) * np;
+}
+__host__ __device__ inline int64_t backwardStage(int nr, int np, int G) {
+  return (int64_t)np * (np | 1) + (int64_t)((np + G - 1) / G) * (nr - np);
+}
+
+// Forward elimination of front t.f, y = L11^-1 v_p, w = v_u - L21 y, by its G
+// blocks: each solves the pivot block itself (no barrier) and takes a slice of
+// the rows below it.  L does not depend on the children: it is staged in shared
+// memory while the block waits for them.  Rows below: a warp takes 32 rows and
+// a quarter of the pivots (a sub-core issues one FP64 instruction per 64
+// cycles, so the pivots are shared out too); the quarters are added in order.
+template <typename T>
+__device__ void forwardLarge(const DevData& d, const LargePlan& lp, const LargeTask& t, const T* Lbase,
+                             const double* rhs, T* X, T* W, T* v, T* part, T* Ls, WaitState& ws) {
+  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+  const int f = t.f, nr = d.fNrow[f], np = d.fNpiv[f], nu = nr - np;
+  const int share = (nu + t.G - 1) / t.G, r0 = np + t.rank * share, r1 = min(nr, r0 + share), ns = max(0, r1 - r0);
   const T* L = Lbase + d.fLOff[f];
   const int* rows = d.frontRows + d.fRowOff[f];
-  __syncthreads();
-  for (int r = tid; r < nr; r += kLT) v[r] = r < np ? (T)rhs[__ldg(rows + r)] : T(0);
-  const int nc = d.fNchild[f];
-  const int64_t co = d.fChildOff[f];
-  for (int c = 0; c < nc; ++c) {
-    __syncthreads();
-    const int ch = d.childList[co + c];
-    const int cu = d.fNrow[ch] - d.fNpiv[ch];
-    const T* wc = W + d.fWOff[ch];
-    const int* rel = d.relIndex + d.fRelOff[ch];
-    for (int a = tid; a < cu; a += kLT) v[__ldg(rel + a)] += ld(wc + a);
+  // pivot block at Ls[i + lds k], rows r0..r1-1 at Lr[(i - r0) + ns k]
+  const bool staged = forwardStage(nr, np, t.G) <= lp.stageCap;
+  const int lds = np | 1;
+  T* Lr = Ls + (int64_t)np * lds;
+  __syncthreads();  // the previous front's reads of the staging area are done
+  if (staged) {
+    for (int k = w; k < np; k += kLW) {
+      for (int i = k + lane; i < np; i += 32) copyAsync(Ls + i + lds * k, L + i + (int64_t)nr * k);
+      for (int i = lane; i < ns; i += 32) copyAsync(Lr + i + ns * k, L + r0 + i + (int64_t)nr * k);
+    }
   }
+  const T* Lp = staged ? Ls : L;
+  const int ldp = staged ? lds : nr;
+  const T* Lq = staged ? Lr : L + r0;
+  const int ldq = staged ? ns : nr;
+  const int nch = d.fNchild[f];
+  const int* chl = d.childList + d.fChildOff[f];
+  const int* inv = lp.inv + lp.invOff[t.li];
+  const int need = lp.expect[t.li];
+  if (need > 0) waitCount(lp.done + t.li, need, ws);
+  // the pivot rows' right-hand side and the children's contributions to the
+  // pivot rows and to this block's rows, in child order
+  for (int q = tid; q < np + ns; q += kLT) {
+    const int r = q < np ? q : r0 + q - np;
+    T x = q < np ? (T)rhs[__ldg(rows + r)] : T(0);
+    for (int c = 0; c < nch; ++c) {
+      const int a = __ldg(inv + (int64_t)c * nr + r);
+      if (a >= 0) x += ld(W + __ldg(d.fWOff + __ldg(chl + c)) + a);
+    }
+    v[q] = x;
+  }
+  if (staged) copyAsyncWait();
   __syncthreads();
   for (int b0 = 0; b0 < np; b0 += 32) {
     const int bs = min(32, np - b0);
-    if (tid < 32) {  // the block's triangle: lane r holds v[b0 + r]
-      // the triangle is staged in shared memory first (eight independent loads
-      // at a time), so that no step of the dependent chain below waits on a load
-      for (int k0 = 0; k0 < bs - 1; k0 += 8) {
-        T t[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int k = k0 + u;
-          t[u] = (k < bs - 1 && lane > k && lane < bs) ? ld(L + (b0 + lane) + (int64_t)nr * (b0 + k)) : T(0);
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) Ltri[(k0 + u) * 32 + lane] = t[u];
-      }
-      __syncwarp();
+    if (w == 0) {  // the block's unit triangle: lane r holds v[b0 + r]
       T x = lane < bs ? v[b0 + lane] : T(0);
-      for (int k = 0; k < bs - 1; ++k) {
-        const T yk = __shfl_sync(0xffffffffu, x, k);
-        if (lane > k && lane < bs) x -= Ltri[k * 32 + lane] * yk;
+      const T* Lb = Lp + b0 + (int64_t)ldp * b0;
+      if (staged) {
+#pragma unroll 4
+        for (int k = 0; k < bs - 1; ++k) {
+          const T l = lane > k && lane < bs ? Lb[lane + ldp * k] : T(0);
+          x -= l * __shfl_sync(0xffffffffu, x, k);
+        }
+      } else {
+        for (int k1 = 0; k1 < bs - 1; k1 += 8) {
+          T l[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            const int k = k1 + u;
+            l[u] = (k < bs - 1 && lane > k && lane < bs) ? Lb[lane + (int64_t)ldp * k] : T(0);
+          }
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+            if (k1 + u < bs - 1) x -= l[u] * __shfl_sync(0xffffffffu, x, k1 + u);
+        }
       }
       if (lane < bs) v[b0 + lane] = x;
     }
     __syncthreads();
-    for (int i = b0 + bs + tid; i < nr; i += kLT) {
-      T s = v[i];
-      for (int k0 = 0; k0 < bs; k0 += 8) {  // eight loads in flight, then the ordered updates
-        T t[8];
+    // the later pivot rows: four lanes a row, each a quarter of the block's pivots
+    const int left = np - b0 - bs;
+    for (int q = tid; q < ((4 * left + 31) & ~31); q += kLT) {
+      const int i = b0 + bs + (q >> 2), h = q & 3;
+      T a = T(0);
+      if (i < np)
+        for (int k = 8 * h; k < min(bs, 8 * h + 8); ++k) a += Lp[i + (int64_t)ldp * (b0 + k)] * v[b0 + k];
+      T sum = __shfl_sync(0xffffffffu, a, lane & ~3);
 #pragma unroll
-        for (int u = 0; u < 8; ++u) t[u] = k0 + u < bs ? ld(L + i + (int64_t)nr * (b0 + k0 + u)) : T(0);
-#pragma unroll
-        for (int u = 0; u < 8; ++u)
-          if (k0 + u < bs) s -= t[u] * v[b0 + k0 + u];
-      }
-      v[i] = s;
+      for (int o = 1; o < 4; ++o) sum += __shfl_sync(0xffffffffu, a, (lane & ~3) + o);
+      if (h == 0 && i < np) v[i] -= sum;
     }
     __syncthreads();
   }
-  for (int r = tid; r < np; r += kLT) X[__ldg(rows + r)] = v[r] / ld(L + r + (int64_t)nr * r);
-  T* wo = W + d.fWOff[f];
-  for (int a = tid; a < nu; a += kLT) st(wo + a, v[np + a]);
-}
-
-// after large front f: count it at its (large) parent; returns the parent when
-// this block completed the count, else -1
-__device__ inline int climbLarge(const DevData& d, const PersistentPlan& p, int f, int* cnt, int* shNext) {
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int next = -1;
-    const int par = d.fParent[f];
-    if (par >= 0) {
-      int old;
-      asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;\n" : "=r"(old) : "l"(cnt + par) : "memory");
-      if (old == p.fNlarge[par] - 1) next = par;
+  if (t.rank == 0)
+    for (int r = tid; r < np; r += kLT) st(X + __ldg(rows + r), v[r] / Lp[r + (int64_t)ldp * r]);
+  // rows below: quarter h of the pivots of 32 rows per warp, two row groups at a time
+  const int qn = (np + 3) >> 2;
+  T* wo = W + d.fWOff[f] + (r0 - np);
+  for (int g0 = 0; g0 < ns; g0 += 64) {
+    const int g = g0 + 32 * (w >> 2), h = w & 3, i = g + lane;
+    T a = T(0);
+    if (i < ns) {
+      const int ke = min(np, (h + 1) * qn);
+#pragma unroll 8
+      for (int k = h * qn; k < ke; ++k) a += Lq[i + (int64_t)ldq * k] * v[k];
     }
-    *shNext = next;
+    part[tid] = a;
+    __syncthreads();
+    if (h == 0 && i < ns) {
+      T sum = a;
+#pragma unroll
+      for (int o = 1; o < 4; ++o) sum += part[tid + 32 * o];
+      st(wo + i, v[np + i] - sum);
+    }
+    __syncthreads();
   }
-  __syncthreads();
-  return *shNext;
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kLT) kLargeFactorForward(DevData d, PersistentPlan p, const T* asmVal, T* Lbase,
-                                                            T* Ubase, double tolFact, const double* rhs, T* X, T* W,
-                                                            int* cnt, int doFactor, int panel) {
+__global__ void __launch_bounds__(kLT) kLargeForward(DevData d, LargePlan lp, const T* Lbase, const double* rhs, T* X,
+                                                      T* W) {
   pdlEntry();
   extern __shared__ __align__(16) unsigned char smraw[];
-  const int ldp = (p.maxRowLarge + 3) & ~3;
   T* v = reinterpret_cast<T*>(smraw);
-  T* diag0 = v + ldp;
-  T* dpan = diag0 + ldp;
-  T* Ltri = dpan + 32;  // 32 x 32 staging of a forward elimination's triangle
-  T* P = Ltri + 32 * 32;
-  __shared__ int shIdx, shNext;
-  cg::cluster_group cluster = cg::this_cluster();
-  const int crank = (int)cluster.block_rank(), csize = (int)cluster.num_blocks();
-  int* const next = cnt + d.nfrontTot;
-  for (;;) {
-    // block 0 of the cluster takes the task; every block reads it from there
-    if (crank == 0 && threadIdx.x == 0) shIdx = atomicAdd(next, 1);
-    cluster.sync();
-    const int idx = *cluster.map_shared_rank(&shIdx, 0);
-    cluster.sync();
-    if (idx >= p.nLargeTasks) break;
-    int f = p.largeTasks[idx];
-    const int fl = d.m.flags[d.fModel[f]];
-    const bool factor = doFactor && (fl & FL_TANGENT);
-    while ((fl & FL_ACTIVE) && f >= 0) {
-      if (factor) factorLarge<T>(d, f, asmVal, Lbase, Ubase, tolFact, P, ldp, panel, diag0, dpan, crank, csize);
-      if (crank == 0) {
-        forwardLarge<T>(d, f, Lbase, rhs, X, W, v, Ltri);
-        f = climbLarge(d, p, f, cnt, &shNext);
+  T* part = v + lp.maxRow;
+  T* Ls = part + kLT;
+  WaitState ws{lp.err, lp.spinLimit, false};
+  __shared__ unsigned char todo[kLT];
+  for (int wv = 0; wv < lp.nWaves; ++wv) {
+    if (wv % kLT == 0) scanWaves(d, lp, wv, FL_ACTIVE, todo);
+    if (!todo[wv % kLT]) {
+      if (wv % kLT == kLT - 1) __syncthreads();
+      continue;
+    }
+    const LargeTask t = lp.tasks[(int64_t)wv * gridDim.x + blockIdx.x];
+    forwardLarge<T>(d, lp, t, Lbase, rhs, X, W, v, part, Ls, ws);
+    __syncthreads();
+    const int par = lp.parent[t.li];
+    if (threadIdx.x == 0 && par >= 0) signalCount(lp.done + par);
+  }
+}
+
+// Back substitution of front t.f, x_p = L11^-T (v_p - L21^T x_u), waves taken
+// from the last: its blocks share out the pivot columns (a warp per column),
+// block 0 then solves the pivot block and signals the children.  L is staged
+// while the block waits for the parent.
+template <typename T>
+__device__ void backwardLarge(const DevData& d, const LargePlan& lp, const LargeTask& t, const T* Lbase, T* X, int acc,
+                              int finalize, T* xs, T* part, T* Ls, WaitState& ws) {
+  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+  const int f = t.f, nr = d.fNrow[f], np = d.fNpiv[f], nu = nr - np;
+  const T* L = Lbase + d.fLOff[f];
+  const int* rows = d.frontRows + d.fRowOff[f];
+  const int cshare = (np + t.G - 1) / t.G, k0 = t.rank * cshare, k1 = min(np, k0 + cshare), nc = max(0, k1 - k0);
+  const bool staged = backwardStage(nr, np, t.G) <= lp.stageCap;
+  const int lds = np | 1;
+  T* Lc = Ls + (t.rank == 0 ? (int64_t)np * lds : 0);  // columns k0..k1-1 below the pivot block, nu values each
+  __syncthreads();
+  if (staged) {
+    for (int k = w; k < nc; k += kLW)
+      for (int i = lane; i < nu; i += 32) copyAsync(Lc + i + nu * k, L + np + i + (int64_t)nr * (k0 + k));
+    if (t.rank == 0)
+      for (int k = w; k < np; k += kLW)
+        for (int i = k + 1 + lane; i < np; i += 32) copyAsync(Ls + i + lds * k, L + i + (int64_t)nr * k);
+  }
+  const T* Lq = staged ? Lc : L + np + (int64_t)nr * k0;
+  const int ldq = staged ? nu : nr;
+  const int par = lp.parent[t.li];
+  if (par >= 0) waitCount(lp.done + par, 1, ws);
+  for (int r = np + tid; r < nr; r += kLT) xs[r] = ld(X + __ldg(rows + r));
+  if (staged) copyAsyncWait();
+  __syncthreads();
+  for (int k = w; k < nc; k += kLW) {
+    T a = T(0);
+#pragma unroll 4
+    for (int i = lane; i < nu; i += 32) a += Lq[i + (int64_t)ldq * k] * xs[np + i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+    if (lane == 0) {
+      T* q = X + __ldg(rows + k0 + k);
+      st(q, ld(q) - a);
+    }
+  }
+  __syncthreads();
+  if (t.rank != 0) {
+    if (tid == 0) signalCount(lp.bar + t.li);
+    return;
+  }
+  if (t.G > 1) waitCount(lp.bar + t.li, t.G - 1, ws);
+  for (int r = tid; r < np; r += kLT) xs[r] = ld(X + __ldg(rows + r));
+  __syncthreads();
+  const T* Lp = staged ? Ls : L;
+  const int ldp = staged ? lds : nr;
+  // the unit upper triangle L11^T, blocks of 32 pivots from the last: warp 0
+  // solves the block with shuffles, then the pivots above it are updated with
+  // the block's values
+  for (int bEnd = np; bEnd > 0; bEnd -= 32) {
+    const int b0 = bEnd > 32 ? bEnd - 32 : 0, bs = bEnd - b0;
+    if (w == 0) {
+      T x = lane < bs ? xs[b0 + lane] : T(0);
+      const T* Lb = Lp + b0 + (int64_t)ldp * (b0 + (lane < bs ? lane : 0));
+      if (staged) {
+#pragma unroll 4
+        for (int j = bs - 1; j > 0; --j) {
+          const T l = lane < j ? Lb[j] : T(0);
+          x -= l * __shfl_sync(0xffffffffu, x, j);
+        }
+      } else {
+        for (int j1 = bs - 1; j1 > 0; j1 -= 8) {
+          T l[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) l[u] = (j1 - u > 0 && lane < j1 - u) ? Lb[j1 - u] : T(0);
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+            if (j1 - u > 0) x -= l[u] * __shfl_sync(0xffffffffu, x, j1 - u);
+        }
       }
-      cluster.sync();
-      f = *cluster.map_shared_rank(&shNext, 0);
-      cluster.sync();
+      if (lane < bs) xs[b0 + lane] = x;
+    }
+    __syncthreads();
+    // pivots above the block: four lanes a pivot, each a quarter of the block's rows
+    for (int q = tid; q < ((4 * b0 + 31) & ~31); q += kLT) {
+      const int k = q >> 2, h = q & 3;
+      T a = T(0);
+      if (k < b0)
+        for (int j = 8 * h; j < min(bs, 8 * h + 8); ++j) a += Lp[b0 + j + (int64_t)ldp * k] * xs[b0 + j];
+      T sum = __shfl_sync(0xffffffffu, a, lane & ~3);
+#pragma unroll
+      for (int o = 1; o < 4; ++o) sum += __shfl_sync(0xffffffffu, a, (lane & ~3) + o);
+      if (h == 0 && k < b0) xs[k] -= sum;
+    }
+    __syncthreads();
+  }
+  for (int r = tid; r < np; r += kLT) st(X + __ldg(rows + r), xs[r]);
+  __syncthreads();
+  if (tid == 0) signalCount(lp.done + t.li);
+  for (int r = tid; r < np; r += kLT) {
+    const int row = __ldg(rows + r);
+    const T x = xs[r];
+    if (acc == 0) {
+      d.del[row] = (double)x;
+    } else {
+      const double xr = acc == 1 ? (double)x : d.xref[row] + (double)x;
+      d.xref[row] = xr;
+      if (finalize) d.del[row] = xr;
     }
   }
 }
 
-// Top-down queue of large fronts (see front_cascade.cu's kBackwardQueue for
-// the protocol): a block takes the next slot, waits (bounded) until a front is
-// stored there, solves it, stores its large children but the first in fresh
-// slots and continues with the first; the small children are left to the warp
-// queue launched afterwards.  acc as kBackwardQueue.
 template <typename T>
-__global__ void __launch_bounds__(kLT) kLargeBackward(DevData d, PersistentPlan p, const T* Lbase, T* X, int* queue,
-                                                       int* ctr, int* errFlag, int acc, int finalize) {
+__global__ void __launch_bounds__(kLT) kLargeBackward(DevData d, LargePlan lp, const T* Lbase, T* X, int acc,
+                                                       int finalize) {
   pdlEntry();
   extern __shared__ __align__(16) unsigned char smraw[];
   T* xs = reinterpret_cast<T*>(smraw);
-  T* Ltri = xs + ((p.maxRowLarge + 3) & ~3);  // 32 x 32 staging of a block's triangle
-  __shared__ int shSlot, shF, shOk;
-  const int tid = threadIdx.x;
-  const int w = tid >> 5, lane = tid & 31;
-  const int total = *(volatile const int*)(ctr + 2);
-  for (;;) {
-    if (tid == 0) shSlot = atomicAdd(ctr, 1);
-    __syncthreads();
-    const int slot = shSlot;
-    __syncthreads();
-    if (slot >= total) break;
-    if (tid == 0) {
-      int f = -1, ok = 1;
-      long long spins = 0;
-      while ((f = *(volatile const int*)(queue + slot)) < 0) {
-        __nanosleep(32);
-        if (++spins > p.spinLimit) {
-          atomicOr(errFlag, 1);
-          ok = 0;
-          break;
-        }
-      }
-      __threadfence();
-      shF = f;
-      shOk = ok;
+  T* part = xs + lp.maxRow;
+  T* Ls = part + kLT;
+  WaitState ws{lp.err, lp.spinLimit, false};
+  __shared__ unsigned char todo[kLT];
+  for (int wv = lp.nWaves - 1; wv >= 0; --wv) {
+    if (wv == lp.nWaves - 1 || wv % kLT == kLT - 1) {
+      __syncthreads();
+      scanWaves(d, lp, wv - wv % kLT, FL_ACTIVE, todo);
     }
-    __syncthreads();
-    int f = shF;
-    if (!shOk) break;
-    while (f >= 0) {
-      const int nr = d.fNrow[f], np = d.fNpiv[f];
-      const T* L = Lbase + d.fLOff[f];
-      const int* rows = d.frontRows + d.fRowOff[f];
-      for (int r = tid; r < nr; r += kLT) xs[r] = ld(X + __ldg(rows + r));
-      __syncthreads();
-      // the update rows' contribution for every pivot: one warp per pivot, the
-      // lanes over the rows in a fixed pattern, a fixed shuffle tree
-      for (int k = w; k < np; k += kLT / 32) {
-        T a = T(0);
-        for (int i = np + lane; i < nr; i += 32) a += ld(L + i + (int64_t)nr * k) * xs[i];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
-        if (lane == 0) xs[k] -= a;
-      }
-      __syncthreads();
-      // the unit upper triangle L11^T, blocks of 32 pivots from the last: warp
-      // 0 solves the block with shuffles, then the pivots above it are updated
-      // with the block's values (one warp per pivot)
-      for (int bEnd = np; bEnd > 0; bEnd -= 32) {
-        const int b0 = bEnd > 32 ? bEnd - 32 : 0, bs = bEnd - b0;
-        if (tid < 32) {
-          // lane r's column of the triangle staged first (rows j > r), eight
-          // independent loads at a time
-          for (int j0 = 0; j0 < bs; j0 += 8) {
-            T t[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-              const int j = j0 + u;
-              t[u] = (j < bs && lane < j) ? ld(L + (b0 + j) + (int64_t)nr * (b0 + lane)) : T(0);
-            }
-#pragma unroll
-            for (int u = 0; u < 8; ++u) Ltri[(j0 + u) * 32 + lane] = t[u];
-          }
-          __syncwarp();
-          T x = lane < bs ? xs[b0 + lane] : T(0);
-          for (int j = bs - 1; j > 0; --j) {
-            const T xj = __shfl_sync(0xffffffffu, x, j);
-            if (lane < j) x -= Ltri[j * 32 + lane] * xj;
-          }
-          if (lane < bs) xs[b0 + lane] = x;
-        }
-        __syncthreads();
-        for (int k = w; k < b0; k += kLT / 32) {
-          T a = lane < bs ? ld(L + (b0 + lane) + (int64_t)nr * k) * xs[b0 + lane] : T(0);
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
-          if (lane == 0) xs[k] -= a;
-        }
-        __syncthreads();
-      }
-      for (int r = tid; r < np; r += kLT) {
-        const int row = __ldg(rows + r);
-        const T x = xs[r];
-        st(X + row, x);
-        if (acc == 0) {
-          d.del[row] = (double)x;
-        } else {
-          const double xr = acc == 1 ? (double)x : d.xref[row] + (double)x;
-          d.xref[row] = xr;
-          if (finalize) d.del[row] = xr;
-        }
-      }
-      __threadfence();
-      __syncthreads();
-      // large children: the first continues here, the others go to fresh slots
-      const int nch = d.fNchild[f];
-      const int* chl = d.childList + d.fChildOff[f];
-      if (tid == 0) {
-        int first = -1, nl = 0;
-        for (int c = 0; c < nch; ++c)
-          if (p.fLarge[chl[c]]) {
-            if (first < 0) first = chl[c];
-            else ++nl;
-          }
-        if (nl > 0) {
-          int base = atomicAdd(ctr + 1, nl);
-          bool skip = true;
-          for (int c = 0; c < nch; ++c)
-            if (p.fLarge[chl[c]]) {
-              if (skip) { skip = false; continue; }
-              atomicExch(queue + base++, chl[c]);
-            }
-        }
-        shF = first;
-      }
-      __syncthreads();
-      f = shF;
-      __syncthreads();
-    }
+    if (!todo[wv % kLT]) continue;
+    const LargeTask t = lp.tasks[(int64_t)wv * gridDim.x + blockIdx.x];
+    backwardLarge<T>(d, lp, t, Lbase, X, acc, finalize, xs, part, Ls, ws);
   }
 }
 
-int smCount() {
-  // engines may be built on several host threads at once
-  static std::atomic<int> cached{0};
-  int n = cached.load(std::memory_order_relaxed);
-  if (n == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    if (n <= 0) n = 1;
-    cached.store(n, std::memory_order_relaxed);
-  }
-  return n;
-}
-
-template <typename K>
-int gridFor(K kernel, size_t smem, int needed) {
-  int perSm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, kLT, smem) != cudaSuccess || perSm < 1) perSm = 1;
-  const int cap = perSm * smCount();
-  return needed < 1 ? 1 : (needed < cap ? needed : cap);
-}
-
-template <typename K>
-void bigSmem(K kernel, size_t bytes) {
-  if (bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
-
-// panel width: 32 pivots, fewer when the panel of the largest front would not
-// fit the shared memory (about 200 KB)
-template <typename T>
-int panelWidth(int maxRow) {
-  const size_t ldp = (size_t)((maxRow + 3) & ~3);
-  int kb = 32;
-  while (kb > 4 && (2 * ldp + 32 + 32 * 32 + (size_t)kb * ldp) * sizeof(T) > 200 * 1024) kb -= 4;
-  return kb;
-}
-
-// clusters of csize blocks the device can hold at once with the factorisation's
-// shared memory (0: none; sizes above 8 need the non-portable cluster opt-in)
-template <typename T>
-int largeClusterCapacity(const PersistentPlan& p, int csize) {
-  const size_t ldp = (size_t)((p.maxRowLarge + 3) & ~3);
-  const int kb = panelWidth<T>(p.maxRowLarge);
-  const size_t sm = (2 * ldp + 32 + 32 * 32 + (size_t)kb * ldp) * sizeof(T);
-  bigSmem(kLargeFactorForward<T>, sm);
-  if (csize > 8 && cudaFuncSetAttribute(kLargeFactorForward<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-                       cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  cudaLaunchConfig_t cfg = {};
+// cooperative launch (all blocks resident), ordered like any launch of the stream
+template <typename... KArgs, typename... Args>
+void coopLaunch(void (*kernel)(KArgs...), int grid, size_t smem, cudaStream_t s, Args... args) {
+  if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = csize;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.blockDim = dim3(kLT);
-  cfg.dynamicSmemBytes = sm;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cfg.gridDim = dim3(csize);
-  int clusters = 0;
-  if (cudaOccupancyMaxActiveClusters(&clusters, kLargeFactorForward<T>, &cfg) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  return clusters;
-}
-
-// Factorisations run as clusters of p.largeCluster blocks per front (a grid of
-// as many clusters as fit at once, at most one per start task); forward
-// eliminations alone as single blocks.
-template <typename T>
-void factorForwardLarge(const DevData& d, const PersistentPlan& p, const T* asmVal, T* L, T* U, const double* rhs,
-                        T* X, T* W, int* cnt, bool factor, cudaStream_t s) {
-  const size_t ldp = (size_t)((p.maxRowLarge + 3) & ~3);
-  const int kb = panelWidth<T>(p.maxRowLarge);
-  const size_t sm = (2 * ldp + 32 + 32 * 32 + (factor ? (size_t)kb * ldp : 0)) * sizeof(T);
-  bigSmem(kLargeFactorForward<T>, sm);
-  if (!factor) {
-    const int grid = gridFor(kLargeFactorForward<T>, sm, p.nLargeTasks);
-    pdlLaunch(kLargeFactorForward<T>, grid, kLT, sm, s, d, p, asmVal, L, U, 1.0e-12, rhs, X, W, cnt, 0, kb);
-    return;
-  }
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  int csize = p.largeCluster;
-  // 16 blocks per cluster is beyond the portable size: allowed per kernel, and
-  // only taken when the device can hold such a cluster with this shared memory
-  if (csize > 8 && largeClusterCapacity<T>(p, csize) < 1) csize = 8;
-  attr[0].val.clusterDim.x = csize;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(kLT);
-  cfg.dynamicSmemBytes = sm;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cfg.attrs = attr;
-  cfg.numAttrs = 2;
-  cfg.gridDim = dim3(csize * p.nLargeTasks);
-  int clusters = 0;
-  if (cudaOccupancyMaxActiveClusters(&clusters, kLargeFactorForward<T>, &cfg) != cudaSuccess || clusters < 1)
-    clusters = 1;
-  clusters = std::min(clusters, p.nLargeTasks);
-  cfg.gridDim = dim3(csize * clusters);
-  cudaLaunchKernelEx(&cfg, kLargeFactorForward<T>, d, p, asmVal, L, U, 1.0e-12, rhs, X, W, cnt, 1, kb);
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+template <typename T>
+size_t solveShared(const LargePlan& lp) {
+  return (size_t)(lp.maxRow + kLT + lp.stageCap) * sizeof(T);
 }
 
 }  // namespace
 
-int largeClusterCapacity(const PersistentPlan& p, bool fp32, int csize) {
-  if (p.nLargeTasks <= 0) return 0;
-  return fp32 ? largeClusterCapacity<float>(p, csize) : largeClusterCapacity<double>(p, csize);
+// at most about 200 KB of staged L per block
+int64_t largeSolveStage(int nr, int np, int G, size_t elemBytes) {
+  const int64_t want = std::max(forwardStage(nr, np, G), backwardStage(nr, np, G));
+  return std::min<int64_t>(want, (int64_t)(200 * 1024 / elemBytes));
 }
 
-void launchLargeFactorForward(const DevData& d, const PersistentPlan& p, bool fp32, const double* rhs,
-                              cudaStream_t s) {
-  if (p.nLargeTasks <= 0) return;
-  if (fp32) factorForwardLarge<float>(d, p, d.asmVal32, d.L32, d.U32, rhs, d.x32, d.w32, p.cntLargeFactor, true, s);
-  else factorForwardLarge<double>(d, p, d.asmVal64, d.L64, d.U64, rhs, d.x64, d.w64, p.cntLargeFactor, true, s);
+void launchLargeFactor(const DevData& d, const PersistentPlan& p, bool fp32, cudaStream_t s) {
+  if (p.nLarge <= 0) return;
+  int shape = 0;
+  for (int k = 0; k < 4; ++k)
+    if (p.largeCluster == (2 << k)) shape = k;
+  LargePlan lp = p.large[shape];
+  lp.spinLimit = p.spinLimit;
+  lp.done = p.cntLarge;
+  lp.bar = p.cntLarge + p.nLarge;
+  if (fp32)
+    coopLaunch(kLargeFactor<float>, lp.grid, sizeof(FactorShared<float>), s, d, lp, (const float*)d.asmVal32, d.L32,
+               d.U32, 1.0e-12);
+  else
+    coopLaunch(kLargeFactor<double>, lp.grid, sizeof(FactorShared<double>), s, d, lp, (const double*)d.asmVal64, d.L64,
+               d.U64, 1.0e-12);
 }
 
 void launchLargeForward(const DevData& d, const PersistentPlan& p, bool fp32, const double* rhs, int sweep,
                         cudaStream_t s) {
-  if (p.nLargeTasks <= 0) return;
-  int* cnt = p.cntLargeForward + (size_t)(sweep - 1) * ((size_t)d.nfrontTot + 1);
-  if (fp32) factorForwardLarge<float>(d, p, d.asmVal32, d.L32, d.U32, rhs, d.x32, d.w32, cnt, false, s);
-  else factorForwardLarge<double>(d, p, d.asmVal64, d.L64, d.U64, rhs, d.x64, d.w64, cnt, false, s);
+  if (p.nLarge <= 0) return;
+  LargePlan lp = p.large[4];
+  lp.spinLimit = p.spinLimit;
+  lp.done = p.cntLarge + (size_t)(2 + 3 * sweep) * p.nLarge;
+  if (fp32)
+    coopLaunch(kLargeForward<float>, lp.grid, solveShared<float>(lp), s, d, lp, (const float*)d.L32, rhs, d.x32, d.w32);
+  else
+    coopLaunch(kLargeForward<double>, lp.grid, solveShared<double>(lp), s, d, lp, (const double*)d.L64, rhs, d.x64,
+               d.w64);
 }
 
 void launchLargeBackward(const DevData& d, const PersistentPlan& p, bool fp32, int sweep, bool last, cudaStream_t s) {
-  if (p.nLargeTasks <= 0) return;
+  if (p.nLarge <= 0) return;
   const int acc = !fp32 ? 0 : (sweep == 0 ? 1 : 2);
   const int fin = (fp32 && last) ? 1 : 0;
-  int* queue = p.bwLQueue + (size_t)sweep * p.largeStride;
-  int* ctr = p.bwLCtr + 4 * sweep;
-  if (fp32) {
-    const size_t sm = ((size_t)((p.maxRowLarge + 3) & ~3) + 32 * 32) * sizeof(float);
-    bigSmem(kLargeBackward<float>, sm);
-    const int grid = gridFor(kLargeBackward<float>, sm, p.nLargeTasks);
-    pdlLaunch(kLargeBackward<float>, grid, kLT, sm, s, d, p, d.L32, d.x32, queue, ctr, p.errFlag, acc, fin);
-  } else {
-    const size_t sm = ((size_t)((p.maxRowLarge + 3) & ~3) + 32 * 32) * sizeof(double);
-    bigSmem(kLargeBackward<double>, sm);
-    const int grid = gridFor(kLargeBackward<double>, sm, p.nLargeTasks);
-    pdlLaunch(kLargeBackward<double>, grid, kLT, sm, s, d, p, d.L64, d.x64, queue, ctr, p.errFlag, acc, fin);
-  }
+  LargePlan lp = p.large[4];
+  lp.spinLimit = p.spinLimit;
+  lp.done = p.cntLarge + (size_t)(3 + 3 * sweep) * p.nLarge;
+  lp.bar = p.cntLarge + (size_t)(4 + 3 * sweep) * p.nLarge;
+  if (fp32)
+    coopLaunch(kLargeBackward<float>, lp.grid, solveShared<float>(lp), s, d, lp, (const float*)d.L32, d.x32, acc, fin);
+  else
+    coopLaunch(kLargeBackward<double>, lp.grid, solveShared<double>(lp), s, d, lp, (const double*)d.L64, d.x64, acc,
+               fin);
 }
 
 }  // namespace fgpu

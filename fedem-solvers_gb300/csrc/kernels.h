@@ -64,14 +64,6 @@ struct BackwardSeed {
   const int* slotCnt = nullptr;
   int* queue = nullptr;
   int* ctr = nullptr;
-  // the same for the large-front queues (seeded with the large roots; chains
-  // end at large fronts without large children); strideL = 0: no large fronts
-  int strideL = 0;
-  const int* rootOffL = nullptr;
-  const int* rootsL = nullptr;
-  const int* slotCntL = nullptr;
-  int* queueL = nullptr;
-  int* ctrL = nullptr;
 };
 void launchBeginStep(const DevData& d, int* activeCount, long long* activeEl, const BackwardSeed& seed,
                      cudaStream_t s);
@@ -113,6 +105,32 @@ void launchPartsNewton(const DevData& d, cudaStream_t s);
 void launchPartsStepEnd(const DevData& d, cudaStream_t s);
 
 // --- front_cascade.cu: one launch per phase over all fronts of all models ----
+// Large fronts: the blocks of a launch work through waves; tasks[wave * grid +
+// block] is the block's front in that wave (f < 0: none), the front's ordinal
+// among the large ones, the block's rank and the number of blocks on the front.
+struct LargeTask {
+  int f, li, rank, G;
+};
+struct LargePlan {
+  const LargeTask* tasks = nullptr;
+  int nWaves = 0, grid = 0;
+  const int* expect = nullptr;   // per large front: signals of its large children's blocks
+  const int* parent = nullptr;   // per large front: its (large) parent's ordinal, or -1
+  // inverse row maps: inv[invOff[li] + c * nrow + i] = update row of child c at row i, or -1
+  const int* inv = nullptr;
+  const int64_t* invOff = nullptr;
+  // original entries of each pivot column: asmCol[asmColOff[li] + j] .. [+ j + 1]
+  // (offsets from the front's first entry), and each pivot's diagonal entry
+  // (index into the assembled values)
+  const int* asmCol = nullptr;
+  const int* asmColOff = nullptr;
+  const int* diagAsm = nullptr;
+  const int* diagOff = nullptr;
+  int maxRow = 0;                // largest large front (rows)
+  int64_t stageCap = 0;          // values of L a block of the solves can stage
+  int *done = nullptr, *bar = nullptr, *err = nullptr;
+  long long spinLimit = 0;
+};
 struct PersistentPlan {
   const int* leaves;  // fronts without children, longest root path first (factorisation)
   int nLeaves;
@@ -137,21 +155,16 @@ struct PersistentPlan {
   // polls of a bounded wait in the back substitution before it gives up and
   // sets errFlag (about 1-2 s at the default)
   long long spinLimit = 1LL << 23;
-  // large fronts (more than kLargeFrontRows rows, and all their ancestors),
-  // one thread block each (front_large.cu): the number of large children of
-  // every front (d.fNlarge, global), the cascade's start tasks (large fronts
-  // without large children, longest root path first), the largest large front,
-  // their counters (factor, then one set per refinement forward elimination,
-  // nfrontTot + 1 apart) and backward queues (largeStride slots per solve, 4
-  // counters per solve)
+  // large fronts (more than kLargeFrontRows rows, and all their ancestors;
+  // front_large.cu): their number, the plans of the factorisation for the four
+  // shares of the GPU's blocks (largeCluster 2, 4, 8, 16) and of the solves
+  // (large[4]), and their counters (nLarge each: factorisation signals and
+  // barriers, then per solve forward signals, backward signals, backward
+  // barriers), zeroed with the other iteration counters
   const unsigned char* fLarge = nullptr;
-  const int* fNlarge = nullptr;
-  const int* largeTasks = nullptr;
-  int nLargeTasks = 0;
-  int maxRowLarge = 0;
-  int *cntLargeFactor = nullptr, *cntLargeForward = nullptr;
-  int *bwLQueue = nullptr, *bwLCtr = nullptr;
-  int largeStride = 0;
+  int nLarge = 0;
+  LargePlan large[5];
+  int* cntLarge = nullptr;
   // Launch shapes, picked per batch by the engine's autotuner.  No choice
   // changes a result bit: tasks are taken dynamically, and each front's
   // arithmetic is the same whichever warp, block or cluster does it.
@@ -159,22 +172,20 @@ struct PersistentPlan {
                            // (blocks of 8), 2 register-blocked (blocks of 4, fronts up to 32 rows)
   int forwardWarps = 8;    // warps per block of the forward-elimination cascade
   int backwardWarps = 8;   // warps per block of the back-substitution queue
-  int largeCluster = 8;    // blocks per cluster of the large-front factorisation (2, 4, 8 or 16)
+  int largeCluster = 16;   // sixteenths of the GPU's SMs the large-front factorisation runs on (2, 4, 8 or 16)
 };
 // fronts with more rows than this are factored and solved by a thread block
 // each (front_large.cu); smaller ones by one warp each in shared memory
 constexpr int kLargeFrontRows = 96;
-// the large-front kernels: factorisation (tangent models) fused with the first
-// forward elimination, a further forward elimination (refinement sweep), and
-// the back substitution of the large fronts (before the warp queue's)
-void launchLargeFactorForward(const DevData& d, const PersistentPlan& p, bool fp32, const double* rhs,
-                              cudaStream_t s);
-// clusters of csize blocks (2 to 16) the device can hold at once for the
-// large-front factorisation of this plan (0: none)
-int largeClusterCapacity(const PersistentPlan& p, bool fp32, int csize);
+// the large-front kernels: factorisation (tangent models), forward elimination
+// of rhs and back substitution (active models; before the warp queue's small
+// fronts) of solve `sweep` of the iteration
+void launchLargeFactor(const DevData& d, const PersistentPlan& p, bool fp32, cudaStream_t s);
 void launchLargeForward(const DevData& d, const PersistentPlan& p, bool fp32, const double* rhs, int sweep,
                         cudaStream_t s);
 void launchLargeBackward(const DevData& d, const PersistentPlan& p, bool fp32, int sweep, bool last, cudaStream_t s);
+// values of L a block of the large-front solves stages for a front shared by G blocks
+int64_t largeSolveStage(int nr, int np, int G, size_t elemBytes);
 // values of one front's L block the solve kernels stage in shared memory
 int stagingCapacity(const PersistentPlan& p, size_t elemBytes);
 // The first solve's back substitution run by the factorisation's own launch
