@@ -1044,7 +1044,7 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
       lparent.assign(nL, -1);
       level.assign(nL, 0);
       std::vector<int64_t> invOff(nL);
-      std::vector<int> inv, asmCol, asmColOff(nL), diagAsm, diagOff(nL);
+      std::vector<int> inv, asmCol, asmColOff(nL), diagAsm, diagOff(nL), gOff, gSrc, gRow(nL);
       for (int li = 0; li < nL; ++li) {  // children precede their parents
         const int f = lf[li];
         if (parent[f] >= 0) {
@@ -1058,6 +1058,16 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
           inv.resize(base + nrow[f], -1);
           for (int a = 0; a < nrow[ch] - npiv[ch]; ++a) inv[base + relIndex[relOffV[ch] + a]] = a;
         }
+        // the children's update-vector entries of each row
+        gRow[li] = (int)gOff.size();
+        for (int i = 0; i < nrow[f]; ++i) {
+          gOff.push_back((int)gSrc.size());
+          for (int c = 0; c < nchild[f]; ++c) {
+            const int a = inv[(size_t)invOff[li] + (size_t)c * nrow[f] + i];
+            if (a >= 0) gSrc.push_back((int)(wOffV[childList[childOffV[f] + c]] + a));
+          }
+        }
+        gOff.push_back((int)gSrc.size());
         // the original entries lie column by column
         asmColOff[li] = (int)asmCol.size();
         diagOff[li] = (int)diagAsm.size();
@@ -1083,6 +1093,9 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
         UPV(dao, int, asmColOff); UPV(dd, int, diagAsm); UPV(ddo, int, diagOff);
         base.parent = dp; base.inv = di; base.invOff = dio; base.asmCol = da; base.asmColOff = dao;
         base.diagAsm = dd; base.diagOff = ddo;
+        int *dg = nullptr, *dgs = nullptr, *dgr = nullptr;
+        UPV(dg, int, gOff); UPV(dgs, int, gSrc); UPV(dgr, int, gRow);
+        base.gOff = dg; base.gSrc = dgs; base.gRow = dgr;
       }
       int sms = 0;
       FG_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
@@ -1094,10 +1107,10 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
         const int cap = std::max(1, solve ? sms : sms * (2 << shape) / 16);
         // blocks a front can use: factorisation, four trailing blocks of the first
         // panel per thread block (one per sub-core); solves, 64 rows below the
-        // pivots per thread block, at most 8
+        // pivots or 8 pivots (a warp each) per thread block, at most 16
         auto wanted = [&](int li) {
           const int f = lf[li], nr = nrow[f], np = npiv[f];
-          if (solve) return std::min(8, std::max(1, (nr - np + 63) / 64));
+          if (solve) return std::min(16, std::max({1, (nr - np + 63) / 64, (np + 7) / 8}));
           const int nb = (nr - std::min(32, np) + 15) / 16, tasks = nb * (nb + 1) / 2 * (opt_.fp32Factor ? 1 : 2);
           return std::max(1, std::min(cap, (tasks + 3) / 4));
         };
@@ -1127,18 +1140,23 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
             waves.push_back(w);
           }
         }
+        // the solves take the blocks in turn from wave to wave: a block that waits
+        // for its next front has the waves between to load that front's L
+        if (solve) width = cap;
         tasks.assign(waves.size() * (size_t)width, LargeTask{-1, 0, 0, 1});
+        int next = 0;
         for (size_t w = 0; w < waves.size(); ++w) {
-          int b = 0;
+          int b = solve ? next : 0;
           for (const auto& q : waves[w])
             for (int r = 0; r < q.second; ++r) {
-              tasks[w * width + b++] = LargeTask{lf[q.first], q.first, r, q.second};
+              tasks[w * width + (size_t)(b++ % width)] = LargeTask{lf[q.first], q.first, r, q.second};
               if (lparent[q.first] >= 0) ++expect[lparent[q.first]];
               if (solve)
                 pplan_.large[4].stageCap =
                     std::max(pplan_.large[4].stageCap,
                              largeSolveStage(nrow[lf[q.first]], npiv[lf[q.first]], q.second, elemB));
             }
+          next = b % width;
         }
         const int64_t stageCap = pplan_.large[4].stageCap;
         LargeTask* dt = nullptr;

@@ -66,9 +66,6 @@ struct Front {
   }
 };
 
-__device__ inline bool singularPivot(float dk, float d0, double tol) { return !(fabsf(dk) > (float)tol * fabsf(d0)); }
-__device__ inline bool singularPivot(double dk, double d0, double tol) { return !(fabs(dk) > tol * fabs(d0)); }
-
 template <typename T>
 __device__ inline T ld(const T* p) {
   return __ldcg(p);
@@ -148,59 +145,97 @@ __device__ inline void mmaTf32(float* c, const uint32_t* a, const uint32_t* b) {
 }
 
 // shared memory of the factorisation: the panel's factored diagonal block
-// (Lt[k][i] = l_ik), its pivots, their reciprocals and the original diagonal,
-// the elimination's column buffers, and per warp the staged operand rows of one
-// trailing block (k-major: 16 rows, and 16 or 8 columns)
+// (Lt[k][i] = l_ik), its pivots, their reciprocals and singularity thresholds
+// (two panels'), the elimination's column buffers, and per warp the staged
+// operand rows of one trailing block (k-major: 16 rows, and 16 or 8 columns)
 template <typename T>
 struct FactorShared {
   T Lt[kPanel][kPanel];
-  T d[kPanel], dinv[kPanel], diag0[kPanel];
-  T ubuf[2][kPanel];
+  T d[kPanel], dinv[kPanel], diag0[2][kPanel];
+  T ubuf[2][kPanel], uk[2][kPanel];
   T A[kLW][kPanel][16 + (sizeof(T) == 4 ? 4 : 0)];
   T B[kLW][kPanel][std::is_same<T, float>::value ? 20 : 8];
 };
 
+// 1 / d.  FP64: the hardware's approximate reciprocal and one third-order Newton
+// step (e = 1 - d r; r (1 + e + e^2)), three multiply-adds on the critical chain
+// in place of the division's five; the division itself outside the normal range.
+__device__ inline float recip(float d) { return 1.0f / d; }
+__device__ inline double recip(double d) {
+  const unsigned ex = ((unsigned)__double2hiint(d) >> 20) & 0x7ffu;
+  if (ex - 64u > 1918u) return 1.0 / d;
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+  const double e = fma(-d, r, 1.0);
+  const double t = fma(e, e, e);
+  return fma(r, t, r);
+}
+// tests on the bit patterns of |x| (the order of non-negative patterns is the
+// numeric order): they keep the FP64 pipe, one instruction per 64 cycles, free
+__device__ inline bool absGreater(double a, double b) {
+  const long long m = 0x7fffffffffffffffll;
+  const long long x = __double_as_longlong(a) & m, y = __double_as_longlong(b) & m;
+  return x > y && x <= 0x7ff0000000000000ll;
+}
+__device__ inline bool absGreater(float a, float b) { return fabsf(a) > fabsf(b); }
+__device__ inline bool negative(double a) { return __double_as_longlong(a) < 0 && (__double_as_longlong(a) << 1) != 0; }
+__device__ inline bool negative(float a) { return a < 0.0f; }
+
 // Partial LDL^T of the kb x kb diagonal block (lower triangle in s.Lt[col][row],
-// unscaled) by warps 0 to 3: columns c = 4 q + w in the registers of warp w, one
-// row per lane.  Each step publishes its column through shared memory; the four
-// warps then scale it and update their own columns, the next pivot's first.
-// The chain per pivot is one reciprocal, a product and a multiply-subtract (about
-// 0.3 us in FP64), so a second warp per sub-core would only queue behind it.
+// unscaled; diag0: the singularity thresholds) by warps 0 to 3, one row per
+// lane, in steps with one barrier each.  In step k warp 0 applies the update of
+// pivot k - 1 to column k, takes its pivot and scales it; warps 1 to 3, which own
+// the later columns c = 3 q + w - 1, meanwhile apply pivot k - 1 to them, column
+// k + 1 first, which they pass on.  The chain of a pivot (a multiply-subtract, a
+// reciprocal, a product) so has a sub-core's FP64 pipe to itself: with the
+// columns on all four warps and every warp computing the reciprocal a block took
+// 26,300 cycles in FP64.
 template <typename T>
-__device__ void factorDiagonal(FactorShared<T>& s, int kb, double tolFact, int& neg, bool& sing) {
+__device__ void factorDiagonal(FactorShared<T>& s, const T* diag0, int kb, int& neg, bool& sing) {
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (w < 4) {
-    T a[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int c = 4 * q + w;
-      a[q] = (c < kb && lane < kb && lane >= c) ? s.Lt[c][lane] : T(0);
+  if (w == 0) {
+    T u = lane < kb ? s.Lt[0][lane] : T(0), l = T(0);
+    for (int k = 0; k < kb; ++k) {
+      if (k > 0) {
+        const T uk = __shfl_sync(0xffffffffu, u, k);  // pivot k - 1's unscaled value of row k
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        u = s.ubuf[k & 1][lane] - l * uk;
+      }
+      const T dk = __shfl_sync(0xffffffffu, u, k);
+      const bool bad = !absGreater(dk, diag0[k]);
+      const T inv = bad ? T(0) : recip(dk);
+      if (negative(dk)) ++neg;
+      sing |= bad;
+      l = u * inv;
+      // for the others' step k + 1 (and the panel): l below the diagonal, u
+      s.Lt[k][lane] = lane > k ? l : T(0);
+      s.uk[k & 1][lane] = u;
+      if (lane == 0) {
+        s.d[k] = dk;
+        s.dinv[k] = inv;
+      }
     }
-    if (w == 0) s.ubuf[0][lane] = a[0];
+  } else if (w < 4) {
+    // columns c = 3 q + w - 1 (c >= 1); a[q] holds the row's value of column c
+    T a[11];
 #pragma unroll
-    for (int k = 0; k < kPanel; ++k) {
+    for (int q = 0; q < 11; ++q) {
+      const int c = 3 * q + w - 1;
+      a[q] = (c > 0 && c < kb && lane < kb && lane >= c) ? s.Lt[c][lane] : T(0);
+      if (c == 1) s.ubuf[1][lane] = a[q];
+    }
+#pragma unroll
+    for (int k = 1; k < kPanel; ++k) {  // step k: pivot k - 1 applied to columns above k
       if (k >= kb) break;
       asm volatile("bar.sync 1, 128;" ::: "memory");
-      const T u = s.ubuf[k & 1][lane];
-      const T dk = s.ubuf[k & 1][k];
-      const bool bad = singularPivot(dk, s.diag0[k], tolFact);
-      const T inv = bad ? T(0) : T(1) / dk;
-      if (dk < T(0)) ++neg;
-      sing |= bad;
-      const T l = u * inv;
+      const T l = s.Lt[k - 1][lane];
+      const T* u = s.uk[(k - 1) & 1];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int c = 4 * q + w;
-        if (4 * q + 3 > k && c > k && c < kb) {
-          a[q] -= l * s.ubuf[k & 1][c];  // rows above the column hold unused values
+      for (int q = 0; q < 11; ++q) {
+        const int c = 3 * q + w - 1;
+        if (3 * q + 2 > k && c > k && c < kb) {
+          a[q] -= l * u[c];
           if (c == k + 1) s.ubuf[(k + 1) & 1][lane] = a[q];
-        }
-      }
-      if ((k & 3) == w) {
-        s.Lt[k][lane] = lane > k ? l : T(0);
-        if (lane == 0) {
-          s.d[k] = dk;
-          s.dinv[k] = inv;
         }
       }
     }
@@ -338,40 +373,47 @@ __device__ void assembleLarge(const DevData& d, const LargePlan& lp, const Large
   for (int u = t.rank + t.G * w; u < nr * nrb; u += t.G * kLW) {
     const int j = u / nrb, i0 = (u - j * nrb) << 7;
     if (i0 + 127 < j) continue;
+    const int k0 = j < np ? __ldg(colPtr + j) : 0, k1 = j < np ? __ldg(colPtr + j + 1) : 0;
     T v[4] = {T(0), T(0), T(0), T(0)};
-    for (int c = 0; c < nch; ++c) {
-      const int* ic = inv + (int64_t)c * nr;
-      const int b = __ldg(ic + j);
-      if (b < 0) continue;
-      const int ch = __ldg(chl + c);
-      const int cu = __ldg(d.fNrow + ch) - __ldg(d.fNpiv + ch);
-      const T* U = Ubase + __ldg(d.fUOff + ch) + ((int64_t)b * cu - (int64_t)b * (b - 1) / 2 - b);
-      int a[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int i = i0 + 32 * q + lane;
-        a[q] = (i < nr && i >= j) ? __ldg(ic + i) : -1;
+    for (int c0 = 0; c0 < nch; c0 += 32) {
+      // lane c: child c0 + c's update row at row j and the start of its column,
+      // shifted so that [row] addresses it; then the children that have row j, in order
+      int b = -1;
+      long long off = 0;
+      if (c0 + lane < nch) {
+        b = __ldg(inv + (int64_t)(c0 + lane) * nr + j);
+        const int ch = __ldg(chl + c0 + lane);
+        const int cu = __ldg(d.fNrow + ch) - __ldg(d.fNpiv + ch);
+        off = __ldg(d.fUOff + ch) + ((int64_t)b * cu - (int64_t)b * (b - 1) / 2 - b);
       }
-      T x[4];
+      for (unsigned m = __ballot_sync(0xffffffffu, b >= 0); m; m &= m - 1) {
+        const int c = __ffs(m) - 1;
+        const int* ic = inv + (int64_t)(c0 + c) * nr;
+        const T* U = Ubase + __shfl_sync(0xffffffffu, off, c);
+        int a[4];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) x[q] = a[q] >= 0 ? ld(U + a[q]) : T(0);
+        for (int q = 0; q < 4; ++q) {
+          const int i = i0 + 32 * q + lane;
+          a[q] = (i < nr && i >= j) ? __ldg(ic + i) : -1;
+        }
+        T x[4];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) v[q] += x[q];
+        for (int q = 0; q < 4; ++q) x[q] = a[q] >= 0 ? ld(U + a[q]) : T(0);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] += x[q];
+      }
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int i = i0 + 32 * q + lane;
       if (i < nr && i >= j) st(F.at(i, j), v[q]);
     }
-    if (j < np) {
-      __syncwarp();
-      const int k1 = __ldg(colPtr + j + 1);
-      for (int k = __ldg(colPtr + j) + lane; k < k1; k += 32) {
-        const int i = __ldg(d.asmPos + ao + k) - nr * j;
-        if (i >= i0 && i < i0 + 128) {
-          T* q = F.L + i + (int64_t)nr * j;
-          st(q, ld(q) + ld(asmVal + ao + k));
-        }
+    __syncwarp();
+    for (int k = k0 + lane; k < k1; k += 32) {
+      const int i = __ldg(d.asmPos + ao + k) - nr * j;
+      if (i >= i0 && i < i0 + 128) {
+        T* q = F.L + i + (int64_t)nr * j;
+        st(q, ld(q) + ld(asmVal + ao + k));
       }
     }
   }
@@ -387,23 +429,30 @@ __device__ void factorLarge(const DevData& d, const LargePlan& lp, const LargeTa
   const int nr = F.nr, np = F.np;
   int* bar = lp.bar + t.li;
   const int gw = t.rank + G * w, nw = G * kLW;  // warps numbered across the blocks first: one per sub-core
+  // a pivot is singular when |d_k| <= tolFactorize |a_kk| (the original entry);
+  // the thresholds of a panel are loaded ahead of it
+  auto threshold = [&](int k) {
+    const T a = ld(asmVal + __ldg(lp.diagAsm + lp.diagOff[t.li] + k));
+    return (T)tolFact * (a < T(0) ? -a : a);
+  };
+  if (tid < min(kPanel, np)) s.diag0[0][tid] = threshold(tid);
   assembleLarge<T>(d, lp, t, F, asmVal, Ubase);
   int phase = 0, neg = 0;
   bool sing = false;
   for (int k0 = 0; k0 < np; k0 += kPanel) {
     groupBarrier(bar, G, ++phase, ws);  // the panel's columns complete (assembly, earlier trailing updates)
     const int kb = min(kPanel, np - k0);
+    T* diag0 = s.diag0[(k0 / kPanel) & 1];
     for (int q = tid; q < kPanel * kPanel; q += kLT) {
       const int c = q >> 5, r = q & 31;
       if (c < kb && r < kb && r >= c) s.Lt[c][r] = ld(F.L + (k0 + r) + (int64_t)nr * (k0 + c));
     }
-    if (tid < kb) s.diag0[tid] = ld(asmVal + lp.diagAsm[lp.diagOff[t.li] + k0 + tid]);
     // this warp's first row below the block, loaded beside the block's factorisation
     const int rBelow = k0 + kb;
     T a0 = T(0);
     if (rBelow + gw < nr && lane < kb) a0 = ld(F.L + (rBelow + gw) + (int64_t)nr * (k0 + lane));
     __syncthreads();
-    factorDiagonal<T>(s, kb, tolFact, neg, sing);
+    factorDiagonal<T>(s, diag0, kb, neg, sing);
     // rows below the block: lane j holds column j; for k in order a_j -= a_k l_jk, then l_j = a_j / d_j
     const T di = lane < kb ? s.dinv[lane] : T(0);
     for (int r = rBelow + gw; r < nr; r += nw) {
@@ -424,6 +473,7 @@ __device__ void factorLarge(const DevData& d, const LargePlan& lp, const LargeTa
       }
     const int nt = nr - rBelow;
     if (nt <= 0) break;
+    if (tid < min(kPanel, np - rBelow)) s.diag0[(rBelow / kPanel) & 1][tid] = threshold(rBelow + tid);
     // trailing lower triangle in 16 x 16 blocks (row block rb >= column block cb)
     constexpr int kHalves = std::is_same<T, float>::value ? 1 : 2;
     const int nb = (nt + 15) >> 4, ntask = kHalves * (nb * (nb + 1) / 2);
@@ -534,21 +584,40 @@ __device__ void forwardLarge(const DevData& d, const LargePlan& lp, const LargeT
   const int ldp = staged ? lds : nr;
   const T* Lq = staged ? Lr : L + r0;
   const int ldq = staged ? ns : nr;
-  const int nch = d.fNchild[f];
-  const int* chl = d.childList + d.fChildOff[f];
-  const int* inv = lp.inv + lp.invOff[t.li];
+  // the right-hand side of the pivot rows, and where the children's
+  // contributions to the pivot rows and to this block's rows come from (in
+  // child order), before the wait; their values after it
+  const int* gOff = lp.gOff + lp.gRow[t.li];
+  const int nv = np + ns;
+  int p0 = 0, p1 = 0, src[4] = {0, 0, 0, 0};
+  T x = T(0);
+  if (tid < nv) {
+    const int r = tid < np ? tid : r0 + tid - np;
+    p0 = __ldg(gOff + r);
+    p1 = __ldg(gOff + r + 1);
+    if (tid < np) x = (T)rhs[__ldg(rows + r)];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) src[q] = p0 + q < p1 ? __ldg(lp.gSrc + p0 + q) : -1;
+  }
   const int need = lp.expect[t.li];
   if (need > 0) waitCount(lp.done + t.li, need, ws);
-  // the pivot rows' right-hand side and the children's contributions to the
-  // pivot rows and to this block's rows, in child order
-  for (int q = tid; q < np + ns; q += kLT) {
-    const int r = q < np ? q : r0 + q - np;
-    T x = q < np ? (T)rhs[__ldg(rows + r)] : T(0);
-    for (int c = 0; c < nch; ++c) {
-      const int a = __ldg(inv + (int64_t)c * nr + r);
-      if (a >= 0) x += ld(W + __ldg(d.fWOff + __ldg(chl + c)) + a);
+  for (int q0 = tid; q0 < nv; q0 += kLT) {
+    if (q0 != tid) {
+      const int r = q0 < np ? q0 : r0 + q0 - np;
+      p0 = __ldg(gOff + r);
+      p1 = __ldg(gOff + r + 1);
+      x = q0 < np ? (T)rhs[__ldg(rows + r)] : T(0);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) src[q] = p0 + q < p1 ? __ldg(lp.gSrc + p0 + q) : -1;
     }
-    v[q] = x;
+    T c[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) c[q] = src[q] >= 0 && p0 + q < p1 ? ld(W + src[q]) : T(0);
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (p0 + q < p1) x += c[q];
+    for (int p = p0 + 4; p < p1; ++p) x += ld(W + __ldg(lp.gSrc + p));
+    v[q0] = x;
   }
   if (staged) copyAsyncWait();
   __syncthreads();
@@ -558,7 +627,7 @@ __device__ void forwardLarge(const DevData& d, const LargePlan& lp, const LargeT
       T x = lane < bs ? v[b0 + lane] : T(0);
       const T* Lb = Lp + b0 + (int64_t)ldp * b0;
       if (staged) {
-#pragma unroll 4
+#pragma unroll 8
         for (int k = 0; k < bs - 1; ++k) {
           const T l = lane > k && lane < bs ? Lb[lane + ldp * k] : T(0);
           x -= l * __shfl_sync(0xffffffffu, x, k);
@@ -667,9 +736,18 @@ __device__ void backwardLarge(const DevData& d, const LargePlan& lp, const Large
   }
   const T* Lq = staged ? Lc : L + np + (int64_t)nr * k0;
   const int ldq = staged ? nu : nr;
+  // row indices and this warp's first pivot value before the wait
   const int par = lp.parent[t.li];
+  int row[2];
+#pragma unroll
+  for (int q = 0; q < 2; ++q) row[q] = np + tid + kLT * q < nr ? __ldg(rows + np + tid + kLT * q) : -1;
+  const int rowk = w < nc ? __ldg(rows + k0 + w) : 0, rowp = tid < np ? __ldg(rows + tid) : 0;
+  const T yk = w < nc ? ld(X + rowk) : T(0);
   if (par >= 0) waitCount(lp.done + par, 1, ws);
-  for (int r = np + tid; r < nr; r += kLT) xs[r] = ld(X + __ldg(rows + r));
+#pragma unroll
+  for (int q = 0; q < 2; ++q)
+    if (row[q] >= 0) xs[np + tid + kLT * q] = ld(X + row[q]);
+  for (int r = np + tid + 2 * kLT; r < nr; r += kLT) xs[r] = ld(X + __ldg(rows + r));
   if (staged) copyAsyncWait();
   __syncthreads();
   for (int k = w; k < nc; k += kLW) {
@@ -679,8 +757,12 @@ __device__ void backwardLarge(const DevData& d, const LargePlan& lp, const Large
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
     if (lane == 0) {
-      T* q = X + __ldg(rows + k0 + k);
-      st(q, ld(q) - a);
+      if (k == w) {
+        st(X + rowk, yk - a);
+      } else {
+        T* q = X + __ldg(rows + k0 + k);
+        st(q, ld(q) - a);
+      }
     }
   }
   __syncthreads();
@@ -689,7 +771,7 @@ __device__ void backwardLarge(const DevData& d, const LargePlan& lp, const Large
     return;
   }
   if (t.G > 1) waitCount(lp.bar + t.li, t.G - 1, ws);
-  for (int r = tid; r < np; r += kLT) xs[r] = ld(X + __ldg(rows + r));
+  for (int r = tid; r < np; r += kLT) xs[r] = ld(X + (r == tid ? rowp : __ldg(rows + r)));
   __syncthreads();
   const T* Lp = staged ? Ls : L;
   const int ldp = staged ? lds : nr;
@@ -702,7 +784,7 @@ __device__ void backwardLarge(const DevData& d, const LargePlan& lp, const Large
       T x = lane < bs ? xs[b0 + lane] : T(0);
       const T* Lb = Lp + b0 + (int64_t)ldp * (b0 + (lane < bs ? lane : 0));
       if (staged) {
-#pragma unroll 4
+#pragma unroll 8
         for (int j = bs - 1; j > 0; --j) {
           const T l = lane < j ? Lb[j] : T(0);
           x -= l * __shfl_sync(0xffffffffu, x, j);

@@ -119,6 +119,11 @@ struct LargePlan {
   // inverse row maps: inv[invOff[li] + c * nrow + i] = update row of child c at row i, or -1
   const int* inv = nullptr;
   const int64_t* invOff = nullptr;
+  // the children's update-vector entries of each row, in child order:
+  // gSrc[gOff[gRow[li] + i]] .. up to gOff[gRow[li] + i + 1]
+  const int* gOff = nullptr;
+  const int* gSrc = nullptr;
+  const int* gRow = nullptr;
   // original entries of each pivot column: asmCol[asmColOff[li] + j] .. [+ j + 1]
   // (offsets from the front's first entry), and each pivot's diagonal entry
   // (index into the assembled values)
