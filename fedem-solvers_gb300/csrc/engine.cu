@@ -942,7 +942,7 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
     auto fastFront = [&](int f) { return nrow[f] <= 64 && (long long)nrow[f] * npiv[f] <= capL; };
     std::vector<char> inGroup(nfr, 0), isHead(nfr, 0);
     for (int f = 0; f < nfr; ++f) {
-      if (nchild[f] == 0 || nchild[f] > 8 || !fastFront(f)) continue;
+      if (large[f] || nchild[f] == 0 || nchild[f] > 8 || !fastFront(f)) continue;
       bool ok = true;
       int ncg = 0;
       for (int c = 0; c < nchild[f] && ok; ++c) {
@@ -957,7 +957,7 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
     std::vector<int> tasks, taskLen;
     for (int f = 0; f < nfr; ++f) {
       if (isHead[f]) { tasks.push_back(f | (1 << 30)); taskLen.push_back(pathLen[f] + 1); }
-      else if (nchild[f] == 0 && !inGroup[f]) { tasks.push_back(f); taskLen.push_back(pathLen[f]); }
+      else if (nchild[f] == 0 && !large[f] && !inGroup[f]) { tasks.push_back(f); taskLen.push_back(pathLen[f]); }
     }
     if (nfr >= (1 << 30)) { err = "too many fronts for the task encoding"; return -910; }
     std::vector<int> order(tasks.size());
@@ -999,6 +999,104 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
       std::vector<int> fill(rootOff.begin(), rootOff.end() - 1);
       for (int f = 0; f < nfr; ++f)
         if (smallTop(f)) roots[fill[fmodel[f]]++] = f;
+    }
+    const int tw = treeWarps((int)leaves.size(), maxRowAll, opt_.fp32Factor);
+    if (tw > 0) {
+      // ---- trees on thread blocks: the small fronts cut into chunks of at most tw
+      // fronts: tiers of as many tree levels as a full binary piece of tw fronts has
+      // (so that a root path crosses few chunks), and where a piece is larger, its
+      // largest children to chunks of their own
+      int tier = 1;
+      while ((2 << tier) - 1 <= tw) ++tier;
+      std::vector<int> size(nfr, 0), chunkOf(nfr, -1), height(nfr, 0);
+      std::vector<char> cut(nfr, 0), lev(nfr, 0);
+      for (int f = 0; f < nfr; ++f) {
+        if (large[f]) continue;
+        std::vector<int> kids;
+        int sum = 1;
+        for (int c = 0; c < nchild[f]; ++c)
+          height[f] = std::max(height[f], height[childList[childOffV[f] + c]] + 1);
+        for (int c = 0; c < nchild[f]; ++c) {
+          const int k = childList[childOffV[f] + c];
+          if (height[k] / tier != height[f] / tier) {
+            cut[k] = 1;
+            continue;
+          }
+          kids.push_back(k);
+          sum += size[k];
+        }
+        std::stable_sort(kids.begin(), kids.end(), [&](int a, int b) { return size[a] > size[b]; });
+        for (size_t k = 0; k < kids.size() && sum > tw; ++k) {
+          cut[kids[k]] = 1;
+          sum -= size[kids[k]];
+        }
+        size[f] = sum;
+        for (int k : kids)
+          if (!cut[k]) lev[f] = std::max<char>(lev[f], lev[k] + 1);
+        if (parent[f] < 0 || large[parent[f]]) cut[f] = 1;
+      }
+      // chunks numbered by their root front; members by level
+      std::vector<TreeChunk> chunks;
+      std::vector<std::vector<int>> members;
+      std::vector<int> root;
+      for (int f = nfr - 1; f >= 0; --f) {  // parents precede their children here
+        if (large[f]) continue;
+        if (cut[f]) {
+          chunkOf[f] = (int)chunks.size();
+          TreeChunk ch{};
+          ch.model = fmodel[f];
+          ch.levels = lev[f] + 1;
+          ch.parent = parent[f] >= 0 && !large[parent[f]] ? chunkOf[parent[f]] : -1;
+          chunks.push_back(ch);
+          members.emplace_back();
+          root.push_back(f);
+        } else {
+          chunkOf[f] = chunkOf[parent[f]];
+        }
+        members[chunkOf[f]].push_back(f);
+      }
+      const int nc = (int)chunks.size();
+      std::vector<int> fronts, kids, start, need(nc, 0);
+      std::vector<unsigned char> level;
+      std::vector<std::vector<int>> kidsOf(nc);
+      for (int c = 0; c < nc; ++c)
+        if (chunks[c].parent >= 0) {
+          ++need[chunks[c].parent];
+          kidsOf[chunks[c].parent].push_back(c);
+        }
+      for (int c = 0; c < nc; ++c) {
+        std::vector<int>& m = members[c];
+        std::stable_sort(m.begin(), m.end(), [&](int a, int b) { return lev[a] < lev[b]; });
+        chunks[c].off = (int)fronts.size();
+        chunks[c].n = (int)m.size();
+        for (int f : m) {
+          fronts.push_back(f);
+          level.push_back((unsigned char)lev[f]);
+        }
+        chunks[c].parentNeed = chunks[c].parent >= 0 ? need[chunks[c].parent] : 0;
+        chunks[c].kidOff = (int)kids.size();
+        chunks[c].nKids = (int)kidsOf[c].size();
+        kids.insert(kids.end(), kidsOf[c].begin(), kidsOf[c].end());
+        if (kidsOf[c].empty()) start.push_back(c);
+      }
+      std::stable_sort(start.begin(), start.end(), [&](int a, int b) {
+        return pathLen[root[a]] + chunks[a].levels > pathLen[root[b]] + chunks[b].levels;
+      });
+      TreeChunk* dc = nullptr;
+      int *df = nullptr, *dk = nullptr, *ds = nullptr;
+      unsigned char* dl = nullptr;
+      if (kids.empty()) kids.push_back(-1);
+      UPV(dc, TreeChunk, chunks); UPV(df, int, fronts); UPV(dl, unsigned char, level); UPV(dk, int, kids);
+      UPV(ds, int, start);
+      pplan_.tree.chunks = dc; pplan_.tree.fronts = df; pplan_.tree.level = dl; pplan_.tree.kids = dk;
+      pplan_.tree.start = ds;
+      pplan_.tree.nStart = (int)start.size();
+      pplan_.tree.warps = tw;
+      // the back substitution's queue holds chunks: its roots are the top chunks,
+      // its chains end at the chunks without child chunks
+      for (int& r : roots) r = chunkOf[r];
+      std::fill(leafCnt.begin(), leafCnt.end(), 0);
+      for (int c : start) ++leafCnt[chunks[c].model];
     }
     int *dRootOff = nullptr, *dRoots = nullptr, *dLeafCnt = nullptr;
     UPV(dRootOff, int, rootOff);
@@ -1503,7 +1601,7 @@ int Engine::autotune() {
     pplan_.largeCluster = pick;
   }
   // 3. forward elimination of a refinement sweep: warps per block
-  if (ok && f32 && opt_.refineSweeps > 1) {
+  if (ok && f32 && opt_.refineSweeps > 1 && pplan_.tree.warps == 0) {
     float best = -1.f;
     int pick = 8;
     for (int w : {8, 4, 16}) {
@@ -1519,7 +1617,7 @@ int Engine::autotune() {
     pplan_.forwardWarps = pick;
   }
   // 4. back substitution: warps per block (queues seeded for every model)
-  if (ok) {
+  if (ok && pplan_.tree.warps == 0) {
     float best = -1.f;
     int pick = 8;
     for (int w : {8, 4, 16}) {
@@ -1600,13 +1698,16 @@ void Engine::enqueueSolve(cudaStream_t s, bool timedForward, bool backwardDone) 
     // the first forward elimination ran with the factorisation
     if (sweep > 0) launchRefineResidual(d_, s);
     if (sweep == 1 && timedForward) recordPhase(ev_[5], s);
+    // trees on thread blocks: a refinement solve's back substitution in the launch
+    // of its forward elimination too
+    const bool fused = sweep == 0 ? backwardDone : pplan_.tree.warps > 0 && pplan_.nLarge == 0;
     if (sweep > 0) {
-      launchForwardCascade(d_, pplan_, f32, f32 ? d_.rref : d_.del, sweep, s);
+      launchForwardCascade(d_, pplan_, f32, f32 ? d_.rref : d_.del, sweep, s, fused, sweep == sw - 1);
       launchLargeForward(d_, pplan_, f32, f32 ? d_.rref : d_.del, sweep, s);
     }
     if (sweep == 1 && timedForward) recordPhase(ev_[6], s);
     if (sweep == timedBackward && timedForward) recordPhase(ev_[7], s);
-    if (!(sweep == 0 && backwardDone)) {
+    if (!fused) {
       launchLargeBackward(d_, pplan_, f32, sweep, sweep == sw - 1, s);
       launchBackward(d_, pplan_, f32, sweep, sweep == sw - 1, s);
     }
@@ -2015,7 +2116,8 @@ void Engine::enqueueIteration(cudaStream_t s) {
   // elimination + a back substitution per solve (the first solve's inside the
   // factorisation's launch when fused) + for large fronts their factorisation and a
   // forward elimination and a back substitution per solve
-  launchesPerIter_ = (d_.beamSparse ? 11 : 12) + 1 + 2 * (sw - 1) + sw - (fuseBackward_ ? 1 : 0) +
+  launchesPerIter_ = (d_.beamSparse ? 11 : 12) + 1 + 2 * (sw - 1) + sw -
+                     (fuseBackward_ ? 1 : 0) - (pplan_.tree.warps > 0 && pplan_.nLarge == 0 ? sw - 1 : 0) +
                      (pplan_.nLarge > 0 ? 1 + 2 * sw : 0) +
                      (d_.urQs ? 1 : 0) +
                      (d_.nmotTot > 0 ? 1 : 0) + (d_.nmrTot > 0 ? 1 : 0) + (d_.naxTot > 0 ? 3 : 0) +

@@ -25,9 +25,11 @@
 // Mixed precision: FP32 factor and correction solves; the FP64 refinement
 // residual is in front_kernels.cu.
 
+#include <algorithm>
 #include <atomic>
 
 #include "kernels.h"
+#include "pivot.cuh"
 
 namespace fgpu {
 namespace {
@@ -41,11 +43,6 @@ namespace {
 // the unit L below it in the panel; the unscaled panel values of the update
 // rows (L d) are kept in the unused upper triangle (row k, column i) for the
 // rank-np pass.
-// a pivot counts as singular when |d_k| <= tolFactorize * |a_kk| (the FP32
-// factor tests in FP32, keeping the FP64 pipe free)
-__device__ inline bool singularPivot(float dk, float d0, double tol) { return !(fabsf(dk) > (float)tol * fabsf(d0)); }
-__device__ inline bool singularPivot(double dk, double d0, double tol) { return !(fabs(dk) > tol * fabs(d0)); }
-
 // Panel factorisations of the small fronts, all with the same arithmetic in
 // the same order (so the same factor to the last bit), picked per batch by the
 // engine's autotuner: pivot by pivot with the multipliers passed by shuffles
@@ -59,14 +56,14 @@ constexpr int kPanelRegisters4 = 2;  // blocks of 4 pivots, one row per lane (fr
 // pivot by pivot: rows lane and lane + 32 in shared memory; the multipliers of
 // the pivot rows (lanes below np) are passed by shuffles, one barrier per pivot
 template <typename T>
-__device__ void panelShuffle(T* F, const T* diag0, int nr, int np, int lane, double tolFact, int& neg, bool& sing) {
+__device__ void panelShuffle(T* F, const T* diag0, int nr, int np, int lane, int& neg, bool& sing) {
   const int i0 = lane, i1 = lane + 32;
   for (int k = 0; k < np; ++k) {
     const T dk = F[k + nr * k];
-    const bool bad = singularPivot(dk, diag0[k], tolFact);
+    const bool bad = !absGreater(dk, diag0[k]);
     sing |= bad;
-    if (dk < T(0)) ++neg;
-    const T inv = bad ? T(0) : T(1) / dk;
+    if (negative(dk)) ++neg;
+    const T inv = bad ? T(0) : recip(dk);
     const bool r0 = i0 > k && i0 < nr, r1 = i1 > k && i1 < nr;
     const T f0 = r0 ? F[i0 + nr * k] : T(0), f1 = r1 ? F[i1 + nr * k] : T(0);
     const T l0 = f0 * inv, l1 = f1 * inv;
@@ -90,8 +87,7 @@ __device__ void panelShuffle(T* F, const T* diag0, int nr, int np, int lane, dou
 // register-blocked in blocks of PB pivots (TWO: a second row per lane, fronts
 // of up to 64 rows; else at most 32 rows)
 template <typename T, int PB, bool TWO>
-__device__ void panelRegisters(T* F, const T* diag0, int nr, int np, int lane, double tolFact, int& neg,
-                               bool& sing) {
+__device__ void panelRegisters(T* F, const T* diag0, int nr, int np, int lane, int& neg, bool& sing) {
   // Register-blocked panel: lane r owns rows r and r + 32; the pivot columns
   // are taken PB at a time.  Inside a block the row values sit in
   // registers and each multiplier l_jk is passed by a shuffle from the lane
@@ -120,10 +116,10 @@ __device__ void panelRegisters(T* F, const T* diag0, int nr, int np, int lane, d
       if (kk >= kb) break;  // warp-uniform
       const int k = k0 + kk;
       const T dk = __shfl_sync(0xffffffffu, a0[kk], k);  // row k < 32 is lane k's first row
-      const bool bad = singularPivot(dk, diag0[k], tolFact);
+      const bool bad = !absGreater(dk, diag0[k]);
       sing |= bad;
-      if (dk < T(0)) ++neg;
-      const T inv = bad ? T(0) : T(1) / dk;
+      if (negative(dk)) ++neg;
+      const T inv = bad ? T(0) : recip(dk);
       const bool r0 = i0 > k && i0 < nr;
       const T f0 = r0 ? a0[kk] : T(0), f1 = h1 ? a1[kk] : T(0);
       const T l0 = f0 * inv, l1 = f1 * inv;
@@ -172,24 +168,23 @@ __device__ void panelRegisters(T* F, const T* diag0, int nr, int np, int lane, d
 }
 
 template <typename T, int PANEL>
-__device__ void factorBlocked(T* F, T* lcol, const T* diag0, int nr, int np, int lane, double tolFact, int& neg,
-                              bool& sing, T* Uout) {
+__device__ void factorBlocked(T* F, T* lcol, const T* diag0, int nr, int np, int lane, int& neg, bool& sing, T* Uout) {
   if (np <= 32 && nr <= 64) {
     if constexpr (PANEL == kPanelRegisters) {
-      panelRegisters<T, 8, true>(F, diag0, nr, np, lane, tolFact, neg, sing);
+      panelRegisters<T, 8, true>(F, diag0, nr, np, lane, neg, sing);
     } else if constexpr (PANEL == kPanelRegisters4) {
-      if (nr <= 32) panelRegisters<T, 4, false>(F, diag0, nr, np, lane, tolFact, neg, sing);
-      else panelShuffle<T>(F, diag0, nr, np, lane, tolFact, neg, sing);
+      if (nr <= 32) panelRegisters<T, 4, false>(F, diag0, nr, np, lane, neg, sing);
+      else panelShuffle<T>(F, diag0, nr, np, lane, neg, sing);
     } else {
-      panelShuffle<T>(F, diag0, nr, np, lane, tolFact, neg, sing);
+      panelShuffle<T>(F, diag0, nr, np, lane, neg, sing);
     }
   } else {
     for (int k = 0; k < np; ++k) {
       const T dk = F[k + nr * k];
-      const bool bad = singularPivot(dk, diag0[k], tolFact);
+      const bool bad = !absGreater(dk, diag0[k]);
       sing |= bad;
-      if (dk < T(0)) ++neg;
-      const T inv = bad ? T(0) : T(1) / dk;
+      if (negative(dk)) ++neg;
+      const T inv = bad ? T(0) : recip(dk);
       for (int i = k + 1 + lane; i < nr; i += 32) lcol[i] = F[i + nr * k] * inv;
       __syncwarp();
       for (int i = k + 1 + lane; i < nr; i += 32) {
@@ -248,7 +243,8 @@ __device__ void factorOneFront(const DevData& d, int f, T* F, T* lcol, T* diag0,
       if (pos[u] >= 0) F[pos[u]] = val[u];
   }
   __syncwarp();
-  for (int k = lane; k < np; k += 32) diag0[k] = F[k + nr * k];
+  // a pivot counts as singular when |d_k| <= tolFactorize * |a_kk|
+  for (int k = lane; k < np; k += 32) diag0[k] = singularBound(F[k + nr * k], (T)tolFact);
   __syncwarp();
   // extend-add of the children's update matrices, child by child
   for (int k0 = 0; k0 < ns; k0 += 32 * kFrontBatch) {
@@ -269,7 +265,7 @@ __device__ void factorOneFront(const DevData& d, int f, T* F, T* lcol, T* diag0,
   }
   int neg = 0;
   bool sing = false;
-  factorBlocked<T, PANEL>(F, lcol, diag0, nr, np, lane, tolFact, neg, sing, Uout);
+  factorBlocked<T, PANEL>(F, lcol, diag0, nr, np, lane, neg, sing, Uout);
   T* Lout = Lbase + d.fLOff[f];
   for (int k = lane; k < nr * np; k += 32) Lout[k] = F[k];
   if (lane == 0) {
@@ -332,7 +328,7 @@ __device__ void forwardOneFront(const DevData& d, int f, T* v, T* Ls, int capL, 
     for (int i = k + 1 + lane; i < nr; i += 32) v[i] -= L[i + (size_t)nr * k] * yk;
     __syncwarp();
   }
-  for (int r = lane; r < np; r += 32) X[rows[r]] = v[r] / L[r + (size_t)nr * r];
+  for (int r = lane; r < np; r += 32) X[rows[r]] = quotient(v[r], L[r + (size_t)nr * r]);
   T* wo = W + d.fWOff[f];
   for (int a = lane; a < nu; a += 32) wo[a] = v[np + a];
 }
@@ -368,6 +364,39 @@ __device__ inline SolveDesc solveDesc(const DevData& d, int f) {
   return q;
 }
 
+// the arithmetic of a forward elimination (fronts of at most 64 rows and 64
+// child update rows) on loaded values: lane r has rows and child entries r, r + 32
+template <typename T>
+__device__ void forwardRun(const SolveDesc& q, const int* row, const int* dst, const int* src, const double* b,
+                           const T* wv, T* v, const T* L, T* X, int lane, T* Wout) {
+  const int nr = q.nr, np = q.np, nch = q.nch;
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int r = lane + 32 * u;
+    if (r < nr) v[r] = r < np ? (T)b[u] : T(0);
+  }
+  __syncwarp();
+  for (int c = 0; c < nch; ++c) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+      if (src[u] >= 0 && (dst[u] >> 16) == c) v[dst[u] & 0xffff] += wv[u];
+    __syncwarp();
+  }
+  // the elimination with the rows in registers (lane r: rows r and r + 32), the
+  // pivot value of each step passed by a shuffle: no barrier between steps
+  T v0 = lane < nr ? v[lane] : T(0), v1 = lane + 32 < nr ? v[lane + 32] : T(0);
+  for (int k = 0; k < np; ++k) {
+    const T yk = __shfl_sync(0xffffffffu, k < 32 ? v0 : v1, k & 31);
+    const T* Lk = L + (size_t)nr * k;
+    if (lane > k && lane < nr) v0 -= Lk[lane] * yk;
+    if (lane + 32 > k && lane + 32 < nr) v1 -= Lk[lane + 32] * yk;
+  }
+  if (lane >= np && lane < nr) Wout[lane - np] = v0;
+  if (lane + 32 >= np && lane + 32 < nr) Wout[lane + 32 - np] = v1;
+  if (lane < np) X[row[0]] = quotient(v0, L[lane + (size_t)nr * lane]);
+  if (lane + 32 < np) X[row[1]] = quotient(v1, L[(lane + 32) + (size_t)nr * (lane + 32)]);
+}
+
 template <typename T>
 __device__ bool forwardOneFrontFast(const DevData& d, const SolveDesc& q, T* v, T* Ls, int capL, const T* Lbase,
                                     const double* rhs, T* X, const T* W, int lane, const T* Lres, T* Wout,
@@ -399,32 +428,7 @@ __device__ bool forwardOneFrontFast(const DevData& d, const SolveDesc& q, T* v, 
     wv[u] = src[u] < 0 ? T(0) : Win ? Win[lane + 32 * u] : __ldcg(W + src[u]);
   }
   if (!Lres) copyAsyncWait();
-  const T* L = Lres ? Lres : Ls;
-#pragma unroll
-  for (int u = 0; u < 2; ++u) {
-    const int r = lane + 32 * u;
-    if (r < nr) v[r] = r < np ? (T)b[u] : T(0);
-  }
-  __syncwarp();
-  for (int c = 0; c < nch; ++c) {
-#pragma unroll
-    for (int u = 0; u < 2; ++u)
-      if (src[u] >= 0 && (dst[u] >> 16) == c) v[dst[u] & 0xffff] += wv[u];
-    __syncwarp();
-  }
-  // the elimination with the rows in registers (lane r: rows r and r + 32), the
-  // pivot value of each step passed by a shuffle: no barrier between steps
-  T v0 = lane < nr ? v[lane] : T(0), v1 = lane + 32 < nr ? v[lane + 32] : T(0);
-  for (int k = 0; k < np; ++k) {
-    const T yk = __shfl_sync(0xffffffffu, k < 32 ? v0 : v1, k & 31);
-    const T* Lk = L + (size_t)nr * k;
-    if (lane > k && lane < nr) v0 -= Lk[lane] * yk;
-    if (lane + 32 > k && lane + 32 < nr) v1 -= Lk[lane + 32] * yk;
-  }
-  if (lane >= np && lane < nr) Wout[lane - np] = v0;
-  if (lane + 32 >= np && lane + 32 < nr) Wout[lane + 32 - np] = v1;
-  if (lane < np) X[row[0]] = v0 / L[lane + (size_t)nr * lane];
-  if (lane + 32 < np) X[row[1]] = v1 / L[(lane + 32) + (size_t)nr * (lane + 32)];
+  forwardRun<T>(q, row, dst, src, b, wv, v, Lres ? Lres : Ls, X, lane, Wout);
   return true;
 }
 
@@ -626,27 +630,11 @@ __device__ inline BackDesc backDesc(const DevData& d, const unsigned char* bwInl
 // is staged through L2 loads; an L1 line filled earlier in the launch by a
 // neighbouring front's solve could hold its old values (fusableBackward
 // guarantees that every block fits the staging area)
+// the arithmetic of a back substitution: xs holds the front's solution values
+// (pivots: the eliminated right-hand side), L its block; stores the pivots'
 template <typename T>
-__device__ void backwardOneFront(const DevData& d, const BackDesc& q, T* xs, T* Ls, int capL, const T* Lbase, T* X,
-                                 int acc, bool finalize, int lane, bool l2Only = false) {
-  const int nr = q.nr, np = q.np;
-  const int* rows = d.frontRows + q.rowOff;
-  const T* L;
-  if (l2Only) {
-    const T* Lg = Lbase + q.lOff;
-    const int cnt = nr * np;
-    if (cnt > capL) {
-      L = Lg;
-    } else {
-      for (int k = lane; k < cnt; k += 32) Ls[k] = __ldcg(Lg + k);
-      L = Ls;
-    }
-  } else {
-    L = stageL(Lbase + q.lOff, nr * np, Ls, capL, lane);
-  }
-  for (int r = lane; r < nr; r += 32) xs[r] = __ldcg(X + __ldg(rows + r));
-  copyAsyncWait();
-  __syncwarp();
+__device__ void backwardSolve(const DevData& d, const int* rows, int nr, int np, T* xs, const T* L, T* X, int acc,
+                              bool finalize, int lane) {
   if (np <= 32) {
     // one pivot per lane in a register; the back substitution passes each
     // solved value by a shuffle (no barrier between steps)
@@ -686,6 +674,30 @@ __device__ void backwardOneFront(const DevData& d, const BackDesc& q, T* xs, T* 
       if (finalize) d.del[row] = xr;
     }
   }
+}
+
+template <typename T>
+__device__ void backwardOneFront(const DevData& d, const BackDesc& q, T* xs, T* Ls, int capL, const T* Lbase, T* X,
+                                 int acc, bool finalize, int lane, bool l2Only = false) {
+  const int nr = q.nr, np = q.np;
+  const int* rows = d.frontRows + q.rowOff;
+  const T* L;
+  if (l2Only) {
+    const T* Lg = Lbase + q.lOff;
+    const int cnt = nr * np;
+    if (cnt > capL) {
+      L = Lg;
+    } else {
+      for (int k = lane; k < cnt; k += 32) Ls[k] = __ldcg(Lg + k);
+      L = Ls;
+    }
+  } else {
+    L = stageL(Lbase + q.lOff, nr * np, Ls, capL, lane);
+  }
+  for (int r = lane; r < nr; r += 32) xs[r] = __ldcg(X + __ldg(rows + r));
+  copyAsyncWait();
+  __syncwarp();
+  backwardSolve<T>(d, rows, nr, np, xs, L, X, acc, finalize, lane);
 }
 
 // Top-down work queue.  The step-start kernel puts the roots of the active
@@ -789,6 +801,278 @@ __global__ void kBackwardQueue(DevData d, int maxRow, int capL, const T* Lbase, 
                        lane, nullptr);
 }
 
+// ---- trees on thread blocks ----------------------------------------------------
+// Batches of few small fronts (a single model, a few models) are bound by the
+// latency of their assembly trees: in the cascades every level costs a front's
+// loads in four dependent rounds and a release-acquire through L2 (about 9 us a
+// level in the factorisation, 4 us in the solves, on a chain of 3,826 beams).
+// Here the host cuts the trees into chunks, connected pieces of at most as many
+// fronts as a block has warps, and a block takes a chunk with one warp per front:
+// every warp loads all that does not depend on its children (descriptors,
+// original entries, extend-add map, right-hand side, or the factor block) at
+// the chunk's start, then the levels follow one another at block barriers.
+// Between chunks the cascades' protocol applies, a chunk in the place of a
+// front: the block that completes a parent chunk's count goes on with it;
+// the back substitution is handed down through the queue, a block holding one
+// chunk at a time and going on with its first child chunk.  The arithmetic of
+// every front is that of the cascades (the same device functions), so both give
+// the same bits and the choice is the launch's alone.
+
+// loads of a front's forward elimination that do not depend on its children
+template <typename T>
+struct ForwardIn {
+  int row[2], src[2], dst[2];
+  double b[2];
+};
+
+template <typename T, int PANEL>
+__global__ void __launch_bounds__(512, 1) kTree(DevData d, TreePlan tp, int maxRow, const T* asmVal, T* Lbase, T* Ubase,
+                                              double tolFact, const double* rhs, T* X, T* Wv, int* cnt,
+                                              FusedBackward fb, int up, int mayFactor) {
+  pdlEntry();
+  extern __shared__ __align__(16) unsigned char smraw[];
+  __shared__ int shNext;
+  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+  T* F = reinterpret_cast<T*>(smraw) + (size_t)w * ((size_t)maxRow * maxRow + 3 * maxRow);
+  T* lcol = F + (size_t)maxRow * maxRow;
+  T* diag0 = lcol + maxRow;
+  T* v = diag0 + maxRow;
+  if (up) {
+    int* const start = cnt + d.nfrontTot;
+    auto take = [&]() {
+      const int i = atomicAdd(start, 1);
+      return i < tp.nStart ? tp.start[i] : -1;
+    };
+    if (tid == 0) shNext = take();
+    __syncthreads();
+    int c = shNext;
+    while (c >= 0) {
+      const TreeChunk ch = tp.chunks[c];
+      const int fl = d.m.flags[ch.model];
+      const bool active = fl & FL_ACTIVE, factor = mayFactor && (fl & FL_TANGENT);
+      if (active) {
+        const bool mine = w < ch.n;
+        const int f = mine ? tp.fronts[ch.off + w] : -1;
+        const int level = mine ? tp.level[ch.off + w] : -1;
+        SolveDesc q{};
+        ForwardIn<T> in;
+        constexpr int kSeg = 8;  // extend-add entries per lane loaded ahead
+        int sp[kSeg];
+        int ns = 0;
+        const T* segIn = nullptr;
+        const int* segPos = nullptr;
+        bool fast = false;
+        if (mine) {
+          q = solveDesc(d, f);
+          const int nr = q.nr, np = q.np;
+          fast = nr <= 64 && q.ncg <= 64;
+          if (factor) {
+            const int64_t ao = d.fAsmOff[f], so = d.fSegOff[f];
+            const int na = d.fNasm[f];
+            ns = d.fSegLen[f];
+            segIn = Ubase + so;
+            segPos = d.segPos + so;
+#pragma unroll
+            for (int u = 0; u < kSeg; ++u) {
+              const int k = lane + 32 * u;
+              sp[u] = k < ns ? __ldg(segPos + k) : -1;
+            }
+            for (int k = lane; k < nr * nr; k += 32) F[k] = T(0);
+            for (int k0 = 0; k0 < na; k0 += 32 * kFrontBatch) {
+              T val[kFrontBatch];
+              int pos[kFrontBatch];
+#pragma unroll
+              for (int u = 0; u < kFrontBatch; ++u) {
+                const int k = k0 + 32 * u + lane;
+                pos[u] = k < na ? __ldg(d.asmPos + ao + k) : -1;
+                val[u] = k < na ? __ldg(asmVal + ao + k) : T(0);
+              }
+              __syncwarp();
+#pragma unroll
+              for (int u = 0; u < kFrontBatch; ++u)
+                if (pos[u] >= 0) F[pos[u]] = val[u];
+            }
+            __syncwarp();
+            for (int k = lane; k < np; k += 32) diag0[k] = singularBound(F[k + nr * k], (T)tolFact);
+          } else {
+            const T* Lg = Lbase + q.lOff;
+            for (int k = lane; k < nr * np; k += 32) copyAsync(F + k, Lg + k);
+          }
+          if (fast) {
+            const int* rows = d.frontRows + q.rowOff;
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+              const int r = lane + 32 * u;
+              in.row[u] = r < np ? __ldg(rows + r) : -1;
+              in.src[u] = r < q.ncg ? __ldg(d.cgSrc + q.cg0 + r) : -1;
+              in.dst[u] = r < q.ncg ? __ldg(d.cgDst + q.cg0 + r) : 0;
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) in.b[u] = in.row[u] >= 0 ? rhs[in.row[u]] : 0.0;
+          }
+          if (!factor) copyAsyncWait();
+          __syncwarp();
+        }
+        for (int l = 0; l < ch.levels; ++l) {
+          if (level == l) {
+            const int nr = q.nr, np = q.np;
+            T wv[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) wv[u] = fast && in.src[u] >= 0 ? __ldcg(Wv + in.src[u]) : T(0);
+            if (factor) {
+              // extend-add of the children's update matrices, child by child
+              T sv[kSeg];
+#pragma unroll
+              for (int u = 0; u < kSeg; ++u) sv[u] = sp[u] >= 0 ? __ldcg(segIn + lane + 32 * u) : T(0);
+              for (int c1 = 0; c1 < q.nch; ++c1) {
+#pragma unroll
+                for (int u = 0; u < kSeg; ++u)
+                  if (sp[u] >= 0 && (sp[u] >> 20) == c1) F[sp[u] & 0xfffff] += sv[u];
+                __syncwarp();
+              }
+              for (int k0 = 32 * kSeg; k0 < ns; k0 += 32 * kFrontBatch) {
+                T val[kFrontBatch];
+                int pc[kFrontBatch];
+#pragma unroll
+                for (int u = 0; u < kFrontBatch; ++u) {
+                  const int k = k0 + 32 * u + lane;
+                  pc[u] = k < ns ? __ldg(segPos + k) : -1;
+                  val[u] = k < ns ? __ldcg(segIn + k) : T(0);
+                }
+                for (int c1 = 0; c1 < q.nch; ++c1) {
+#pragma unroll
+                  for (int u = 0; u < kFrontBatch; ++u)
+                    if (pc[u] >= 0 && (pc[u] >> 20) == c1) F[pc[u] & 0xfffff] += val[u];
+                  __syncwarp();
+                }
+              }
+              int neg = 0;
+              bool sing = false;
+              factorBlocked<T, PANEL>(F, lcol, diag0, nr, np, lane, neg, sing, Ubase + d.fUOff[f]);
+              if (lane == 0) {
+                if (neg) atomicAdd(&d.m.negPiv[ch.model], neg);
+                if (sing) atomicOr(&d.m.status[ch.model], SS_SINGULAR);
+              }
+            }
+            if (fast) forwardRun<T>(q, in.row, in.dst, in.src, in.b, wv, v, F, X, lane, Wv + q.wOff);
+            else forwardOneFront<T>(d, f, v, F, 0, Lbase, rhs, X, Wv, lane, F);
+            if (factor) {
+              T* Lout = Lbase + q.lOff;
+              for (int k = lane; k < nr * np; k += 32) Lout[k] = F[k];
+            }
+          }
+          __syncthreads();
+        }
+      }
+      __syncthreads();
+      if (tid == 0) {
+        int nx = -1;
+        if (active) {
+          if (ch.parent >= 0) {
+            int old;
+            asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;\n" : "=r"(old) : "l"(cnt + ch.parent) : "memory");
+            if (old == ch.parentNeed - 1) nx = ch.parent;
+          } else if (fb.queue) {
+            asm volatile("red.release.gpu.global.add.s32 [%0], %1;\n" ::"l"(cnt + c), "r"(kRootDone) : "memory");
+          }
+        }
+        shNext = nx >= 0 ? nx : take();
+      }
+      __syncthreads();
+      c = shNext;
+    }
+  }
+  if (!fb.queue) return;
+  // back substitution: the queue of kBackwardQueue with chunks in the place of
+  // fronts.  With the elimination in the same launch (up), the roots' done marks
+  // are waited for, and L, written in this launch, is read through L2.
+  const int total = *(volatile const int*)(fb.ctr + 2);
+  for (;;) {
+    __syncthreads();
+    if (tid == 0) {
+      int c = -1;
+      const int slot = atomicAdd(fb.ctr, 1);
+      if (slot < total) {
+        long long spins = 0;
+        bool ok = true;
+        while ((c = *(volatile const int*)(fb.queue + slot)) < 0) {
+          __nanosleep(20);
+          if (++spins > fb.spinLimit) {
+            atomicOr(fb.errFlag, 1);
+            ok = false;
+            break;
+          }
+        }
+        __threadfence();
+        if (ok && up && tp.chunks[c].parent < 0 && (d.m.flags[tp.chunks[c].model] & FL_ACTIVE)) {
+          while (acquireCount(cnt + c) < kRootDone) {
+            __nanosleep(20);
+            if (++spins > fb.spinLimit) {
+              atomicOr(fb.errFlag, 1);
+              ok = false;
+              break;
+            }
+          }
+        }
+        if (!ok) c = -1;
+      }
+      shNext = c;
+    }
+    __syncthreads();
+    int c = shNext;
+    if (c < 0) break;
+    while (c >= 0) {
+      const TreeChunk ch = tp.chunks[c];
+      const bool mine = w < ch.n;
+      const int f = mine ? tp.fronts[ch.off + w] : -1;
+      const int level = mine ? tp.level[ch.off + w] : -1;
+      const int* rows = nullptr;
+      int nr = 0, np = 0, rr[3];
+      if (mine) {
+        nr = d.fNrow[f];
+        np = d.fNpiv[f];
+        rows = d.frontRows + d.fRowOff[f];
+        const T* Lg = Lbase + d.fLOff[f];
+#pragma unroll
+        for (int u = 0; u < 3; ++u) rr[u] = lane + 32 * u < nr ? __ldg(rows + lane + 32 * u) : -1;
+        if (up && mayFactor) {
+          for (int k = lane; k < nr * np; k += 32) F[k] = __ldcg(Lg + k);
+        } else {
+          for (int k = lane; k < nr * np; k += 32) copyAsync(F + k, Lg + k);
+          copyAsyncWait();
+        }
+        __syncwarp();
+      }
+      for (int l = ch.levels - 1; l >= 0; --l) {
+        if (level == l) {
+#pragma unroll
+          for (int u = 0; u < 3; ++u)
+            if (rr[u] >= 0) v[lane + 32 * u] = __ldcg(X + rr[u]);
+          for (int r = lane + 96; r < nr; r += 32) v[r] = __ldcg(X + __ldg(rows + r));
+          __syncwarp();
+          backwardSolve<T>(d, rows, nr, np, v, F, X, fb.acc, fb.finalize != 0, lane);
+        }
+        __syncthreads();
+      }
+      if (tid == 0) {
+        int nx = -1;
+        if (ch.nKids > 0) {
+          nx = tp.kids[ch.kidOff];
+          if (ch.nKids > 1) {
+            __threadfence();
+            const int base = atomicAdd(fb.ctr + 1, ch.nKids - 1);
+            for (int k = 1; k < ch.nKids; ++k) atomicExch(fb.queue + base + k - 1, tp.kids[ch.kidOff + k]);
+          }
+        }
+        shNext = nx;
+      }
+      __syncthreads();
+      c = shNext;
+      __syncthreads();
+    }
+  }
+}
+
 int smCountCached() {
   // engines may be built on several host threads at once
   static std::atomic<int> cached{0};
@@ -827,6 +1111,44 @@ void factorCascade(void (*kernel)(DevData, const int*, int, int, const T*, T*, T
   const int blocks = occupancyBlocks(kernel, 32 * wpb, sm, (p.nLeaves + wpb - 1) / wpb);
   pdlLaunch(kernel, blocks, 32 * wpb, sm, s, d, p.leaves, p.nLeaves, p.maxRow, asmVal, L, U, tol, rhs, X, W, p.cntFactor,
             fb);
+}
+
+size_t treeWarpValues(int maxRow) { return (size_t)maxRow * maxRow + 3 * (size_t)maxRow; }
+
+// one launch of the trees on thread blocks (kTree)
+template <typename T>
+void treeLaunch(const DevData& d, const PersistentPlan& p, const T* asmVal, T* L, T* U, const double* rhs, T* X, T* W,
+                int* cnt, const FusedBackward& fb, bool up, bool mayFactor, cudaStream_t s) {
+  const auto kernel = !mayFactor || p.factorPanel == kPanelShuffle ? kTree<T, kPanelShuffle>
+                      : p.factorPanel == kPanelRegisters           ? kTree<T, kPanelRegisters>
+                                                                   : kTree<T, kPanelRegisters4>;
+  const int threads = 32 * p.tree.warps;
+  const size_t sm = p.tree.warps * treeWarpValues(p.maxRow) * sizeof(T);
+  allowBigSmem(kernel, sm);
+  const int blocks = occupancyBlocks(kernel, threads, sm, p.tree.nStart);
+  pdlLaunch(kernel, blocks, threads, sm, s, d, p.tree, p.maxRow, asmVal, L, U, 1.0e-12, rhs, X, W, cnt, fb, up ? 1 : 0,
+            mayFactor ? 1 : 0);
+}
+
+void treeLaunch(const DevData& d, const PersistentPlan& p, bool fp32, const double* rhs, int* cnt,
+                const FusedBackward& fb, bool up, bool mayFactor, cudaStream_t s) {
+  if (fp32)
+    treeLaunch<float>(d, p, d.asmVal32, d.L32, d.U32, rhs, d.x32, d.w32, cnt, fb, up, mayFactor, s);
+  else
+    treeLaunch<double>(d, p, d.asmVal64, d.L64, d.U64, rhs, d.x64, d.w64, cnt, fb, up, mayFactor, s);
+}
+
+// the back substitution of solve `sweep` (launchBackward's arguments)
+FusedBackward backwardOf(const PersistentPlan& p, bool fp32, int sweep, bool last) {
+  FusedBackward fb;
+  fb.queue = p.bwQueue + (size_t)sweep * p.nLeaves;
+  fb.ctr = p.bwCtr + 4 * sweep;
+  fb.bwInline = p.bwInline;
+  fb.errFlag = p.errFlag;
+  fb.spinLimit = p.spinLimit;
+  fb.acc = !fp32 ? ACC_SET : (sweep == 0 ? ACC_FIRST : ACC_ADD);
+  fb.finalize = (fp32 && last) ? 1 : 0;
+  return fb;
 }
 
 int factorWarpsPerBlock(size_t perWarpBytes) {
@@ -869,14 +1191,12 @@ void launchFactorForwardCascade(const DevData& d, const PersistentPlan& p, bool 
   // solve vector and L staging reuse the warp's v and F areas
   FusedBackward fb;
   if (withBackward) {
-    fb.queue = p.bwQueue;
-    fb.ctr = p.bwCtr;
-    fb.bwInline = p.bwInline;
-    fb.errFlag = p.errFlag;
-    fb.spinLimit = p.spinLimit;
-    fb.acc = fp32 ? ACC_FIRST : ACC_SET;
-    fb.finalize = (fp32 && lastSweep) ? 1 : 0;
+    fb = backwardOf(p, fp32, 0, lastSweep);
     fb.capL = stagingCapacity(p, fp32 ? sizeof(float) : sizeof(double));
+  }
+  if (p.tree.warps > 0) {
+    treeLaunch(d, p, fp32, rhs, p.cntFactor, fb, true, true, s);
+    return;
   }
   if (fp32) {
     const int wpb = factorWarpsPerBlock(perWarp * sizeof(float));
@@ -912,16 +1232,37 @@ int stagingCapacity(const PersistentPlan& p, size_t elemBytes) {
   return (int)(want < cap ? want : cap);
 }
 
+// The line between the trees on thread blocks and the cascades, by the batch's
+// leaf fronts (iteration in microseconds, cascades against trees of 16 and 8
+// warps; chains of beams, mixed unless noted): 1,066 leaves 238 / 174 / 183;
+// 3,200: 265 / 221 / 221; 5,333: 360 / 334 / 324 (FP64 368 / 315 / 298); 8,533:
+// 348 / 348 / 334; FP64 10,666: 446 / 524 / 477; 16,000: 556 / 779 / 721.  With
+// more leaves the cascades' warps, which never wait for a level, keep the GPU
+// busier; between 4,096 and 8,192 two blocks of 8 warps share an SM better than
+// one of 16.
+int treeWarps(int nLeaves, int maxRow, bool fp32) {
+  if (nLeaves <= 0 || nLeaves > 8192) return 0;
+  const int fit = (int)(200 * 1024 / (treeWarpValues(maxRow) * (fp32 ? sizeof(float) : sizeof(double))));
+  const int w = std::min(nLeaves <= 4096 ? 16 : 8, fit);
+  return w >= 3 ? w : 0;
+}
+
 bool fusableBackward(const PersistentPlan& p, bool fp32) {
+  if (p.tree.warps > 0) return p.nLeaves > 0 && p.nLarge == 0;
   return p.nLeaves > 0 && p.nLarge == 0 &&
          (long long)stagingCapacity(p, fp32 ? sizeof(float) : sizeof(double)) >= (long long)p.maxRow * p.maxNpiv;
 }
 
 void launchForwardCascade(const DevData& d, const PersistentPlan& p, bool fp32, const double* rhs, int sweep,
-                          cudaStream_t s) {
+                          cudaStream_t s, bool withBackward, bool lastSweep) {
   if (p.nTasks <= 0) return;
   const int wpb = p.forwardWarps;
   int* cnt = p.cntForward + (size_t)(sweep - 1) * ((size_t)d.nfrontTot + 1);
+  if (p.tree.warps > 0) {
+    treeLaunch(d, p, fp32, rhs, cnt, withBackward ? backwardOf(p, fp32, sweep, lastSweep) : FusedBackward{}, true,
+               false, s);
+    return;
+  }
   if (fp32) {
     const int capL = stagingCapacity(p, sizeof(float));
     const size_t sm = (size_t)wpb * (p.maxRow + capL + 64) * sizeof(float);
@@ -943,6 +1284,10 @@ void launchBackward(const DevData& d, const PersistentPlan& p, bool fp32, int sw
   const int acc = !fp32 ? ACC_SET : (sweep == 0 ? ACC_FIRST : ACC_ADD);
   const int fin = (fp32 && last) ? 1 : 0;
   if (p.nLeaves <= 0) return;
+  if (p.tree.warps > 0) {
+    treeLaunch(d, p, fp32, nullptr, p.cntFactor, backwardOf(p, fp32, sweep, last), false, false, s);
+    return;
+  }
   const int wpb = p.backwardWarps;
   int* queue = p.bwQueue + (size_t)sweep * p.nLeaves;
   int* ctr = p.bwCtr + 4 * sweep;

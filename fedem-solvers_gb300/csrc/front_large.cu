@@ -43,6 +43,7 @@
 #include <type_traits>
 
 #include "kernels.h"
+#include "pivot.cuh"
 
 namespace fgpu {
 namespace {
@@ -50,6 +51,7 @@ namespace {
 constexpr int kLT = 256;  // threads per block
 constexpr int kLW = kLT / 32;
 constexpr int kPanel = 32;  // pivots per panel
+constexpr int kMaxShared = 220 * 1024;  // dynamic shared memory a launch may ask for
 
 // lower-triangle entry (ii >= jj) of an nu x nu matrix packed column by column
 __device__ inline int64_t packedAt(int ii, int jj, int nu) {
@@ -156,30 +158,6 @@ struct FactorShared {
   T A[kLW][kPanel][16 + (sizeof(T) == 4 ? 4 : 0)];
   T B[kLW][kPanel][std::is_same<T, float>::value ? 20 : 8];
 };
-
-// 1 / d.  FP64: the hardware's approximate reciprocal and one third-order Newton
-// step (e = 1 - d r; r (1 + e + e^2)), three multiply-adds on the critical chain
-// in place of the division's five; the division itself outside the normal range.
-__device__ inline float recip(float d) { return 1.0f / d; }
-__device__ inline double recip(double d) {
-  const unsigned ex = ((unsigned)__double2hiint(d) >> 20) & 0x7ffu;
-  if (ex - 64u > 1918u) return 1.0 / d;
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-  const double e = fma(-d, r, 1.0);
-  const double t = fma(e, e, e);
-  return fma(r, t, r);
-}
-// tests on the bit patterns of |x| (the order of non-negative patterns is the
-// numeric order): they keep the FP64 pipe, one instruction per 64 cycles, free
-__device__ inline bool absGreater(double a, double b) {
-  const long long m = 0x7fffffffffffffffll;
-  const long long x = __double_as_longlong(a) & m, y = __double_as_longlong(b) & m;
-  return x > y && x <= 0x7ff0000000000000ll;
-}
-__device__ inline bool absGreater(float a, float b) { return fabsf(a) > fabsf(b); }
-__device__ inline bool negative(double a) { return __double_as_longlong(a) < 0 && (__double_as_longlong(a) << 1) != 0; }
-__device__ inline bool negative(float a) { return a < 0.0f; }
 
 // Partial LDL^T of the kb x kb diagonal block (lower triangle in s.Lt[col][row],
 // unscaled; diag0: the singularity thresholds) by warps 0 to 3, one row per
@@ -432,8 +410,7 @@ __device__ void factorLarge(const DevData& d, const LargePlan& lp, const LargeTa
   // a pivot is singular when |d_k| <= tolFactorize |a_kk| (the original entry);
   // the thresholds of a panel are loaded ahead of it
   auto threshold = [&](int k) {
-    const T a = ld(asmVal + __ldg(lp.diagAsm + lp.diagOff[t.li] + k));
-    return (T)tolFact * (a < T(0) ? -a : a);
+    return singularBound(ld(asmVal + __ldg(lp.diagAsm + lp.diagOff[t.li] + k)), (T)tolFact);
   };
   if (tid < min(kPanel, np)) s.diag0[0][tid] = threshold(tid);
   assembleLarge<T>(d, lp, t, F, asmVal, Ubase);
@@ -663,7 +640,7 @@ __device__ void forwardLarge(const DevData& d, const LargePlan& lp, const LargeT
     __syncthreads();
   }
   if (t.rank == 0)
-    for (int r = tid; r < np; r += kLT) st(X + __ldg(rows + r), v[r] / Lp[r + (int64_t)ldp * r]);
+    for (int r = tid; r < np; r += kLT) st(X + __ldg(rows + r), quotient(v[r], Lp[r + (int64_t)ldp * r]));
   // rows below: quarter h of the pivots of 32 rows per warp, two row groups at a time
   const int qn = (np + 3) >> 2;
   T* wo = W + d.fWOff[f] + (r0 - np);
@@ -855,7 +832,9 @@ __global__ void __launch_bounds__(kLT) kLargeBackward(DevData d, LargePlan lp, c
 // cooperative launch (all blocks resident), ordered like any launch of the stream
 template <typename... KArgs, typename... Args>
 void coopLaunch(void (*kernel)(KArgs...), int grid, size_t smem, cudaStream_t s, Args... args) {
-  if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // one value for every batch: the attribute is the function's, and a smaller
+  // batch must not lower it under a larger one's captured launches
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxShared);
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;

@@ -136,7 +136,25 @@ struct LargePlan {
   int *done = nullptr, *bar = nullptr, *err = nullptr;
   long long spinLimit = 0;
 };
+// Small-front trees cut into chunks of at most `warps` fronts (front_cascade.cu,
+// kTree): fronts chunks[c].off .. + n with their levels inside the chunk
+// (children below their parents), ascending.
+struct TreeChunk {
+  int off, n, levels, model;
+  int parent, parentNeed;  // the chunk of the root's parent front (-1: none) and that chunk's child chunks
+  int kidOff, nKids;       // child chunks
+};
+struct TreePlan {
+  const TreeChunk* chunks = nullptr;
+  const int* fronts = nullptr;
+  const unsigned char* level = nullptr;
+  const int* kids = nullptr;
+  const int* start = nullptr;  // chunks without child chunks, longest root path first
+  int nStart = 0;
+  int warps = 0;  // fronts per chunk at most, and warps per block (0: the cascades are used)
+};
 struct PersistentPlan {
+  TreePlan tree;
   const int* leaves;  // fronts without children, longest root path first (factorisation)
   int nLeaves;
   // forward-elimination tasks, longest root path first: a leaf, or a front
@@ -191,6 +209,9 @@ void launchLargeForward(const DevData& d, const PersistentPlan& p, bool fp32, co
 void launchLargeBackward(const DevData& d, const PersistentPlan& p, bool fp32, int sweep, bool last, cudaStream_t s);
 // values of L a block of the large-front solves stages for a front shared by G blocks
 int64_t largeSolveStage(int nr, int np, int G, size_t elemBytes);
+// warps per block (and fronts per chunk) of the trees on thread blocks for a batch
+// of nLeaves leaf fronts and fronts of at most maxRow rows; 0: not used
+int treeWarps(int nLeaves, int maxRow, bool fp32);
 // values of one front's L block the solve kernels stage in shared memory
 int stagingCapacity(const PersistentPlan& p, size_t elemBytes);
 // The first solve's back substitution run by the factorisation's own launch
@@ -215,8 +236,10 @@ bool fusableBackward(const PersistentPlan& p, bool fp32);
 void launchFactorForwardCascade(const DevData& d, const PersistentPlan& p, bool fp32, const double* rhs,
                                 cudaStream_t s, bool withBackward = false, bool lastSweep = false);
 // forward elimination of the right-hand side rhs (FP64, rounded to the solve precision)
+// (withBackward, trees on thread blocks only: the back substitution of that
+// sweep too, in place of launchBackward; lastSweep: it is the iteration's last)
 void launchForwardCascade(const DevData& d, const PersistentPlan& p, bool fp32, const double* rhs, int sweep,
-                          cudaStream_t s);
+                          cudaStream_t s, bool withBackward = false, bool lastSweep = false);
 // back substitution; stores the solution in del (FP64 solve) or accumulates it in xref
 // (FP32 refinement sweep `sweep`; the last sweep also copies xref to del)
 void launchBackward(const DevData& d, const PersistentPlan& p, bool fp32, int sweep, bool last, cudaStream_t s);
