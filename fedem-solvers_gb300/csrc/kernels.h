@@ -197,9 +197,13 @@ struct PersistentPlan {
   int backwardWarps = 8;   // warps per block of the back-substitution queue
   int largeCluster = 16;   // sixteenths of the GPU's SMs the large-front factorisation runs on (2, 4, 8 or 16)
 };
-// fronts with more rows than this are factored and solved by a thread block
-// each (front_large.cu); smaller ones by one warp each in shared memory
-constexpr int kLargeFrontRows = 96;
+// fronts with more rows than this are factored and solved by several thread
+// blocks each (front_large.cu); smaller ones by one warp each in shared memory.
+// 8 steps of the space-frame tower with the line at 96 / 64 / 48 rows: FP64 16.1 /
+// 15.6 / 13.8 ms, mixed 14.7 / 14.1 / 13.0; 20 steps of 16 reduced parts, FP64 (80
+// row leaf fronts): 24.4 / 19.9 / 19.0 ms.  Fronts of beam chains (up to 36 rows)
+// stay below it: there the trees' parallelism suffices.
+constexpr int kLargeFrontRows = 48;
 // the large-front kernels: factorisation (tangent models), forward elimination
 // of rhs and back substitution (active models; before the warp queue's small
 // fronts) of solve `sweep` of the iteration
