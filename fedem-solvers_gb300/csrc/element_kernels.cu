@@ -1137,7 +1137,7 @@ __global__ void __launch_bounds__(CHUNK_TPB) kNormsPartial(DevData d) {
 // norms, convergence test (normTypeModule.f90:196-249) and iteration counters
 // one warp per model: lane k combines partial value k over the model's chunks
 // in chunk order, lane 0 evaluates the norms and the test
-__global__ void kControl(DevData d) {
+__global__ void kControl(DevData d, int* tally) {
   pdlEntry();
   const int m = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
@@ -1203,19 +1203,53 @@ __global__ void kControl(DevData d) {
     if (exists2) conv = conv && oneOf;
     if (exists1) conv = conv && allOf;
   }
+  // would the model start a step at time t after n steps (kBeginStep's test)
+  auto starts = [&](long long n, double t) {
+    return n < d.m.stepLimit[m] && !(d.m.tStart[m] <= d.m.tEnd[m] && t + 0.1 * d.m.minInc[m] > d.m.tEnd[m]);
+  };
   if (conv) {
-    d.m.nStep[m] += 1;
+    const long long n = d.m.nStep[m] + 1;
+    d.m.nStep[m] = n;
     d.m.state[m] = ST_NEED_STEP;
     d.m.flags[m] = fl | FL_STEPDONE;
+    if (starts(n, d.m.time[m])) {
+      atomicAdd(tally, 1);
+      if (starts(n + 1, d.m.time[m] + d.m.dt[m])) atomicAdd(tally + 1, 1);
+    }
+  } else if (d.m.state[m] == ST_ITER) {
+    atomicAdd(tally, 1);
+    if (starts(d.m.nStep[m] + 1, d.m.time[m])) atomicAdd(tally + 1, 1);
   }
 }
 
 // terminateStep (solverRoutinesModule.f90:728-827): orthonormalise the triad
 // rotations of models that finished a step; keep their deformation for the next one
 // threads [0, ntriTot) a triad each, threads [ntriTot, ntriTot + nelTot) an element each
-__global__ void kStepEnd(DevData d) {
+// (and, see IterationEnd, counters reset and the iteration reported)
+__global__ void kStepEnd(DevData d, IterationEnd e) {
   pdlEntry();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  // thread 0 reads the counters it reports before zeroing them; the others skip them
+  const int kept = e.elements ? 4 : 0;
+  const long long nt = (long long)gridDim.x * blockDim.x;
+  for (long long k = kept + t; k < e.ctrInts; k += nt) e.ctr[k] = 0;
+  for (long long k = t; k < e.queueInts; k += nt) e.queue[k] = -1;
+  if (t == 0 && e.tally) {
+    const int active = *e.active, remaining = e.tally[0], more = e.tally[1];
+    const long long elements = *e.elements;
+    for (int k = 0; k < kept; ++k) e.ctr[k] = 0;
+    e.tally[0] = 0;
+    e.tally[1] = 0;
+    e.tally[2] = active;
+    const long long serial = ++*reinterpret_cast<long long*>(e.tally + 4);
+    volatile IterationReport* h = e.host;
+    h->elements = elements;
+    h->active = active;
+    h->remaining = remaining;
+    h->more = more;
+    __threadfence_system();
+    h->serial = serial;
+  }
   if (t < d.ntriTot) {
     if ((d.m.flags[d.triModel[t]] & FL_STEPDONE) && d.triNdof[t] == 6) orthonormRot(d.ur + 12 * (size_t)t);
     return;
@@ -1426,16 +1460,16 @@ void launchCsrGather(const DevData& d, cudaStream_t s) {
 void launchIncrement(const DevData& d, cudaStream_t s) {
   pdlLaunch(kIncrement, blocksFor(d.ntriTot + d.ndofTot), TPB, 0, s, d);
 }
-void launchNormsControl(const DevData& d, cudaStream_t s) {
+void launchNormsControl(const DevData& d, const IterationEnd& e, cudaStream_t s) {
   launchNormsPartial(d, s);
-  launchControlStepEnd(d, s);
+  launchControlStepEnd(d, e, s);
 }
 void launchNormsPartial(const DevData& d, cudaStream_t s) {
   if (d.nchunkTot > 0) pdlLaunch(kNormsPartial, d.nchunkTot, CHUNK_TPB, 0, s, d);
 }
-void launchControlStepEnd(const DevData& d, cudaStream_t s) {
-  pdlLaunch(kControl, blocksFor(32LL * d.m.n, 128), 128, 0, s, d);
-  pdlLaunch(kStepEnd, blocksFor(d.ntriTot + d.nelTot), TPB, 0, s, d);
+void launchControlStepEnd(const DevData& d, const IterationEnd& e, cudaStream_t s) {
+  pdlLaunch(kControl, blocksFor(32LL * d.m.n, 128), 128, 0, s, d, e.tally);
+  pdlLaunch(kStepEnd, blocksFor(d.ntriTot + d.nelTot), TPB, 0, s, d, e);
   launchPartsStepEnd(d, s);
 }
 void launchLoads(const DevData& d, cudaStream_t s) {

@@ -45,8 +45,7 @@ Engine::~Engine() {
     std::string err;
     resultsClose(err);
   }
-  if (graphExec_) cudaGraphExecDestroy(graphExec_);
-  if (graph_) cudaGraphDestroy(graph_);
+  dropGraphs();
   if (stream_) cudaStreamSynchronize(stream_);
   for (cudaEvent_t ev : ev_)
     if (ev) cudaEventDestroy(ev);
@@ -56,6 +55,7 @@ Engine::~Engine() {
   for (void* p : allocs_) cudaFree(p);
   if (hActive_) cudaFreeHost(hActive_);
   if (hStates_) cudaFreeHost(hStates_);
+  if (hReport_) cudaFreeHost(hReport_);
   if (side_) cudaStreamSynchronize(side_);
   if (evFork_) cudaEventDestroy(evFork_);
   if (evJoin_) cudaEventDestroy(evJoin_);
@@ -1111,7 +1111,10 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
     const size_t largeInts = (size_t)nLargeFronts * (2 + 3 * (size_t)nq);
     ctrInts_ = 4 + 4 * (size_t)nq + (size_t)nq * (nfr + 1) + largeInts;
     ctrBlock_ = alloc<int>(ctrInts_);
-    if (!ctrBlock_) { err = "out of device memory (counters)"; return -906; }
+    // remaining, more, last active count; serial number (8-byte aligned)
+    end_.tally = alloc<int>(6);
+    if (!ctrBlock_ || !end_.tally) { err = "out of device memory (counters)"; return -906; }
+    if (ctrInts_ > INT_MAX || (size_t)nq * leaves.size() > INT_MAX) { err = "too many fronts for the counters"; return -910; }
     dActive_ = ctrBlock_;
     dActiveEl_ = reinterpret_cast<long long*>(ctrBlock_ + 2);
     pplan_.bwCtr = ctrBlock_ + 4;
@@ -1274,7 +1277,15 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
   if (allocFailed_) { err = "out of device memory"; return -906; }
   FG_CHECK(cudaMallocHost(&hActive_, sizeof(int)));
   FG_CHECK(cudaMallocHost(&hStates_, sizeof(int) * (size_t)std::max(nm, 1)));
-  FG_CHECK(cudaMallocHost(&hActiveEl_, sizeof(long long)));
+  FG_CHECK(cudaMallocHost(&hReport_, sizeof(IterationReport)));
+  *hReport_ = IterationReport{};
+  end_.ctr = ctrBlock_;
+  end_.ctrInts = (int)ctrInts_;
+  end_.queue = pplan_.bwQueue;
+  end_.queueInts = (int)queueInts_;
+  end_.active = dActive_;
+  end_.elements = dActiveEl_;
+  end_.host = hReport_;
   for (cudaEvent_t& ev : ev_) FG_CHECK(cudaEventCreate(&ev));
   // mutable state for snapshot/restore (everything a run changes that is read
   // before it is rewritten), with the layout of each array's per-model slices
@@ -1739,9 +1750,9 @@ bool Engine::sideReady() {
   return true;
 }
 
-void Engine::enqueueAssembly(cudaStream_t s) {
+void Engine::enqueueAssembly(cudaStream_t s, bool reset) {
   iterated_ = true;
-  resetIterationCounters(s);
+  if (reset) resetIterationCounters(s);
   launchBeginStep(d_, dActive_, dActiveEl_, seed_, s);
   launchQsRestore(d_, s);
   // Beam-only batches: the element Newton matrices and their CSR gather read
@@ -1776,18 +1787,21 @@ void Engine::enqueueAssembly(cudaStream_t s) {
 
 // second half: factorisation and solves, the increment, the element pass and
 // the convergence test
-void Engine::enqueueSolveUpdate(cudaStream_t s) {
+void Engine::enqueueSolveUpdate(cudaStream_t s, bool timed) {
   // Batches without large fronts run the first solve's back substitution in
   // the factorisation's launch: a model's back substitution starts as soon as
   // its own elimination is done, beside the other models' factorisations.
   const bool fuse = fuseBackward_;
-  recordPhase(ev_[0], s);
+  auto mark = [&](int k) {
+    if (timed) recordPhase(ev_[k], s);
+  };
+  mark(0);
   enqueueFactor(s, fuse);
-  recordPhase(ev_[1], s);
-  enqueueSolve(s, true, fuse);
-  recordPhase(ev_[2], s);
+  mark(1);
+  enqueueSolve(s, timed, fuse);
+  mark(2);
   launchIncrement(d_, s);
-  recordPhase(ev_[3], s);
+  mark(3);
   // the partial norms read the increments and the residual, which the element
   // pass does not touch; the convergence test after the join also sees every
   // status bit the element pass set (a failed corotation)
@@ -1799,24 +1813,24 @@ void Engine::enqueueSolveUpdate(cudaStream_t s) {
     cudaEventRecord(evJoin2_, side_);
   }
   launchElements(d_, EM_INC, s);
-  recordPhase(ev_[4], s);
+  mark(4);
   if (fork) {
     cudaStreamWaitEvent(s, evJoin2_, 0);
-    launchControlStepEnd(d_, s);
+    launchControlStepEnd(d_, end_, s);
   } else {
-    launchNormsControl(d_, s);
+    launchNormsControl(d_, end_, s);
   }
   if (rec_.on) launchRecordStep(d_, rec_.plan, false, s);
 }
 
 int Engine::assembleIteration() {
   ensureTuned();
-  enqueueAssembly(stream_);
+  enqueueAssembly(stream_, true);
   return cudaStreamSynchronize(stream_) == cudaSuccess ? 0 : -940;
 }
 
 int Engine::solveUpdateIteration() {
-  enqueueSolveUpdate(stream_);
+  enqueueSolveUpdate(stream_, false);
   if (cudaStreamSynchronize(stream_) != cudaSuccess) return -941;
   std::string err;
   return resultsDrain(err) ? -942 : 0;
@@ -2105,9 +2119,9 @@ int Engine::parkModels(const std::vector<int>& ms) {
   return cudaStreamSynchronize(stream_) == cudaSuccess ? 0 : -949;
 }
 
-void Engine::enqueueIteration(cudaStream_t s) {
-  enqueueAssembly(s);
-  enqueueSolveUpdate(s);
+void Engine::enqueueIteration(cudaStream_t s, bool timed, bool reset) {
+  enqueueAssembly(s, reset);
+  enqueueSolveUpdate(s, timed);
   const int sw = opt_.refineSweeps;
   // kernels per batched iteration: 12 fixed (begin step, predict, elements x2, residual,
   // element Newton build + rotate (one fused kernel for compressed beams), CSR gather,
@@ -2231,55 +2245,127 @@ int Engine::probeRootWaitTimeout(long long spins, int* flag) {
   return 0;
 }
 
+void Engine::dropGraphs() {
+  for (int k = 0; k < 2; ++k) {
+    if (graphExec_[k]) cudaGraphExecDestroy(graphExec_[k]);
+    if (graph_[k]) cudaGraphDestroy(graph_[k]);
+    graphExec_[k] = nullptr;
+    graph_[k] = nullptr;
+  }
+}
+
+// the captured iteration (timed: with the phase-timing events, about 2 us each)
+int Engine::graphReady(bool timed) {
+  const int k = timed ? 1 : 0;
+  if (!opt_.useGraph || graphExec_[k]) return 0;
+  cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal);
+  enqueueIteration(stream_, timed, false);
+  if (cudaStreamEndCapture(stream_, &graph_[k]) != cudaSuccess) return -920;
+  if (cudaGraphInstantiate(&graphExec_[k], graph_[k], 0) != cudaSuccess) return -921;
+  return 0;
+}
+
+int Engine::launchIteration(bool timed) {
+  if (!opt_.useGraph) {
+    enqueueIteration(stream_, timed, false);
+    return 0;
+  }
+  const int rc = graphReady(timed);
+  if (rc) return rc;
+  return cudaGraphLaunch(graphExec_[timed ? 1 : 0], stream_) == cudaSuccess ? 0 : -922;
+}
+
+// Waits for the step end's report of iteration `serial` (false: the stream
+// failed or drained without it).
+bool Engine::waitReport(long long serial) {
+  const volatile IterationReport* h = hReport_;
+  for (int spins = 0; h->serial < serial; ++spins) {
+    if ((spins & 1023) != 1023) continue;
+    const cudaError_t q = cudaStreamQuery(stream_);
+    if (q == cudaSuccess) return h->serial >= serial;
+    if (q != cudaErrorNotReady) return false;
+    std::this_thread::yield();
+  }
+  std::atomic_thread_fence(std::memory_order_acquire);
+  return true;
+}
+
+// the phase durations of the last timed iteration
+void Engine::samplePhases(long long elements, int active) {
+  float t0 = 0.f, t1 = 0.f, t2 = 0.f;
+  if (!(elements > 0 || (active > 0 && d_.npartTot > 0)) ||
+      cudaEventElapsedTime(&t0, ev_[3], ev_[4]) != cudaSuccess ||
+      cudaEventElapsedTime(&t1, ev_[0], ev_[1]) != cudaSuccess || cudaEventElapsedTime(&t2, ev_[1], ev_[2]) != cudaSuccess)
+    return;
+  phaseMs_[0] += t0;
+  phaseMs_[1] += t1;
+  phaseMs_[2] += t2;
+  float t3 = 0.0f;
+  if (opt_.refineSweeps > 1 && cudaEventElapsedTime(&t3, ev_[5], ev_[6]) == cudaSuccess) phaseMs_[3] += t3;
+  float t4 = 0.0f;
+  if (cudaEventElapsedTime(&t4, ev_[7], ev_[8]) == cudaSuccess) phaseMs_[4] += t4;
+  phaseElems_ += elements;
+  ++phaseSamples_;
+}
+
+// The iterations are launched one ahead of the device: the step end of each
+// reports (IterationReport) how many models go on, so the host needs no copy and
+// no synchronisation between them, and none is launched that would find nothing
+// to do, as long as some model is known to start another step.  While every
+// remaining model is in its last step, an iteration is launched only when the
+// one before asks for it.  (Seven at a time, with a synchronisation after each
+// seven, ran up to six idle iterations at the end: the 20-beam cantilever driven
+// step by step took 0.59 ms a step for two iterations of 0.13 ms.)  Every
+// seventh iteration is timed: an odd distance, so that with two iterations per
+// step predictors and correctors are both sampled.
 int Engine::run(long long maxBatched, RunStats* stats) {
   ensureTuned();
-  if (opt_.useGraph && !graphExec_) {
-    cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal);
-    enqueueIteration(stream_);
-    if (cudaStreamEndCapture(stream_, &graph_) != cudaSuccess) return -920;
-    if (cudaGraphInstantiate(&graphExec_, graph_, 0) != cudaSuccess) return -921;
-  }
+  int rc = graphReady(false);
+  if (rc) return rc;
   if (!evRun_[0]) {
     cudaEventCreate(&evRun_[0]);
     cudaEventCreate(&evRun_[1]);
   }
   auto t0 = std::chrono::steady_clock::now();
   cudaEventRecord(evRun_[0], stream_);
-  long long done = 0;
-  // an odd chunk length: the phase durations are sampled from the last
-  // iteration of each chunk, and with two iterations per time step an even
-  // length would always sample the same kind (predictor or corrector)
-  const int chunk = 7;
-  while (done < maxBatched) {
-    int n = (int)std::min<long long>(chunk, maxBatched - done);
-    for (int k = 0; k < n; ++k) {
-      if (opt_.useGraph) cudaGraphLaunch(graphExec_, stream_);
-      else enqueueIteration(stream_);
+  resetIterationCounters(stream_);
+  cudaMemsetAsync(end_.tally, 0, sizeof(int) * 6, stream_);
+  *hReport_ = IterationReport{};
+  const int every = 7;
+  long long launched = 0, seen = 0, done = 0;
+  // the first two at once: a step takes at least two iterations, but for linear
+  // quasi-static and fixed-iteration ones
+  long long ahead = 2;
+  while (launched < maxBatched || seen < launched) {
+    for (; launched < std::min(maxBatched, ahead); ++launched) {
+      rc = launchIteration((launched + 1) % every == 0);
+      if (rc) return rc;
     }
-    done += n;
-    cudaMemcpyAsync(hActiveEl_, dActiveEl_, sizeof(long long), cudaMemcpyDeviceToHost, stream_);
-    int active = readActive();
-    // sample the phase durations of the last iteration of this chunk
-    float t0 = 0.f, t1 = 0.f, t2 = 0.f;
-    if (cudaEventElapsedTime(&t0, ev_[3], ev_[4]) == cudaSuccess &&
-        cudaEventElapsedTime(&t1, ev_[0], ev_[1]) == cudaSuccess &&
-        cudaEventElapsedTime(&t2, ev_[1], ev_[2]) == cudaSuccess && (*hActiveEl_ > 0 || (active > 0 && d_.npartTot > 0))) {
-      phaseMs_[0] += t0;
-      phaseMs_[1] += t1;
-      phaseMs_[2] += t2;
-      float t3 = 0.0f;
-      if (opt_.refineSweeps > 1 && cudaEventElapsedTime(&t3, ev_[5], ev_[6]) == cudaSuccess)
-        phaseMs_[3] += t3;
-      float t4 = 0.0f;
-      if (cudaEventElapsedTime(&t4, ev_[7], ev_[8]) == cudaSuccess) phaseMs_[4] += t4;
-      phaseElems_ += *hActiveEl_;
-      ++phaseSamples_;
-    }
-    if (rec_.on) {
+    if (!waitReport(seen + 1)) return -922;
+    // (a later iteration may have reported meanwhile)
+    seen = hReport_->serial;
+    const int remaining = hReport_->remaining, more = hReport_->more, active = hReport_->active;
+    if (active > 0) done = seen;
+    if (seen % every == 0) samplePhases(hReport_->elements, active);
+    if (rec_.on && seen % every == 0) {
+      // records are drained before a model's ring can fill: nothing runs meanwhile
+      if (cudaStreamSynchronize(stream_) != cudaSuccess) return -922;
       std::string err;
       if (resultsDrain(err)) return -924;
     }
-    if (active == 0) break;
+    if (remaining == 0) break;
+    ahead = seen + (more > 0 && !(rec_.on && (seen + 1) % every == 0) ? 2 : 1);
+  }
+  // the models that reached their end leave the active set (kBeginStep's
+  // bookkeeping, which an iteration without work would do)
+  if (seen > 0 && hReport_->remaining == 0) {
+    resetIterationCounters(stream_);
+    launchBeginStep(d_, dActive_, dActiveEl_, seed_, stream_);
+  }
+  if (rec_.on) {
+    if (cudaStreamSynchronize(stream_) != cudaSuccess) return -922;
+    std::string err;
+    if (resultsDrain(err)) return -924;
   }
   cudaEventRecord(evRun_[1], stream_);
   if (cudaStreamSynchronize(stream_) != cudaSuccess) return -922;
@@ -2310,18 +2396,16 @@ int Engine::run(long long maxBatched, RunStats* stats) {
 
 int Engine::launchChunk(int n) {
   ensureTuned();
-  if (opt_.useGraph && !graphExec_) {
-    cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal);
-    enqueueIteration(stream_);
-    if (cudaStreamEndCapture(stream_, &graph_) != cudaSuccess) return -920;
-    if (cudaGraphInstantiate(&graphExec_, graph_, 0) != cudaSuccess) return -921;
-  }
+  const int rc = graphReady(false);
+  if (rc) return rc;
   if (!evChunk_ && cudaEventCreateWithFlags(&evChunk_, cudaEventDisableTiming) != cudaSuccess) return -924;
+  resetIterationCounters(stream_);
   for (int k = 0; k < n; ++k) {
-    if (opt_.useGraph) cudaGraphLaunch(graphExec_, stream_);
-    else enqueueIteration(stream_);
+    const int rl = launchIteration(false);
+    if (rl) return rl;
   }
-  cudaMemcpyAsync(hActive_, dActive_, sizeof(int), cudaMemcpyDeviceToHost, stream_);
+  // the models that took part in the chunk's last iteration
+  cudaMemcpyAsync(hActive_, end_.tally + 2, sizeof(int), cudaMemcpyDeviceToHost, stream_);
   cudaMemcpyAsync(hStates_, d_.m.state, sizeof(int) * (size_t)d_.m.n, cudaMemcpyDeviceToHost, stream_);
   cudaEventRecord(evChunk_, stream_);
   chunkPending_ = true;

@@ -172,9 +172,16 @@ class Engine {
  private:
   template <typename T>
   T* alloc(size_t n);
-  void enqueueIteration(cudaStream_t s);
-  void enqueueAssembly(cudaStream_t s);
-  void enqueueSolveUpdate(cudaStream_t s);
+  // timed: with the phase-timing events; reset: with the iteration counters'
+  // reset (between iterations the step end does it)
+  void enqueueIteration(cudaStream_t s, bool timed, bool reset);
+  void enqueueAssembly(cudaStream_t s, bool reset);
+  void enqueueSolveUpdate(cudaStream_t s, bool timed);
+  int launchIteration(bool timed);
+  int graphReady(bool timed);
+  void dropGraphs();
+  bool waitReport(long long serial);
+  void samplePhases(long long elements, int active);
   // backwardDone: the first solve's back substitution already ran in the
   // factorisation's launch (enqueueFactor with withBackward)
   void enqueueSolve(cudaStream_t s, bool timedForward = false, bool backwardDone = false);
@@ -217,8 +224,11 @@ class Engine {
   // pass after the increment (they read the increments and the residual only)
   cudaEvent_t evFork2_ = nullptr, evJoin2_ = nullptr;
   bool sideReady();
-  cudaGraph_t graph_ = nullptr;
-  cudaGraphExec_t graphExec_ = nullptr;
+  // the captured iteration, without and with the phase-timing events
+  cudaGraph_t graph_[2] = {nullptr, nullptr};
+  cudaGraphExec_t graphExec_[2] = {nullptr, nullptr};
+  IterationEnd end_;
+  IterationReport* hReport_ = nullptr;  // pinned, written by the step end
   std::vector<int> modelTriOff_, modelDofOff_, modelEqOff_, modelElOff_;
   std::vector<int64_t> modelSlotOff_;
   std::vector<int> normChunkOff_, normChunkCnt_;
@@ -256,7 +266,6 @@ class Engine {
   // phase timing events (recorded as external event nodes inside the graph)
   cudaEvent_t ev_[9] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   long long* dActiveEl_ = nullptr;
-  long long* hActiveEl_ = nullptr;
   cudaEvent_t evRun_[2] = {nullptr, nullptr};
   double lastRunDevSec_ = 0.0;
   long long uploadedBytes_ = 0;

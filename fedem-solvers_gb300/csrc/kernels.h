@@ -65,6 +65,28 @@ struct BackwardSeed {
   int* queue = nullptr;
   int* ctr = nullptr;
 };
+// What the last kernel of an iteration does beside the step end: the iteration's
+// counters and backward queues reset for the next one (in place of memset nodes),
+// and a report into host memory, its serial number last, that the host can follow
+// without a copy or a synchronisation.
+struct IterationReport {
+  long long serial;    // iterations finished since the counters' last reset by the host
+  long long elements;  // elements of the models that took part
+  int active;          // models that took part
+  int remaining;       // models with another iteration to do
+  int more;            // of them, models with a further step after the one they are in (or about to start)
+};
+struct IterationEnd {
+  int* ctr = nullptr;  // counters to zero
+  int ctrInts = 0;
+  int* queue = nullptr;  // queue slots to empty (-1)
+  int queueInts = 0;
+  const int* active = nullptr;          // (inside ctr)
+  const long long* elements = nullptr;  // (inside ctr)
+  int* tally = nullptr;                 // remaining, more (counted by the convergence test), kept: active of
+                                        // the last iteration; then the serial number
+  IterationReport* host = nullptr;      // pinned host memory
+};
 void launchBeginStep(const DevData& d, int* activeCount, long long* activeEl, const BackwardSeed& seed,
                      cudaStream_t s);
 void launchPredictDofs(const DevData& d, cudaStream_t s);
@@ -74,11 +96,11 @@ void launchBuildElementNewton(const DevData& d, cudaStream_t s);
 void launchRotateElementNewton(const DevData& d, cudaStream_t s);
 void launchCsrGather(const DevData& d, cudaStream_t s);
 void launchIncrement(const DevData& d, cudaStream_t s);
-void launchNormsControl(const DevData& d, cudaStream_t s);
+void launchNormsControl(const DevData& d, const IterationEnd& e, cudaStream_t s);
 // the same in two parts: the per-chunk partial norms (reading the increments
 // and the residual only), then the convergence test and the step end
 void launchNormsPartial(const DevData& d, cudaStream_t s);
-void launchControlStepEnd(const DevData& d, cudaStream_t s);
+void launchControlStepEnd(const DevData& d, const IterationEnd& e, cudaStream_t s);
 // static equilibrium helpers
 void launchStaticBegin(const DevData& d, int* activeCount, const BackwardSeed& seed, cudaStream_t s);
 void launchSeedBackward(const DevData& d, const BackwardSeed& seed, cudaStream_t s);

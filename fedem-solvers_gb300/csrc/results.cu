@@ -180,8 +180,7 @@ int Engine::resultsOpen(const std::string& dir, bool asDouble, std::string& err,
   rec_.written.assign(nm, 0);
   rec_.on = true;
   // the batched iteration is captured again with the record kernel in it
-  if (graphExec_) cudaGraphExecDestroy(graphExec_), graphExec_ = nullptr;
-  if (graph_) cudaGraphDestroy(graph_), graph_ = nullptr;
+  dropGraphs();
   // the current state: the initial configuration, or where the models are now
   launchRecordStep(d_, r, true, stream_);
   return resultsDrain(err);
@@ -256,8 +255,7 @@ int Engine::resultsClose(std::string& err) {
       f = nullptr;
     }
   rec_.on = false;
-  if (graphExec_) cudaGraphExecDestroy(graphExec_), graphExec_ = nullptr;
-  if (graph_) cudaGraphDestroy(graph_), graph_ = nullptr;
+  dropGraphs();
   return rc;
 }
 
