@@ -19,6 +19,8 @@
 
 #include <cmath>
 
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <mutex>
 
@@ -100,47 +102,63 @@ __device__ inline void seedBackward(const BackwardSeed& b, int i) {
   }
 }
 
+// One warp per model: lane 0 keeps the books, lanes 0 to 5 take one of the
+// step's six quotients each (an FP64 division is some 560 cycles; one after the
+// other they were most of the launch).
 __global__ void kBeginStep(DevModels m, int* activeCount, long long* activeEl, BackwardSeed bs) {
   pdlEntry();
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (i >= m.n) return;
-  int st = m.state[i], fl = 0;
+  const int st = m.state[i];
+  int fl = 0;
   if (st == ST_NEED_STEP) {
-    if (m.nStep[i] >= m.stepLimit[i]) { m.flags[i] = 0; return; }
-    double t = m.time[i];
-    if (m.tStart[i] <= m.tEnd[i] && t + 0.1 * m.minInc[i] > m.tEnd[i]) {
-      m.state[i] = ST_DONE;
-      m.flags[i] = 0;
+    const double t = m.time[i];
+    const bool limit = m.nStep[i] >= m.stepLimit[i];
+    __syncwarp();  // every lane has read the books before lane 0 writes them
+    if (limit || (m.tStart[i] <= m.tEnd[i] && t + 0.1 * m.minInc[i] > m.tEnd[i])) {
+      if (lane == 0) {
+        if (!limit) m.state[i] = ST_DONE;
+        m.flags[i] = 0;
+      }
       return;
     }
-    double dt = m.dt[i], be = m.beta[i], ga = m.gamma[i];
-    m.time[i] = t + dt;
-    m.iter[i] = 0;
-    m.nSeqNoUpd[i] = 0;
-    m.negPiv[i] = 0;
+    const double dt = m.dt[i], be = m.beta[i], ga = m.gamma[i];
+    const bool qs = t + dt < m.tQs[i] + 0.1 * m.minInc[i];
+    const int qsCount = m.qsCount[i];
+    __syncwarp();
     fl = FL_ACTIVE | FL_PRED;
-    if (t + dt < m.tQs[i] + 0.1 * m.minInc[i]) {
+    if (qs) {
       // quasi-static load step (solverModule.f90:826-841, isQuasiStatic)
       fl |= FL_QSTATIC;
       if (m.fixedIt[i] == -1) fl |= FL_LINEAR;
-      m.qsCount[i] += 1;
     } else {
-      if (m.qsCount[i] > 0) fl |= FL_QS2DYN;
-      m.qsCount[i] = 0;
-      m.pc[4 * i + 0] = ga / be - 1.0;
-      m.pc[4 * i + 1] = (0.5 * ga / be - 1.0) * dt;
-      m.pc[4 * i + 2] = 1.0 / (be * dt);
-      m.pc[4 * i + 3] = 0.5 / be - 1.0;
-      m.sacc[i] = 1.0 / (be * dt * dt);
-      m.svel[i] = ga / (be * dt);
+      if (qsCount > 0) fl |= FL_QS2DYN;
+      // DD, DA, AD, AA of the predictor; sacc, svel
+      const double num = lane == 0 || lane == 5 ? ga : lane == 1 ? 0.5 * ga : lane == 3 ? 0.5 : 1.0;
+      const double den = lane == 2 || lane == 5 ? be * dt : lane == 4 ? be * dt * dt : be;
+      double v = num / den;
+      if (lane == 0 || lane == 1 || lane == 3) v -= 1.0;
+      if (lane == 1) v *= dt;
+      if (lane < 4) m.pc[4 * i + lane] = v;
+      if (lane == 4) m.sacc[i] = v;
+      if (lane == 5) m.svel[i] = v;
     }
-    m.state[i] = ST_ITER;
+    if (lane == 0) {
+      m.time[i] = t + dt;
+      m.iter[i] = 0;
+      m.nSeqNoUpd[i] = 0;
+      m.negPiv[i] = 0;
+      m.qsCount[i] = qs ? qsCount + 1 : 0;
+      m.state[i] = ST_ITER;
+    }
+    __syncwarp();
   } else if (st == ST_ITER) {
     fl = FL_ACTIVE | (m.flags[i] & (FL_QSTATIC | FL_LINEAR));
   } else {
-    m.flags[i] = 0;
+    if (lane == 0) m.flags[i] = 0;
     return;
   }
+  if (lane != 0) return;
   int it = m.iter[i];
   bool tangent = it < max(1, m.nUpdat[i]) || m.nSeqNoUpd[i] >= m.maxSeq[i];
   if (tangent) {
@@ -444,6 +462,240 @@ __global__ void __launch_bounds__(128) kElements(DevData d, int mode) {
     y[r] = ss * (d.fg[(size_t)r * nel + e] * gl0 + d.fg[(size_t)(r + 12) * nel + e] * gl1 +
                  d.fg[(size_t)(r + 24) * nel + e] * gl2);
   rotateStore(S, y, Qo, nel, e);
+}
+
+// ---- the beam element pass and Newton matrices, four lanes per element -------
+// A sub-core issues one FP64 instruction per 64 cycles whether one lane is active
+// or 32, so with fewer warps than sub-cores an element's 440 instructions set the
+// launch's time. Here the four lanes of an element take a node's translations or
+// rotations each (lane g: DOFs 3 g .. 3 g + 2): its accelerations, a reference
+// point, a column of the new frame, two columns of a node's local position, its
+// rows of the products and of the rotations; the frame's axes are formed by all
+// four. About 180 instructions instead of 440 (1.6 times as many in all), every
+// value by the same operations in the same order: the same bits. The pass after
+// the increment, with the partial norms beside it: 20 beams 24.2 -> 13.8 us, 3,827
+// beams 26.3 -> 18.4. From about 9,700 beams (16 lanes' worth of elements for each
+// of the 608 sub-cores, two rounds of 180) one thread per element is ahead.
+constexpr int kWideElements = 8192;
+
+__device__ __forceinline__ double quad(double v, int g, unsigned mask) { return __shfl_sync(mask, v, g, 4); }
+__device__ __forceinline__ int pick(unsigned table, int g) { return (int)((table >> (8 * g)) & 0xffu); }
+
+// rows 3 g .. 3 g + 2 of s A x (26-value pattern; see matvecBeam), x distributed
+__device__ inline void matvecBeamRows(const double* __restrict__ A26, int nel, int e, int g, unsigned mask,
+                                      const double* x, double s, double* y) {
+  auto a = [&](unsigned table) { return A26[(size_t)pick(table, g) * nel + e]; };
+  const bool rot = g & 1;
+  // value indices of the rows' nonzeros for g = 0 .. 3 (lowest byte first)
+  const double c0 = a(0x0b010a00u), c1 = a(0x17120b01u);
+  const double b0 = a(0x09040702u), b1 = a(0x0e100c03u), b2 = a(0x16130d04u), b3 = a(0x18140e05u);
+  const double d0 = a(0x05080306u), d1 = a(0x110d0f07u), d2 = a(0x14151008u), d3 = a(0x19161109u);
+  const double xa = quad(x[0], rot ? 1 : 0, mask), xb = quad(x[0], rot ? 3 : 2, mask);
+  // columns 1, 5, 7, 11 and 2, 4, 8, 10
+  const double u0 = quad(x[1], 0, mask), u1 = quad(x[2], 1, mask), u2 = quad(x[1], 2, mask), u3 = quad(x[2], 3, mask);
+  const double w0 = quad(x[2], 0, mask), w1 = quad(x[1], 1, mask), w2 = quad(x[2], 2, mask), w3 = quad(x[1], 3, mask);
+  y[0] = c0 * xa;
+  y[0] += c1 * xb;
+  y[1] = b0 * (rot ? w0 : u0);
+  y[1] += b1 * (rot ? w1 : u1);
+  y[1] += b2 * (rot ? w2 : u2);
+  y[1] += b3 * (rot ? w3 : u3);
+  y[2] = d0 * (rot ? u0 : w0);
+  y[2] += d1 * (rot ? u1 : w1);
+  y[2] += d2 * (rot ? u2 : w2);
+  y[2] += d3 * (rot ? u3 : w3);
+#pragma unroll
+  for (int r = 0; r < 3; ++r) y[r] *= s;
+}
+
+__device__ inline void rotateStoreRows(const double* S, const double* f, double* out, int nel, int e, int g) {
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+    out[(size_t)(3 * g + r) * nel + e] = S[r] * f[0] + S[r + 3] * f[1] + S[r + 6] * f[2];
+}
+
+__global__ void __launch_bounds__(128) kElementsWide(DevData d, int mode) {
+  pdlEntry();
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, e = t >> 2, g = t & 3;
+  const int nel = d.nelTot;
+  if (e >= nel) return;
+  const unsigned mask = 0xfu << (threadIdx.x & 28);
+  const int m = d.elModel[e];
+  const int fl = d.m.flags[m];
+  if (mode == EM_PRED) {
+    if (!(fl & FL_PRED)) return;
+  } else {
+    if (!(fl & FL_ACTIVE)) return;
+  }
+  const bool qs = fl & FL_QSTATIC;
+  const int n = g >> 1;
+  const bool rot = g & 1;
+  double S[12];
+#pragma unroll
+  for (int k = 0; k < 12; ++k) S[k] = d.supTr[(size_t)k * nel + e];
+  const int tri[2] = {d.elTri[e], d.elTri[nel + e]};
+  double uld[3], uldd[3];
+  const double dt = d.m.dt[m];
+  const bool vldActive = d.hasVld[e] && dt > 0.0;
+  const bool needUld = !qs && (d.hasC[e] || vldActive);
+  if (!qs) {
+    const double* vs = mode == EM_PRED ? d.dk : d.urd;
+    const double* as = mode == EM_PRED ? d.ak : d.urdd;
+    const int d0 = d.triFirstDof[tri[n]] + (rot ? 3 : 0);
+    const double a0 = as[d0], a1 = as[d0 + 1], a2 = as[d0 + 2];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) uldd[r] = S[3 * r] * a0 + S[3 * r + 1] * a1 + S[3 * r + 2] * a2;
+    if (needUld) {
+      const double v0 = vs[d0], v1 = vs[d0 + 1], v2 = vs[d0 + 2];
+#pragma unroll
+      for (int r = 0; r < 3; ++r) uld[r] = S[3 * r] * v0 + S[3 * r + 1] * v1 + S[3 * r + 2] * v2;
+    }
+  }
+  const bool newPositions = mode == EM_INC && !(qs && (fl & FL_LINEAR));
+  double fin[3];
+  if (newPositions) {
+    // reference point j of lane j (lane 3: point 0 again)
+    const int j = g < 3 ? g : 0;
+    const int node = d.elRef[(size_t)j * nel + e];
+    const double* U = d.ur + 12 * (size_t)(node ? tri[1] : tri[0]);
+    const double o0 = d.offset[(size_t)(3 * j) * nel + e], o1 = d.offset[(size_t)(3 * j + 1) * nel + e],
+                 o2 = d.offset[(size_t)(3 * j + 2) * nel + e];
+    double pj[3], p[3][3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) pj[q] = U[q] * o0 + U[q + 3] * o1 + U[q + 6] * o2 + U[q + 9];
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+#pragma unroll
+      for (int q = 0; q < 3; ++q) p[k][q] = quad(pj[q], k, mask);
+    double ex[3], v2[3], ez[3], ey[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) { ex[k] = p[1][k] - p[0][k]; v2[k] = p[2][k] - p[0][k]; }
+    crossd(ex, v2, ez);
+    double lx = ex[0] * ex[0] + ex[1] * ex[1] + ex[2] * ex[2];
+    double lz = ez[0] * ez[0] + ez[1] * ez[1] + ez[2] * ez[2];
+    if (!(lx > 1.0e-16) || !(lz > 1.0e-16)) {  // the same for the four lanes
+      if (g == 0) atomicOr(&d.m.status[m], SS_COROT);
+      return;
+    }
+    const double ilx = rsqrt(lx), ilz = rsqrt(lz);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) { ex[k] *= ilx; ez[k] *= ilz; }
+    crossd(ez, ex, ey);
+    // column g of the new frame
+    double b[3], col[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) b[k] = d.triRelSup[(size_t)(3 * g + k) * nel + e];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      double v = ex[r] * b[0] + ey[r] * b[1] + ez[r] * b[2];
+      if (g == 3) v += p[0][r];
+      col[r] = v;
+      d.supTr[(size_t)(3 * g + r) * nel + e] = v;
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int r = 0; r < 3; ++r) S[3 * c + r] = quad(col[r], c, mask);
+  }
+  if (newPositions || qs) {
+    double inv[12];
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) inv[r + 3 * c] = S[c + 3 * r];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) inv[9 + r] = -(inv[r] * S[9] + inv[r + 3] * S[10] + inv[r + 6] * S[11]);
+    // the node's local position: the rotation lane forms columns 0 and 1, the
+    // translation lane columns 2 and 3
+    const double* U = d.ur + 12 * (size_t)tri[n];
+    const double* Tu = d.trUnd + (size_t)(12 * n) * nel + e;
+    double la[3], lb[3], lc[3];
+    {
+      const double* Ua = U + (rot ? 0 : 6);
+      const double* Ub = U + (rot ? 3 : 9);
+      const double a0 = Ua[0], a1 = Ua[1], a2 = Ua[2], b0 = Ub[0], b1 = Ub[1], b2 = Ub[2];
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        la[r] = inv[r] * a0 + inv[r + 3] * a1 + inv[r + 6] * a2;
+        double v = inv[r] * b0 + inv[r + 3] * b1 + inv[r + 6] * b2;
+        if (!rot) v += inv[r + 9];
+        lb[r] = v;
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 3; ++r) lc[r] = quad(la[r], 2 * n, mask);  // column 2 from the translation lane
+    if (rot) {
+      // dR = loc(:,1:3) * Tu(:,1:3)^T; entries (3,2), (1,3), (2,1)
+      fin[0] = la[2] * Tu[3 * (size_t)nel] + lb[2] * Tu[4 * (size_t)nel] + lc[2] * Tu[5 * (size_t)nel];
+      fin[1] = la[0] * Tu[6 * (size_t)nel] + lb[0] * Tu[7 * (size_t)nel] + lc[0] * Tu[8 * (size_t)nel];
+      fin[2] = la[1] * Tu[0] + lb[1] * Tu[(size_t)nel] + lc[1] * Tu[2 * (size_t)nel];
+    } else {
+#pragma unroll
+      for (int r = 0; r < 3; ++r) fin[r] = lb[r] - Tu[(size_t)(9 + r) * nel];
+    }
+    __syncwarp(mask);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) d.finit[(size_t)(3 * g + k) * nel + e] = fin[k];
+  } else {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) fin[k] = d.finit[(size_t)(3 * g + k) * nel + e];
+  }
+  const double ss = d.stifScl[e];
+  double y[3];
+  double* FSo = d.Fel;
+  double* FDo = d.Fel + (size_t)12 * nel;
+  double* FIo = d.Fel + (size_t)24 * nel;
+  double* Qo = d.Fel + (size_t)36 * nel;
+  const bool keepFsQ = mode == EM_PRED && !qs;
+  if (!keepFsQ) {
+    matvecBeamRows(d.K26, nel, e, g, mask, fin, ss, y);
+    rotateStoreRows(S, y, FSo, nel, e, g);
+  }
+  if (qs) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) { FDo[(size_t)(3 * g + k) * nel + e] = 0.0; FIo[(size_t)(3 * g + k) * nel + e] = 0.0; }
+  } else {
+    matvecBeamRows(d.M26, nel, e, g, mask, uldd, 1.0, y);
+    rotateStoreRows(S, y, FIo, nel, e, g);
+    if (d.hasC[e] || vldActive) {
+      if (d.hasC[e]) {
+        matvecBeamRows(d.C26, nel, e, g, mask, uld, ss, y);
+      } else {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) y[k] = 0.0;
+      }
+      if (vldActive) {
+        double tmp[3], yk[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) tmp[k] = uld[k] - (fin[k] - d.finitPrev[(size_t)(3 * g + k) * nel + e]) / dt;
+        matvecBeamRows(d.K26, nel, e, g, mask, tmp, ss, yk);
+        const double kd = d.kDmp[e];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) y[k] -= kd * yk[k];
+      }
+      rotateStoreRows(S, y, FDo, nel, e, g);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) FDo[(size_t)(3 * g + k) * nel + e] = 0.0;
+    }
+  }
+  if (keepFsQ) return;
+  const double* gv = d.m.gravity + 3 * m;
+  if (gv[0] == 0.0 && gv[1] == 0.0 && gv[2] == 0.0) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) Qo[(size_t)(3 * g + k) * nel + e] = 0.0;
+    return;
+  }
+  double gl0 = gv[0] * S[0] + gv[1] * S[1] + gv[2] * S[2];
+  double gl1 = gv[0] * S[3] + gv[1] * S[4] + gv[2] * S[5];
+  double gl2 = gv[0] * S[6] + gv[1] * S[7] + gv[2] * S[8];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const int r = 3 * g + k;
+    y[k] = ss * (d.fg[(size_t)r * nel + e] * gl0 + d.fg[(size_t)(r + 12) * nel + e] * gl1 +
+                 d.fg[(size_t)(r + 24) * nel + e] * gl2);
+  }
+  rotateStoreRows(S, y, Qo, nel, e, g);
 }
 
 // axial springs and dampers: direction, length, forces (UpdateSprings/UpdateDampers,
@@ -778,6 +1030,43 @@ __global__ void __launch_bounds__(128) kNewtonBeam(DevData d) {
   rotDiag(R, a[23], a[24], a[25], S); storeBlock(out, nel, e, 3, 3, S);
 }
 
+// four lanes per element: lane g forms the pair block g and the diagonal block g
+// of storeBlock's ten, lanes 0 and 1 also the diagonal blocks 4 and 5 (about 100
+// FP64 instructions instead of 330; the same operations, the same bits)
+__global__ void __launch_bounds__(128) kNewtonBeamWide(DevData d) {
+  pdlEntry();
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, e = t >> 2, g = t & 3;
+  const int nel = d.nelTot;
+  if (e >= nel) return;
+  const int m = d.elModel[e];
+  if (!(d.m.flags[m] & FL_TANGENT)) return;
+  const double* sn = d.m.scaleN + 3 * m;
+  const double ss = d.stifScl[e];
+  const double sM = sn[0], sK = sn[1] * ss, sC = sn[2] * ss;
+  const bool hc = d.hasC[e];
+  auto value = [&](int k) {
+    const size_t ix = (size_t)k * nel + e;
+    double v = sM * d.M26[ix];
+    if (hc) v += sC * d.C26[ix];
+    v += sK * d.K26[ix];
+    return v;
+  };
+  double R[9], S[9];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) R[k] = d.supTr[(size_t)k * nel + e];
+  double* out = d.elMat;
+  // pair blocks (0,1), (0,3), (1,2), (2,3)
+  rotPair(R, value(pick(0x140d0503u, g)), value(pick(0x16100907u, g)), S);
+  storeBlock(out, nel, e, pick(0x02010000u, g), pick(0x03020301u, g), S);
+  // diagonal-type blocks (0,0), (0,2), (1,1), (1,3), then (2,2), (3,3)
+  rotDiag(R, value(pick(0x0b0a0100u, g)), value(pick(0x0e0c0402u, g)), value(pick(0x110f0806u, g)), S);
+  storeBlock(out, nel, e, pick(0x01010000u, g), pick(0x03010200u, g), S);
+  if (g < 2) {
+    rotDiag(R, value(g ? 23 : 18), value(g ? 24 : 19), value(g ? 25 : 21), S);
+    storeBlock(out, nel, e, 2 + g, 2 + g, S);
+  }
+}
+
 // CSR slot gather (deterministic segmented reduction over element contributions)
 // The block of kSlotBlock slots runs on kSlotBlock / 4 threads, four slots a thread.
 // Each CSR slot of a beam chain has one or two contributions, so the slot pointers,
@@ -1032,6 +1321,10 @@ __device__ inline bool isBad(double v) { return !(fabs(v) <= 1.0e300); }
 // types), 20 NaN/Inf seen.
 constexpr int NPART = 21;
 constexpr int CHUNK_TPB = 256;
+// at most so many chunks as clusters of one-warp blocks (a chain of 3,827 beams, 12
+// chunks: 15.9 us a launch with 8-warp blocks; with 98 chunks, 784 warps for 608
+// sub-cores, the pass and its neighbours lost 6 us)
+constexpr int kWideNormChunks = 48;
 
 // |x| as a bit pattern: for non-negative doubles the order of the patterns is
 // the numeric order (NaN patterns are above infinity), so the maxima and the
@@ -1041,12 +1334,19 @@ __device__ inline unsigned long long absBits(double x) {
 }
 __device__ inline unsigned long long umax64(unsigned long long a, unsigned long long b) { return a > b ? a : b; }
 
-__global__ void __launch_bounds__(CHUNK_TPB) kNormsPartial(DevData d) {
+// A chunk by a block of 8 warps or, with few chunks, by a cluster of 8 one-warp
+// blocks (WIDE): a warp's sums then have a sub-core's FP64 pipe to themselves
+// instead of sharing it with another. Each warp takes the same DOFs in the same
+// order either way, and the warps are combined in order: the same bits.
+template <bool WIDE>
+__global__ void __launch_bounds__(WIDE ? 32 : CHUNK_TPB) kNormsPartial(DevData d) {
   pdlEntry();
-  __shared__ double sh[CHUNK_TPB / 32][NPART];
-  const int c = blockIdx.x;
+  __shared__ double sh[WIDE ? 1 : CHUNK_TPB / 32][NPART];
+  constexpr int kWarps = CHUNK_TPB / 32;
+  const int c = WIDE ? blockIdx.x / kWarps : blockIdx.x;
+  const int w = WIDE ? blockIdx.x % kWarps : threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m = d.chunkModel[c];
-  if (!(d.m.flags[m] & FL_ACTIVE)) return;
+  if (!(d.m.flags[m] & FL_ACTIVE)) return;  // (the same for a whole cluster)
   const double* wD = d.m.wDisp + 3 * m;
   const double* wF = d.m.wForce + 3 * m;
   const unsigned long long badBits = absBits(1.0e300);
@@ -1059,7 +1359,7 @@ __global__ void __launch_bounds__(CHUNK_TPB) kNormsPartial(DevData d) {
   for (int k = 0; k < 13; ++k) mx[k] = 0ull;
   bool bad = false;
   const int cEnd = d.chunkEnd[c];
-  for (int i0 = d.chunkStart[c] + threadIdx.x; i0 < cEnd; i0 += 4 * CHUNK_TPB) {
+  for (int i0 = d.chunkStart[c] + 32 * w + lane; i0 < cEnd; i0 += 4 * CHUNK_TPB) {
     // four DOFs per pass: all loads issued before the ordered accumulation
     int eqs[4], ts[4];
     double a0[4], a1[4], a2[4], rr[4];
@@ -1111,28 +1411,39 @@ __global__ void __launch_bounds__(CHUNK_TPB) kNormsPartial(DevData d) {
     for (int k = 0; k < 13; ++k) mx[k] = umax64(mx[k], __shfl_down_sync(0xffffffffu, mx[k], o));
   }
   bad = __any_sync(0xffffffffu, bad);
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (lane == 0) {
-    sh[w][0] = 0.0;
-    sh[w][1] = 0.0;
-    sh[w][2] = v2;
-    sh[w][3] = v3;
-    sh[w][4] = v4;
-    sh[w][5] = v5;
-    sh[w][6] = v6;
+    double* o = sh[WIDE ? 0 : w];
+    o[0] = 0.0;
+    o[1] = 0.0;
+    o[2] = v2;
+    o[3] = v3;
+    o[4] = v4;
+    o[5] = v5;
+    o[6] = v6;
 #pragma unroll
-    for (int k = 0; k < 13; ++k) sh[w][7 + k] = __longlong_as_double((long long)mx[k]);
-    sh[w][20] = bad ? 1.0 : 0.0;
+    for (int k = 0; k < 13; ++k) o[7 + k] = __longlong_as_double((long long)mx[k]);
+    o[20] = bad ? 1.0 : 0.0;
   }
-  __syncthreads();
-  if (threadIdx.x < NPART) {
+  if constexpr (WIDE) cooperative_groups::this_cluster().sync();
+  else __syncthreads();
+  if (threadIdx.x < NPART && (!WIDE || w == 0)) {
     const int k = threadIdx.x;
-    double x = sh[0][k];
-    for (int ww = 1; ww < CHUNK_TPB / 32; ++ww)
-      x = (k <= 6) ? x + sh[ww][k] : __longlong_as_double((long long)umax64(absBits(x), absBits(sh[ww][k])));
+    double y[kWarps];
+#pragma unroll
+    for (int ww = 0; ww < kWarps; ++ww) {
+      if constexpr (WIDE) y[ww] = cooperative_groups::this_cluster().map_shared_rank(&sh[0][0], ww)[k];
+      else y[ww] = sh[ww][k];
+    }
+    double x = y[0];
+#pragma unroll
+    for (int ww = 1; ww < kWarps; ++ww)
+      x = (k <= 6) ? x + y[ww] : __longlong_as_double((long long)umax64(absBits(x), absBits(y[ww])));
     d.partial[(size_t)c * NPART + k] = x;
   }
+  // the other blocks' shared memory stays until it has been read
+  if constexpr (WIDE) cooperative_groups::this_cluster().sync();
 }
+
 
 // norms, convergence test (normTypeModule.f90:196-249) and iteration counters
 // one warp per model: lane k combines partial value k over the model's chunks
@@ -1154,26 +1465,33 @@ __global__ void kControl(DevData d, int* tally) {
       acc = (lane <= 6) ? acc + x : __longlong_as_double((long long)umax64(absBits(acc), absBits(x)));
     }
   }
-  double v[NPART];
-#pragma unroll
-  for (int k = 0; k < NPART; ++k) v[k] = __shfl_sync(0xffffffffu, acc, k);
-  if (lane != 0) return;
-  double* nv = d.m.normVal + 18 * m;
-  v[0] = d.m.sumWd2[m];
-  v[1] = d.m.sumWf2[m];
-  nv[0] = v[0] > 0 ? sqrt(v[2] / v[0]) : 0.0;
-  nv[4] = v[0] > 0 ? sqrt(v[3] / v[0]) : 0.0;
-  nv[8] = v[0] > 0 ? sqrt(v[4] / v[0]) : 0.0;
-  nv[12] = v[1] > 0 ? sqrt(v[5] / v[1]) : 0.0;
-  for (int t = 0; t < 3; ++t) {
-    nv[1 + t] = v[8 + t];
-    nv[5 + t] = v[11 + t];
-    nv[9 + t] = v[14 + t];
-    nv[13 + t] = v[17 + t];
-  }
+  // lane k forms norm k (0-3 displacement, 4-7 velocity, 8-11 acceleration,
+  // 12-15 residual: L2 and the three maxima; 16 energy maximum, 17 mean) and its
+  // test, all at once
+  const int from = lane < 16 ? ((lane & 3) ? 8 + 3 * (lane >> 2) + (lane & 3) - 1 : 2 + (lane >> 2))
+                             : (lane == 16 ? 7 : 6);
+  double value = __shfl_sync(0xffffffffu, acc, from);
+  const bool bad = __shfl_sync(0xffffffffu, acc, 20) > 0.0;
   const int neq = d.m.neq[m], nd = d.m.ndof[m];
-  nv[16] = v[7];
-  nv[17] = (nd > 1 && neq > 0) ? v[6] / (double)neq : v[6];
+  if (lane < 16 && (lane & 3) == 0) {
+    const double w = lane < 12 ? d.m.sumWd2[m] : d.m.sumWf2[m];
+    value = w > 0 ? sqrt(value / w) : 0.0;
+  } else if (lane == 17 && nd > 1 && neq > 0) {
+    value = value / (double)neq;
+  }
+  bool below = false;
+  int code = 0;
+  if (lane < 18) {
+    d.m.normVal[18 * m + lane] = value;
+    code = d.m.tolCode[18 * m + lane];
+    below = value < d.m.tolVal[18 * m + lane];
+  }
+  const bool exists1 = __any_sync(0xffffffffu, code == 1), exists2 = __any_sync(0xffffffffu, code == 2);
+  const bool oneOf = __any_sync(0xffffffffu, code == 2 && below);
+  // (a norm that is NaN does not count as at or above its tolerance, as before)
+  const bool above = lane < 18 && code == 1 && value >= d.m.tolVal[18 * m + lane];
+  const bool allOf = !__any_sync(0xffffffffu, above);
+  if (lane != 0) return;
   const int it = d.m.iter[m] + 1;
   d.m.iter[m] = it;
   d.m.nIter[m] += 1;
@@ -1181,8 +1499,8 @@ __global__ void kControl(DevData d, int* tally) {
   else d.m.nSeqNoUpd[m] += 1;
   bool conv = false;
   if (d.errFlag && *d.errFlag) d.m.status[m] |= SS_TIMEOUT;
-  if (v[20] > 0.0 || (d.m.status[m] & (SS_SINGULAR | SS_COROT | SS_TIMEOUT))) {
-    d.m.status[m] |= v[20] > 0.0 ? SS_NAN : 0;
+  if (bad || (d.m.status[m] & (SS_SINGULAR | SS_COROT | SS_TIMEOUT))) {
+    d.m.status[m] |= bad ? SS_NAN : 0;
     d.m.state[m] = ST_ERROR;
   } else if (fl & FL_LINEAR) {
     conv = it == d.linearIters;  // pure linear quasi-static step: one solve (+ refinement)
@@ -1192,13 +1510,6 @@ __global__ void kControl(DevData d, int* tally) {
     d.m.status[m] |= SS_MAXIT;
     d.m.state[m] = ST_ERROR;
   } else if (it >= max(2, d.m.minIt[m])) {
-    bool exists1 = false, exists2 = false, oneOf = false, allOf = true;
-    const int* code = d.m.tolCode + 18 * m;
-    const double* tol = d.m.tolVal + 18 * m;
-    for (int k = 0; k < 18; ++k) {
-      if (code[k] == 2) { exists2 = true; if (nv[k] < tol[k]) oneOf = true; }
-      else if (code[k] == 1) { exists1 = true; if (nv[k] >= tol[k]) allOf = false; }
-    }
     conv = true;
     if (exists2) conv = conv && oneOf;
     if (exists1) conv = conv && allOf;
@@ -1406,11 +1717,13 @@ __global__ void kStaticFinish(DevModels m) {
   if (it >= m.maxIt[i]) m.staticDone[i] = 1;  // accepted without full convergence
 }
 
+bool wideElements(const DevData& d) { return d.beamSparse && d.nelTot <= kWideElements; }
+
 }  // namespace
 
 void launchBeginStep(const DevData& d, int* activeCount, long long* activeEl, const BackwardSeed& seed,
                      cudaStream_t s) {
-  pdlLaunch(kBeginStep, blocksFor(d.m.n, 128), 128, 0, s, d.m, activeCount, activeEl, seed);
+  pdlLaunch(kBeginStep, blocksFor(32LL * d.m.n, 128), 128, 0, s, d.m, activeCount, activeEl, seed);
 }
 void launchPredictDofs(const DevData& d, cudaStream_t s) {
   long long n = d.ndofTot > d.neqTot ? d.ndofTot : d.neqTot;
@@ -1418,7 +1731,10 @@ void launchPredictDofs(const DevData& d, cudaStream_t s) {
 }
 void launchElements(const DevData& d, int mode, cudaStream_t s) {
   launchJoints(d, mode, s);  // dependent triads first, as UpdateMechanism updates the joints first
-  if (d.nelTot > 0) pdlLaunch(kElements, blocksFor(d.nelTot, 128), 128, 0, s, d, mode);
+  if (d.nelTot > 0 && wideElements(d) && (mode == EM_PRED || mode == EM_INC))
+    pdlLaunch(kElementsWide, blocksFor(4LL * d.nelTot, 128), 128, 0, s, d, mode);
+  else if (d.nelTot > 0)
+    pdlLaunch(kElements, blocksFor(d.nelTot, 128), 128, 0, s, d, mode);
   launchParts(d, mode, s);
   if (d.naxTot > 0) pdlLaunch(kAxial, blocksFor(d.naxTot, 128), 128, 0, s, d, mode);
   launchExpandForces(d, mode, s);
@@ -1431,7 +1747,9 @@ void launchBuildElementNewton(const DevData& d, cudaStream_t s) {
   if (d.nelTot > 0 && !d.beamSparse) pdlLaunch(kBuildElementNewton, blocksFor(d.nelTot), TPB, 0, s, d);
 }
 void launchRotateElementNewton(const DevData& d, cudaStream_t s) {
-  if (d.nelTot > 0 && d.beamSparse) pdlLaunch(kNewtonBeam, blocksFor(d.nelTot, 128), 128, 0, s, d);
+  if (d.nelTot > 0 && wideElements(d))
+    pdlLaunch(kNewtonBeamWide, blocksFor(4LL * d.nelTot, 128), 128, 0, s, d);
+  else if (d.nelTot > 0 && d.beamSparse) pdlLaunch(kNewtonBeam, blocksFor(d.nelTot, 128), 128, 0, s, d);
   else if (d.nelTot > 0) pdlLaunch(kRotateElementNewton, blocksFor(d.nelTot, 128), 128, 0, s, d);
   if (d.naxTot > 0) pdlLaunch(kAxialNewton, blocksFor(d.naxTot, 128), 128, 0, s, d);
   launchExpandElements(d, s);
@@ -1465,7 +1783,25 @@ void launchNormsControl(const DevData& d, const IterationEnd& e, cudaStream_t s)
   launchControlStepEnd(d, e, s);
 }
 void launchNormsPartial(const DevData& d, cudaStream_t s) {
-  if (d.nchunkTot > 0) pdlLaunch(kNormsPartial, d.nchunkTot, CHUNK_TPB, 0, s, d);
+  if (d.nchunkTot <= 0) return;
+  if (d.nchunkTot > kWideNormChunks) {
+    pdlLaunch(kNormsPartial<false>, d.nchunkTot, CHUNK_TPB, 0, s, d);
+    return;
+  }
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = CHUNK_TPB / 32;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(d.nchunkTot * (CHUNK_TPB / 32));
+  cfg.blockDim = dim3(32);
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  cudaLaunchKernelEx(&cfg, kNormsPartial<true>, d);
 }
 void launchControlStepEnd(const DevData& d, const IterationEnd& e, cudaStream_t s) {
   pdlLaunch(kControl, blocksFor(32LL * d.m.n, 128), 128, 0, s, d, e.tally);

@@ -30,14 +30,16 @@ __device__ inline void crossd(const double* a, const double* b, double* c) {
 // root each.
 __device__ inline void rotvecToMat(const double* rv, double sinEpsOverEps, double* R /* col-major 3x3 */) {
   const double epsTh2 = 0.0005;
-  double thh = 0.5 * sqrt(rv[0] * rv[0] + rv[1] * rv[1] + rv[2] * rv[2]);
+  const double h2 = 0.25 * (rv[0] * rv[0] + rv[1] * rv[1] + rv[2] * rv[2]);
   double cthh, fac;
-  if (thh < epsTh2) {
-    const double h2 = thh * thh;
+  if (h2 < epsTh2 * epsTh2) {
     cthh = 1.0 - h2 * (0.5 - h2 * (1.0 / 24.0 - h2 * (1.0 / 720.0)));
-    double f1 = thh / epsTh2;
+    // f1 = h / eps; it weighs 1 - sin(eps)/eps = 4e-8, so h = h2 rsqrt(h2) and the
+    // product with 1 / eps (in place of a root and a division) do not show
+    const double f1 = (h2 > 0.0 ? h2 * rsqrt(h2) : 0.0) * (1.0 / epsTh2);
     fac = f1 * sinEpsOverEps + 1.0 - f1;
   } else {
+    const double thh = sqrt(h2);
     double sthh;
     sincos(thh, &sthh, &cthh);
     fac = sthh / thh;
