@@ -90,15 +90,25 @@ __device__ inline double dependentValue(const DevData& d, int dd, const double* 
 // ---------------------------------------------------------------------------
 // per-model control at the start of a batched iteration
 // ---------------------------------------------------------------------------
-// the roots of model i into every backward queue, and its chain count
-__device__ inline void seedBackward(const BackwardSeed& b, int i) {
+// the roots of model i into every backward queue, and its chain count, by the
+// lanes of a warp (a model whose upper levels go to the trees on thread blocks
+// has thousands of roots below them)
+__device__ inline void seedQueue(int* ctr, int* queue, const int* off, const int* roots, int chains, int i, int lane) {
+  const int r0 = off[i], nr = off[i + 1] - r0;
+  int base = 0;
+  if (lane == 0) {
+    base = atomicAdd(ctr + 1, nr);
+    atomicAdd(ctr + 2, chains);
+  }
+  base = __shfl_sync(0xffffffffu, base, 0);
+#pragma unroll 4
+  for (int k = lane; k < nr; k += 32) queue[base + k] = roots[r0 + k];
+}
+__device__ inline void seedBackward(const BackwardSeed& b, int i, int lane) {
   for (int q = 0; q < b.nq; ++q) {
-    const int r0 = b.rootOff[i], nr = b.rootOff[i + 1] - r0;
-    int* ctr = b.ctr + 4 * q;
-    int* queue = b.queue + (size_t)q * b.stride;
-    const int base = atomicAdd(ctr + 1, nr);
-    for (int k = 0; k < nr; ++k) queue[base + k] = b.roots[r0 + k];
-    atomicAdd(ctr + 2, b.slotCnt[i]);
+    seedQueue(b.ctr + 4 * q, b.queue + (size_t)q * b.stride, b.rootOff, b.roots, b.slotCnt[i], i, lane);
+    if (b.strideT > 0)  // the top chunks into the trees' queue
+      seedQueue(b.ctrT + 4 * q, b.queueT + (size_t)q * b.strideT, b.rootOffT, b.rootsT, b.slotCntT[i], i, lane);
   }
 }
 
@@ -158,6 +168,7 @@ __global__ void kBeginStep(DevModels m, int* activeCount, long long* activeEl, B
     if (lane == 0) m.flags[i] = 0;
     return;
   }
+  seedBackward(bs, i, lane);
   if (lane != 0) return;
   int it = m.iter[i];
   bool tangent = it < max(1, m.nUpdat[i]) || m.nSeqNoUpd[i] >= m.maxSeq[i];
@@ -174,7 +185,6 @@ __global__ void kBeginStep(DevModels m, int* activeCount, long long* activeEl, B
   m.flags[i] = fl;
   atomicAdd(activeCount, 1);
   atomicAdd(reinterpret_cast<unsigned long long*>(activeEl), (unsigned long long)m.nel[i]);
-  seedBackward(bs, i);
 }
 
 // predicted velocity/acceleration increments and the actual inertia force
@@ -1583,15 +1593,22 @@ __global__ void kStepEnd(DevData d, IterationEnd e) {
 // backward queues of the active models, for solves outside a step start
 __global__ void kSeedBackward(DevModels m, BackwardSeed bs) {
   pdlEntry();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < m.n && (m.flags[i] & FL_ACTIVE)) seedBackward(bs, i);
+  const int i = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5);  // a warp per model
+  if (i < m.n && (m.flags[i] & FL_ACTIVE)) seedBackward(bs, i, threadIdx.x & 31);
 }
 
 __global__ void kStaticBegin(DevModels m, int* activeCount, BackwardSeed bs) {
   pdlEntry();
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;  // a warp per model
   if (i >= m.n) return;
-  if (m.staticDone[i] || m.state[i] == ST_ERROR) { m.flags[i] = 0; return; }
+  const bool skip = m.staticDone[i] || m.state[i] == ST_ERROR;
+  __syncwarp();
+  if (skip) {
+    if (lane == 0) m.flags[i] = 0;
+    return;
+  }
+  seedBackward(bs, i, lane);
+  if (lane != 0) return;
   int fl = FL_ACTIVE | FL_STATIC | FL_TANGENT;
   double* sn = m.scaleN + 3 * i;
   if (fabs(0.0 - sn[0]) + fabs(1.0 - sn[1]) + fabs(0.0 - sn[2]) > 1.0e-16) {
@@ -1600,7 +1617,6 @@ __global__ void kStaticBegin(DevModels m, int* activeCount, BackwardSeed bs) {
   }
   m.flags[i] = fl;
   atomicAdd(activeCount, 1);
-  seedBackward(bs, i);
 }
 
 __global__ void kStaticResidual(DevData d) {
@@ -1823,10 +1839,10 @@ void launchQsRestore(const DevData& d, cudaStream_t s) {
   pdlLaunch(kQsRestore, blocksFor(n), TPB, 0, s, d);
 }
 void launchSeedBackward(const DevData& d, const BackwardSeed& seed, cudaStream_t s) {
-  pdlLaunch(kSeedBackward, blocksFor(d.m.n, 128), 128, 0, s, d.m, seed);
+  pdlLaunch(kSeedBackward, blocksFor(32LL * d.m.n, 128), 128, 0, s, d.m, seed);
 }
 void launchStaticBegin(const DevData& d, int* activeCount, const BackwardSeed& seed, cudaStream_t s) {
-  pdlLaunch(kStaticBegin, blocksFor(d.m.n, 128), 128, 0, s, d.m, activeCount, seed);
+  pdlLaunch(kStaticBegin, blocksFor(32LL * d.m.n, 128), 128, 0, s, d.m, activeCount, seed);
 }
 void launchStaticResidual(const DevData& d, cudaStream_t s) {
   if (d.neqTot > 0) pdlLaunch(kStaticResidual, blocksFor(d.neqTot), TPB, 0, s, d);

@@ -910,8 +910,6 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
       return -905;
     }
     if (maxRowLarge >= 1024) { err = "front of 1024 rows or more"; return -905; }
-    UPV(d_.fLarge, uint8_t, large);
-    pplan_.fLarge = d_.fLarge;
     pplan_.nLarge = nLargeFronts;
     // leaf-to-root path lengths: parents follow their children in each model's order
     std::vector<int> pathLen(nfr, 1);
@@ -921,9 +919,36 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
     }
     // tasks with the longest paths first: the cascades' critical paths (the
     // deep trees of the large models) start in the first wave of warps
+    // classes of fronts: 0 the cascades', 1 large, 2 the trees on thread blocks'
+    // (all small fronts of a small batch; of a larger one the upper levels, from the
+    // lowest height above which few enough subtrees are left)
+    std::vector<int> height(nfr, 0);
+    int smallLeaves = 0, maxHeight = 0;
+    for (int f = 0; f < nfr; ++f) {
+      if (large[f]) continue;
+      for (int c = 0; c < nchild[f]; ++c)
+        height[f] = std::max(height[f], height[childList[childOffV[f] + c]] + 1);
+      smallLeaves += nchild[f] == 0;
+      maxHeight = std::max(maxHeight, height[f]);
+    }
+    const int treeHeight = treeFromHeight(smallLeaves, maxHeight, [&](int h) {
+      // fronts of at least height h without a child of at least height h
+      long long n = 0;
+      for (int f = 0; f < nfr; ++f) {
+        if (large[f] || height[f] < h) continue;
+        bool lowest = true;
+        for (int c = 0; c < nchild[f] && lowest; ++c) lowest = height[childList[childOffV[f] + c]] < h;
+        n += lowest;
+      }
+      return n;
+    });
+    const int tw = treeHeight < 0 ? 0 : treeWarps(treeHeight == 0 ? smallLeaves : 0, maxRowAll, opt_.fp32Factor);
+    std::vector<unsigned char> cls(nfr, 0);
+    for (int f = 0; f < nfr; ++f) cls[f] = large[f] ? 1 : (tw > 0 && height[f] >= treeHeight ? 2 : 0);
+    UPV(d_.fLarge, uint8_t, cls);
     std::vector<int> leaves;
     for (int f = 0; f < nfr; ++f)
-      if (nchild[f] == 0 && !large[f]) leaves.push_back(f);
+      if (nchild[f] == 0 && cls[f] == 0) leaves.push_back(f);
     std::stable_sort(leaves.begin(), leaves.end(), [&](int a, int b) { return pathLen[a] > pathLen[b]; });
     int* dLeaves = nullptr;
     UPV(dLeaves, int, leaves);
@@ -942,7 +967,7 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
     auto fastFront = [&](int f) { return nrow[f] <= 64 && (long long)nrow[f] * npiv[f] <= capL; };
     std::vector<char> inGroup(nfr, 0), isHead(nfr, 0);
     for (int f = 0; f < nfr; ++f) {
-      if (large[f] || nchild[f] == 0 || nchild[f] > 8 || !fastFront(f)) continue;
+      if (cls[f] != 0 || nchild[f] == 0 || nchild[f] > 8 || !fastFront(f)) continue;
       bool ok = true;
       int ncg = 0;
       for (int c = 0; c < nchild[f] && ok; ++c) {
@@ -957,7 +982,7 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
     std::vector<int> tasks, taskLen;
     for (int f = 0; f < nfr; ++f) {
       if (isHead[f]) { tasks.push_back(f | (1 << 30)); taskLen.push_back(pathLen[f] + 1); }
-      else if (nchild[f] == 0 && !large[f] && !inGroup[f]) { tasks.push_back(f); taskLen.push_back(pathLen[f]); }
+      else if (nchild[f] == 0 && cls[f] == 0 && !inGroup[f]) { tasks.push_back(f); taskLen.push_back(pathLen[f]); }
     }
     if (nfr >= (1 << 30)) { err = "too many fronts for the task encoding"; return -910; }
     std::vector<int> order(tasks.size());
@@ -975,17 +1000,17 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
     // a chain ends at a leaf not solved inline or at an inline front
     std::vector<unsigned char> bwInline(nfr, 0);
     for (int f = 0; f < nfr; ++f) {
-      bool all = nchild[f] > 0 && !large[f];
+      bool all = nchild[f] > 0 && cls[f] == 0;
       for (int c = 0; c < nchild[f] && all; ++c) all = nchild[childList[childOffV[f] + c]] == 0;
       bwInline[f] = all ? 1 : 0;
     }
-    // the warp queue starts at the tops of the small subtrees (roots, or fronts
-    // under a large parent)
-    auto smallTop = [&](int f) { return !large[f] && (parent[f] < 0 || large[parent[f]]); };
+    // the warp queue starts at the tops of the cascades' subtrees (roots, or fronts
+    // under a parent of another class)
+    auto smallTop = [&](int f) { return cls[f] == 0 && (parent[f] < 0 || cls[parent[f]] != 0); };
     std::vector<int> rootOff(nm + 1, 0), roots, leafCnt(nm, 0);
     for (int f = 0; f < nfr; ++f) {
       if (smallTop(f)) ++rootOff[fmodel[f] + 1];
-      if (!large[f] && (bwInline[f] || (nchild[f] == 0 && !(parent[f] >= 0 && bwInline[parent[f]]))))
+      if (cls[f] == 0 && (bwInline[f] || (nchild[f] == 0 && !(parent[f] >= 0 && bwInline[parent[f]]))))
         ++leafCnt[fmodel[f]];
     }
     {
@@ -1000,7 +1025,8 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
       for (int f = 0; f < nfr; ++f)
         if (smallTop(f)) roots[fill[fmodel[f]]++] = f;
     }
-    const int tw = treeWarps((int)leaves.size(), maxRowAll, opt_.fp32Factor);
+    std::vector<int> treeRootOff(nm + 1, 0), treeRoots, treeChains(nm, 0);
+    int nChunks = 0;
     if (tw > 0) {
       // ---- trees on thread blocks: the small fronts cut into chunks of at most tw
       // fronts: tiers of as many tree levels as a full binary piece of tw fronts has
@@ -1008,17 +1034,16 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
       // largest children to chunks of their own
       int tier = 1;
       while ((2 << tier) - 1 <= tw) ++tier;
-      std::vector<int> size(nfr, 0), chunkOf(nfr, -1), height(nfr, 0);
+      std::vector<int> size(nfr, 0), chunkOf(nfr, -1);
       std::vector<char> cut(nfr, 0), lev(nfr, 0);
       for (int f = 0; f < nfr; ++f) {
-        if (large[f]) continue;
+        if (cls[f] != 2) continue;
         std::vector<int> kids;
         int sum = 1;
-        for (int c = 0; c < nchild[f]; ++c)
-          height[f] = std::max(height[f], height[childList[childOffV[f] + c]] + 1);
         for (int c = 0; c < nchild[f]; ++c) {
           const int k = childList[childOffV[f] + c];
-          if (height[k] / tier != height[f] / tier) {
+          if (cls[k] != 2) continue;  // done by the cascades before
+          if ((height[k] - treeHeight) / tier != (height[f] - treeHeight) / tier) {
             cut[k] = 1;
             continue;
           }
@@ -1033,20 +1058,20 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
         size[f] = sum;
         for (int k : kids)
           if (!cut[k]) lev[f] = std::max<char>(lev[f], lev[k] + 1);
-        if (parent[f] < 0 || large[parent[f]]) cut[f] = 1;
+        if (parent[f] < 0 || cls[parent[f]] != 2) cut[f] = 1;
       }
       // chunks numbered by their root front; members by level
       std::vector<TreeChunk> chunks;
       std::vector<std::vector<int>> members;
       std::vector<int> root;
       for (int f = nfr - 1; f >= 0; --f) {  // parents precede their children here
-        if (large[f]) continue;
+        if (cls[f] != 2) continue;
         if (cut[f]) {
           chunkOf[f] = (int)chunks.size();
           TreeChunk ch{};
           ch.model = fmodel[f];
           ch.levels = lev[f] + 1;
-          ch.parent = parent[f] >= 0 && !large[parent[f]] ? chunkOf[parent[f]] : -1;
+          ch.parent = parent[f] >= 0 && cls[parent[f]] == 2 ? chunkOf[parent[f]] : -1;
           chunks.push_back(ch);
           members.emplace_back();
           root.push_back(f);
@@ -1092,16 +1117,27 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
       pplan_.tree.start = ds;
       pplan_.tree.nStart = (int)start.size();
       pplan_.tree.warps = tw;
-      // the back substitution's queue holds chunks: its roots are the top chunks,
+      pplan_.tree.nChunks = nChunks = nc;
+      // their back substitution's queue holds chunks: it starts at the top chunks,
       // its chains end at the chunks without child chunks
-      for (int& r : roots) r = chunkOf[r];
-      std::fill(leafCnt.begin(), leafCnt.end(), 0);
-      for (int c : start) ++leafCnt[chunks[c].model];
+      for (const TreeChunk& ch : chunks)
+        if (ch.parent < 0) ++treeRootOff[ch.model + 1];
+      for (int m = 0; m < nm; ++m) treeRootOff[m + 1] += treeRootOff[m];
+      treeRoots.resize(treeRootOff[nm]);
+      std::vector<int> fill(treeRootOff.begin(), treeRootOff.end() - 1);
+      for (int c = 0; c < nc; ++c)
+        if (chunks[c].parent < 0) treeRoots[fill[chunks[c].model]++] = c;
+      for (int c : start) ++treeChains[chunks[c].model];
     }
     int *dRootOff = nullptr, *dRoots = nullptr, *dLeafCnt = nullptr;
     UPV(dRootOff, int, rootOff);
     UPV(dRoots, int, roots);
     UPV(dLeafCnt, int, leafCnt);
+    int *dTreeRootOff = nullptr, *dTreeRoots = nullptr, *dTreeChains = nullptr;
+    if (treeRoots.empty()) treeRoots.push_back(-1);
+    UPV(dTreeRootOff, int, treeRootOff);
+    UPV(dTreeRoots, int, treeRoots);
+    UPV(dTreeChains, int, treeChains);
     // iteration counters in one block, zeroed by one memset per iteration:
     // active models (int) and elements (long long), the backward queues'
     // counters (4 per solve), the factorisation's per-front counters and one set
@@ -1109,20 +1145,35 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
     const int nq = std::max(1, opt_.fp32Factor ? opt_.refineSweeps : 1);
     // with large fronts: their signals and barriers (PersistentPlan::cntLarge) follow
     const size_t largeInts = (size_t)nLargeFronts * (2 + 3 * (size_t)nq);
-    ctrInts_ = 4 + 4 * (size_t)nq + (size_t)nq * (nfr + 1) + largeInts;
+    // the trees' per-chunk counters (one set per solve, each + its start counter) and
+    // queue counters (4 per solve) come last
+    const size_t treeInts = tw > 0 ? (size_t)nq * (nChunks + 1) + 4 * (size_t)nq : 0;
+    ctrInts_ = 4 + 4 * (size_t)nq + (size_t)nq * (nfr + 1) + largeInts + treeInts;
     ctrBlock_ = alloc<int>(ctrInts_);
     // remaining, more, last active count; serial number (8-byte aligned)
     end_.tally = alloc<int>(6);
     if (!ctrBlock_ || !end_.tally) { err = "out of device memory (counters)"; return -906; }
-    if (ctrInts_ > INT_MAX || (size_t)nq * leaves.size() > INT_MAX) { err = "too many fronts for the counters"; return -910; }
+    const size_t treeSlots = tw > 0 ? (size_t)std::max(pplan_.tree.nStart, 1) : 0;
+    if (ctrInts_ > INT_MAX || (size_t)nq * (leaves.size() + treeSlots) > INT_MAX) { err = "too many fronts for the counters"; return -910; }
     dActive_ = ctrBlock_;
     dActiveEl_ = reinterpret_cast<long long*>(ctrBlock_ + 2);
     pplan_.bwCtr = ctrBlock_ + 4;
     pplan_.cntFactor = ctrBlock_ + 4 + 4 * nq;
     pplan_.cntForward = pplan_.cntFactor + (nfr + 1);
     pplan_.cntLarge = pplan_.cntFactor + (size_t)nq * (nfr + 1);
-    pplan_.bwQueue = alloc<int>((size_t)nq * std::max<size_t>(leaves.size(), 1));
-    queueInts_ = (size_t)nq * std::max<size_t>(leaves.size(), 1);
+    queueInts_ = (size_t)nq * (std::max<size_t>(leaves.size(), 1) + treeSlots);
+    pplan_.bwQueue = alloc<int>(queueInts_);
+    pplan_.cntTree = pplan_.cntLarge + largeInts;
+    pplan_.treeCtr = pplan_.cntTree + (size_t)nq * (nChunks + 1);
+    pplan_.treeQueue = pplan_.bwQueue + (size_t)nq * std::max<size_t>(leaves.size(), 1);
+    if (tw > 0) {
+      seed_.strideT = (int)treeSlots;
+      seed_.rootOffT = dTreeRootOff;
+      seed_.rootsT = dTreeRoots;
+      seed_.slotCntT = dTreeChains;
+      seed_.queueT = pplan_.treeQueue;
+      seed_.ctrT = pplan_.treeCtr;
+    }
     seed_.nq = nq;
     seed_.stride = (int)std::max<size_t>(leaves.size(), 1);
     seed_.rootOff = dRootOff;
@@ -1457,6 +1508,8 @@ int Engine::timeFactor(int reps, double* msPerLaunch, double* bytes) {
   const size_t cntBytes = sizeof(int) * ((size_t)d_.nfrontTot + 1);
   auto clear = [&]() {
     cudaMemsetAsync(pplan_.cntFactor, 0, cntBytes, stream_);
+    if (pplan_.tree.warps > 0)
+      cudaMemsetAsync(pplan_.cntTree, 0, sizeof(int) * ((size_t)pplan_.tree.nChunks + 1), stream_);
     if (pplan_.nLarge > 0)  // the factorisation's and the first forward elimination's
       cudaMemsetAsync(pplan_.cntLarge, 0, sizeof(int) * 3 * (size_t)pplan_.nLarge, stream_);
   };
@@ -1538,7 +1591,8 @@ int Engine::autotune() {
   char key[256];
   snprintf(key, sizeof key, "dev%d f%d s%d r%d p%d L%d n%d l%d t%d", device_, opt_.fp32Factor ? 1 : 0,
            opt_.refineSweeps, pplan_.maxRow, pplan_.maxNpiv, pplan_.nLarge > 0 ? pplan_.large[4].maxRow : 0,
-           (int)std::lround(std::log2((double)d_.nfrontTot + 1.0)), (int)std::lround(std::log2(pplan_.nLeaves + 1.0)),
+           (int)std::lround(std::log2((double)d_.nfrontTot + 1.0)),
+           (int)std::lround(std::log2(pplan_.nLeaves + pplan_.tree.nStart + 1.0)),
            pplan_.nLarge > 0 ? (int)std::lround(std::log2(pplan_.nLarge + 1.0)) : -1);
   {
     std::lock_guard<std::mutex> lk(g_shapeMutex);
@@ -1612,7 +1666,7 @@ int Engine::autotune() {
     pplan_.largeCluster = pick;
   }
   // 3. forward elimination of a refinement sweep: warps per block
-  if (ok && f32 && opt_.refineSweeps > 1 && pplan_.tree.warps == 0) {
+  if (ok && f32 && opt_.refineSweeps > 1 && pplan_.nLeaves > 0) {
     float best = -1.f;
     int pick = 8;
     for (int w : {8, 4, 16}) {
@@ -1628,7 +1682,7 @@ int Engine::autotune() {
     pplan_.forwardWarps = pick;
   }
   // 4. back substitution: warps per block (queues seeded for every model)
-  if (ok && pplan_.tree.warps == 0) {
+  if (ok && pplan_.nLeaves > 0) {
     float best = -1.f;
     int pick = 8;
     for (int w : {8, 4, 16}) {
@@ -1710,18 +1764,17 @@ void Engine::enqueueSolve(cudaStream_t s, bool timedForward, bool backwardDone) 
     if (sweep > 0) launchRefineResidual(d_, s);
     if (sweep == 1 && timedForward) recordPhase(ev_[5], s);
     // trees on thread blocks: a refinement solve's back substitution in the launch
-    // of its forward elimination too
+    // of its forward elimination too (the cascades' part, below the trees, follows)
     const bool fused = sweep == 0 ? backwardDone : pplan_.tree.warps > 0 && pplan_.nLarge == 0;
+    const bool below = fused && pplan_.tree.warps > 0 && pplan_.nLeaves > 0;
     if (sweep > 0) {
       launchForwardCascade(d_, pplan_, f32, f32 ? d_.rref : d_.del, sweep, s, fused, sweep == sw - 1);
       launchLargeForward(d_, pplan_, f32, f32 ? d_.rref : d_.del, sweep, s);
     }
     if (sweep == 1 && timedForward) recordPhase(ev_[6], s);
     if (sweep == timedBackward && timedForward) recordPhase(ev_[7], s);
-    if (!fused) {
-      launchLargeBackward(d_, pplan_, f32, sweep, sweep == sw - 1, s);
-      launchBackward(d_, pplan_, f32, sweep, sweep == sw - 1, s);
-    }
+    if (!fused) launchLargeBackward(d_, pplan_, f32, sweep, sweep == sw - 1, s);
+    if (!fused || below) launchBackward(d_, pplan_, f32, sweep, sweep == sw - 1, s, below);
     if (sweep == timedBackward && timedForward) recordPhase(ev_[8], s);
   }
 }
@@ -2132,6 +2185,7 @@ void Engine::enqueueIteration(cudaStream_t s, bool timed, bool reset) {
   // forward elimination and a back substitution per solve
   launchesPerIter_ = (d_.beamSparse ? 11 : 12) + 1 + 2 * (sw - 1) + sw -
                      (fuseBackward_ ? 1 : 0) - (pplan_.tree.warps > 0 && pplan_.nLarge == 0 ? sw - 1 : 0) +
+                     (pplan_.tree.warps > 0 && pplan_.nLeaves > 0 ? 2 * sw : 0) +
                      (pplan_.nLarge > 0 ? 1 + 2 * sw : 0) +
                      (d_.urQs ? 1 : 0) +
                      (d_.nmotTot > 0 ? 1 : 0) + (d_.nmrTot > 0 ? 1 : 0) + (d_.naxTot > 0 ? 3 : 0) +

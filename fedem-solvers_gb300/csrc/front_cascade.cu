@@ -838,7 +838,7 @@ __global__ void __launch_bounds__(512, 1) kTree(DevData d, TreePlan tp, int maxR
   T* diag0 = lcol + maxRow;
   T* v = diag0 + maxRow;
   if (up) {
-    int* const start = cnt + d.nfrontTot;
+    int* const start = cnt + tp.nChunks;
     auto take = [&]() {
       const int i = atomicAdd(start, 1);
       return i < tp.nStart ? tp.start[i] : -1;
@@ -1113,6 +1113,9 @@ void factorCascade(void (*kernel)(DevData, const int*, int, int, const T*, T*, T
             fb);
 }
 
+// subtrees' lowest fronts from which a larger batch's upper levels go to the trees
+constexpr long long kTreeTops = 1500;
+
 size_t treeWarpValues(int maxRow) { return (size_t)maxRow * maxRow + 3 * (size_t)maxRow; }
 
 // one launch of the trees on thread blocks (kTree)
@@ -1138,11 +1141,12 @@ void treeLaunch(const DevData& d, const PersistentPlan& p, bool fp32, const doub
     treeLaunch<double>(d, p, d.asmVal64, d.L64, d.U64, rhs, d.x64, d.w64, cnt, fb, up, mayFactor, s);
 }
 
-// the back substitution of solve `sweep` (launchBackward's arguments)
-FusedBackward backwardOf(const PersistentPlan& p, bool fp32, int sweep, bool last) {
+// the back substitution of solve `sweep` (launchBackward's arguments), the
+// cascades' or the trees'
+FusedBackward backwardOf(const PersistentPlan& p, bool fp32, int sweep, bool last, bool tree) {
   FusedBackward fb;
-  fb.queue = p.bwQueue + (size_t)sweep * p.nLeaves;
-  fb.ctr = p.bwCtr + 4 * sweep;
+  fb.queue = tree ? p.treeQueue + (size_t)sweep * p.tree.nStart : p.bwQueue + (size_t)sweep * p.nLeaves;
+  fb.ctr = (tree ? p.treeCtr : p.bwCtr) + 4 * sweep;
   fb.bwInline = p.bwInline;
   fb.errFlag = p.errFlag;
   fb.spinLimit = p.spinLimit;
@@ -1173,31 +1177,12 @@ __global__ void kProbeEntries(DevData d, T* asmVal) {
   }
 }
 
-}  // namespace
-
-void launchProbeEntries(const DevData& d, bool fp32, cudaStream_t s) {
-  if (d.nfrontTot <= 0) return;
-  const int blocks = (d.nfrontTot + 127) / 128;
-  if (fp32) pdlLaunch(kProbeEntries<float>, blocks, 128, 0, s, d, d.asmVal32);
-  else pdlLaunch(kProbeEntries<double>, blocks, 128, 0, s, d, d.asmVal64);
-}
-
-void launchFactorForwardCascade(const DevData& d, const PersistentPlan& p, bool fp32, const double* rhs,
-                                cudaStream_t s, bool withBackward, bool lastSweep) {
-  if (p.nLeaves <= 0) return;
+// the cascades' factorisation with the first forward elimination (and the back
+// substitution fb, if any)
+void factorForwardCascade(const DevData& d, const PersistentPlan& p, bool fp32, const double* rhs,
+                          const FusedBackward& fb, cudaStream_t s) {
   const double tol = 1.0e-12;
   const size_t perWarp = (size_t)p.maxRow * p.maxRow + 3 * p.maxRow;
-  // the fused back substitution of solve 0 (launchBackward's arguments); its
-  // solve vector and L staging reuse the warp's v and F areas
-  FusedBackward fb;
-  if (withBackward) {
-    fb = backwardOf(p, fp32, 0, lastSweep);
-    fb.capL = stagingCapacity(p, fp32 ? sizeof(float) : sizeof(double));
-  }
-  if (p.tree.warps > 0) {
-    treeLaunch(d, p, fp32, rhs, p.cntFactor, fb, true, true, s);
-    return;
-  }
   if (fp32) {
     const int wpb = factorWarpsPerBlock(perWarp * sizeof(float));
     const size_t sm = (size_t)wpb * perWarp * sizeof(float);
@@ -1225,44 +1210,12 @@ void launchFactorForwardCascade(const DevData& d, const PersistentPlan& p, bool 
   }
 }
 
-// staging capacity (values) of one front's L block per warp
-int stagingCapacity(const PersistentPlan& p, size_t elemBytes) {
-  long long want = (long long)p.maxRow * p.maxNpiv;
-  long long cap = (long long)(12 * 1024 / elemBytes);
-  return (int)(want < cap ? want : cap);
-}
 
-// The line between the trees on thread blocks and the cascades, by the batch's
-// leaf fronts (iteration in microseconds, cascades against trees of 16 and 8
-// warps; chains of beams, mixed unless noted): 1,066 leaves 238 / 174 / 183;
-// 3,200: 265 / 221 / 221; 5,333: 360 / 334 / 324 (FP64 368 / 315 / 298); 8,533:
-// 348 / 348 / 334; FP64 10,666: 446 / 524 / 477; 16,000: 556 / 779 / 721.  With
-// more leaves the cascades' warps, which never wait for a level, keep the GPU
-// busier; between 4,096 and 8,192 two blocks of 8 warps share an SM better than
-// one of 16.
-int treeWarps(int nLeaves, int maxRow, bool fp32) {
-  if (nLeaves <= 0 || nLeaves > 8192) return 0;
-  const int fit = (int)(200 * 1024 / (treeWarpValues(maxRow) * (fp32 ? sizeof(float) : sizeof(double))));
-  const int w = std::min(nLeaves <= 4096 ? 16 : 8, fit);
-  return w >= 3 ? w : 0;
-}
-
-bool fusableBackward(const PersistentPlan& p, bool fp32) {
-  if (p.tree.warps > 0) return p.nLeaves > 0 && p.nLarge == 0;
-  return p.nLeaves > 0 && p.nLarge == 0 &&
-         (long long)stagingCapacity(p, fp32 ? sizeof(float) : sizeof(double)) >= (long long)p.maxRow * p.maxNpiv;
-}
-
-void launchForwardCascade(const DevData& d, const PersistentPlan& p, bool fp32, const double* rhs, int sweep,
-                          cudaStream_t s, bool withBackward, bool lastSweep) {
-  if (p.nTasks <= 0) return;
+// the cascades' forward elimination of a refinement solve
+void forwardCascade(const DevData& d, const PersistentPlan& p, bool fp32, const double* rhs, int sweep,
+                    cudaStream_t s) {
   const int wpb = p.forwardWarps;
   int* cnt = p.cntForward + (size_t)(sweep - 1) * ((size_t)d.nfrontTot + 1);
-  if (p.tree.warps > 0) {
-    treeLaunch(d, p, fp32, rhs, cnt, withBackward ? backwardOf(p, fp32, sweep, lastSweep) : FusedBackward{}, true,
-               false, s);
-    return;
-  }
   if (fp32) {
     const int capL = stagingCapacity(p, sizeof(float));
     const size_t sm = (size_t)wpb * (p.maxRow + capL + 64) * sizeof(float);
@@ -1280,14 +1233,93 @@ void launchForwardCascade(const DevData& d, const PersistentPlan& p, bool fp32, 
   }
 }
 
-void launchBackward(const DevData& d, const PersistentPlan& p, bool fp32, int sweep, bool last, cudaStream_t s) {
-  const int acc = !fp32 ? ACC_SET : (sweep == 0 ? ACC_FIRST : ACC_ADD);
-  const int fin = (fp32 && last) ? 1 : 0;
-  if (p.nLeaves <= 0) return;
+}  // namespace
+
+void launchProbeEntries(const DevData& d, bool fp32, cudaStream_t s) {
+  if (d.nfrontTot <= 0) return;
+  const int blocks = (d.nfrontTot + 127) / 128;
+  if (fp32) pdlLaunch(kProbeEntries<float>, blocks, 128, 0, s, d, d.asmVal32);
+  else pdlLaunch(kProbeEntries<double>, blocks, 128, 0, s, d, d.asmVal64);
+}
+
+void launchFactorForwardCascade(const DevData& d, const PersistentPlan& p, bool fp32, const double* rhs,
+                                cudaStream_t s, bool withBackward, bool lastSweep) {
+  // the cascades below the trees first; the back substitution of the trees is part
+  // of their launch, the cascades' follows on its own
   if (p.tree.warps > 0) {
-    treeLaunch(d, p, fp32, nullptr, p.cntFactor, backwardOf(p, fp32, sweep, last), false, false, s);
+    if (p.nLeaves > 0) factorForwardCascade(d, p, fp32, rhs, FusedBackward{}, s);
+    treeLaunch(d, p, fp32, rhs, p.cntTree, withBackward ? backwardOf(p, fp32, 0, lastSweep, true) : FusedBackward{},
+               true, true, s);
     return;
   }
+  if (p.nLeaves <= 0) return;
+  FusedBackward fb;
+  if (withBackward) {
+    // (its solve vector and L staging reuse the warp's v and F areas)
+    fb = backwardOf(p, fp32, 0, lastSweep, false);
+    fb.capL = stagingCapacity(p, fp32 ? sizeof(float) : sizeof(double));
+  }
+  factorForwardCascade(d, p, fp32, rhs, fb, s);
+}
+
+// staging capacity (values) of one front's L block per warp
+int stagingCapacity(const PersistentPlan& p, size_t elemBytes) {
+  long long want = (long long)p.maxRow * p.maxNpiv;
+  long long cap = (long long)(12 * 1024 / elemBytes);
+  return (int)(want < cap ? want : cap);
+}
+
+// The line between the trees on thread blocks and the cascades, by the batch's
+// leaf fronts (iteration in microseconds, cascades against trees of 16 and 8
+// warps; chains of beams, mixed unless noted): 1,066 leaves 238 / 174 / 183;
+// 3,200: 265 / 221 / 221; 5,333: 360 / 334 / 324 (FP64 368 / 315 / 298); 8,533:
+// 348 / 348 / 334; FP64 10,666: 446 / 524 / 477; 16,000: 556 / 779 / 721.  With
+// more leaves the cascades' warps, which never wait for a level, keep the GPU
+// busier; between 4,096 and 8,192 two blocks of 8 warps share an SM better than
+// one of 16.  Larger batches up to 32,768 leaves take both: the cascades up to the
+// height above which at most kTreeTops subtrees begin, the trees from there, where
+// the cascades run out of fronts and pay their latency level by level (cascades
+// alone against both: one chain of 33,333 beams 595 / 498; 24 of 2,000 550 / 485;
+// 8 of 8,000 657 / 571; 64 of 1,000 586 / 562; FP64 32 of 1,000 424 / 414; with
+// 300, 600 or 3,000 subtrees up to 9 % slower than with 1,500).  Above, other
+// models' fronts fill the cascades' upper levels (64,000 leaves: 675 / 689, FP64
+// 727 / 749).
+int treeFromHeight(int nLeaves, int maxHeight, const std::function<long long(int)>& lowest) {
+  if (nLeaves <= 0) return -1;
+  if (nLeaves <= 8192) return 0;
+  if (nLeaves <= 32768)
+    for (int h = 1; h + 2 <= maxHeight; ++h)
+      if (lowest(h) <= kTreeTops) return h;
+  return -1;
+}
+
+int treeWarps(int nLeaves, int maxRow, bool fp32) {
+  const int fit = (int)(200 * 1024 / (treeWarpValues(maxRow) * (fp32 ? sizeof(float) : sizeof(double))));
+  const int w = std::min(nLeaves <= 4096 ? 16 : 8, fit);
+  return w >= 3 ? w : 0;
+}
+
+bool fusableBackward(const PersistentPlan& p, bool fp32) {
+  if (p.tree.warps > 0) return p.nLarge == 0;
+  return p.nLeaves > 0 && p.nLarge == 0 &&
+         (long long)stagingCapacity(p, fp32 ? sizeof(float) : sizeof(double)) >= (long long)p.maxRow * p.maxNpiv;
+}
+
+void launchForwardCascade(const DevData& d, const PersistentPlan& p, bool fp32, const double* rhs, int sweep,
+                          cudaStream_t s, bool withBackward, bool lastSweep) {
+  if (p.nTasks > 0) forwardCascade(d, p, fp32, rhs, sweep, s);
+  if (p.tree.warps > 0)
+    treeLaunch(d, p, fp32, rhs, p.cntTree + (size_t)sweep * (p.tree.nChunks + 1),
+               withBackward ? backwardOf(p, fp32, sweep, lastSweep, true) : FusedBackward{}, true, false, s);
+}
+
+void launchBackward(const DevData& d, const PersistentPlan& p, bool fp32, int sweep, bool last, cudaStream_t s,
+                    bool treeDone) {
+  const int acc = !fp32 ? ACC_SET : (sweep == 0 ? ACC_FIRST : ACC_ADD);
+  const int fin = (fp32 && last) ? 1 : 0;
+  if (p.tree.warps > 0 && !treeDone)
+    treeLaunch(d, p, fp32, nullptr, p.cntTree, backwardOf(p, fp32, sweep, last, true), false, false, s);
+  if (p.nLeaves <= 0) return;
   const int wpb = p.backwardWarps;
   int* queue = p.bwQueue + (size_t)sweep * p.nLeaves;
   int* ctr = p.bwCtr + 4 * sweep;

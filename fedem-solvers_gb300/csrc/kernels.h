@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <functional>
 #include <string>
 
 #include "engine_dev.cuh"
@@ -56,14 +57,22 @@ enum ElemMode : int {
 struct BackwardSeed {
   int nq = 0;      // queues (solves per iteration)
   int stride = 0;  // slots per queue
-  // per model: the tops of its small-front subtrees (fronts whose parent is a
-  // large front, or roots) in roots[rootOff[m]..rootOff[m+1]), and its number
+  // per model: the tops of the cascades' subtrees (fronts whose parent is not the
+  // cascades', or roots) in roots[rootOff[m]..rootOff[m+1]), and its number
   // of chains
   const int* rootOff = nullptr;
   const int* roots = nullptr;
   const int* slotCnt = nullptr;
   int* queue = nullptr;
   int* ctr = nullptr;
+  // the same for the queues of the trees on thread blocks (chunks in the place of
+  // fronts); strideT = 0: none
+  int strideT = 0;
+  const int* rootOffT = nullptr;
+  const int* rootsT = nullptr;
+  const int* slotCntT = nullptr;
+  int* queueT = nullptr;
+  int* ctrT = nullptr;
 };
 // What the last kernel of an iteration does beside the step end: the iteration's
 // counters and backward queues reset for the next one (in place of memset nodes),
@@ -173,7 +182,8 @@ struct TreePlan {
   const int* kids = nullptr;
   const int* start = nullptr;  // chunks without child chunks, longest root path first
   int nStart = 0;
-  int warps = 0;  // fronts per chunk at most, and warps per block (0: the cascades are used)
+  int nChunks = 0;
+  int warps = 0;  // fronts per chunk at most, and warps per block (0: no such trees)
 };
 struct PersistentPlan {
   TreePlan tree;
@@ -206,10 +216,12 @@ struct PersistentPlan {
   // (large[4]), and their counters (nLarge each: factorisation signals and
   // barriers, then per solve forward signals, backward signals, backward
   // barriers), zeroed with the other iteration counters
-  const unsigned char* fLarge = nullptr;
   int nLarge = 0;
   LargePlan large[5];
   int* cntLarge = nullptr;
+  // the trees' counters (nChunks + 1 per solve: child chunks done, then the start
+  // counter), queues (tree.nStart slots per solve) and queue counters (4 per solve)
+  int *cntTree = nullptr, *treeQueue = nullptr, *treeCtr = nullptr;
   // Launch shapes, picked per batch by the engine's autotuner.  No choice
   // changes a result bit: tasks are taken dynamically, and each front's
   // arithmetic is the same whichever warp, block or cluster does it.
@@ -235,8 +247,12 @@ void launchLargeForward(const DevData& d, const PersistentPlan& p, bool fp32, co
 void launchLargeBackward(const DevData& d, const PersistentPlan& p, bool fp32, int sweep, bool last, cudaStream_t s);
 // values of L a block of the large-front solves stages for a front shared by G blocks
 int64_t largeSolveStage(int nr, int np, int G, size_t elemBytes);
-// warps per block (and fronts per chunk) of the trees on thread blocks for a batch
-// of nLeaves leaf fronts and fronts of at most maxRow rows; 0: not used
+// the height from which a batch's small fronts go to the trees on thread blocks:
+// 0 (all of them), more (the cascades below it), or -1 (none), by its leaf fronts,
+// the largest height and the number of subtrees' lowest fronts from a height on
+int treeFromHeight(int nLeaves, int maxHeight, const std::function<long long(int)>& lowest);
+// their warps per block (and fronts per chunk) for nLeaves leaf fronts (0: the upper
+// levels of a larger batch) and fronts of at most maxRow rows; 0: too few fit
 int treeWarps(int nLeaves, int maxRow, bool fp32);
 // values of one front's L block the solve kernels stage in shared memory
 int stagingCapacity(const PersistentPlan& p, size_t elemBytes);
@@ -268,7 +284,9 @@ void launchForwardCascade(const DevData& d, const PersistentPlan& p, bool fp32, 
                           cudaStream_t s, bool withBackward = false, bool lastSweep = false);
 // back substitution; stores the solution in del (FP64 solve) or accumulates it in xref
 // (FP32 refinement sweep `sweep`; the last sweep also copies xref to del)
-void launchBackward(const DevData& d, const PersistentPlan& p, bool fp32, int sweep, bool last, cudaStream_t s);
+// (treeDone: the trees' part already ran)
+void launchBackward(const DevData& d, const PersistentPlan& p, bool fp32, int sweep, bool last, cudaStream_t s,
+                    bool treeDone = false);
 // One warp of the back-substitution queue kernel on a private queue (4 ints of
 // counters at ctr, the slots at queue), waiting at most `spins` polls: with an
 // empty slot 0 and a slot total of 1 the wait runs out and sets p.errFlag.

@@ -1,9 +1,10 @@
 """Small batches take kernels of their own: four lanes per beam element in the
 element pass and the Newton matrices, clusters of one-warp blocks in the norms,
 and the assembly trees on thread blocks (up to 8,192 elements, 48 norm chunks
-and 8,192 leaf fronts).  They perform the operations of the large batches'
+and 8,192 leaf fronts; up to 32,768 leaf fronts the trees' upper levels only).  They perform the operations of the large batches'
 kernels in the same order, so a model alone and the same model beside two long
-chains, which put the batch above all three lines, must agree to the last bit
+chains (the trees' upper levels) or six (the cascades alone), which put the batch
+above the other lines, must agree to the last bit
 (tolerance zero): chains from a single beam (one front) over the sizes around the
 chunks' tiers, and a gravity-loaded pendulum with a joint (kept frames, gravity
 forces, constraint expansion)."""
@@ -23,13 +24,14 @@ def _cases():
     return out
 
 
+@pytest.mark.parametrize("chains", [2, 6])
 @pytest.mark.parametrize("mixed", [False, True], ids=["fp64", "mixed"])
-def test_alone_and_in_a_large_batch_agree_bitwise(gpu, mixed):
+def test_alone_and_in_a_large_batch_agree_bitwise(gpu, mixed, chains):
     from fedem_gb300 import models
     from fedem_gb300.batch import Batch, create_models
 
     cases = _cases()
-    big = [models.batch_c4(1, seed=s, n_min=30000, n_max=30000, steps=4)[0][:2] for s in (1, 2)]
+    big = [models.batch_c4(1, seed=s, n_min=30000, n_max=30000, steps=4)[0][:2] for s in range(chains)]
     ms = create_models(cases + big)
     together = Batch(ms, mixed=mixed)
     assert together.run()["models_failed"] == 0
