@@ -1248,6 +1248,19 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
         int *dg = nullptr, *dgs = nullptr, *dgr = nullptr;
         UPV(dg, int, gOff); UPV(dgs, int, gSrc); UPV(dgr, int, gRow);
         base.gOff = dg; base.gSrc = dgs; base.gRow = dgr;
+        std::vector<int> invFront, invPart, invBlk(nL);
+        for (int li = 0; li < nL; ++li) {
+          invBlk[li] = (int)invFront.size();
+          for (int k = 0; k < npiv[lf[li]]; k += 32) {
+            invFront.push_back(lf[li]);
+            invPart.push_back(k / 32);
+          }
+        }
+        int *df = nullptr, *dp2 = nullptr, *db = nullptr;
+        UPV(df, int, invFront); UPV(dp2, int, invPart); UPV(db, int, invBlk);
+        base.nInvBlk = (int)invFront.size();
+        base.invFront = df; base.invPart = dp2; base.invBlk = db;
+        base.inverse = alloc<char>(2048 * elemB * invFront.size());
       }
       int sms = 0;
       FG_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
@@ -2186,7 +2199,7 @@ void Engine::enqueueIteration(cudaStream_t s, bool timed, bool reset) {
   launchesPerIter_ = (d_.beamSparse ? 11 : 12) + 1 + 2 * (sw - 1) + sw -
                      (fuseBackward_ ? 1 : 0) - (pplan_.tree.warps > 0 && pplan_.nLarge == 0 ? sw - 1 : 0) +
                      (pplan_.tree.warps > 0 && pplan_.nLeaves > 0 ? 2 * sw : 0) +
-                     (pplan_.nLarge > 0 ? 1 + 2 * sw : 0) +
+                     (pplan_.nLarge > 0 ? 2 + 2 * sw : 0) +
                      (d_.urQs ? 1 : 0) +
                      (d_.nmotTot > 0 ? 1 : 0) + (d_.nmrTot > 0 ? 1 : 0) + (d_.naxTot > 0 ? 3 : 0) +
                      (d_.nldTot > 0 ? 1 : 0) + (d_.njointTot > 0 ? 2 : 0) + (d_.ncxTot > 0 ? 3 : 0) +

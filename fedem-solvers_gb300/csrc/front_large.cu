@@ -486,7 +486,7 @@ __device__ inline void scanWaves(const DevData& d, const LargePlan& lp, int base
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kLT) kLargeFactor(DevData d, LargePlan lp, const T* asmVal, T* Lbase, T* Ubase,
+__global__ void __launch_bounds__(kLT, 1) kLargeFactor(DevData d, LargePlan lp, const T* asmVal, T* Lbase, T* Ubase,
                                                      double tolFact) {
   pdlEntry();
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -532,6 +532,94 @@ __host__ __device__ inline int64_t backwardStage(int nr, int np, int G) {
   return (int64_t)np * (np | 1) + (int64_t)((np + G - 1) / G) * (nr - np);
 }
 
+// ---- inverses of the pivot blocks ----------------------------------------------
+// The solves multiply by the inverse of each 32 x 32 unit lower pivot block instead
+// of substituting through it: 32 dependent steps of a shuffle and a multiply-add
+// (3,000 cycles in FP64) become one product shared by four warps (850).  The space-
+// frame tower's solves, 17 fronts deep, spent more than half their time there.
+// inverse + 2048 blk: the block's inverse column by column (entry (i, k) at
+// 32 k + i), then row by row (1024 + 32 i + k); identity beyond a short block.
+// this lane's (row or column `lane`) eight values 8 h .. 8 h + 7
+template <typename T>
+__device__ inline void loadInverse(T* li, const T* inv, int h, int lane) {
+#pragma unroll
+  for (int q = 0; q < 8; ++q) li[q] = ld(inv + 32 * (8 * h + q) + lane);
+}
+
+// One block of 128 threads per pivot block (of a model that factored): the 8 x 8
+// diagonal blocks by substitution, then twice the size from the halves,
+// [A 0; B C]^-1 = [A' 0; -C' B A' C'].
+template <typename T>
+__global__ void __launch_bounds__(128) kLargeInverse(DevData d, LargePlan lp, const T* Lbase) {
+  pdlEntry();
+  __shared__ T L[32][33], V[32][33], M[16][17];  // [row][column]
+  const int f = lp.invFront[blockIdx.x], k0 = 32 * lp.invPart[blockIdx.x];
+  const int fl = d.m.flags[d.fModel[f]];
+  if (!(fl & FL_ACTIVE) || !(fl & FL_TANGENT)) return;
+  const int nr = d.fNrow[f], kb = min(32, d.fNpiv[f] - k0);
+  const T* Lf = Lbase + d.fLOff[f] + k0 + (int64_t)nr * k0;
+  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+  for (int q = tid; q < 1024; q += 128) {
+    const int i = q & 31, k = q >> 5;
+    L[i][k] = (i > k && i < kb) ? ld(Lf + i + (int64_t)nr * k) : T(0);
+    V[i][k] = T(0);
+  }
+  __syncthreads();
+  if (lane < 8) {  // column `lane` of the inverse of diagonal block w
+    T x[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      T a = T(0);
+#pragma unroll
+      for (int k = 0; k < i; ++k) a += L[8 * w + i][8 * w + k] * x[k];
+      x[i] = i == lane ? T(1) : (i > lane ? -a : T(0));
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) V[8 * w + i][8 * w + lane] = x[i];
+  }
+  __syncthreads();
+  {  // 16: one entry of each product per thread
+    const int p = tid >> 6, i = (tid >> 3) & 7, k = tid & 7, o = 16 * p;
+    T a = T(0);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) a += L[o + 8 + i][o + j] * V[o + j][o + k];
+    M[8 * p + i][k] = a;
+    __syncthreads();
+    a = T(0);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) a += V[o + 8 + i][o + 8 + j] * M[8 * p + j][k];
+    V[o + 8 + i][o + k] = -a;
+  }
+  __syncthreads();
+  {  // 32: two entries of each product per thread
+    const int i = tid >> 3, k = tid & 7;
+    T a = T(0), b = T(0);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      a += L[16 + i][j] * V[j][k];
+      b += L[16 + i][j] * V[j][k + 8];
+    }
+    __syncthreads();
+    M[i][k] = a;
+    M[i][k + 8] = b;
+    __syncthreads();
+    a = b = T(0);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      a += V[16 + i][16 + j] * M[j][k];
+      b += V[16 + i][16 + j] * M[j][k + 8];
+    }
+    V[16 + i][k] = -a;
+    V[16 + i][k + 8] = -b;
+  }
+  __syncthreads();
+  T* out = static_cast<T*>(lp.inverse) + 2048 * (int64_t)blockIdx.x;
+  for (int q = tid; q < 1024; q += 128) {
+    out[q] = V[q & 31][q >> 5];
+    out[1024 + q] = V[q >> 5][q & 31];
+  }
+}
+
 // Forward elimination of front t.f, y = L11^-1 v_p, w = v_u - L21 y, by its G
 // blocks: each solves the pivot block itself (no barrier) and takes a slice of
 // the rows below it.  L does not depend on the children: it is staged in shared
@@ -561,6 +649,9 @@ __device__ void forwardLarge(const DevData& d, const LargePlan& lp, const LargeT
   const int ldp = staged ? lds : nr;
   const T* Lq = staged ? Lr : L + r0;
   const int ldq = staged ? ns : nr;
+  T li[8];  // this lane's share of a pivot block's inverse
+  const T* linv = static_cast<const T*>(lp.inverse) + 2048 * (int64_t)lp.invBlk[t.li];
+  if (w < 4) loadInverse(li, linv, w, lane);
   // the right-hand side of the pivot rows, and where the children's
   // contributions to the pivot rows and to this block's rows come from (in
   // child order), before the wait; their values after it
@@ -600,30 +691,18 @@ __device__ void forwardLarge(const DevData& d, const LargePlan& lp, const LargeT
   __syncthreads();
   for (int b0 = 0; b0 < np; b0 += 32) {
     const int bs = min(32, np - b0);
-    if (w == 0) {  // the block's unit triangle: lane r holds v[b0 + r]
-      T x = lane < bs ? v[b0 + lane] : T(0);
-      const T* Lb = Lp + b0 + (int64_t)ldp * b0;
-      if (staged) {
-#pragma unroll 8
-        for (int k = 0; k < bs - 1; ++k) {
-          const T l = lane > k && lane < bs ? Lb[lane + ldp * k] : T(0);
-          x -= l * __shfl_sync(0xffffffffu, x, k);
-        }
-      } else {
-        for (int k1 = 0; k1 < bs - 1; k1 += 8) {
-          T l[8];
+    // the block's pivots: inverse times right-hand side, a quarter of the columns
+    // per warp (the next block's inverse is loaded meanwhile)
+    if (w < 4) {
+      T a = T(0);
 #pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            const int k = k1 + u;
-            l[u] = (k < bs - 1 && lane > k && lane < bs) ? Lb[lane + (int64_t)ldp * k] : T(0);
-          }
-#pragma unroll
-          for (int u = 0; u < 8; ++u)
-            if (k1 + u < bs - 1) x -= l[u] * __shfl_sync(0xffffffffu, x, k1 + u);
-        }
-      }
-      if (lane < bs) v[b0 + lane] = x;
+      for (int q = 0; q < 8; ++q)
+        if (8 * w + q < bs) a += li[q] * v[b0 + 8 * w + q];
+      part[tid] = a;
+      if (b0 + 32 < np) loadInverse(li, linv + 2048 * (b0 / 32 + 1), w, lane);
     }
+    __syncthreads();
+    if (w == 0 && lane < bs) v[b0 + lane] = ((part[lane] + part[32 + lane]) + part[64 + lane]) + part[96 + lane];
     __syncthreads();
     // the later pivot rows: four lanes a row, each a quarter of the block's pivots
     const int left = np - b0 - bs;
@@ -665,7 +744,7 @@ __device__ void forwardLarge(const DevData& d, const LargePlan& lp, const LargeT
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kLT) kLargeForward(DevData d, LargePlan lp, const T* Lbase, const double* rhs, T* X,
+__global__ void __launch_bounds__(kLT, 1) kLargeForward(DevData d, LargePlan lp, const T* Lbase, const double* rhs, T* X,
                                                       T* W) {
   pdlEntry();
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -720,6 +799,10 @@ __device__ void backwardLarge(const DevData& d, const LargePlan& lp, const Large
   for (int q = 0; q < 2; ++q) row[q] = np + tid + kLT * q < nr ? __ldg(rows + np + tid + kLT * q) : -1;
   const int rowk = w < nc ? __ldg(rows + k0 + w) : 0, rowp = tid < np ? __ldg(rows + tid) : 0;
   const T yk = w < nc ? ld(X + rowk) : T(0);
+  // (block 0) the last pivot block's inverse, row by row
+  T li[8];
+  const T* linv = static_cast<const T*>(lp.inverse) + 2048 * (int64_t)lp.invBlk[t.li] + 1024;
+  if (t.rank == 0 && w < 4) loadInverse(li, linv + 2048 * ((np - 1) / 32), w, lane);
   if (par >= 0) waitCount(lp.done + par, 1, ws);
 #pragma unroll
   for (int q = 0; q < 2; ++q)
@@ -752,32 +835,21 @@ __device__ void backwardLarge(const DevData& d, const LargePlan& lp, const Large
   __syncthreads();
   const T* Lp = staged ? Ls : L;
   const int ldp = staged ? lds : nr;
-  // the unit upper triangle L11^T, blocks of 32 pivots from the last: warp 0
-  // solves the block with shuffles, then the pivots above it are updated with
-  // the block's values
-  for (int bEnd = np; bEnd > 0; bEnd -= 32) {
-    const int b0 = bEnd > 32 ? bEnd - 32 : 0, bs = bEnd - b0;
-    if (w == 0) {
-      T x = lane < bs ? xs[b0 + lane] : T(0);
-      const T* Lb = Lp + b0 + (int64_t)ldp * (b0 + (lane < bs ? lane : 0));
-      if (staged) {
-#pragma unroll 8
-        for (int j = bs - 1; j > 0; --j) {
-          const T l = lane < j ? Lb[j] : T(0);
-          x -= l * __shfl_sync(0xffffffffu, x, j);
-        }
-      } else {
-        for (int j1 = bs - 1; j1 > 0; j1 -= 8) {
-          T l[8];
+  // the unit upper triangle L11^T, the factorisation's blocks of 32 pivots from the
+  // last: the transposed inverse of the block times its values, then the pivots
+  // above it are updated
+  for (int bEnd = np; bEnd > 0; bEnd = (bEnd - 1) & ~31) {
+    const int b0 = (bEnd - 1) & ~31, bs = bEnd - b0;
+    if (w < 4) {
+      T a = T(0);
 #pragma unroll
-          for (int u = 0; u < 8; ++u) l[u] = (j1 - u > 0 && lane < j1 - u) ? Lb[j1 - u] : T(0);
-#pragma unroll
-          for (int u = 0; u < 8; ++u)
-            if (j1 - u > 0) x -= l[u] * __shfl_sync(0xffffffffu, x, j1 - u);
-        }
-      }
-      if (lane < bs) xs[b0 + lane] = x;
+      for (int q = 0; q < 8; ++q)
+        if (8 * w + q < bs) a += li[q] * xs[b0 + 8 * w + q];
+      part[tid] = a;
+      if (b0 > 0) loadInverse(li, linv + 2048 * (b0 / 32 - 1), w, lane);
     }
+    __syncthreads();
+    if (w == 0 && lane < bs) xs[b0 + lane] = ((part[lane] + part[32 + lane]) + part[64 + lane]) + part[96 + lane];
     __syncthreads();
     // pivots above the block: four lanes a pivot, each a quarter of the block's rows
     for (int q = tid; q < ((4 * b0 + 31) & ~31); q += kLT) {
@@ -809,7 +881,7 @@ __device__ void backwardLarge(const DevData& d, const LargePlan& lp, const Large
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kLT) kLargeBackward(DevData d, LargePlan lp, const T* Lbase, T* X, int acc,
+__global__ void __launch_bounds__(kLT, 1) kLargeBackward(DevData d, LargePlan lp, const T* Lbase, T* X, int acc,
                                                        int finalize) {
   pdlEntry();
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -876,6 +948,9 @@ void launchLargeFactor(const DevData& d, const PersistentPlan& p, bool fp32, cud
   else
     coopLaunch(kLargeFactor<double>, lp.grid, sizeof(FactorShared<double>), s, d, lp, (const double*)d.asmVal64, d.L64,
                d.U64, 1.0e-12);
+  // the inverses of the pivot blocks, for the solves
+  if (fp32) pdlLaunch(kLargeInverse<float>, lp.nInvBlk, 128, 0, s, d, lp, (const float*)d.L32);
+  else pdlLaunch(kLargeInverse<double>, lp.nInvBlk, 128, 0, s, d, lp, (const double*)d.L64);
 }
 
 void launchLargeForward(const DevData& d, const PersistentPlan& p, bool fp32, const double* rhs, int sweep,

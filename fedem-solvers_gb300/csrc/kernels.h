@@ -162,6 +162,13 @@ struct LargePlan {
   const int* asmColOff = nullptr;
   const int* diagAsm = nullptr;
   const int* diagOff = nullptr;
+  // pivot blocks of 32: the fronts and their parts of them, each front's first one,
+  // and their inverses (2048 values each; see front_large.cu)
+  int nInvBlk = 0;
+  const int* invFront = nullptr;
+  const int* invPart = nullptr;
+  const int* invBlk = nullptr;
+  void* inverse = nullptr;
   int maxRow = 0;                // largest large front (rows)
   int64_t stageCap = 0;          // values of L a block of the solves can stage
   int *done = nullptr, *bar = nullptr, *err = nullptr;
