@@ -22,6 +22,9 @@ namespace fgpu {
 namespace {
 
 constexpr int kMaxLevels = 7;  // position-matrix levels of a joint (1..6 used)
+// joints up to which four lanes share one: eight joints a warp, a warp per sub-core of
+// 152 SMs; beyond it a second wave of warps costs what the lanes save
+constexpr int kSharedJoints = 4864;
 
 // joint variables of level im (1-based) as a 3x4 position matrix
 __device__ void jointLevel(const DevData& d, int j, int im, double* F) {
@@ -45,79 +48,108 @@ __device__ inline bool modeActive(int mode, int fl) {
   return true;  // EM_FINAL: every model
 }
 
-// One thread per joint: increment of the joint variables (after an increment
-// pass), the dependent triad on its kinematic position, the coefficients T.
-__global__ void kJoints(DevData d, int mode) {
+// Shared working set of a joint: its frame, the dependent triad's position, and per
+// level the position matrix of its variables, the rotation its DOFs act in (csys) and
+// its global position (png)
+struct JointWork {
+  double JG[12], P[12], F[kMaxLevels][12], csys[kMaxLevels][9], png[kMaxLevels][3];
+};
+
+// W lanes per joint: increment of the joint variables (after an increment pass), the
+// dependent triad on its kinematic position, the coefficients T.
+//
+// Bound by FP64 issue (64 cycles a warp instruction whatever its lanes), so while the
+// lanes of a wave of warps outnumber the joints, four lanes share a joint: a column or
+// a row of each 3 x 4 product and a joint DOF each.  Every value is the same expression
+// for any W.
+template <int W>
+__global__ void __launch_bounds__(32) kJoints(DevData d, int mode) {
   pdlEntry();
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  __shared__ JointWork work[32 / W];
+  const int j = (blockIdx.x * 32 + threadIdx.x) / W, lane = threadIdx.x % W;
   if (j >= d.njointTot) return;
   if (!modeActive(mode, d.m.flags[d.jModel[j]])) return;
+  JointWork& w = work[threadIdx.x / W];
+  const unsigned group = W == 32 ? 0xffffffffu : ((1u << W) - 1) << (threadIdx.x & ~(W - 1) & 31);
   const int n0 = d.jDofOff[j], nv = d.jNdof[j], nmats = d.jNmats[j];
   if (mode == EM_INC || mode == EM_STATIC)
-    for (int k = 0; k < nv; ++k) d.jVar[n0 + k] += d.sinc0[d.jFirstDof[j] + k];
+    for (int k = lane; k < nv; k += W) d.jVar[n0 + k] += d.sinc0[d.jFirstDof[j] + k];
+  __syncwarp(group);
   double* US = d.ur + 12 * (size_t)d.jSlave[j];
   const double* UM = d.ur + 12 * (size_t)d.jMaster[j];
-  double M[12], JG[12], JT[12];
+  // joint frame follows the master triad; position matrices of the levels
+  for (int c = lane; c < 4; c += W)
+    for (int r = 0; r < 3; ++r) {
+      const double* JT = d.jPosInT + 12 * j + 3 * c;
+      double v = UM[r] * JT[0] + UM[r + 3] * JT[1] + UM[r + 6] * JT[2];
+      if (c == 3) v += UM[r + 9];
+      w.JG[r + 3 * c] = v;
+    }
+  for (int im = 1 + lane; im <= nmats; im += W) {
+    double F[12];
+    jointLevel(d, j, im, F);
 #pragma unroll
-  for (int k = 0; k < 12; ++k) { M[k] = UM[k]; JT[k] = d.jPosInT[12 * j + k]; }
-  compose34(M, JT, JG);  // joint frame follows the master triad
+    for (int k = 0; k < 12; ++k) w.F[im][k] = F[k];
+  }
   // TR = -spin(e), e the dependent triad's position relative to the master
   // before the dependent triad is moved (SetLinearDependencies)
-  const double e0 = US[9] - M[9], e1 = US[10] - M[10], e2 = US[11] - M[11];
-  double P[12], Q[12], F[12];
-#pragma unroll
-  for (int k = 0; k < 12; ++k) P[k] = d.jSTPos0[12 * j + k];
-  for (int im = 1; im <= nmats; ++im) {
-    jointLevel(d, j, im, F);
-    compose34(F, P, Q);
-#pragma unroll
-    for (int k = 0; k < 12; ++k) P[k] = Q[k];
+  const double e0 = US[9] - UM[9], e1 = US[10] - UM[10], e2 = US[11] - UM[11];
+  __syncwarp(group);
+  // the dependent triad: JG F(nmats) ... F(1) STPos0, a column per lane
+  for (int c = lane; c < 4; c += W) {
+    double p[3], q[3];
+    for (int r = 0; r < 3; ++r) p[r] = d.jSTPos0[12 * j + 3 * c + r];
+    for (int im = 1; im <= nmats + 1; ++im) {
+      const double* F = im <= nmats ? w.F[im] : w.JG;
+      for (int r = 0; r < 3; ++r) {
+        q[r] = F[r] * p[0] + F[r + 3] * p[1] + F[r + 6] * p[2];
+        if (c == 3) q[r] += F[r + 9];
+      }
+      for (int r = 0; r < 3; ++r) p[r] = q[r];
+    }
+    for (int r = 0; r < 3; ++r) w.P[3 * c + r] = US[3 * c + r] = p[r];
   }
-  compose34(JG, P, Q);
-#pragma unroll
-  for (int k = 0; k < 12; ++k) US[k] = Q[k];
+  // accumulated level frames, a row per lane: csys(im) = rotation of the frame the
+  // level's DOFs act in, png(im) = position of level im (global)
+  for (int r = lane; r < 3; r += W) {
+    double a[4];
+    for (int c = 0; c < 4; ++c) a[c] = w.JG[r + 3 * c];
+    for (int im = nmats; im >= 1; --im) {
+      const double* F = w.F[im];
+      for (int c = 0; c < 3; ++c) w.csys[im][r + 3 * c] = a[c];
+      double q[4];
+      for (int c = 0; c < 4; ++c) {
+        q[c] = a[0] * F[3 * c] + a[1] * F[3 * c + 1] + a[2] * F[3 * c + 2];
+        if (c == 3) q[c] += a[3];
+      }
+      for (int c = 0; c < 4; ++c) a[c] = q[c];
+      w.png[im][r] = a[3];
+    }
+  }
   // constraint coefficients (updateDependencies): master block, then joint DOFs
   double* T = d.jT + 72 * (size_t)j;
-#pragma unroll
-  for (int k = 0; k < 72; ++k) T[k] = 0.0;
+  for (int k = lane; k < 72; k += W) T[k] = 0.0;
+  __syncwarp(group);
   const int nM = d.jNM[j];
-  // TR columns: TR(:,c) = -spin(e) e_c = e x e_c
-  const double TR[9] = {0.0, -e2, e1, e2, 0.0, -e0, -e1, e0, 0.0};  // column-major, TR[r + 3c]
-  for (int lm = 0; lm < nM; ++lm)
-    for (int ls = 0; ls < 6; ++ls) {
-      double v = 0.0;
-      if (ls < 3 && lm < 3) v = ls == lm ? 1.0 : 0.0;
-      else if (ls < 3) v = TR[ls + 3 * (lm - 3)];
-      else if (lm >= 3) v = ls == lm ? 1.0 : 0.0;
-      T[12 * ls + lm] = v;
-    }
-  // accumulated level frames: csys(im) = rotation of the frame the level's DOFs
-  // act in, png(im) = position of level im (global)
-  double csys[kMaxLevels][9], png[kMaxLevels][3];
-  double Pacc[12];
-#pragma unroll
-  for (int k = 0; k < 12; ++k) Pacc[k] = JG[k];
-  for (int im = nmats; im >= 1; --im) {
-#pragma unroll
-    for (int k = 0; k < 9; ++k) csys[im][k] = Pacc[k];
-    jointLevel(d, j, im, F);
-    compose34(Pacc, F, Q);
-#pragma unroll
-    for (int k = 0; k < 12; ++k) Pacc[k] = Q[k];
-    png[im][0] = Pacc[9]; png[im][1] = Pacc[10]; png[im][2] = Pacc[11];
+  for (int lm = lane; lm < nM; lm += W) {
+    T[12 * lm + lm] = 1.0;
+    // TR columns: TR(:,c) = -spin(e) e_c = e x e_c
+    if (lm == 3) { T[12 + lm] = -e2; T[24 + lm] = e1; }
+    if (lm == 4) { T[lm] = e2; T[24 + lm] = -e0; }
+    if (lm == 5) { T[lm] = -e1; T[12 + lm] = e0; }
   }
-  for (int k = 0; k < nv; ++k) {
+  for (int k = lane; k < nv; k += W) {
     const int lm = d.jLdof[n0 + k], im = d.jImat[n0 + k];
     double dUS[6];
     if (lm <= 3) {
 #pragma unroll
-      for (int r = 0; r < 3; ++r) { dUS[r] = csys[im][r + 3 * (lm - 1)]; dUS[3 + r] = 0.0; }
+      for (int r = 0; r < 3; ++r) { dUS[r] = w.csys[im][r + 3 * (lm - 1)]; dUS[3 + r] = 0.0; }
     } else {
       double dOm[3], ecc[3], dUG[3];
 #pragma unroll
       for (int r = 0; r < 3; ++r) {
-        dOm[r] = csys[im][r + 3 * (lm - 4)];
-        ecc[r] = US[9 + r] - png[im][r];
+        dOm[r] = w.csys[im][r + 3 * (lm - 4)];
+        ecc[r] = w.P[9 + r] - w.png[im][r];
       }
       crossd(dOm, ecc, dUG);
 #pragma unroll
@@ -220,7 +252,11 @@ __global__ void kExpandForces(DevData d, int mode) {
 }  // namespace
 
 void launchJoints(const DevData& d, int mode, cudaStream_t s) {
-  if (d.njointTot > 0) pdlLaunch(kJoints, (d.njointTot + 63) / 64, 64, 0, s, d, mode);
+  if (d.njointTot <= 0) return;
+  if (d.njointTot <= kSharedJoints)
+    pdlLaunch(kJoints<4>, (d.njointTot + 7) / 8, 32, 0, s, d, mode);
+  else
+    pdlLaunch(kJoints<1>, (d.njointTot + 31) / 32, 32, 0, s, d, mode);
 }
 
 void launchExpandElements(const DevData& d, cudaStream_t s) {

@@ -27,7 +27,7 @@
 namespace fgpu {
 namespace {
 
-constexpr int kPartThreads = 128;
+constexpr int kPartThreads = 256;
 
 __device__ inline bool partModeActive(int mode, int fl) {
   if (mode == EM_PRED) return fl & FL_PRED;
@@ -81,8 +81,11 @@ __global__ void __launch_bounds__(kPartThreads) kParts(DevData d, int mode) {
   double* fin = sh + 12;     // n
   double* uld = fin + n;     // n
   double* uldd = uld + n;    // n
-  double* F = uldd + n;      // 4 n: FS, FD, FI, Q
+  double* F = uldd + n;      // 4 n: FS, FD, FI, Q (12 nt <= 2 n positions before)
+  double* rate = F + 4 * n;  // nd <= n
+  double* filt = rate + n;   // nd
   __shared__ int bad;
+  __shared__ double pt[3][3], invT[3];
   const bool qs = (mode == EM_PRED || mode == EM_INC) && (fl & FL_QSTATIC);
   const bool isStatic = mode == EM_STATIC || mode == EM_STATIC_INIT || qs;
   const bool newPositions = (mode == EM_INC || mode == EM_STATIC || mode == EM_FINAL) && !(qs && (fl & FL_LINEAR));
@@ -114,33 +117,43 @@ __global__ void __launch_bounds__(kPartThreads) kParts(DevData d, int mode) {
     uldd[i] = a;
   }
   __syncthreads();
-  if (tid == 0 && newPositions) {
+  // The frame and the deformation are spread over threads, a column, a point or a
+  // component each: one thread's 230 FP64 instructions, 64 cycles apart, were half
+  // of this launch.  With the products below on a thread per row and matrix, an
+  // iteration of 16 parts of 42 DOFs went from 264 to 245 us (joints included).
+  if (newPositions) {
     // corotated frame through the three reference points (shadowPosAlg = 1)
-    double pt[3][3];
-    for (int j = 0; j < 3; ++j) {
+    if (tid < 9) {
+      const int j = tid / 3, q = tid % 3;
       const double* U = d.ur + 12 * (size_t)d.pTri[t0 + d.pRef[3 * p + j]];
       const double* o = d.pOffset + 9 * (size_t)p + 3 * j;
-      for (int q = 0; q < 3; ++q) pt[j][q] = U[q] * o[0] + U[q + 3] * o[1] + U[q + 6] * o[2] + U[q + 9];
+      pt[j][q] = U[q] * o[0] + U[q + 3] * o[1] + U[q + 6] * o[2] + U[q + 9];
     }
-    double ex[3], v2[3], ez[3], ey[3];
-    for (int k = 0; k < 3; ++k) { ex[k] = pt[1][k] - pt[0][k]; v2[k] = pt[2][k] - pt[0][k]; }
-    crossd(ex, v2, ez);
-    const double lx = ex[0] * ex[0] + ex[1] * ex[1] + ex[2] * ex[2];
-    const double lz = ez[0] * ez[0] + ez[1] * ez[1] + ez[2] * ez[2];
-    if (!(lx > 1.0e-16) || !(lz > 1.0e-16)) {
-      atomicOr(&d.m.status[m], SS_COROT);
-      bad = 1;
-    } else {
-      const double ilx = rsqrt(lx), ilz = rsqrt(lz);
-      for (int k = 0; k < 3; ++k) { ex[k] *= ilx; ez[k] *= ilz; }
-      crossd(ez, ex, ey);
-      double T[12] = {ex[0], ex[1], ex[2], ey[0], ey[1], ey[2], ez[0], ez[1], ez[2], pt[0][0], pt[0][1], pt[0][2]};
-      double Rel[12], Snew[12];
-      for (int k = 0; k < 12; ++k) Rel[k] = d.pTriRelSup[12 * (size_t)p + k];
-      compose34(T, Rel, Snew);
-      for (int k = 0; k < 12; ++k) {
-        S[k] = Snew[k];
-        d.pSupTr[12 * (size_t)p + k] = Snew[k];
+    __syncthreads();
+    if (tid < 4) {
+      double ex[3], v2[3], ez[3], ey[3];
+      for (int k = 0; k < 3; ++k) { ex[k] = pt[1][k] - pt[0][k]; v2[k] = pt[2][k] - pt[0][k]; }
+      crossd(ex, v2, ez);
+      const double lx = ex[0] * ex[0] + ex[1] * ex[1] + ex[2] * ex[2];
+      const double lz = ez[0] * ez[0] + ez[1] * ez[1] + ez[2] * ez[2];
+      if (!(lx > 1.0e-16) || !(lz > 1.0e-16)) {
+        if (tid == 0) {
+          atomicOr(&d.m.status[m], SS_COROT);
+          bad = 1;
+        }
+      } else {
+        const double ilx = rsqrt(lx), ilz = rsqrt(lz);
+        for (int k = 0; k < 3; ++k) { ex[k] *= ilx; ez[k] *= ilz; }
+        crossd(ez, ex, ey);
+        // column tid of the new frame
+        double r[3];
+        for (int k = 0; k < 3; ++k) r[k] = d.pTriRelSup[12 * (size_t)p + 3 * tid + k];
+        for (int k = 0; k < 3; ++k) {
+          double v = ex[k] * r[0] + ey[k] * r[1] + ez[k] * r[2];
+          if (tid == 3) v += pt[0][k];
+          S[3 * tid + k] = v;
+          d.pSupTr[12 * (size_t)p + 3 * tid + k] = v;
+        }
       }
     }
   }
@@ -148,20 +161,29 @@ __global__ void __launch_bounds__(kPartThreads) kParts(DevData d, int mode) {
   if (bad) return;
   // deformation vector in the corotated axes
   if (newPositions || mode == EM_STATIC_INIT || qs) {
-    double inv[12];
-    for (int r = 0; r < 3; ++r)
-      for (int c = 0; c < 3; ++c) inv[r + 3 * c] = S[c + 3 * r];
-    for (int r = 0; r < 3; ++r) inv[9 + r] = -(inv[r] * S[9] + inv[r + 3] * S[10] + inv[r + 6] * S[11]);
-    for (int t = tid; t < nt; t += nth) {
-      const double* U = d.ur + 12 * (size_t)d.pTri[t0 + t];
-      double Uc[12], loc[12], Tu[12];
-      for (int k = 0; k < 12; ++k) { Uc[k] = U[k]; Tu[k] = d.pTrUnd[12 * (size_t)(t0 + t) + k]; }
-      compose34(inv, Uc, loc);
-      for (int r = 0; r < 3; ++r) fin[6 * t + r] = loc[9 + r] - Tu[9 + r];
-      auto dR = [&](int r, int c) { return loc[r] * Tu[3 * c] + loc[r + 3] * Tu[3 * c + 1] + loc[r + 6] * Tu[3 * c + 2]; };
-      fin[6 * t + 3] = dR(2, 1);
-      fin[6 * t + 4] = dR(0, 2);
-      fin[6 * t + 5] = dR(1, 0);
+    // (r, c) of each triad's position in part axes: threads over 12 nt entries; the
+    // frame's inverse is its transpose, its translation column inv[9 + r]
+    if (tid < 3) invT[tid] = -(S[3 * tid] * S[9] + S[3 * tid + 1] * S[10] + S[3 * tid + 2] * S[11]);
+    __syncthreads();
+    double* loc = F;  // 12 nt values (the force vectors come later)
+    for (int q = tid; q < 12 * nt; q += nth) {
+      const int t = q / 12, c = (q % 12) / 3, r = q % 3;
+      const double* U = d.ur + 12 * (size_t)d.pTri[t0 + t] + 3 * c;
+      double v = S[3 * r] * U[0] + S[3 * r + 1] * U[1] + S[3 * r + 2] * U[2];
+      if (c == 3) v += invT[r];
+      loc[q] = v;
+    }
+    __syncthreads();
+    for (int q = tid; q < 6 * nt; q += nth) {
+      const int t = q / 6, k = q % 6;
+      const double* l = loc + 12 * t;
+      const double* Tu = d.pTrUnd + 12 * (size_t)(t0 + t);
+      if (k < 3) {
+        fin[q] = l[9 + k] - Tu[9 + k];
+      } else {  // dR entries (3,2), (1,3), (2,1)
+        const int r = k == 3 ? 2 : k - 4, c = k == 3 ? 1 : (k == 4 ? 2 : 0);
+        fin[q] = l[r] * Tu[3 * c] + l[r + 3] * Tu[3 * c + 1] + l[r + 6] * Tu[3 * c + 2];
+      }
     }
     for (int g = tid; g < ng; g += nth) fin[nd + g] = d.pGen[go + g];
     __syncthreads();
@@ -186,28 +208,42 @@ __global__ void __launch_bounds__(kPartThreads) kParts(DevData d, int mode) {
   const double gl2 = gv[0] * S[6] + gv[1] * S[7] + gv[2] * S[8];
   const double* fg = d.pFg + 3 * (size_t)vo;
   const double* fprev = d.pFinitPrev + vo;
-  for (int i = tid; i < n; i += nth) {
-    double fs = 0.0, fi = 0.0, fd = 0.0;
-    for (int j = 0; j < n; ++j) fs += K[i + (size_t)n * j] * fin[j];
-    fs *= ss;
-    if (!isStatic) {
-      for (int j = 0; j < n; ++j) fi += M[i + (size_t)n * j] * uldd[j];
-      if (hasC) {
-        for (int j = 0; j < n; ++j) fd += C[i + (size_t)n * j] * uld[j];
-        fd *= ss;
-      }
-      if (vldActive && i < nd) {
-        double y = 0.0;
-        for (int j = 0; j < nd; ++j) y += K[i + (size_t)n * j] * (uld[j] - (fin[j] - fprev[j]) / dt);
-        fd -= d.pKDmp[p] * (ss * y);
-      }
+  // the deformation rate the filtered damping takes off (one division each)
+  if (vldActive)
+    for (int j = tid; j < nd; j += nth) rate[j] = uld[j] - (fin[j] - fprev[j]) / dt;
+  __syncthreads();
+  // a row of one product per thread: K fin, M uldd, C uld and the filtered damping's
+  // K rate on the triad DOFs (eight entries of the row loaded ahead of their sum)
+  auto dot = [&](const double* A, const double* x, int i, int cols) {
+    double v = 0.0;
+    for (int j0 = 0; j0 < cols; j0 += 8) {
+      double a[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) a[u] = j0 + u < cols ? A[i + (size_t)n * (j0 + u)] : 0.0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (j0 + u < cols) v += a[u] * x[j0 + u];
     }
-    F[i] = fs;
-    F[n + i] = fd;
-    F[2 * n + i] = fi;
-    F[3 * n + i] = ss * (fg[i] * gl0 + fg[i + n] * gl1 + fg[i + 2 * n] * gl2);
+    return v;
+  };
+  for (int q = tid; q < 3 * n + (vldActive ? nd : 0); q += nth) {
+    const int which = q / n, i = q - which * n;
+    if (which == 0) {
+      F[i] = ss * dot(K, fin, i, n);
+      F[3 * n + i] = ss * (fg[i] * gl0 + fg[i + n] * gl1 + fg[i + 2 * n] * gl2);
+    } else if (which == 1) {
+      F[2 * n + i] = isStatic ? 0.0 : dot(M, uldd, i, n);
+    } else if (which == 2) {
+      F[n + i] = !isStatic && hasC ? ss * dot(C, uld, i, n) : 0.0;
+    } else {
+      filt[i] = dot(K, rate, i, nd);
+    }
   }
   __syncthreads();
+  if (vldActive) {
+    for (int i = tid; i < nd; i += nth) F[n + i] -= d.pKDmp[p] * (ss * filt[i]);
+    __syncthreads();
+  }
   // triad groups to system axes
   for (int w = tid; w < 4 * 2 * nt; w += nth) {
     const int v = w / (2 * nt), g = w % (2 * nt);
@@ -219,18 +255,16 @@ __global__ void __launch_bounds__(kPartThreads) kParts(DevData d, int mode) {
   // expanded forces B^T F
   const int nx = d.pNx[p];
   double* out = d.FelX + d.pXVecOff[p];
-  for (int q = tid; q < nx; q += nth) {
+  for (int w = tid; w < 4 * nx; w += nth) {
     int i0, nb;
     double b[6];
-    partColumn(d, p, q, i0, b, nb);
-    for (int v = 0; v < 4; ++v) {
-      const double* f = F + (size_t)v * n;
-      double s = 0.0;
-      if (nb < 0) s = f[i0];
-      else
-        for (int r = 0; r < 6; ++r) s += b[r] * f[i0 + r];
-      out[4 * q + v] = s;
-    }
+    partColumn(d, p, w >> 2, i0, b, nb);
+    const double* f = F + (size_t)(w & 3) * n;
+    double s = 0.0;
+    if (nb < 0) s = f[i0];
+    else
+      for (int r = 0; r < 6; ++r) s += b[r] * f[i0 + r];
+    out[w] = s;
   }
 }
 
@@ -326,7 +360,7 @@ __global__ void kPartsStepEnd(DevData d) {
   for (int i = threadIdx.x; i < n; i += blockDim.x) d.pFinitPrev[vo + i] = d.pFinit[vo + i];
 }
 
-size_t partSmem(const DevData& d) { return sizeof(double) * (12 + 7 * (size_t)d.partMaxN); }
+size_t partSmem(const DevData& d) { return sizeof(double) * (12 + 9 * (size_t)d.partMaxN); }
 
 size_t partNewtonSmem(const DevData& d) {
   const size_t n = (size_t)d.partMaxN, nx = (size_t)d.partMaxNx;
