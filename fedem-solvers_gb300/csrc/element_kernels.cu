@@ -90,35 +90,60 @@ __device__ inline double dependentValue(const DevData& d, int dd, const double* 
 // ---------------------------------------------------------------------------
 // per-model control at the start of a batched iteration
 // ---------------------------------------------------------------------------
-// the roots of model i into every backward queue, and its chain count, by the
-// lanes of a warp (a model whose upper levels go to the trees on thread blocks
-// has thousands of roots below them)
-__device__ inline void seedQueue(int* ctr, int* queue, const int* off, const int* roots, int chains, int i, int lane) {
-  const int r0 = off[i], nr = off[i + 1] - r0;
+// part `part` of `parts` of the roots of model i into a backward queue, and (part 0)
+// its chain count, by the lanes of a warp (a model whose upper levels go to the trees
+// on thread blocks has thousands of roots below them)
+__device__ inline void seedQueue(int* ctr, int* queue, const int* off, const int* roots, int chains, int i, int lane,
+                                 int part, int parts) {
+  const int n = off[i + 1] - off[i], k0 = (int)((long long)n * part / parts), k1 = (int)((long long)n * (part + 1) / parts);
   int base = 0;
   if (lane == 0) {
-    base = atomicAdd(ctr + 1, nr);
-    atomicAdd(ctr + 2, chains);
+    base = atomicAdd(ctr + 1, k1 - k0);
+    if (part == 0) atomicAdd(ctr + 2, chains);
   }
   base = __shfl_sync(0xffffffffu, base, 0);
+  const int* r = roots + off[i] + k0;
 #pragma unroll 4
-  for (int k = lane; k < nr; k += 32) queue[base + k] = roots[r0 + k];
+  for (int k = lane; k < k1 - k0; k += 32) queue[base + k] = r[k];
 }
-__device__ inline void seedBackward(const BackwardSeed& b, int i, int lane) {
-  for (int q = 0; q < b.nq; ++q) {
-    seedQueue(b.ctr + 4 * q, b.queue + (size_t)q * b.stride, b.rootOff, b.roots, b.slotCnt[i], i, lane);
-    if (b.strideT > 0)  // the top chunks into the trees' queue
-      seedQueue(b.ctrT + 4 * q, b.queueT + (size_t)q * b.strideT, b.rootOffT, b.rootsT, b.slotCntT[i], i, lane);
+// every queue of model i by warp w of `warps`: the queues (and, with the trees' queue of
+// top chunks beside each, twice as many) in parts, a part per warp
+__device__ inline void seedBackward(const BackwardSeed& b, int i, int lane, int w = 0, int warps = 1) {
+  const int kinds = b.strideT > 0 ? 2 : 1, parts = max(1, warps / (kinds * b.nq));
+  for (int t = w; t < kinds * b.nq * parts; t += warps) {
+    const int part = t % parts, q = t / parts % b.nq;
+    if (t / parts < b.nq)
+      seedQueue(b.ctr + 4 * q, b.queue + (size_t)q * b.stride, b.rootOff, b.roots, b.slotCnt[i], i, lane, part, parts);
+    else
+      seedQueue(b.ctrT + 4 * q, b.queueT + (size_t)q * b.strideT, b.rootOffT, b.rootsT, b.slotCntT[i], i, lane, part,
+                parts);
   }
 }
 
 // One warp per model: lane 0 keeps the books, lanes 0 to 5 take one of the
 // step's six quotients each (an FP64 division is some 560 cycles; one after the
 // other they were most of the launch).
-__global__ void kBeginStep(DevModels m, int* activeCount, long long* activeEl, BackwardSeed bs) {
+// With more than kSeedWarpRoots roots in a model's queues (a chain of 33,333 beams has
+// 1,500 in each of two), sixteen warps per model, the books by the first: one warp's
+// rounds of stores took 28.6 us, these 8.
+constexpr int kSeedWarpRoots = 256, kSeedWarps = 16;
+template <int WARPS>
+__global__ void __launch_bounds__(WARPS > 1 ? 32 * WARPS : 128) kBeginStep(DevModels m, int* activeCount, long long* activeEl, BackwardSeed bs) {
   pdlEntry();
-  const int i = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, w = WARPS > 1 ? threadIdx.x >> 5 : 0;
+  const int i = WARPS > 1 ? blockIdx.x : (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5);
   if (i >= m.n) return;
+  if constexpr (WARPS > 1) {
+    // the model starts a step or goes on with one: the same tests as below, on what
+    // every warp has read before the books are written
+    const bool seeds = m.state[i] == ST_ITER || (m.state[i] == ST_NEED_STEP && m.nStep[i] < m.stepLimit[i] &&
+                       !(m.tStart[i] <= m.tEnd[i] && m.time[i] + 0.1 * m.minInc[i] > m.tEnd[i]));
+    __syncthreads();
+    if (w > 0) {
+      if (seeds) seedBackward(bs, i, lane, w, WARPS);
+      return;
+    }
+  }
   const int st = m.state[i];
   int fl = 0;
   if (st == ST_NEED_STEP) {
@@ -168,7 +193,7 @@ __global__ void kBeginStep(DevModels m, int* activeCount, long long* activeEl, B
     if (lane == 0) m.flags[i] = 0;
     return;
   }
-  seedBackward(bs, i, lane);
+  seedBackward(bs, i, lane, 0, WARPS);
   if (lane != 0) return;
   int it = m.iter[i];
   bool tangent = it < max(1, m.nUpdat[i]) || m.nSeqNoUpd[i] >= m.maxSeq[i];
@@ -1469,10 +1494,17 @@ __global__ void kControl(DevData d, int* tally) {
   double acc = 0.0;
   if (lane < NPART) {
     acc = nc > 0 ? d.partial[(size_t)c0 * NPART + lane] : 0.0;
-    for (int c = 1; c < nc; ++c) {
-      double x = d.partial[(size_t)(c0 + c) * NPART + lane];
-      // maxima (and the NaN flag) as |x| bit patterns: a NaN stays in the norm
-      acc = (lane <= 6) ? acc + x : __longlong_as_double((long long)umax64(absBits(acc), absBits(x)));
+    // sixteen chunks' loads at a time (one by one, 98 chunks took 37 us)
+    for (int c = 1; c < nc; c += 16) {
+      double x[16];
+#pragma unroll
+      for (int u = 0; u < 16; ++u) x[u] = c + u < nc ? d.partial[(size_t)(c0 + c + u) * NPART + lane] : 0.0;
+#pragma unroll
+      for (int u = 0; u < 16; ++u) {
+        if (c + u >= nc) break;
+        // maxima (and the NaN flag) as |x| bit patterns: a NaN stays in the norm
+        acc = (lane <= 6) ? acc + x[u] : __longlong_as_double((long long)umax64(absBits(acc), absBits(x[u])));
+      }
     }
   }
   // lane k forms norm k (0-3 displacement, 4-7 velocity, 8-11 acceleration,
@@ -1739,7 +1771,10 @@ bool wideElements(const DevData& d) { return d.beamSparse && d.nelTot <= kWideEl
 
 void launchBeginStep(const DevData& d, int* activeCount, long long* activeEl, const BackwardSeed& seed,
                      cudaStream_t s) {
-  pdlLaunch(kBeginStep, blocksFor(32LL * d.m.n, 128), 128, 0, s, d.m, activeCount, activeEl, seed);
+  if (seed.maxRoots > kSeedWarpRoots)
+    pdlLaunch(kBeginStep<kSeedWarps>, d.m.n, 32 * kSeedWarps, 0, s, d.m, activeCount, activeEl, seed);
+  else
+    pdlLaunch(kBeginStep<1>, blocksFor(32LL * d.m.n, 128), 128, 0, s, d.m, activeCount, activeEl, seed);
 }
 void launchPredictDofs(const DevData& d, cudaStream_t s) {
   long long n = d.ndofTot > d.neqTot ? d.ndofTot : d.neqTot;

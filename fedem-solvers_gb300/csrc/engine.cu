@@ -1175,6 +1175,8 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
       seed_.ctrT = pplan_.treeCtr;
     }
     seed_.nq = nq;
+    for (int m = 0; m < nm; ++m)
+      seed_.maxRoots = std::max({seed_.maxRoots, rootOff[m + 1] - rootOff[m], treeRootOff[m + 1] - treeRootOff[m]});
     seed_.stride = (int)std::max<size_t>(leaves.size(), 1);
     seed_.rootOff = dRootOff;
     seed_.roots = dRoots;

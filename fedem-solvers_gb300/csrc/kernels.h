@@ -57,6 +57,7 @@ enum ElemMode : int {
 struct BackwardSeed {
   int nq = 0;      // queues (solves per iteration)
   int stride = 0;  // slots per queue
+  int maxRoots = 0;  // largest number of entries a model has in one of the queues
   // per model: the tops of the cascades' subtrees (fronts whose parent is not the
   // cascades', or roots) in roots[rootOff[m]..rootOff[m+1]), and its number
   // of chains
