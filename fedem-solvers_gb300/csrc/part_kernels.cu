@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(kPartThreads) kParts(DevData d, int mode) {
   double* rate = F + 4 * n;  // nd <= n
   double* filt = rate + n;   // nd
   __shared__ int bad;
-  __shared__ double pt[3][3], invT[3];
+  __shared__ double pt[3][3];
   const bool qs = (mode == EM_PRED || mode == EM_INC) && (fl & FL_QSTATIC);
   const bool isStatic = mode == EM_STATIC || mode == EM_STATIC_INIT || qs;
   const bool newPositions = (mode == EM_INC || mode == EM_STATIC || mode == EM_FINAL) && !(qs && (fl & FL_LINEAR));
@@ -161,17 +161,15 @@ __global__ void __launch_bounds__(kPartThreads) kParts(DevData d, int mode) {
   if (bad) return;
   // deformation vector in the corotated axes
   if (newPositions || mode == EM_STATIC_INIT || qs) {
-    // (r, c) of each triad's position in part axes: threads over 12 nt entries; the
-    // frame's inverse is its transpose, its translation column inv[9 + r]
-    if (tid < 3) invT[tid] = -(S[3 * tid] * S[9] + S[3 * tid + 1] * S[10] + S[3 * tid + 2] * S[11]);
-    __syncthreads();
+    // (r, c) of each triad's position in part axes (the frame's inverse is its
+    // transpose): threads over 12 nt entries
     double* loc = F;  // 12 nt values (the force vectors come later)
     for (int q = tid; q < 12 * nt; q += nth) {
       const int t = q / 12, c = (q % 12) / 3, r = q % 3;
       const double* U = d.ur + 12 * (size_t)d.pTri[t0 + t] + 3 * c;
-      double v = S[3 * r] * U[0] + S[3 * r + 1] * U[1] + S[3 * r + 2] * U[2];
-      if (c == 3) v += invT[r];
-      loc[q] = v;
+      double u0 = U[0], u1 = U[1], u2 = U[2];
+      if (c == 3) { u0 -= S[9]; u1 -= S[10]; u2 -= S[11]; }
+      loc[q] = S[3 * r] * u0 + S[3 * r + 1] * u1 + S[3 * r + 2] * u2;
     }
     __syncthreads();
     for (int q = tid; q < 6 * nt; q += nth) {
