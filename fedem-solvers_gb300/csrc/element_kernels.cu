@@ -117,7 +117,7 @@ __device__ inline void seedBackward(const BackwardSeed& b, int i, int lane, int 
 // other they were most of the launch).
 // With more than kSeedWarpRoots roots in a model's queues (a chain of 33,333 beams has
 // 1,500 in each of two), sixteen warps per model, the books by the first: one warp's
-// rounds of stores took 28.6 us, these 8.
+// rounds of stores took 28.6 us, these 10.5.
 constexpr int kSeedWarpRoots = 256, kSeedWarps = 16;
 template <int WARPS>
 __global__ void __launch_bounds__(WARPS > 1 ? 32 * WARPS : 128) kBeginStep(DevModels m, int* activeCount, long long* activeEl, BackwardSeed bs) {
@@ -1371,38 +1371,31 @@ __device__ inline bool isBad(double v) { return !(fabs(v) <= 1.0e300); }
 // types), 20 NaN/Inf seen.
 constexpr int NPART = 21;
 constexpr int CHUNK_TPB = 256;
+constexpr int kNormWarps = CHUNK_TPB / 32;
 // at most so many chunks as clusters of one-warp blocks (a chain of 3,827 beams, 12
 // chunks: 15.9 us a launch with 8-warp blocks; with 98 chunks, 784 warps for 608
 // sub-cores, the pass and its neighbours lost 6 us)
 constexpr int kWideNormChunks = 48;
 
-// |x| as a bit pattern: for non-negative doubles the order of the patterns is
-// the numeric order (NaN patterns are above infinity), so the maxima and the
-// finiteness test run on the integer pipe and leave the FP64 pipe to the sums
-__device__ inline unsigned long long absBits(double x) {
-  return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
+// the larger pattern, by 32-bit subtractions with borrow
+__device__ inline unsigned long long umax64(unsigned long long a, unsigned long long b) {
+  const unsigned al = (unsigned)a, ah = (unsigned)(a >> 32), bl = (unsigned)b, bh = (unsigned)(b >> 32);
+  unsigned less;  // all ones where b < a
+  asm("{\n\t.reg .u32 t;\n\tsub.cc.u32 t, %1, %2;\n\tsubc.cc.u32 t, %3, %4;\n\tsubc.u32 %0, 0, 0;\n\t}"
+      : "=r"(less) : "r"(bl), "r"(al), "r"(bh), "r"(ah));
+  const unsigned lo = less ? al : bl, hi = less ? ah : bh;
+  return (unsigned long long)hi << 32 | lo;
 }
-__device__ inline unsigned long long umax64(unsigned long long a, unsigned long long b) { return a > b ? a : b; }
 
-// A chunk by a block of 8 warps or, with few chunks, by a cluster of 8 one-warp
-// blocks (WIDE): a warp's sums then have a sub-core's FP64 pipe to themselves
-// instead of sharing it with another. Each warp takes the same DOFs in the same
-// order either way, and the warps are combined in order: the same bits.
-template <bool WIDE>
-__global__ void __launch_bounds__(WIDE ? 32 : CHUNK_TPB) kNormsPartial(DevData d) {
-  pdlEntry();
-  __shared__ double sh[WIDE ? 1 : CHUNK_TPB / 32][NPART];
-  constexpr int kWarps = CHUNK_TPB / 32;
-  const int c = WIDE ? blockIdx.x / kWarps : blockIdx.x;
-  const int w = WIDE ? blockIdx.x % kWarps : threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m = d.chunkModel[c];
-  if (!(d.m.flags[m] & FL_ACTIVE)) return;  // (the same for a whole cluster)
+// warp w's share of the partial values of chunk c: sums 2-6 (increment, velocity and
+// acceleration increments, residual, energy), maxima 7-19 as bit patterns, 20 the
+// NaN/infinity flag; written to o by lane 0
+__device__ inline void normsWarp(const DevData& d, int m, int c, int w, int lane, double* o) {
   const double* wD = d.m.wDisp + 3 * m;
   const double* wF = d.m.wForce + 3 * m;
-  const unsigned long long badBits = absBits(1.0e300);
-  const bool unit = isOne(wD[0]) && isOne(wD[1]) && isOne(wD[2]) && isOne(wF[0]) && isOne(wF[1]) && isOne(wF[2]);
-  // sums: 2-4 disp/vel/acc, 5 residual, 6 energy; maxima as bit patterns:
-  // mx[0] energy, mx[1 + 3 q + t] vector q of DOF type t; (the weight sums
+  constexpr int kStride = CHUNK_TPB;
+  const unsigned long long badBits = 0x7e37e43c8800759cull;  // 1e300
+  // maxima: mx[0] energy, mx[1 + 3 q + t] vector q of DOF type t; (the weight sums
   // 0 and 1 are per-model constants)
   double v2 = 0.0, v3 = 0.0, v4 = 0.0, v5 = 0.0, v6 = 0.0;
   unsigned long long mx[13];
@@ -1410,13 +1403,13 @@ __global__ void __launch_bounds__(WIDE ? 32 : CHUNK_TPB) kNormsPartial(DevData d
   for (int k = 0; k < 13; ++k) mx[k] = 0ull;
   bool bad = false;
   const int cEnd = d.chunkEnd[c];
-  for (int i0 = d.chunkStart[c] + 32 * w + lane; i0 < cEnd; i0 += 4 * CHUNK_TPB) {
+  for (int i0 = d.chunkStart[c] + 32 * w + lane; i0 < cEnd; i0 += 4 * kStride) {
     // four DOFs per pass: all loads issued before the ordered accumulation
     int eqs[4], ts[4];
     double a0[4], a1[4], a2[4], rr[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const int i = i0 + u * CHUNK_TPB;
+      const int i = i0 + u * kStride;
       eqs[u] = i < cEnd ? d.meqn[i] : -1;
       ts[u] = i < cEnd ? d.dofType[i] - 1 : 0;
       a0[u] = i < cEnd ? d.sinc0[i] : 0.0;
@@ -1432,18 +1425,11 @@ __global__ void __launch_bounds__(WIDE ? 32 : CHUNK_TPB) kNormsPartial(DevData d
       const double s0 = a0[u], s1 = a1[u], s2 = a2[u], r = rr[u];
       const unsigned long long b0 = absBits(s0), b1 = absBits(s1), b2 = absBits(s2), br = absBits(r);
       bad |= b0 > badBits || br > badBits;
-      if (unit) {  // weights of one (the default): four of ten FP64 instructions less, the same values
-        v2 += s0 * s0;
-        v3 += s1 * s1;
-        v4 += s2 * s2;
-        v5 += r * r;
-      } else {
-        const double wd = wD[t], wf = wF[t];
-        v2 += (wd * s0) * (wd * s0);
-        v3 += (wd * s1) * (wd * s1);
-        v4 += (wd * s2) * (wd * s2);
-        v5 += (wf * r) * (wf * r);
-      }
+      const double wd = wD[t], wf = wF[t];
+      v2 += (wd * s0) * (wd * s0);
+      v3 += (wd * s1) * (wd * s1);
+      v4 += (wd * s2) * (wd * s2);
+      v5 += (wf * r) * (wf * r);
       const double en = fabs(s0 * r);
       v6 += en;
       mx[0] = umax64(mx[0], absBits(en));
@@ -1470,7 +1456,6 @@ __global__ void __launch_bounds__(WIDE ? 32 : CHUNK_TPB) kNormsPartial(DevData d
   }
   bad = __any_sync(0xffffffffu, bad);
   if (lane == 0) {
-    double* o = sh[WIDE ? 0 : w];
     o[0] = 0.0;
     o[1] = 0.0;
     o[2] = v2;
@@ -1482,6 +1467,28 @@ __global__ void __launch_bounds__(WIDE ? 32 : CHUNK_TPB) kNormsPartial(DevData d
     for (int k = 0; k < 13; ++k) o[7 + k] = __longlong_as_double((long long)mx[k]);
     o[20] = bad ? 1.0 : 0.0;
   }
+}
+// partial value k of a chunk from those of two sets of its warps, or of two chunks
+// (maxima, and the NaN flag, as |x| bit patterns: a NaN stays in the norm)
+__device__ __forceinline__ double combineNorm(int k, double x, double y) {
+  const long long sum = __double_as_longlong(x + y), top = (long long)umax64(absBits(x), absBits(y));
+  return __longlong_as_double(k <= 6 ? sum : top);
+}
+
+// A chunk by a block of 8 warps or, with few chunks, by a cluster of 8 one-warp
+// blocks (WIDE): a warp's sums then have a sub-core's FP64 pipe to themselves
+// instead of sharing it with another. Each warp takes the same DOFs in the same
+// order either way, and the warps are combined in order: the same bits.
+template <bool WIDE>
+__global__ void __launch_bounds__(WIDE ? 32 : CHUNK_TPB) kNormsPartial(DevData d) {
+  pdlEntry();
+  __shared__ double sh[WIDE ? 1 : kNormWarps][NPART];
+  constexpr int kWarps = kNormWarps;
+  const int c = WIDE ? blockIdx.x / kWarps : blockIdx.x;
+  const int w = WIDE ? blockIdx.x % kWarps : threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int m = d.chunkModel[c];
+  if (!(d.m.flags[m] & FL_ACTIVE)) return;  // (the same for a whole cluster)
+  normsWarp(d, m, c, w, lane, sh[WIDE ? 0 : w]);
   if constexpr (WIDE) cooperative_groups::this_cluster().sync();
   else __syncthreads();
   if (threadIdx.x < NPART && (!WIDE || w == 0)) {
@@ -1494,8 +1501,7 @@ __global__ void __launch_bounds__(WIDE ? 32 : CHUNK_TPB) kNormsPartial(DevData d
     }
     double x = y[0];
 #pragma unroll
-    for (int ww = 1; ww < kWarps; ++ww)
-      x = (k <= 6) ? x + y[ww] : __longlong_as_double((long long)umax64(absBits(x), absBits(y[ww])));
+    for (int ww = 1; ww < kWarps; ++ww) x = combineNorm(k, x, y[ww]);
     d.partial[(size_t)c * NPART + k] = x;
   }
   // the other blocks' shared memory stays until it has been read
@@ -1517,16 +1523,15 @@ __global__ void kControl(DevData d, int* tally) {
   double acc = 0.0;
   if (lane < NPART) {
     acc = nc > 0 ? d.partial[(size_t)c0 * NPART + lane] : 0.0;
-    // sixteen chunks' loads at a time (one by one, 98 chunks took 37 us)
+    // sixteen chunks' loads at a time (98 chunks: 37 us one by one, 20.5 so)
     for (int c = 1; c < nc; c += 16) {
       double x[16];
 #pragma unroll
-      for (int u = 0; u < 16; ++u) x[u] = c + u < nc ? d.partial[(size_t)(c0 + c + u) * NPART + lane] : 0.0;
+      for (int u = 0; u < 16; ++u) x[u] = d.partial[(size_t)(c0 + min(c + u, nc - 1)) * NPART + lane];
 #pragma unroll
       for (int u = 0; u < 16; ++u) {
-        if (c + u >= nc) break;
-        // maxima (and the NaN flag) as |x| bit patterns: a NaN stays in the norm
-        acc = (lane <= 6) ? acc + x[u] : __longlong_as_double((long long)umax64(absBits(acc), absBits(x[u])));
+        const double y = combineNorm(lane, acc, x[u]);
+        if (c + u < nc) acc = y;
       }
     }
   }

@@ -34,6 +34,7 @@
 #include <string>
 
 #include "kernels.h"
+#include "pivot.cuh"
 
 namespace fgpu {
 namespace {
@@ -52,12 +53,8 @@ static __device__ __align__(256) unsigned char g_normScratch[kScratchBytes];
 std::mutex g_setupMutex;
 void* g_scratchPtr[kMaxDevices] = {};
 
-// |x| as a bit pattern: for non-negative doubles the order of the patterns is
-// the numeric order and NaN patterns lie above infinity, so a NaN anywhere
-// shows in the maxima exactly as in the batch's own pass
-__device__ inline unsigned long long absBits(double x) {
-  return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
-}
+// (maxima compared as |x| bit patterns: a NaN anywhere shows in them exactly as in the
+// batch's own pass)
 __device__ inline unsigned long long umax64(unsigned long long a, unsigned long long b) { return a > b ? a : b; }
 
 // one block per chunk of the model; the block that completes the count

@@ -26,17 +26,26 @@ __device__ inline double quotient(double v, double d) {
   const double r = recip(d), q = v * r;
   return fma(fma(-d, q, v), r, q);
 }
-// tests on the bit patterns of |x| (the order of non-negative patterns is the
-// numeric order): they keep the FP64 pipe, one instruction per 64 cycles, free
+// |x| as a bit pattern: for non-negative doubles the order of the patterns is the
+// numeric order (NaN patterns are above infinity), so maxima and tests on it keep the
+// FP64 pipe, one instruction per 64 cycles, free.  The sign is cleared on the high
+// half: an AND on the 64-bit pattern is compiled into a floating-point absolute
+// value, an FP64 instruction again.
+__device__ __forceinline__ unsigned long long absBits(double x) {
+  unsigned long long b;
+  asm("{\n\t.reg .b32 lo, hi;\n\tmov.b64 {lo, hi}, %1;\n\tand.b32 hi, hi, 0x7fffffff;\n\tmov.b64 %0, {lo, hi};\n\t}"
+      : "=l"(b) : "d"(x));
+  return b;
+}
+constexpr unsigned long long kInfBits = 0x7ff0000000000000ull;
 __device__ inline bool absGreater(double a, double b) {
-  const long long m = 0x7fffffffffffffffll;
-  const long long x = __double_as_longlong(a) & m, y = __double_as_longlong(b) & m;
-  return x > y && x <= 0x7ff0000000000000ll;
+  const unsigned long long x = absBits(a), y = absBits(b);
+  return x > y && x <= kInfBits;
 }
 __device__ inline bool absGreater(float a, float b) { return fabsf(a) > fabsf(b); }
 __device__ inline bool negative(double a) {
-  const long long b = __double_as_longlong(a), m = b & 0x7fffffffffffffffll;
-  return b < 0 && m != 0 && m <= 0x7ff0000000000000ll;
+  const unsigned long long m = absBits(a);
+  return __double2hiint(a) < 0 && m != 0 && m <= kInfBits;
 }
 __device__ inline bool negative(float a) { return a < 0.0f; }
 // the bound |d_k| must exceed for pivot k to count as regular
