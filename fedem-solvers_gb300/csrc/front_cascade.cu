@@ -63,10 +63,10 @@ __device__ void panelShuffle(T* F, const T* diag0, int nr, int np, int lane, int
     const bool bad = !absGreater(dk, diag0[k]);
     sing |= bad;
     if (negative(dk)) ++neg;
-    const T inv = bad ? T(0) : recip(dk);
+    const typename PivotScaleOf<T>::type scale(dk, bad);
     const bool r0 = i0 > k && i0 < nr, r1 = i1 > k && i1 < nr;
     const T f0 = r0 ? F[i0 + nr * k] : T(0), f1 = r1 ? F[i1 + nr * k] : T(0);
-    const T l0 = f0 * inv, l1 = f1 * inv;
+    const T l0 = scale(f0), l1 = nr > 32 ? scale(f1) : T(0);
     for (int j = k + 1; j < np; ++j) {
       const T lj = __shfl_sync(0xffffffffu, l0, j);
       if (r0 && j <= i0) F[i0 + nr * j] -= f0 * lj;
@@ -119,10 +119,10 @@ __device__ void panelRegisters(T* F, const T* diag0, int nr, int np, int lane, i
       const bool bad = !absGreater(dk, diag0[k]);
       sing |= bad;
       if (negative(dk)) ++neg;
-      const T inv = bad ? T(0) : recip(dk);
+      const typename PivotScaleOf<T>::type scale(dk, bad);
       const bool r0 = i0 > k && i0 < nr;
       const T f0 = r0 ? a0[kk] : T(0), f1 = h1 ? a1[kk] : T(0);
-      const T l0 = f0 * inv, l1 = f1 * inv;
+      const T l0 = scale(f0), l1 = two ? scale(f1) : T(0);
 #pragma unroll
       for (int jj = kk + 1; jj < PB; ++jj) {
         if (jj >= kb) break;
@@ -204,13 +204,23 @@ __device__ void factorBlocked(T* F, T* lcol, const T* diag0, int nr, int np, int
   while (b < nu && t >= nu - b) { t -= nu - b; ++b; }
   for (int e = lane; b < nu; e += 32) {
     const int i = np + b + t, j = np + b;
-    T acc = T(0);
-    for (int k = 0; k < np; ++k) acc += F[k + nr * i] * F[j + nr * k];
-    Uout[e] = F[i + nr * j] - acc;
+    T v = F[i + nr * j];
+    for (int k = 0; k < np; ++k) v -= F[k + nr * i] * F[j + nr * k];
+    Uout[e] = v;
     t += 32;
     while (b < nu && t >= nu - b) { t -= nu - b; ++b; }
   }
   __syncwarp();
+}
+
+// one entry per lane of child c's update matrix (pos: child << 20 | position, or -1).
+// FP64: not at all when no lane's entry is of this child -- the addition would take the
+// pipe for 64 cycles with no lane active
+template <typename T>
+__device__ __forceinline__ void extendAdd(T* F, int pos, int c, T val) {
+  const bool on = pos >= 0 && (pos >> 20) == c;
+  if (sizeof(T) == 8 && !__any_sync(0xffffffffu, on)) return;
+  if (on) F[pos & 0xfffff] += val;
 }
 
 // partial LDL^T of front f in shared memory (F: maxRow^2, lcol/diag0: maxRow).
@@ -258,8 +268,7 @@ __device__ void factorOneFront(const DevData& d, int f, T* F, T* lcol, T* diag0,
     }
     for (int c = 0; c < nch; ++c) {
 #pragma unroll
-      for (int u = 0; u < kFrontBatch; ++u)
-        if (pc[u] >= 0 && (pc[u] >> 20) == c) F[pc[u] & 0xfffff] += val[u];
+      for (int u = 0; u < kFrontBatch; ++u) extendAdd(F, pc[u], c, val[u]);
       __syncwarp();
     }
   }
@@ -385,11 +394,18 @@ __device__ void forwardRun(const SolveDesc& q, const int* row, const int* dst, c
   // the elimination with the rows in registers (lane r: rows r and r + 32), the
   // pivot value of each step passed by a shuffle: no barrier between steps
   T v0 = lane < nr ? v[lane] : T(0), v1 = lane + 32 < nr ? v[lane + 32] : T(0);
-  for (int k = 0; k < np; ++k) {
-    const T yk = __shfl_sync(0xffffffffu, k < 32 ? v0 : v1, k & 31);
-    const T* Lk = L + (size_t)nr * k;
-    if (lane > k && lane < nr) v0 -= Lk[lane] * yk;
-    if (lane + 32 > k && lane + 32 < nr) v1 -= Lk[lane + 32] * yk;
+  if (nr <= 32) {
+    for (int k = 0; k < np; ++k) {
+      const T yk = __shfl_sync(0xffffffffu, v0, k);
+      if (lane > k && lane < nr) v0 -= L[lane + (size_t)nr * k] * yk;
+    }
+  } else {
+    for (int k = 0; k < np; ++k) {
+      const T yk = __shfl_sync(0xffffffffu, k < 32 ? v0 : v1, k & 31);
+      const T* Lk = L + (size_t)nr * k;
+      if (lane > k && lane < nr) v0 -= Lk[lane] * yk;
+      if (lane + 32 > k && lane + 32 < nr) v1 -= Lk[lane + 32] * yk;
+    }
   }
   if (lane >= np && lane < nr) Wout[lane - np] = v0;
   if (lane + 32 >= np && lane + 32 < nr) Wout[lane + 32 - np] = v1;
@@ -637,12 +653,16 @@ __device__ void backwardSolve(const DevData& d, const int* rows, int nr, int np,
                               bool finalize, int lane) {
   if (np <= 32) {
     // one pivot per lane in a register; the back substitution passes each
-    // solved value by a shuffle (no barrier between steps)
-    T a = T(0);
-    if (lane < np) {
-      a = xs[lane];
-      for (int i = np; i < nr; ++i) a -= L[i + (size_t)nr * lane] * xs[i];
-    }
+    // solved value by a shuffle (no barrier between steps).  The update rows' share
+    // is split over 4 groups of 8 lanes (up to 8 pivots) or 2 of 16: a front of 6
+    // pivots and 12 update rows takes 3 multiply-subtracts and 2 additions one after
+    // the other in place of 12
+    const int width = np <= 8 ? 8 : np <= 16 ? 16 : 32;
+    const int p = lane & (width - 1);
+    T a = lane < np ? xs[lane] : T(0);
+    if (p < np)
+      for (int i = np + lane / width; i < nr; i += 32 / width) a -= L[i + (size_t)nr * p] * xs[i];
+    for (int o = width; o < 32; o <<= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
     for (int j = np - 1; j > 0; --j) {
       const T xj = __shfl_sync(0xffffffffu, a, j);
       if (lane < j) a -= L[j + (size_t)nr * lane] * xj;
@@ -927,7 +947,7 @@ __global__ void __launch_bounds__(512, 1) kTree(DevData d, TreePlan tp, int maxR
               for (int c1 = 0; c1 < q.nch; ++c1) {
 #pragma unroll
                 for (int u = 0; u < kSeg; ++u)
-                  if (sp[u] >= 0 && (sp[u] >> 20) == c1) F[sp[u] & 0xfffff] += sv[u];
+                  extendAdd(F, sp[u], c1, sv[u]);
                 __syncwarp();
               }
               for (int k0 = 32 * kSeg; k0 < ns; k0 += 32 * kFrontBatch) {
@@ -942,7 +962,7 @@ __global__ void __launch_bounds__(512, 1) kTree(DevData d, TreePlan tp, int maxR
                 for (int c1 = 0; c1 < q.nch; ++c1) {
 #pragma unroll
                   for (int u = 0; u < kFrontBatch; ++u)
-                    if (pc[u] >= 0 && (pc[u] >> 20) == c1) F[pc[u] & 0xfffff] += val[u];
+                    extendAdd(F, pc[u], c1, val[u]);
                   __syncwarp();
                 }
               }

@@ -20,6 +20,36 @@ __device__ inline double recip(double d) {
   const double t = fma(e, e, e);
   return fma(r, t, r);
 }
+// f / d for the multipliers of a pivot (0 when bad), as f r (1 + e + e^2) with the
+// product f r beside the reciprocal's own Newton step: one multiply-add less on the
+// pivot's critical chain than through recip(d)
+struct PivotScale32 {
+  float inv;
+  __device__ PivotScale32(float d, bool bad) : inv(bad ? 0.0f : recip(d)) {}
+  __device__ float operator()(float f) const { return f * inv; }
+};
+struct PivotScale64 {
+  double r, t;
+  __device__ PivotScale64(double d, bool bad) {
+    const unsigned ex = ((unsigned)__double2hiint(d) >> 20) & 0x7ffu;
+    if (bad) {
+      r = t = 0.0;
+    } else if (ex - 64u > 1918u) {
+      r = 1.0 / d;
+      t = 0.0;
+    } else {
+      asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+      const double e = fma(-d, r, 1.0);
+      t = fma(e, e, e);
+    }
+  }
+  __device__ double operator()(double f) const {
+    const double q = f * r;
+    return fma(q, t, q);
+  }
+};
+template <typename T> struct PivotScaleOf { using type = PivotScale32; };
+template <> struct PivotScaleOf<double> { using type = PivotScale64; };
 // v / d: the product with the reciprocal and one correction by its remainder
 __device__ inline float quotient(float v, float d) { return v / d; }
 __device__ inline double quotient(double v, double d) {
