@@ -863,6 +863,9 @@ __global__ void kAxialNewton(DevData d) {
     }
 }
 
+__device__ __forceinline__ double turned(double x, bool neg) {
+  return __hiloint2double(__double2hiint(x) ^ (neg ? (int)0x80000000 : 0), __double2loint(x));
+}
 // residual: force predictor (7.53) or corrector (7.55); RHS del = residual
 __global__ void kResidual(DevData d) {
   pdlEntry();
@@ -927,10 +930,8 @@ __global__ void kResidual(DevData d) {
   double a = d.m.alpha[m], sstif = a + 1.0, r;
   if (fl & FL_QSTATIC)  // staticEquilibriumModule.f90 (staticInt): Q alone in a pure linear step
     r = ((fl & FL_LINEAR) && (fl & FL_PRED)) ? q : q - fs;
-  else if (fl & FL_PRED)
-    r = sstif * (q - fs + fd) + fi - a * d.FIact[i];
-  else
-    r = sstif * (q - fs - fd) - fi - a * d.FIact[i];
+  else  // (the predictor's signs turned on the bit patterns: one set of FP64 instructions)
+    r = sstif * (q - fs - turned(fd, fl & FL_PRED)) - turned(fi, fl & FL_PRED) - a * d.FIact[i];
   d.res[i] = r;
   d.del[i] = r;
 }
