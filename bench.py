@@ -486,7 +486,7 @@ def single_model_leg(fsi, opts, steps, desc, pending=None):
             achieved = flops / (f_ms * 1e-3) / 1e12
             leg["roofline_factor"] = {"bound": "fp64", "achieved": achieved, "peak": peak_tf, "unit": "TFLOP/s",
                                       "frac": achieved / peak_tf, "traffic": None,
-                                      "kernel": "kFactorForwardCascade<double> (+ kLargeFactorForward<double>)",
+                                      "kernel": "kFactorForwardCascade<double> (+ kLargeFactor<double>)",
                                       "timing": "10 launches after the run, CUDA events on the engine stream"}
         else:
             leg["factor_gflops"] = flops / (f_ms * 1e-3) / 1e9
@@ -497,7 +497,7 @@ def single_model_leg(fsi, opts, steps, desc, pending=None):
             leg["roofline_factor"] = {"bound": "tensor", "achieved": achieved, "peak": eff, "unit": "TFLOP/s",
                                       "frac": achieved / eff, "traffic": None,
                                       "peak_definition": "measured mma.sync TF32 rate / 3 (3xTF32 split)",
-                                      "kernel": "kFactorForwardCascade<float> (+ kLargeFactorForward<float>)",
+                                      "kernel": "kFactorForwardCascade<float> (+ kLargeFactor<float>)",
                                       "timing": "10 launches after the run, CUDA events on the engine stream"}
         out[key] = leg
         b.close()

@@ -1553,9 +1553,9 @@ int Engine::timeFactor(int reps, double* msPerLaunch, double* bytes) {
 // ---- autotuner ------------------------------------------------------------
 // Launch shapes are timed on the batch's own fronts before its first batched
 // iteration and the fastest kept.  Only shapes that give the same results to
-// the last bit are candidates (panel variant, warps per block, cluster size),
+// the last bit are candidates (panel variant, warps per block, large fronts' SMs),
 // so the choice -- which depends on timing -- never changes a result.  Front
-// bucketing (which fronts go to warps, which to clusters) changes the
+// bucketing (which fronts go to warps, which to whole-GPU waves) changes the
 // arithmetic and is therefore fixed (kLargeFrontRows), not tuned.
 // The probe runs while no model has started a step: the factors and solve
 // vectors it overwrites are scratch until the first iteration's

@@ -150,7 +150,7 @@ class Engine {
   int probeRootWaitTimeout(long long spins, int* flag);
 
   // Launch shapes of the multifrontal kernels (PersistentPlan: factor panel
-  // variant, forward and backward warps per block, large-front cluster size).
+  // variant, forward and backward warps per block, large fronts' share of the SMs).
   // Before the first batched iteration the autotuner times the candidates on
   // this batch's own fronts and keeps the fastest; shapes already tuned for a
   // batch of the same structure are reused.  setLaunchShape (before the first

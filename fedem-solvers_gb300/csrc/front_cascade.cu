@@ -11,6 +11,8 @@
 // be filled, by warps that are running and never wait themselves, so the wait
 // ends whatever the residency.  Each wait is still bounded and sets errFlag
 // when it runs out.
+// Batches of up to 32,768 leaf fronts pay the cascades' latency per tree level, not
+// their work; there whole subtrees go to thread blocks, a warp per front (kTree).
 // The forward and backward solves stage each front's L block in shared memory
 // first (one burst of loads instead of one load latency per pivot).
 //

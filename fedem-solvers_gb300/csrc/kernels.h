@@ -232,7 +232,7 @@ struct PersistentPlan {
   int *cntTree = nullptr, *treeQueue = nullptr, *treeCtr = nullptr;
   // Launch shapes, picked per batch by the engine's autotuner.  No choice
   // changes a result bit: tasks are taken dynamically, and each front's
-  // arithmetic is the same whichever warp, block or cluster does it.
+  // arithmetic is the same whichever warp or block does it.
   int factorPanel = 0;     // small-front panel factorisation: 0 shuffles, 1 register-blocked
                            // (blocks of 8), 2 register-blocked (blocks of 4, fronts up to 32 rows)
   int forwardWarps = 8;    // warps per block of the forward-elimination cascade

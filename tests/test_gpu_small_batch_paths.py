@@ -1,13 +1,14 @@
 """Small batches take kernels of their own: four lanes per beam element in the
-element pass and the Newton matrices, clusters of one-warp blocks in the norms,
-and the assembly trees on thread blocks (up to 8,192 elements, 48 norm chunks
-and 8,192 leaf fronts; up to 32,768 leaf fronts the trees' upper levels only).  They perform the operations of the large batches'
-kernels in the same order, so a model alone and the same model beside two long
-chains (the trees' upper levels) or six (the cascades alone), which put the batch
-above the other lines, must agree to the last bit
-(tolerance zero): chains from a single beam (one front) over the sizes around the
-chunks' tiers, and a gravity-loaded pendulum with a joint (kept frames, gravity
-forces, constraint expansion)."""
+element pass and the Newton matrices (up to 8,192 elements), clusters of one-warp
+blocks in the norms (up to 48 chunks), four lanes per joint, and the assembly trees on
+thread blocks (up to 8,192 leaf fronts; up to 32,768 the trees' upper levels only,
+their many backward roots seeded by sixteen warps).  They perform the operations of
+the large batches' kernels in the same order, so a model alone and the same model
+beside two long chains (the trees' upper levels) or six (the cascades alone), which
+put the batch above the other lines, must agree to the last bit (tolerance zero):
+chains from a single beam (one front) over the sizes around the chunks' tiers, and a
+gravity-loaded pendulum with a joint (kept frames, gravity forces, constraint
+expansion)."""
 import numpy as np
 import pytest
 
