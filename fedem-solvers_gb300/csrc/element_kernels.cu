@@ -1596,11 +1596,15 @@ __global__ void kControl(DevData d, int* tally) {
     d.m.flags[m] = fl | FL_STEPDONE;
     if (starts(n, d.m.time[m])) {
       atomicAdd(tally, 1);
+      const int k = kIterationsAhead - 1;
       if (starts(n + 1, d.m.time[m] + d.m.dt[m])) atomicAdd(tally + 1, 1);
+      if (starts(n + k, d.m.time[m] + k * d.m.dt[m])) atomicAdd(tally + 3, 1);
     }
   } else if (d.m.state[m] == ST_ITER) {
     atomicAdd(tally, 1);
+    const int k = kIterationsAhead - 1;
     if (starts(d.m.nStep[m] + 1, d.m.time[m])) atomicAdd(tally + 1, 1);
+    if (starts(d.m.nStep[m] + k, d.m.time[m] + (k - 1) * d.m.dt[m])) atomicAdd(tally + 3, 1);
   }
 }
 
@@ -1617,18 +1621,20 @@ __global__ void kStepEnd(DevData d, IterationEnd e) {
   for (long long k = kept + t; k < e.ctrInts; k += nt) e.ctr[k] = 0;
   for (long long k = t; k < e.queueInts; k += nt) e.queue[k] = -1;
   if (t == 0 && e.tally) {
-    const int active = *e.active, remaining = e.tally[0], more = e.tally[1];
+    const int active = *e.active, remaining = e.tally[0], more = e.tally[1], far = e.tally[3];
     const long long elements = *e.elements;
     for (int k = 0; k < kept; ++k) e.ctr[k] = 0;
     e.tally[0] = 0;
     e.tally[1] = 0;
     e.tally[2] = active;
+    e.tally[3] = 0;
     const long long serial = ++*reinterpret_cast<long long*>(e.tally + 4);
-    volatile IterationReport* h = e.host;
+    volatile IterationReport* h = e.host + serial % kReports;
     h->elements = elements;
     h->active = active;
     h->remaining = remaining;
     h->more = more;
+    h->far = far;
     __threadfence_system();
     h->serial = serial;
   }

@@ -1343,8 +1343,8 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
   if (allocFailed_) { err = "out of device memory"; return -906; }
   FG_CHECK(cudaMallocHost(&hActive_, sizeof(int)));
   FG_CHECK(cudaMallocHost(&hStates_, sizeof(int) * (size_t)std::max(nm, 1)));
-  FG_CHECK(cudaMallocHost(&hReport_, sizeof(IterationReport)));
-  *hReport_ = IterationReport{};
+  FG_CHECK(cudaMallocHost(&hReport_, kReports * sizeof(IterationReport)));
+  std::fill_n(hReport_, kReports, IterationReport{});
   end_.ctr = ctrBlock_;
   end_.ctrInts = (int)ctrInts_;
   end_.queue = pplan_.bwQueue;
@@ -2347,13 +2347,12 @@ int Engine::launchIteration(bool timed) {
 // Waits for the step end's report of iteration `serial` (false: the stream
 // failed or drained without it).
 bool Engine::waitReport(long long serial) {
-  const volatile IterationReport* h = hReport_;
+  const volatile IterationReport* h = hReport_ + serial % kReports;
   for (int spins = 0; h->serial < serial; ++spins) {
     if ((spins & 1023) != 1023) continue;
     const cudaError_t q = cudaStreamQuery(stream_);
     if (q == cudaSuccess) return h->serial >= serial;
     if (q != cudaErrorNotReady) return false;
-    std::this_thread::yield();
   }
   std::atomic_thread_fence(std::memory_order_acquire);
   return true;
@@ -2377,16 +2376,20 @@ void Engine::samplePhases(long long elements, int active) {
   ++phaseSamples_;
 }
 
-// The iterations are launched one ahead of the device: the step end of each
-// reports (IterationReport) how many models go on, so the host needs no copy and
-// no synchronisation between them, and none is launched that would find nothing
-// to do, as long as some model is known to start another step.  While every
-// remaining model is in its last step, an iteration is launched only when the
-// one before asks for it.  (Seven at a time, with a synchronisation after each
+// The iterations are launched ahead of the device: the step end of each reports
+// (IterationReport) how many models go on, so the host needs no copy and no
+// synchronisation between them, and none is launched that would find nothing to
+// do.  While some model has kIterationsAhead - 1 further steps or more (an
+// iteration each at least), so many are in flight: a host thread that loses its
+// core for a scheduler tick of 4 ms does not leave the GPU idle (one ahead, a run of 16
+// parts beside spinning BLAS threads took 58 ms for 15).  With fewer steps left it is
+// one ahead, and while every remaining model is in its last step an iteration is
+// launched only when the one before asks for it.  (Seven at a time, with a synchronisation after each
 // seven, ran up to six idle iterations at the end: the 20-beam cantilever driven
 // step by step took 0.59 ms a step for two iterations of 0.13 ms.)  Every
 // seventh iteration is timed: an odd distance, so that with two iterations per
-// step predictors and correctors are both sampled.
+// step predictors and correctors are both sampled, and farther apart than
+// kIterationsAhead, so that its events are read before the next records them.
 int Engine::run(long long maxBatched, RunStats* stats) {
   ensureTuned();
   int rc = graphReady(false);
@@ -2399,9 +2402,10 @@ int Engine::run(long long maxBatched, RunStats* stats) {
   cudaEventRecord(evRun_[0], stream_);
   resetIterationCounters(stream_);
   cudaMemsetAsync(end_.tally, 0, sizeof(int) * 6, stream_);
-  *hReport_ = IterationReport{};
+  std::fill_n(hReport_, kReports, IterationReport{});
   const int every = 7;
   long long launched = 0, seen = 0, done = 0;
+  int remaining = 0;
   // the first two at once: a step takes at least two iterations, but for linear
   // quasi-static and fixed-iteration ones
   long long ahead = 2;
@@ -2411,11 +2415,10 @@ int Engine::run(long long maxBatched, RunStats* stats) {
       if (rc) return rc;
     }
     if (!waitReport(seen + 1)) return -922;
-    // (a later iteration may have reported meanwhile)
-    seen = hReport_->serial;
-    const int remaining = hReport_->remaining, more = hReport_->more, active = hReport_->active;
-    if (active > 0) done = seen;
-    if (seen % every == 0) samplePhases(hReport_->elements, active);
+    const IterationReport r = hReport_[++seen % kReports];
+    remaining = r.remaining;
+    if (r.active > 0) done = seen;
+    if (seen % every == 0) samplePhases(r.elements, r.active);
     if (rec_.on && seen % every == 0) {
       // records are drained before a model's ring can fill: nothing runs meanwhile
       if (cudaStreamSynchronize(stream_) != cudaSuccess) return -922;
@@ -2423,11 +2426,12 @@ int Engine::run(long long maxBatched, RunStats* stats) {
       if (resultsDrain(err)) return -924;
     }
     if (remaining == 0) break;
-    ahead = seen + (more > 0 && !(rec_.on && (seen + 1) % every == 0) ? 2 : 1);
+    ahead = seen + (r.far > 0 ? kIterationsAhead : r.more > 0 ? 2 : 1);
+    if (rec_.on) ahead = std::min(ahead, (seen / every + 1) * every);
   }
   // the models that reached their end leave the active set (kBeginStep's
   // bookkeeping, which an iteration without work would do)
-  if (seen > 0 && hReport_->remaining == 0) {
+  if (seen > 0 && remaining == 0) {
     resetIterationCounters(stream_);
     launchBeginStep(d_, dActive_, dActiveEl_, seed_, stream_);
   }

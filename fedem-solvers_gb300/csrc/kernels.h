@@ -79,12 +79,16 @@ struct BackwardSeed {
 // counters and backward queues reset for the next one (in place of memset nodes),
 // and a report into host memory, its serial number last, that the host can follow
 // without a copy or a synchronisation.
+constexpr int kIterationsAhead = 6;
+// reports in turn, more than iterations in flight: one is not overwritten while it is read
+constexpr int kReports = 8;
 struct IterationReport {
   long long serial;    // iterations finished since the counters' last reset by the host
   long long elements;  // elements of the models that took part
   int active;          // models that took part
   int remaining;       // models with another iteration to do
   int more;            // of them, models with a further step after the one they are in (or about to start)
+  int far;             // of them, models with kIterationsAhead - 1 further steps or more
 };
 struct IterationEnd {
   int* ctr = nullptr;  // counters to zero
@@ -94,8 +98,8 @@ struct IterationEnd {
   const int* active = nullptr;          // (inside ctr)
   const long long* elements = nullptr;  // (inside ctr)
   int* tally = nullptr;                 // remaining, more (counted by the convergence test), kept: active of
-                                        // the last iteration; then the serial number
-  IterationReport* host = nullptr;      // pinned host memory
+                                        // the last iteration; far; then the serial number
+  IterationReport* host = nullptr;      // pinned host memory, kReports
 };
 void launchBeginStep(const DevData& d, int* activeCount, long long* activeEl, const BackwardSeed& seed,
                      cudaStream_t s);
