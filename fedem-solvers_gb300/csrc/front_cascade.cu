@@ -215,14 +215,24 @@ __device__ void factorBlocked(T* F, T* lcol, const T* diag0, int nr, int np, int
   __syncwarp();
 }
 
-// one entry per lane of child c's update matrix (pos: child << 20 | position, or -1).
-// FP64: not at all when no lane's entry is of this child -- the addition would take the
-// pipe for 64 cycles with no lane active
-template <typename T>
-__device__ __forceinline__ void extendAdd(T* F, int pos, int c, T val) {
-  const bool on = pos >= 0 && (pos >> 20) == c;
-  if (sizeof(T) == 8 && !__any_sync(0xffffffffu, on)) return;
-  if (on) F[pos & 0xfffff] += val;
+// extend-add of N entries per lane, entry u of lane l the (32 u + l)-th of the front's
+// children segment (pos: child << 20 | position, or -1 past its end).  The segment holds
+// the children in order, so 32 entries are of one child, or of two or a few at a seam:
+// they are added child by child, positions of one child being distinct.  (One pass over
+// all N per child took twice the instructions, half of them without an active lane.)
+template <typename T, int N>
+__device__ __forceinline__ void extendAdd(T* F, const int* pos, const T* val) {
+#pragma unroll
+  for (int u = 0; u < N; ++u) {
+    unsigned left = __ballot_sync(0xffffffffu, pos[u] >= 0);
+    while (left) {
+      const int c = __shfl_sync(0xffffffffu, pos[u], __ffs(left) - 1) >> 20;
+      const bool on = pos[u] >= 0 && (pos[u] >> 20) == c;
+      if (on) F[pos[u] & 0xfffff] += val[u];
+      __syncwarp();
+      left &= ~__ballot_sync(0xffffffffu, on);
+    }
+  }
 }
 
 // partial LDL^T of front f in shared memory (F: maxRow^2, lcol/diag0: maxRow).
@@ -238,7 +248,7 @@ __device__ void factorOneFront(const DevData& d, int f, T* F, T* lcol, T* diag0,
   const int m = d.fModel[f];
   const int nr = d.fNrow[f], np = d.fNpiv[f];
   const int64_t ao = d.fAsmOff[f], so = d.fSegOff[f];
-  const int na = d.fNasm[f], ns = d.fSegLen[f], nch = d.fNchild[f];
+  const int na = d.fNasm[f], ns = d.fSegLen[f];
   for (int k = lane; k < nr * nr; k += 32) F[k] = T(0);
   for (int k0 = 0; k0 < na; k0 += 32 * kFrontBatch) {
     T val[kFrontBatch];
@@ -268,11 +278,7 @@ __device__ void factorOneFront(const DevData& d, int f, T* F, T* lcol, T* diag0,
       pc[u] = k < ns ? __ldg(d.segPos + so + k) : -1;
       val[u] = k < ns ? __ldcg(segIn + k) : T(0);
     }
-    for (int c = 0; c < nch; ++c) {
-#pragma unroll
-      for (int u = 0; u < kFrontBatch; ++u) extendAdd(F, pc[u], c, val[u]);
-      __syncwarp();
-    }
+    extendAdd<T, kFrontBatch>(F, pc, val);
   }
   int neg = 0;
   bool sing = false;
@@ -946,12 +952,7 @@ __global__ void __launch_bounds__(512, 1) kTree(DevData d, TreePlan tp, int maxR
               T sv[kSeg];
 #pragma unroll
               for (int u = 0; u < kSeg; ++u) sv[u] = sp[u] >= 0 ? __ldcg(segIn + lane + 32 * u) : T(0);
-              for (int c1 = 0; c1 < q.nch; ++c1) {
-#pragma unroll
-                for (int u = 0; u < kSeg; ++u)
-                  extendAdd(F, sp[u], c1, sv[u]);
-                __syncwarp();
-              }
+              extendAdd<T, kSeg>(F, sp, sv);
               for (int k0 = 32 * kSeg; k0 < ns; k0 += 32 * kFrontBatch) {
                 T val[kFrontBatch];
                 int pc[kFrontBatch];
@@ -961,12 +962,7 @@ __global__ void __launch_bounds__(512, 1) kTree(DevData d, TreePlan tp, int maxR
                   pc[u] = k < ns ? __ldg(segPos + k) : -1;
                   val[u] = k < ns ? __ldcg(segIn + k) : T(0);
                 }
-                for (int c1 = 0; c1 < q.nch; ++c1) {
-#pragma unroll
-                  for (int u = 0; u < kFrontBatch; ++u)
-                    extendAdd(F, pc[u], c1, val[u]);
-                  __syncwarp();
-                }
+                extendAdd<T, kFrontBatch>(F, pc, val);
               }
               int neg = 0;
               bool sing = false;
