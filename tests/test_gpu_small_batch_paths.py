@@ -44,3 +44,19 @@ def test_alone_and_in_a_large_batch_agree_bitwise(gpu, mixed, chains):
         assert together.info(k)["iterations"] == alone.info(0)["iterations"]
         alone.close()
     together.close()
+
+
+def test_many_joints_agree_bitwise_with_one(gpu):
+    """Beyond 4,864 joints a joint has one lane; 4,900 pendulums against one alone (the
+    joint's four lanes, and every other small-batch kernel)."""
+    from fedem_gb300 import models
+    from fedem_gb300.batch import Batch, Model
+
+    m = Model(models.pendulum(n_el=2)[0], OPTS)
+    alone, many = Batch([m]), Batch([m] * 4900)
+    assert alone.run()["models_failed"] == 0 and many.run()["models_failed"] == 0
+    for k in (0, 1, 2500, 4899):
+        np.testing.assert_array_equal(many.triads(k), alone.triads(0))
+        np.testing.assert_array_equal(many.norms(k), alone.norms(0))
+    alone.close()
+    many.close()
