@@ -248,11 +248,6 @@ __global__ void kPredictDofs(DevData d) {
 // ---------------------------------------------------------------------------
 // element pass: corotated frame, deformation, internal and inertia forces
 // ---------------------------------------------------------------------------
-// v / d with r = recip(d) for several v: the product and one correction by its remainder
-__device__ __forceinline__ double over(double v, double d, double r) {
-  const double q = v * r;
-  return fma(fma(-d, q, v), r, q);
-}
 // tests on bit patterns, off the FP64 pipe: a stiffness scale, or norm weight, of one
 // needs no product, a reference point at its triad no rotated offset
 __device__ __forceinline__ bool isOne(double s) { return __double_as_longlong(s) == 0x3ff0000000000000ll; }
@@ -476,9 +471,8 @@ __global__ void __launch_bounds__(128) kElements(DevData d, int mode) {
       }
       if (vldActive) {
         double tmp[12], yk[12];
-        const double rdt = recip(dt);
 #pragma unroll
-        for (int k = 0; k < 12; ++k) tmp[k] = uld[k] - over(fin[k] - d.finitPrev[(size_t)k * nel + e], dt, rdt);
+        for (int k = 0; k < 12; ++k) tmp[k] = uld[k] - (fin[k] - d.finitPrev[(size_t)k * nel + e]) / dt;
         elemMatvec(d, 0, e, tmp, ss, yk);
         double kd = d.kDmp[e];
 #pragma unroll
@@ -704,9 +698,8 @@ __global__ void __launch_bounds__(128) kElementsWide(DevData d, int mode) {
       }
       if (vldActive) {
         double tmp[3], yk[3];
-        const double rdt = recip(dt);
 #pragma unroll
-        for (int k = 0; k < 3; ++k) tmp[k] = uld[k] - over(fin[k] - d.finitPrev[(size_t)(3 * g + k) * nel + e], dt, rdt);
+        for (int k = 0; k < 3; ++k) tmp[k] = uld[k] - (fin[k] - d.finitPrev[(size_t)(3 * g + k) * nel + e]) / dt;
         matvecBeamRows(d.K26, nel, e, g, mask, tmp, ss, yk);
         const double kd = d.kDmp[e];
 #pragma unroll

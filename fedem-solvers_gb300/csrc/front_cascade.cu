@@ -65,10 +65,10 @@ __device__ void panelShuffle(T* F, const T* diag0, int nr, int np, int lane, int
     const bool bad = !absGreater(dk, diag0[k]);
     sing |= bad;
     if (negative(dk)) ++neg;
-    const typename PivotScaleOf<T>::type scale(dk, bad);
+    const T inv = bad ? T(0) : T(1) / dk;
     const bool r0 = i0 > k && i0 < nr, r1 = i1 > k && i1 < nr;
     const T f0 = r0 ? F[i0 + nr * k] : T(0), f1 = r1 ? F[i1 + nr * k] : T(0);
-    const T l0 = scale(f0), l1 = nr > 32 ? scale(f1) : T(0);
+    const T l0 = f0 * inv, l1 = nr > 32 ? f1 * inv : T(0);
     for (int j = k + 1; j < np; ++j) {
       const T lj = __shfl_sync(0xffffffffu, l0, j);
       if (r0 && j <= i0) F[i0 + nr * j] -= f0 * lj;
@@ -121,10 +121,10 @@ __device__ void panelRegisters(T* F, const T* diag0, int nr, int np, int lane, i
       const bool bad = !absGreater(dk, diag0[k]);
       sing |= bad;
       if (negative(dk)) ++neg;
-      const typename PivotScaleOf<T>::type scale(dk, bad);
+      const T inv = bad ? T(0) : T(1) / dk;
       const bool r0 = i0 > k && i0 < nr;
       const T f0 = r0 ? a0[kk] : T(0), f1 = h1 ? a1[kk] : T(0);
-      const T l0 = scale(f0), l1 = two ? scale(f1) : T(0);
+      const T l0 = f0 * inv, l1 = two ? f1 * inv : T(0);
 #pragma unroll
       for (int jj = kk + 1; jj < PB; ++jj) {
         if (jj >= kb) break;
@@ -186,7 +186,7 @@ __device__ void factorBlocked(T* F, T* lcol, const T* diag0, int nr, int np, int
       const bool bad = !absGreater(dk, diag0[k]);
       sing |= bad;
       if (negative(dk)) ++neg;
-      const T inv = bad ? T(0) : recip(dk);
+      const T inv = bad ? T(0) : T(1) / dk;
       for (int i = k + 1 + lane; i < nr; i += 32) lcol[i] = F[i + nr * k] * inv;
       __syncwarp();
       for (int i = k + 1 + lane; i < nr; i += 32) {
@@ -345,7 +345,7 @@ __device__ void forwardOneFront(const DevData& d, int f, T* v, T* Ls, int capL, 
     for (int i = k + 1 + lane; i < nr; i += 32) v[i] -= L[i + (size_t)nr * k] * yk;
     __syncwarp();
   }
-  for (int r = lane; r < np; r += 32) X[rows[r]] = quotient(v[r], L[r + (size_t)nr * r]);
+  for (int r = lane; r < np; r += 32) X[rows[r]] = v[r] / L[r + (size_t)nr * r];
   T* wo = W + d.fWOff[f];
   for (int a = lane; a < nu; a += 32) wo[a] = v[np + a];
 }
@@ -417,8 +417,8 @@ __device__ void forwardRun(const SolveDesc& q, const int* row, const int* dst, c
   }
   if (lane >= np && lane < nr) Wout[lane - np] = v0;
   if (lane + 32 >= np && lane + 32 < nr) Wout[lane + 32 - np] = v1;
-  if (lane < np) X[row[0]] = quotient(v0, L[lane + (size_t)nr * lane]);
-  if (lane + 32 < np) X[row[1]] = quotient(v1, L[(lane + 32) + (size_t)nr * (lane + 32)]);
+  if (lane < np) X[row[0]] = v0 / L[lane + (size_t)nr * lane];
+  if (lane + 32 < np) X[row[1]] = v1 / L[(lane + 32) + (size_t)nr * (lane + 32)];
 }
 
 template <typename T>

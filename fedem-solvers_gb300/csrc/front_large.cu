@@ -181,7 +181,7 @@ __device__ void factorDiagonal(FactorShared<T>& s, const T* diag0, int kb, int& 
       }
       const T dk = __shfl_sync(0xffffffffu, u, k);
       const bool bad = !absGreater(dk, diag0[k]);
-      const T inv = bad ? T(0) : recip(dk);
+      const T inv = bad ? T(0) : T(1) / dk;
       if (negative(dk)) ++neg;
       sing |= bad;
       l = u * inv;
@@ -719,7 +719,7 @@ __device__ void forwardLarge(const DevData& d, const LargePlan& lp, const LargeT
     __syncthreads();
   }
   if (t.rank == 0)
-    for (int r = tid; r < np; r += kLT) st(X + __ldg(rows + r), quotient(v[r], Lp[r + (int64_t)ldp * r]));
+    for (int r = tid; r < np; r += kLT) st(X + __ldg(rows + r), v[r] / Lp[r + (int64_t)ldp * r]);
   // rows below: quarter h of the pivots of 32 rows per warp, two row groups at a time
   const int qn = (np + 3) >> 2;
   T* wo = W + d.fWOff[f] + (r0 - np);
