@@ -1114,18 +1114,13 @@ int occupancyBlocks(K kernel, int threads, size_t smem, int needed) {
   return needed < cap ? (needed > 0 ? needed : 1) : cap;
 }
 
-template <typename K>
-void allowBigSmem(K kernel, size_t bytes) {
-  if (bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
-
 // one launch of a factor cascade kernel (either panel variant)
 template <typename T>
 void factorCascade(void (*kernel)(DevData, const int*, int, int, const T*, T*, T*, double, const double*, T*, T*,
                                   int*, FusedBackward),
                    int wpb, size_t sm, const DevData& d, const PersistentPlan& p, const T* asmVal, T* L, T* U,
                    double tol, const double* rhs, T* X, T* W, const FusedBackward& fb, cudaStream_t s) {
-  allowBigSmem(kernel, sm);
+  if (sm > 48 * 1024) allowBigShared(kernel);
   const int blocks = occupancyBlocks(kernel, 32 * wpb, sm, (p.nLeaves + wpb - 1) / wpb);
   pdlLaunch(kernel, blocks, 32 * wpb, sm, s, d, p.leaves, p.nLeaves, p.maxRow, asmVal, L, U, tol, rhs, X, W, p.cntFactor,
             fb);
@@ -1145,7 +1140,7 @@ void treeLaunch(const DevData& d, const PersistentPlan& p, const T* asmVal, T* L
                                                                    : kTree<T, kPanelRegisters4>;
   const int threads = 32 * p.tree.warps;
   const size_t sm = p.tree.warps * treeWarpValues(p.maxRow) * sizeof(T);
-  allowBigSmem(kernel, sm);
+  if (sm > 48 * 1024) allowBigShared(kernel);
   const int blocks = occupancyBlocks(kernel, threads, sm, p.tree.nStart);
   pdlLaunch(kernel, blocks, threads, sm, s, d, p.tree, p.maxRow, asmVal, L, U, 1.0e-12, rhs, X, W, cnt, fb, up ? 1 : 0,
             mayFactor ? 1 : 0);
@@ -1237,14 +1232,14 @@ void forwardCascade(const DevData& d, const PersistentPlan& p, bool fp32, const 
   if (fp32) {
     const int capL = stagingCapacity(p, sizeof(float));
     const size_t sm = (size_t)wpb * (p.maxRow + capL + 64) * sizeof(float);
-    allowBigSmem(kForwardCascade<float>, sm);
+    if (sm > 48 * 1024) allowBigShared(kForwardCascade<float>);
     const int blocks = occupancyBlocks(kForwardCascade<float>, 32 * wpb, sm, (p.nTasks + wpb - 1) / wpb);
     pdlLaunch(kForwardCascade<float>, blocks, 32 * wpb, sm, s, d, p.tasks, p.nTasks, p.maxRow, capL, d.L32, rhs, d.x32,
                                                        d.w32, cnt);
   } else {
     const int capL = stagingCapacity(p, sizeof(double));
     const size_t sm = (size_t)wpb * (p.maxRow + capL + 64) * sizeof(double);
-    allowBigSmem(kForwardCascade<double>, sm);
+    if (sm > 48 * 1024) allowBigShared(kForwardCascade<double>);
     const int blocks = occupancyBlocks(kForwardCascade<double>, 32 * wpb, sm, (p.nTasks + wpb - 1) / wpb);
     pdlLaunch(kForwardCascade<double>, blocks, 32 * wpb, sm, s, d, p.tasks, p.nTasks, p.maxRow, capL, d.L64, rhs, d.x64,
                                                          d.w64, cnt);
@@ -1345,14 +1340,14 @@ void launchBackward(const DevData& d, const PersistentPlan& p, bool fp32, int sw
   if (fp32) {
     const int capL = stagingCapacity(p, sizeof(float));
     const size_t sm = (size_t)wpb * (p.maxRow + capL) * sizeof(float);
-    allowBigSmem(kBackwardQueue<float>, sm);
+    if (sm > 48 * 1024) allowBigShared(kBackwardQueue<float>);
     const int blocks = occupancyBlocks(kBackwardQueue<float>, 32 * wpb, sm, needed);
     pdlLaunch(kBackwardQueue<float>, blocks, 32 * wpb, sm, s, d, p.maxRow, capL, d.L32, d.x32, queue, ctr, p.bwInline,
                                                       p.errFlag, acc, fin, p.spinLimit);
   } else {
     const int capL = stagingCapacity(p, sizeof(double));
     const size_t sm = (size_t)wpb * (p.maxRow + capL) * sizeof(double);
-    allowBigSmem(kBackwardQueue<double>, sm);
+    if (sm > 48 * 1024) allowBigShared(kBackwardQueue<double>);
     const int blocks = occupancyBlocks(kBackwardQueue<double>, 32 * wpb, sm, needed);
     pdlLaunch(kBackwardQueue<double>, blocks, 32 * wpb, sm, s, d, p.maxRow, capL, d.L64, d.x64, queue, ctr, p.bwInline,
                                                         p.errFlag, acc, fin, p.spinLimit);
@@ -1364,7 +1359,7 @@ void launchBackwardWaitProbe(const DevData& d, const PersistentPlan& p, int* que
   // one warp; it waits on slot 0 and touches no front (the wait gives up first)
   const int capL = stagingCapacity(p, sizeof(double));
   const size_t sm = (size_t)(p.maxRow + capL) * sizeof(double);
-  allowBigSmem(kBackwardQueue<double>, sm);
+  if (sm > 48 * 1024) allowBigShared(kBackwardQueue<double>);
   pdlLaunch(kBackwardQueue<double>, 1, 32, sm, s, d, p.maxRow, capL, d.L64, d.x64, queue, ctr, p.bwInline, p.errFlag,
                                            ACC_SET, 0, spins);
 }
@@ -1384,7 +1379,7 @@ void launchRootWaitProbe(const DevData& d, const PersistentPlan& p, int* queue, 
   fb.spinLimit = spins;
   fb.acc = ACC_SET;
   fb.capL = stagingCapacity(p, sizeof(double));
-  allowBigSmem(kFactorForwardCascade<double, kPanelShuffle>, sm);
+  if (sm > 48 * 1024) allowBigShared(kFactorForwardCascade<double, kPanelShuffle>);
   pdlLaunch(kFactorForwardCascade<double, kPanelShuffle>, 1, 32, sm, s, d, p.leaves, 0, p.maxRow,
             (const double*)d.asmVal64, d.L64, d.U64, 1.0e-12, (const double*)d.del, d.x64, d.w64, cnt, fb);
 }

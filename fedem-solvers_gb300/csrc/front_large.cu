@@ -51,7 +51,6 @@ namespace {
 constexpr int kLT = 256;  // threads per block
 constexpr int kLW = kLT / 32;
 constexpr int kPanel = 32;  // pivots per panel
-constexpr int kMaxShared = 220 * 1024;  // dynamic shared memory a launch may ask for
 
 // lower-triangle entry (ii >= jj) of an nu x nu matrix packed column by column
 __device__ inline int64_t packedAt(int ii, int jj, int nu) {
@@ -904,9 +903,7 @@ __global__ void __launch_bounds__(kLT, 1) kLargeBackward(DevData d, LargePlan lp
 // cooperative launch (all blocks resident), ordered like any launch of the stream
 template <typename... KArgs, typename... Args>
 void coopLaunch(void (*kernel)(KArgs...), int grid, size_t smem, cudaStream_t s, Args... args) {
-  // one value for every batch: the attribute is the function's, and a smaller
-  // batch must not lower it under a larger one's captured launches
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxShared);
+  allowBigShared(kernel);
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;

@@ -38,6 +38,16 @@ inline void pdlLaunch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t sm
   cfg.numAttrs = 1;
   cudaLaunchKernelEx(&cfg, kernel, args...);
 }
+
+// Dynamic shared memory a launch may ask for.  The limit is an attribute of the
+// function, shared by every batch and host thread of the process: a kernel that can
+// need more than the default 48 KB always gets this one value, since a limit set to one
+// batch's need could be lowered under another batch's launch, or captured graph.
+constexpr int kMaxDynamicShared = 220 * 1024;
+template <typename K>
+inline cudaError_t allowBigShared(K kernel) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicShared);
+}
 #endif
 
 // element pass modes

@@ -369,11 +369,7 @@ size_t partNewtonSmem(const DevData& d) {
 
 int preparePartKernels(const DevData& d) {
   if (d.npartTot <= 0) return 0;
-  if (cudaFuncSetAttribute(kParts, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)partSmem(d)) != cudaSuccess)
-    return -1;
-  if (cudaFuncSetAttribute(kPartsNewton, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)partNewtonSmem(d)) !=
-      cudaSuccess)
-    return -1;
+  if (allowBigShared(kPartsNewton) != cudaSuccess) return -1;
   return 0;
 }
 
