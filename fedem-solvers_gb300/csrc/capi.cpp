@@ -997,6 +997,12 @@ int fgpu_batch_probe_root_wait_timeout(fgpu_batch* b, long long spins, int* flag
   return rc ? fail(rc, "root wait probe failed") : 0;
 }
 
+int fgpu_probe_refuse_launch(int n) {
+  const int left = t_refuseLaunch;
+  t_refuseLaunch = n;
+  return left;
+}
+
 int fgpu_set_device(int ordinal) {
   int n = 0;
   cudaError_t e = cudaGetDeviceCount(&n);

@@ -1874,13 +1874,7 @@ void launchNormsPartial(const DevData& d, cudaStream_t s) {
   attr[1].val.clusterDim.x = CHUNK_TPB / 32;
   attr[1].val.clusterDim.y = 1;
   attr[1].val.clusterDim.z = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(d.nchunkTot * (CHUNK_TPB / 32));
-  cfg.blockDim = dim3(32);
-  cfg.stream = s;
-  cfg.attrs = attr;
-  cfg.numAttrs = 2;
-  cudaLaunchKernelEx(&cfg, kNormsPartial<true>, d);
+  launchWith(attr, 2, kNormsPartial<true>, dim3(d.nchunkTot * (CHUNK_TPB / 32)), dim3(32), 0, s, d);
 }
 void launchControlStepEnd(const DevData& d, const IterationEnd& e, cudaStream_t s) {
   pdlLaunch(kControl, blocksFor(32LL * d.m.n, 128), 128, 0, s, d, e.tally);

@@ -1528,6 +1528,7 @@ int Engine::timeFactor(int reps, double* msPerLaunch, double* bytes) {
     if (pplan_.nLarge > 0)  // the factorisation's and the first forward elimination's
       cudaMemsetAsync(pplan_.cntLarge, 0, sizeof(int) * 3 * (size_t)pplan_.nLarge, stream_);
   };
+  takeLaunchError();
   clear();
   enqueueFactor(stream_);  // warm-up
   cudaEventRecord(e0, stream_);
@@ -1544,7 +1545,7 @@ int Engine::timeFactor(int reps, double* msPerLaunch, double* bytes) {
   cudaMemcpyAsync(d_.m.flags, flags.data(), sizeof(int) * nm, cudaMemcpyHostToDevice, stream_);
   cudaMemcpyAsync(d_.m.status, status.data(), sizeof(int) * nm, cudaMemcpyHostToDevice, stream_);
   cudaMemcpyAsync(d_.m.negPiv, neg.data(), sizeof(int) * nm, cudaMemcpyHostToDevice, stream_);
-  if (cudaStreamSynchronize(stream_) != cudaSuccess) return -946;
+  if (cudaStreamSynchronize(stream_) != cudaSuccess || takeLaunchError() != cudaSuccess) return -946;
   if (msPerLaunch) *msPerLaunch = reps > 0 ? ms / reps : 0.0;
   if (bytes) *bytes = factorBytes_;
   return 0;
@@ -1628,6 +1629,7 @@ int Engine::autotune() {
   cudaMemcpyAsync(neg.data(), d_.m.negPiv, sizeof(int) * nm, cudaMemcpyDeviceToHost, stream_);
   if (cudaStreamSynchronize(stream_) != cudaSuccess) return -1;
   cudaMemcpyAsync(d_.m.flags, all.data(), sizeof(int) * nm, cudaMemcpyHostToDevice, stream_);
+  takeLaunchError();
   launchProbeEntries(d_, f32, stream_);
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
@@ -1641,7 +1643,7 @@ int Engine::autotune() {
       cudaEventRecord(e0, stream_);
       work();
       cudaEventRecord(e1, stream_);
-      if (cudaEventSynchronize(e1) != cudaSuccess) return -1.f;
+      if (cudaEventSynchronize(e1) != cudaSuccess || takeLaunchError() != cudaSuccess) return -1.f;
       float ms = 0.f;
       cudaEventElapsedTime(&ms, e0, e1);
       if (r > 0) tot += ms;
@@ -1893,13 +1895,15 @@ void Engine::enqueueSolveUpdate(cudaStream_t s, bool timed) {
 
 int Engine::assembleIteration() {
   ensureTuned();
+  takeLaunchError();
   enqueueAssembly(stream_, true);
-  return cudaStreamSynchronize(stream_) == cudaSuccess ? 0 : -940;
+  return cudaStreamSynchronize(stream_) == cudaSuccess && takeLaunchError() == cudaSuccess ? 0 : -940;
 }
 
 int Engine::solveUpdateIteration() {
+  takeLaunchError();
   enqueueSolveUpdate(stream_, false);
-  if (cudaStreamSynchronize(stream_) != cudaSuccess) return -941;
+  if (cudaStreamSynchronize(stream_) != cudaSuccess || takeLaunchError() != cudaSuccess) return -941;
   std::string err;
   return resultsDrain(err) ? -942 : 0;
 }
@@ -1924,6 +1928,7 @@ int Engine::seamAssemble(int m, double sM, double sC, double sK) {
   if (m < 0 || m >= d_.m.n) return -1;
   if (modelState(m) == ST_ITER) return -2;  // inside a step: its factor is in use
   ensureTuned();
+  takeLaunchError();
   seamFlags(d_, m, FL_ACTIVE | FL_TANGENT | FL_REBUILD, stream_);
   // scale factors as the element kernels read them: M, K, C
   const double sc[3] = {sM, sK, sC};
@@ -1931,7 +1936,7 @@ int Engine::seamAssemble(int m, double sM, double sC, double sK) {
   launchBuildElementNewton(d_, stream_);
   launchRotateElementNewton(d_, stream_);
   launchCsrGather(d_, stream_);
-  return cudaStreamSynchronize(stream_) == cudaSuccess ? 0 : -3;
+  return cudaStreamSynchronize(stream_) == cudaSuccess && takeLaunchError() == cudaSuccess ? 0 : -3;
 }
 
 int Engine::seamFactor(int m) {
@@ -1945,6 +1950,7 @@ int Engine::seamFactor(int m) {
   cudaMemcpyAsync(d_.m.status + m, &zero, sizeof(int), cudaMemcpyHostToDevice, stream_);
   cudaMemcpyAsync(d_.m.negPiv + m, &zero, sizeof(int), cudaMemcpyHostToDevice, stream_);
   seamFlags(d_, m, FL_ACTIVE | FL_TANGENT, stream_);
+  takeLaunchError();
   resetIterationCounters(stream_);
   enqueueFactor(stream_);
   cudaMemcpyAsync(&st, d_.m.status + m, sizeof(int), cudaMemcpyDeviceToHost, stream_);
@@ -1953,7 +1959,7 @@ int Engine::seamFactor(int m) {
   // the model's own status and pivot count are its stepping's, not the seam's
   cudaMemcpyAsync(d_.m.status + m, &st0, sizeof(int), cudaMemcpyHostToDevice, stream_);
   cudaMemcpyAsync(d_.m.negPiv + m, &neg0, sizeof(int), cudaMemcpyHostToDevice, stream_);
-  if (cudaStreamSynchronize(stream_) != cudaSuccess) return -4;
+  if (cudaStreamSynchronize(stream_) != cudaSuccess || takeLaunchError() != cudaSuccess) return -4;
   return (st & SS_SINGULAR) ? -3 : neg;
 }
 
@@ -1962,6 +1968,7 @@ int Engine::seamSolve(int m, double* rhs, int nrhs) {
   if (modelState(m) == ST_ITER) return -2;
   const int n = hm_[m]->neq;
   seamFlags(d_, m, FL_ACTIVE, stream_);
+  takeLaunchError();
   for (int r = 0; r < nrhs; ++r) {
     double* b = rhs + (size_t)r * n;
     cudaMemcpyAsync(d_.del + modelEqOff_[m], b, sizeof(double) * n, cudaMemcpyHostToDevice, stream_);
@@ -1970,7 +1977,7 @@ int Engine::seamSolve(int m, double* rhs, int nrhs) {
     enqueueFactor(stream_);  // forward elimination only (no tangent flag)
     enqueueSolve(stream_);
     cudaMemcpyAsync(b, d_.del + modelEqOff_[m], sizeof(double) * n, cudaMemcpyDeviceToHost, stream_);
-    if (cudaStreamSynchronize(stream_) != cudaSuccess) return -4;
+    if (cudaStreamSynchronize(stream_) != cudaSuccess || takeLaunchError() != cudaSuccess) return -4;
   }
   int err = 0;
   cudaMemcpyAsync(&err, pplan_.errFlag, sizeof(int), cudaMemcpyDeviceToHost, stream_);
@@ -1988,6 +1995,7 @@ int Engine::prepareStiffnessSolves() {
   for (int k = 0; k < nm; ++k) { sc[3 * k] = 0.0; sc[3 * k + 1] = 1.0; sc[3 * k + 2] = 0.0; }
   cudaMemcpyAsync(d_.m.flags, fl.data(), sizeof(int) * nm, cudaMemcpyHostToDevice, stream_);
   cudaMemcpyAsync(d_.m.scaleN, sc.data(), sizeof(double) * sc.size(), cudaMemcpyHostToDevice, stream_);
+  takeLaunchError();
   launchBuildElementNewton(d_, stream_);
   launchRotateElementNewton(d_, stream_);
   launchCsrGather(d_, stream_);
@@ -1996,7 +2004,7 @@ int Engine::prepareStiffnessSolves() {
   // solves from here on: active, no tangent update
   std::fill(fl.begin(), fl.end(), FL_ACTIVE);
   cudaMemcpyAsync(d_.m.flags, fl.data(), sizeof(int) * nm, cudaMemcpyHostToDevice, stream_);
-  if (cudaStreamSynchronize(stream_) != cudaSuccess) return -948;
+  if (cudaStreamSynchronize(stream_) != cudaSuccess || takeLaunchError() != cudaSuccess) return -948;
   std::vector<int> st(nm);
   cudaMemcpy(st.data(), d_.m.status, sizeof(int) * nm, cudaMemcpyDeviceToHost);
   for (int k = 0; k < nm; ++k)
@@ -2006,13 +2014,14 @@ int Engine::prepareStiffnessSolves() {
 
 int Engine::solveStiffness(int m, const double* b, double* x) {
   const int n = hm_[m]->neq;
+  takeLaunchError();
   cudaMemcpyAsync(d_.del + modelEqOff_[m], b, sizeof(double) * n, cudaMemcpyHostToDevice, stream_);
   resetIterationCounters(stream_);
   launchSeedBackward(d_, seed_, stream_);
   enqueueFactor(stream_);  // forward elimination only (no tangent flag)
   enqueueSolve(stream_);
   cudaMemcpyAsync(x, d_.del + modelEqOff_[m], sizeof(double) * n, cudaMemcpyDeviceToHost, stream_);
-  return cudaStreamSynchronize(stream_) == cudaSuccess ? 0 : -949;
+  return cudaStreamSynchronize(stream_) == cudaSuccess && takeLaunchError() == cudaSuccess ? 0 : -949;
 }
 
 int Engine::endStiffnessSolves() {
@@ -2216,6 +2225,7 @@ int Engine::readActive() {
 
 int Engine::initialState(std::string& err) {
   SetupTrace trace;
+  takeLaunchError();
   // staticEquilibriumModule.f90:50-437: iterate the models that asked for it
   launchStaticBegin(d_, dActive_, BackwardSeed{}, stream_);
   launchElements(d_, EM_STATIC_INIT, stream_);
@@ -2253,6 +2263,7 @@ int Engine::initialState(std::string& err) {
     FG_CHECK(cudaMemcpyAsync(d_.urddQs, d_.urdd, D * (size_t)d_.ndofTot, cudaMemcpyDeviceToDevice, stream_));
   }
   FG_CHECK(cudaStreamSynchronize(stream_));
+  FG_CHECK(takeLaunchError());
   FG_CHECK(cudaGetLastError());
   // a model whose initial equilibrium failed (singular, NaN, no convergence)
   // stays in its error state with its status bits; the others go on
@@ -2270,12 +2281,13 @@ int Engine::probeWaitTimeout(long long spins, int* flag) {
   if (cudaMalloc(&q, sizeof(int) * 8) != cudaSuccess) return -955;
   const int init[8] = {-1, 0, 0, 0, 0, 0, 1, 0};  // queue slot 0 empty; ctr = {take 0, fill 0, total 1}
   cudaMemcpyAsync(q, init, sizeof(init), cudaMemcpyHostToDevice, stream_);
+  takeLaunchError();
   launchBackwardWaitProbe(d_, pplan_, q, q + 4, spins, stream_);
   int f = 0;
   cudaMemcpyAsync(&f, pplan_.errFlag, sizeof(int), cudaMemcpyDeviceToHost, stream_);
   const cudaError_t e = cudaStreamSynchronize(stream_);
   cudaFree(q);
-  if (e != cudaSuccess) return -956;
+  if (e != cudaSuccess || takeLaunchError() != cudaSuccess) return -956;
   if (flag) *flag = f;
   return 0;
 }
@@ -2303,13 +2315,14 @@ int Engine::probeRootWaitTimeout(long long spins, int* flag) {
   cudaMemcpyAsync(q, init, sizeof(init), cudaMemcpyHostToDevice, stream_);
   const int act = fl0 | FL_ACTIVE;
   cudaMemcpyAsync(d_.m.flags, &act, sizeof(int), cudaMemcpyHostToDevice, stream_);
+  takeLaunchError();
   launchRootWaitProbe(d_, pplan_, q, q + 4, q + 8, spins, stream_);
   cudaMemcpyAsync(d_.m.flags, &fl0, sizeof(int), cudaMemcpyHostToDevice, stream_);
   int f = 0;
   cudaMemcpyAsync(&f, pplan_.errFlag, sizeof(int), cudaMemcpyDeviceToHost, stream_);
   const cudaError_t e = cudaStreamSynchronize(stream_);
   cudaFree(q);
-  if (e != cudaSuccess) return -956;
+  if (e != cudaSuccess || takeLaunchError() != cudaSuccess) return -956;
   if (flag) *flag = f;
   return 0;
 }
@@ -2327,17 +2340,27 @@ void Engine::dropGraphs() {
 int Engine::graphReady(bool timed) {
   const int k = timed ? 1 : 0;
   if (!opt_.useGraph || graphExec_[k]) return 0;
+  takeLaunchError();
   cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal);
   enqueueIteration(stream_, timed, false);
-  if (cudaStreamEndCapture(stream_, &graph_[k]) != cudaSuccess) return -920;
-  if (cudaGraphInstantiate(&graphExec_[k], graph_[k], 0) != cudaSuccess) return -921;
-  return 0;
+  const cudaError_t ended = cudaStreamEndCapture(stream_, &graph_[k]);
+  int rc = 0;
+  if (takeLaunchError() != cudaSuccess || ended != cudaSuccess) rc = -920;  // not with a kernel missing
+  else if (cudaGraphInstantiate(&graphExec_[k], graph_[k], 0) != cudaSuccess) rc = -921;
+  if (rc) {
+    cudaGetLastError();
+    if (graph_[k]) cudaGraphDestroy(graph_[k]);
+    graph_[k] = nullptr;
+    graphExec_[k] = nullptr;
+  }
+  return rc;
 }
 
 int Engine::launchIteration(bool timed) {
   if (!opt_.useGraph) {
+    takeLaunchError();
     enqueueIteration(stream_, timed, false);
-    return 0;
+    return takeLaunchError() == cudaSuccess ? 0 : -922;
   }
   const int rc = graphReady(timed);
   if (rc) return rc;
@@ -2412,7 +2435,10 @@ int Engine::run(long long maxBatched, RunStats* stats) {
   while (launched < maxBatched || seen < launched) {
     for (; launched < std::min(maxBatched, ahead); ++launched) {
       rc = launchIteration((launched + 1) % every == 0);
-      if (rc) return rc;
+      if (rc) {
+        cudaStreamSynchronize(stream_);  // the iterations in flight report into host memory
+        return rc;
+      }
     }
     if (!waitReport(seen + 1)) return -922;
     const IterationReport r = hReport_[++seen % kReports];
@@ -2432,8 +2458,10 @@ int Engine::run(long long maxBatched, RunStats* stats) {
   // the models that reached their end leave the active set (kBeginStep's
   // bookkeeping, which an iteration without work would do)
   if (seen > 0 && remaining == 0) {
+    takeLaunchError();
     resetIterationCounters(stream_);
     launchBeginStep(d_, dActive_, dActiveEl_, seed_, stream_);
+    rc = takeLaunchError() == cudaSuccess ? 0 : -923;
   }
   if (rec_.on) {
     if (cudaStreamSynchronize(stream_) != cudaSuccess) return -922;
@@ -2442,7 +2470,7 @@ int Engine::run(long long maxBatched, RunStats* stats) {
   }
   cudaEventRecord(evRun_[1], stream_);
   if (cudaStreamSynchronize(stream_) != cudaSuccess) return -922;
-  if (cudaGetLastError() != cudaSuccess) return -923;
+  if (rc || cudaGetLastError() != cudaSuccess) return -923;
   lastRunSec_ = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
   float devMs = 0.f;
   cudaEventElapsedTime(&devMs, evRun_[0], evRun_[1]);
@@ -2475,7 +2503,10 @@ int Engine::launchChunk(int n) {
   resetIterationCounters(stream_);
   for (int k = 0; k < n; ++k) {
     const int rl = launchIteration(false);
-    if (rl) return rl;
+    if (rl) {
+      cudaStreamSynchronize(stream_);
+      return rl;
+    }
   }
   // the models that took part in the chunk's last iteration
   cudaMemcpyAsync(hActive_, end_.tally + 2, sizeof(int), cudaMemcpyDeviceToHost, stream_);

@@ -907,14 +907,7 @@ void coopLaunch(void (*kernel)(KArgs...), int grid, size_t smem, cudaStream_t s,
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(kLT);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, args...);
+  launchWith(attr, 1, kernel, dim3(grid), dim3(kLT), smem, s, args...);
 }
 
 template <typename T>

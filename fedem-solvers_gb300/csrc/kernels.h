@@ -10,6 +10,30 @@
 
 namespace fgpu {
 
+// Refused launches.  The launch wrappers return nothing: the first launch of a host
+// thread that the runtime refuses is kept until the thread's next takeLaunchError(),
+// which every call that enqueues kernels asks before it reports success (and, at its
+// start, to begin afresh).  Until then the thread launches nothing more: no kernel runs
+// on what a missing one should have written.  The runtime's own last error is cleared,
+// so that it does not turn up in another batch's call.
+inline thread_local cudaError_t t_launchError = cudaSuccess;
+inline void noteLaunch(cudaError_t e) {
+  if (e == cudaSuccess) return;
+  cudaGetLastError();
+  if (t_launchError == cudaSuccess) t_launchError = e;
+}
+inline cudaError_t takeLaunchError() {
+  const cudaError_t e = t_launchError;
+  t_launchError = cudaSuccess;
+  return e;
+}
+// Test hook: the t_refuseLaunch-th launch of this host thread from now asks for more
+// shared memory than any device has, which the runtime refuses (0: off).
+inline thread_local int t_refuseLaunch = 0;
+inline size_t launchShared(size_t smem) {
+  return t_refuseLaunch > 0 && --t_refuseLaunch == 0 ? (size_t)1 << 30 : smem;
+}
+
 // Programmatic dependent launch.  Every kernel of the engine is launched with
 // programmatic stream serialization (pdlLaunch) and calls pdlEntry() first:
 // it waits until the previous kernel of its stream has completed and its
@@ -23,20 +47,28 @@ __device__ __forceinline__ void pdlEntry() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// One launch (none after one that the runtime refused, see above, or of an empty grid).
+template <typename... KArgs, typename... Args>
+inline void launchWith(cudaLaunchAttribute* attrs, int nAttrs, void (*kernel)(KArgs...), dim3 grid, dim3 block,
+                       size_t smem, cudaStream_t s, Args... args) {
+  if (t_launchError != cudaSuccess || grid.x == 0) return;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = launchShared(smem);
+  cfg.stream = s;
+  cfg.attrs = attrs;
+  cfg.numAttrs = nAttrs;
+  noteLaunch(cudaLaunchKernelEx(&cfg, kernel, args...));
+}
+
 template <typename... KArgs, typename... Args>
 inline void pdlLaunch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
                       Args... args) {
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, args...);
+  launchWith(attr, 1, kernel, grid, block, smem, s, args...);
 }
 
 // Dynamic shared memory a launch may ask for.  The limit is an attribute of the

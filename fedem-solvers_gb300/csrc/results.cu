@@ -182,7 +182,14 @@ int Engine::resultsOpen(const std::string& dir, bool asDouble, std::string& err,
   // the batched iteration is captured again with the record kernel in it
   dropGraphs();
   // the current state: the initial configuration, or where the models are now
+  takeLaunchError();
   launchRecordStep(d_, r, true, stream_);
+  if (takeLaunchError() != cudaSuccess) {
+    std::string ignored;
+    resultsClose(ignored);
+    err = "results: launch refused";
+    return -4;
+  }
   return resultsDrain(err);
 }
 

@@ -202,6 +202,12 @@ int fgpu_batch_probe_wait_timeout(fgpu_batch* b, long long spins, int* flag);
  * polls and sets the wait-error flag (*flag = 1).  No front is touched; the
  * running models then fail with status 16 as above. */
 int fgpu_batch_probe_root_wait_timeout(fgpu_batch* b, long long spins, int* flag);
+/* Test hook of the failure path of a launch: the n-th kernel launch that the
+ * calling host thread makes from now asks for more shared memory than any
+ * device has, which the runtime refuses on the host (n = 0: off).  The call
+ * that made it must fail.  Returns what was left of an earlier count: 0 when
+ * that launch has been made. */
+int fgpu_probe_refuse_launch(int n);
 
 /* Measured FP64 fused multiply-add rate of the library's current device:
  * eight independent FMA chains per thread, eight 256-thread blocks per SM,
