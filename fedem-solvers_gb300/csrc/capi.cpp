@@ -863,6 +863,12 @@ int fgpu_batch_set_launch_shape(fgpu_batch* b, const int* shape4) {
   return 0;
 }
 
+int fgpu_batch_front_plan(const fgpu_batch* b, long long* p5) {
+  if (!b || !p5) return fail(-1, "bad argument");
+  b->engine.frontPlan(p5);
+  return 0;
+}
+
 int fgpu_batch_results_open(fgpu_batch* b, const char* dir, int doublePrecision) {
   if (!b || !dir) return fail(-1, "bad argument");
   OnDevice onDev(b->engine.device());

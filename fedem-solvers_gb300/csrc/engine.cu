@@ -1266,6 +1266,10 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
       }
       int sms = 0;
       FG_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
+      // (FGPU_LARGE_SMS set at batch creation: as on a partition of so many SMs)
+      if (const char* e = std::getenv("FGPU_LARGE_SMS")) sms = std::max(1, std::min(sms, std::atoi(e)));
+      sms = largeBlocks(opt_.fp32Factor, sms);
+      if (sms < 1) { err = "large-front kernels do not fit on the device"; return -905; }
       const int levels = 1 + *std::max_element(level.begin(), level.end());
       std::vector<std::vector<int>> byLevel(levels);
       for (int li = 0; li < nL; ++li) byLevel[level[li]].push_back(li);
@@ -1589,6 +1593,14 @@ int Engine::launchShape(int* sh, double* probeMs) const {
   sh[3] = pplan_.largeCluster;
   if (probeMs) *probeMs = probeMs_;
   return tuned_ ? 1 : 0;
+}
+
+void Engine::frontPlan(long long* p5) const {
+  p5[0] = d_.nfrontTot;
+  p5[1] = pplan_.nLarge;
+  p5[2] = pplan_.nLarge > 0 ? std::max(pplan_.large[3].grid, pplan_.large[4].grid) : 0;
+  p5[3] = pplan_.tree.nChunks;
+  p5[4] = pplan_.tree.warps;
 }
 
 void Engine::ensureTuned() {

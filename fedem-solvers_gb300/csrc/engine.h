@@ -149,6 +149,10 @@ class Engine {
   // the same for the fused back substitution's wait for a root's elimination
   int probeRootWaitTimeout(long long spins, int* flag);
 
+  // fronts, large fronts, blocks of the large fronts' launches, chunks and warps per
+  // block of the trees on thread blocks (0: none)
+  void frontPlan(long long* p5) const;
+
   // Launch shapes of the multifrontal kernels (PersistentPlan: factor panel
   // variant, forward and backward warps per block, large fronts' share of the SMs).
   // Before the first batched iteration the autotuner times the candidates on

@@ -917,6 +917,28 @@ size_t solveShared(const LargePlan& lp) {
 
 }  // namespace
 
+// Blocks of a cooperative launch must all be resident: at most as many as the device
+// (or the partition of it that this process has) holds of each kernel at once, and one
+// per SM.  The solves are asked with the most shared memory they can take.
+int largeBlocks(bool fp32, int sms) {
+  auto resident = [&](auto kernel, size_t smem) {
+    int perSm = 0;
+    if (allowBigShared(kernel) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, kLT, smem) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    return perSm * sms;
+  };
+  if (fp32)
+    return std::min({sms, resident(kLargeFactor<float>, sizeof(FactorShared<float>)),
+                     resident(kLargeForward<float>, kMaxDynamicShared),
+                     resident(kLargeBackward<float>, kMaxDynamicShared)});
+  return std::min({sms, resident(kLargeFactor<double>, sizeof(FactorShared<double>)),
+                   resident(kLargeForward<double>, kMaxDynamicShared),
+                   resident(kLargeBackward<double>, kMaxDynamicShared)});
+}
+
 // at most about 200 KB of staged L per block
 int64_t largeSolveStage(int nr, int np, int G, size_t elemBytes) {
   const int64_t want = std::max(forwardStage(nr, np, G), backwardStage(nr, np, G));

@@ -299,6 +299,8 @@ void launchLargeFactor(const DevData& d, const PersistentPlan& p, bool fp32, cud
 void launchLargeForward(const DevData& d, const PersistentPlan& p, bool fp32, const double* rhs, int sweep,
                         cudaStream_t s);
 void launchLargeBackward(const DevData& d, const PersistentPlan& p, bool fp32, int sweep, bool last, cudaStream_t s);
+// blocks the large-front launches may have on a device of `sms` SMs (0: they do not fit)
+int largeBlocks(bool fp32, int sms);
 // values of L a block of the large-front solves stages for a front shared by G blocks
 int64_t largeSolveStage(int nr, int np, int G, size_t elemBytes);
 // the height from which a batch's small fronts go to the trees on thread blocks:

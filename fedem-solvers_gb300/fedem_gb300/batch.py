@@ -243,6 +243,15 @@ class Batch:
         keys = ("panel", "forward_warps", "backward_warps", "large_cluster")
         return dict(zip(keys, list(sh))), ms.value, tuned == 1
 
+    def front_plan(self):
+        """How the fronts are spread over the kernels: all fronts, the large ones and
+        the blocks of their launches, chunks and warps per chunk of the small-front
+        trees on thread blocks (0: the cascades take the small fronts)."""
+        p = (ctypes.c_longlong * 5)()
+        if self._lib.fgpu_batch_front_plan(self._h, p) != 0:
+            raise FedemException("front_plan failed: " + self._lib.fgpu_last_error().decode())
+        return dict(zip(("fronts", "large", "large_blocks", "tree_chunks", "tree_warps"), list(p)))
+
     def assemble_newton(self, model, sM, sC, sK):
         """N = sM M + sC C + sK K of the model's current state, assembled on the
         GPU (read it with newton_values); between the model's steps."""

@@ -145,6 +145,11 @@ int fgpu_batch_time_factor(fgpu_batch* b, int reps, double* out2);
  * no GPU kernels to shape). */
 int fgpu_batch_set_launch_shape(fgpu_batch* b, const int* shape4);
 int fgpu_batch_launch_shape(fgpu_batch* b, int* shape4, double* probeMs);
+/* How the batch's fronts are spread over the kernels: {fronts, large fronts
+ * (several blocks each), blocks of their launches, chunks of the small-front
+ * trees that run on thread blocks, warps per chunk (both 0 where the cascades
+ * take the small fronts)}. */
+int fgpu_batch_front_plan(const fgpu_batch* b, long long* p5);
 
 /* The linear-solver seam of one model, at the granularity of the reference's
  * csAddEM + csSolve (src/vpmCommon/vpmLinAlg/asmExtensionModule.f90:1227,
