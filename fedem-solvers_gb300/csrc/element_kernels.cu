@@ -101,7 +101,7 @@ __device__ inline void seedQueue(int* ctr, int* queue, const int* off, const int
 // every queue of model i by warp w of `warps`: the queues (and, with the trees' queue of
 // top chunks beside each, twice as many) in parts, a part per warp
 __device__ inline void seedBackward(const BackwardSeed& b, int i, int lane, int w = 0, int warps = 1) {
-  const int kinds = b.strideT > 0 ? 2 : 1, parts = max(1, warps / (kinds * b.nq));
+  const int kinds = b.strideT > 0 ? 2 : 1, parts = seedParts(warps, kinds * b.nq);
   for (int t = w; t < kinds * b.nq * parts; t += warps) {
     const int part = t % parts, q = t / parts % b.nq;
     if (t / parts < b.nq)

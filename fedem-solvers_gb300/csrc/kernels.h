@@ -117,6 +117,11 @@ struct BackwardSeed {
   int* queueT = nullptr;
   int* ctrT = nullptr;
 };
+// parts that each of `queues` queues of a model is cut into when `warps` warps seed
+// them, a part per warp (no queues: nothing to seed)
+inline __host__ __device__ int seedParts(int warps, int queues) {
+  return queues <= 0 ? 0 : warps > queues ? warps / queues : 1;
+}
 // What the last kernel of an iteration does beside the step end: the iteration's
 // counters and backward queues reset for the next one (in place of memset nodes),
 // and a report into host memory, its serial number last, that the host can follow
