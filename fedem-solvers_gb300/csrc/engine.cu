@@ -2383,7 +2383,7 @@ int Engine::launchIteration(bool timed) {
 // failed or drained without it).
 bool Engine::waitReport(long long serial) {
   const volatile IterationReport* h = hReport_ + serial % kReports;
-  for (int spins = 0; h->serial < serial; ++spins) {
+  for (unsigned spins = 0; h->serial < serial; ++spins) {  // (wraps around)
     if ((spins & 1023) != 1023) continue;
     const cudaError_t q = cudaStreamQuery(stream_);
     if (q == cudaSuccess) return h->serial >= serial;
@@ -2438,7 +2438,7 @@ int Engine::run(long long maxBatched, RunStats* stats) {
   resetIterationCounters(stream_);
   cudaMemsetAsync(end_.tally, 0, sizeof(int) * 6, stream_);
   std::fill_n(hReport_, kReports, IterationReport{});
-  const int every = 7;
+  const int every = kTimedEvery;
   long long launched = 0, seen = 0, done = 0;
   int remaining = 0;
   // the first two at once: a step takes at least two iterations, but for linear

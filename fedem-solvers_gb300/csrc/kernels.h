@@ -129,6 +129,11 @@ inline __host__ __device__ int seedParts(int warps, int queues) {
 constexpr int kIterationsAhead = 6;
 // reports in turn, more than iterations in flight: one is not overwritten while it is read
 constexpr int kReports = 8;
+static_assert(kIterationsAhead < kReports, "a report would be overwritten before it is read");
+// every so many iterations one is timed, farther apart than iterations in flight: its
+// events are read before the next timed one records them
+constexpr int kTimedEvery = 7;
+static_assert(kIterationsAhead < kTimedEvery, "phase events would be recorded again before they are read");
 struct IterationReport {
   long long serial;    // iterations finished since the counters' last reset by the host
   long long elements;  // elements of the models that took part
