@@ -2425,6 +2425,7 @@ void Engine::samplePhases(long long elements, int active) {
 // seventh iteration is timed: an odd distance, so that with two iterations per
 // step predictors and correctors are both sampled, and farther apart than
 // kIterationsAhead, so that its events are read before the next records them.
+// The last iteration of a run of limited length is timed too.
 int Engine::run(long long maxBatched, RunStats* stats) {
   ensureTuned();
   int rc = graphReady(false);
@@ -2439,14 +2440,17 @@ int Engine::run(long long maxBatched, RunStats* stats) {
   cudaMemsetAsync(end_.tally, 0, sizeof(int) * 6, stream_);
   std::fill_n(hReport_, kReports, IterationReport{});
   const int every = kTimedEvery;
-  long long launched = 0, seen = 0, done = 0;
+  long long launched = 0, seen = 0, done = 0, lastTimed = 0;
   int remaining = 0;
   // the first two at once: a step takes at least two iterations, but for linear
   // quasi-static and fixed-iteration ones
   long long ahead = 2;
   while (launched < maxBatched || seen < launched) {
     for (; launched < std::min(maxBatched, ahead); ++launched) {
-      rc = launchIteration((launched + 1) % every == 0);
+      const bool timed = (launched + 1) % every == 0 || launched + 1 == maxBatched;
+      if (timed && lastTimed > seen) break;  // the events of the timed one before are still to be read
+      rc = launchIteration(timed);
+      if (timed) lastTimed = launched + 1;
       if (rc) {
         cudaStreamSynchronize(stream_);  // the iterations in flight report into host memory
         return rc;
@@ -2456,7 +2460,7 @@ int Engine::run(long long maxBatched, RunStats* stats) {
     const IterationReport r = hReport_[++seen % kReports];
     remaining = r.remaining;
     if (r.active > 0) done = seen;
-    if (seen % every == 0) samplePhases(r.elements, r.active);
+    if (seen == lastTimed) samplePhases(r.elements, r.active);
     if (rec_.on && seen % every == 0) {
       // records are drained before a model's ring can fill: nothing runs meanwhile
       if (cudaStreamSynchronize(stream_) != cudaSuccess) return -922;
