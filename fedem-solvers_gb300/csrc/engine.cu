@@ -931,18 +931,79 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
       smallLeaves += nchild[f] == 0;
       maxHeight = std::max(maxHeight, height[f]);
     }
-    const int treeHeight = treeFromHeight(smallLeaves, maxHeight, [&](int h) {
-      // fronts of at least height h without a child of at least height h
-      long long n = 0;
+    // cut of the small fronts from height h on into chunks of at most warps fronts:
+    // tiers of as many tree levels as a full binary piece of that many fronts has (so
+    // that a root path crosses few chunks), and where a piece is larger, its largest
+    // children to chunks of their own
+    struct TreeCut {
+      int height = -1, warps = 0, chunks = 0;
+      long long fronts = 0;
+      std::vector<char> cut, lev;  // chunk roots; levels inside the chunk
+    };
+    auto cutTrees = [&](int h, int warps) {
+      TreeCut t;
+      t.height = h;
+      t.warps = warps;
+      t.cut.assign(nfr, 0);
+      t.lev.assign(nfr, 0);
+      auto in = [&](int f) { return !large[f] && height[f] >= h; };
+      int tier = 1;
+      while ((2 << tier) - 1 <= warps) ++tier;
+      std::vector<int> size(nfr, 0), kids;
       for (int f = 0; f < nfr; ++f) {
-        if (large[f] || height[f] < h) continue;
-        bool lowest = true;
-        for (int c = 0; c < nchild[f] && lowest; ++c) lowest = height[childList[childOffV[f] + c]] < h;
-        n += lowest;
+        if (!in(f)) continue;
+        kids.clear();
+        int sum = 1;
+        for (int c = 0; c < nchild[f]; ++c) {
+          const int k = childList[childOffV[f] + c];
+          if (!in(k)) continue;  // done by the cascades before
+          if ((height[k] - h) / tier != (height[f] - h) / tier) {
+            t.cut[k] = 1;
+            continue;
+          }
+          kids.push_back(k);
+          sum += size[k];
+        }
+        std::stable_sort(kids.begin(), kids.end(), [&](int a, int b) { return size[a] > size[b]; });
+        for (size_t k = 0; k < kids.size() && sum > warps; ++k) {
+          t.cut[kids[k]] = 1;
+          sum -= size[kids[k]];
+        }
+        size[f] = sum;
+        for (int k : kids)
+          if (!t.cut[k]) t.lev[f] = std::max<char>(t.lev[f], t.lev[k] + 1);
+        if (parent[f] < 0 || large[parent[f]]) t.cut[f] = 1;
       }
-      return n;
-    });
-    const int tw = treeHeight < 0 ? 0 : treeWarps(treeHeight == 0 ? smallLeaves : 0, maxRowAll, opt_.fp32Factor);
+      for (int f = 0; f < nfr; ++f) {
+        t.chunks += t.cut[f];
+        t.fronts += in(f);
+      }
+      return t;
+    };
+    TreeCut tree;
+    {
+      // all small fronts, or the upper levels of a larger batch's trees
+      auto consider = [&](int h) {
+        const int warps = h < 0 ? 0 : treeWarps(h == 0 ? smallLeaves : 0, maxRowAll, opt_.fp32Factor);
+        if (warps == 0 || tree.warps > 0) return;
+        TreeCut t = cutTrees(h, warps);
+        if (treesPay(t.chunks, t.fronts, warps, h)) tree = std::move(t);
+      };
+      if (smallLeaves > 0 && smallLeaves <= kTreeAllLeaves) consider(0);
+      if (tree.warps == 0 && smallLeaves > 0 && smallLeaves <= kTreeTopLeaves)
+        consider(treeTopHeight(maxHeight, [&](int h) {
+          // fronts of at least height h without a child of at least height h
+          long long n = 0;
+          for (int f = 0; f < nfr; ++f) {
+            if (large[f] || height[f] < h) continue;
+            bool lowest = true;
+            for (int c = 0; c < nchild[f] && lowest; ++c) lowest = height[childList[childOffV[f] + c]] < h;
+            n += lowest;
+          }
+          return n;
+        }));
+    }
+    const int treeHeight = tree.height, tw = tree.warps;
     std::vector<unsigned char> cls(nfr, 0);
     for (int f = 0; f < nfr; ++f) cls[f] = large[f] ? 1 : (tw > 0 && height[f] >= treeHeight ? 2 : 0);
     UPV(d_.fLarge, uint8_t, cls);
@@ -1028,38 +1089,9 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
     std::vector<int> treeRootOff(nm + 1, 0), treeRoots, treeChains(nm, 0);
     int nChunks = 0;
     if (tw > 0) {
-      // ---- trees on thread blocks: the small fronts cut into chunks of at most tw
-      // fronts: tiers of as many tree levels as a full binary piece of tw fronts has
-      // (so that a root path crosses few chunks), and where a piece is larger, its
-      // largest children to chunks of their own
-      int tier = 1;
-      while ((2 << tier) - 1 <= tw) ++tier;
-      std::vector<int> size(nfr, 0), chunkOf(nfr, -1);
-      std::vector<char> cut(nfr, 0), lev(nfr, 0);
-      for (int f = 0; f < nfr; ++f) {
-        if (cls[f] != 2) continue;
-        std::vector<int> kids;
-        int sum = 1;
-        for (int c = 0; c < nchild[f]; ++c) {
-          const int k = childList[childOffV[f] + c];
-          if (cls[k] != 2) continue;  // done by the cascades before
-          if ((height[k] - treeHeight) / tier != (height[f] - treeHeight) / tier) {
-            cut[k] = 1;
-            continue;
-          }
-          kids.push_back(k);
-          sum += size[k];
-        }
-        std::stable_sort(kids.begin(), kids.end(), [&](int a, int b) { return size[a] > size[b]; });
-        for (size_t k = 0; k < kids.size() && sum > tw; ++k) {
-          cut[kids[k]] = 1;
-          sum -= size[kids[k]];
-        }
-        size[f] = sum;
-        for (int k : kids)
-          if (!cut[k]) lev[f] = std::max<char>(lev[f], lev[k] + 1);
-        if (parent[f] < 0 || cls[parent[f]] != 2) cut[f] = 1;
-      }
+      // ---- trees on thread blocks ------------------------------------------------
+      const std::vector<char>&cut = tree.cut, &lev = tree.lev;
+      std::vector<int> chunkOf(nfr, -1);
       // chunks numbered by their root front; members by level
       std::vector<TreeChunk> chunks;
       std::vector<std::vector<int>> members;
@@ -1617,11 +1649,11 @@ void Engine::ensureTuned() {
 int Engine::autotune() {
   const auto t0 = std::chrono::steady_clock::now();
   char key[256];
-  snprintf(key, sizeof key, "dev%d f%d s%d r%d p%d L%d n%d l%d t%d", device_, opt_.fp32Factor ? 1 : 0,
+  snprintf(key, sizeof key, "dev%d f%d s%d r%d p%d L%d n%d l%d t%d w%d", device_, opt_.fp32Factor ? 1 : 0,
            opt_.refineSweeps, pplan_.maxRow, pplan_.maxNpiv, pplan_.nLarge > 0 ? pplan_.large[4].maxRow : 0,
            (int)std::lround(std::log2((double)d_.nfrontTot + 1.0)),
            (int)std::lround(std::log2(pplan_.nLeaves + pplan_.tree.nStart + 1.0)),
-           pplan_.nLarge > 0 ? (int)std::lround(std::log2(pplan_.nLarge + 1.0)) : -1);
+           pplan_.nLarge > 0 ? (int)std::lround(std::log2(pplan_.nLarge + 1.0)) : -1, pplan_.tree.warps);
   {
     std::lock_guard<std::mutex> lk(g_shapeMutex);
     auto it = g_shapeCache.find(key);

@@ -11,8 +11,9 @@
 // be filled, by warps that are running and never wait themselves, so the wait
 // ends whatever the residency.  Each wait is still bounded and sets errFlag
 // when it runs out.
-// Batches of up to 32,768 leaf fronts pay the cascades' latency per tree level, not
-// their work; there whole subtrees go to thread blocks, a warp per front (kTree).
+// Batches of few or deep trees, up to 32,768 leaf fronts, pay the cascades' latency per
+// tree level, not their work; there whole subtrees go to thread blocks, a warp per front
+// (kTree; treesPay).
 // The forward and backward solves stage each front's L block in shared memory
 // first (one burst of loads instead of one load latency per pivot).
 //
@@ -1282,28 +1283,37 @@ int stagingCapacity(const PersistentPlan& p, size_t elemBytes) {
   return (int)(want < cap ? want : cap);
 }
 
-// The line between the trees on thread blocks and the cascades, by the batch's
-// leaf fronts (iteration in microseconds, cascades against trees of 16 and 8
-// warps; chains of beams, mixed unless noted): 1,066 leaves 238 / 174 / 183;
-// 3,200: 265 / 221 / 221; 5,333: 360 / 334 / 324 (FP64 368 / 315 / 298); 8,533:
-// 348 / 348 / 334; FP64 10,666: 446 / 524 / 477; 16,000: 556 / 779 / 721.  With
-// more leaves the cascades' warps, which never wait for a level, keep the GPU
-// busier; between 4,096 and 8,192 two blocks of 8 warps share an SM better than
-// one of 16.  Larger batches up to 32,768 leaves take both: the cascades up to the
-// height above which at most kTreeTops subtrees begin, the trees from there, where
-// the cascades run out of fronts and pay their latency level by level (cascades
-// alone against both: one chain of 33,333 beams 595 / 498; 24 of 2,000 550 / 485;
-// 8 of 8,000 657 / 571; 64 of 1,000 586 / 562; FP64 32 of 1,000 424 / 414; with
-// 300, 600 or 3,000 subtrees up to 9 % slower than with 1,500).  Above, other
-// models' fronts fill the cascades' upper levels (64,000 leaves: 675 / 689, FP64
-// 727 / 749).
-int treeFromHeight(int nLeaves, int maxHeight, const std::function<long long(int)>& lowest) {
-  if (nLeaves <= 0) return -1;
-  if (nLeaves <= 8192) return 0;
-  if (nLeaves <= 32768)
-    for (int h = 1; h + 2 <= maxHeight; ++h)
-      if (lowest(h) <= kTreeTops) return h;
+// The line between the trees on thread blocks and the cascades (iteration in
+// microseconds on batches of chains, written models x beams; FP64, mixed in brackets).
+// A block takes one chunk at a time whatever its fronts, so many chunks of few fronts
+// each leave most of its warps idle: 4,000 x 1 (one front a chunk) 420 (569) on trees
+// against 184 (210) on cascades, 1,000 x 8 209 (244) / 136 (153), 300 x 12 127 (144) /
+// 112 (128), 128 frames of 3 x 2 with 736 chunks 557 (582) / 526 (469).  Few chunks, or
+// well filled ones, spare the cascades' latency per tree level: 1 x 20 72 (84) / 84
+// (102), 64 chains of 8 reduced parts with 192 chunks 219 (275) / 264 (267), 150 x 20
+// with 246 chunks of 8 fronts 122 (133) / 122 (140), 64 x 150 with 556 of 11 183 (197) /
+// 228 (232).
+//   With more than 4,096 leaf fronts two blocks of 8 warps share an SM better than one
+// of 16, as long as the chunks are few enough: 300 x 40 with 1,572 chunks 196 (210) /
+// 219 (224); 1,000 x 12 with 1,832 187 (211) / 187 (197); 128 x 150 with 2,057 253
+// (273) / 251 (276).
+//   Otherwise the cascades take the fronts up to the height above which at most
+// kTreeTops subtrees begin, and the trees the levels from there, where the cascades run
+// out of fronts: 5 x 4,000 336 (339) / 404 (422), 30 x 600 with 259 chunks 318 (311) /
+// 353 (349), 100 x 300 with 248 375 (364) / 366 (392), but 250 x 100 with 413 265 (284) /
+// 245 (275).  (1,500 subtrees: with 300, 600 or 3,000 up to 9 % slower.)  Above 32,768
+// leaf fronts other models' fronts fill the cascades' upper levels (64,000: 675 / 689,
+// FP64 727 / 749).
+int treeTopHeight(int maxHeight, const std::function<long long(int)>& lowest) {
+  for (int h = 1; h + 2 <= maxHeight; ++h)
+    if (lowest(h) <= kTreeTops) return h;
   return -1;
+}
+
+bool treesPay(int nChunks, long long nFronts, int warps, int fromHeight) {
+  if (fromHeight > 0) return nChunks <= 300;
+  if (warps > 8) return nChunks <= 200 || 2 * nFronts >= (long long)warps * nChunks;
+  return nChunks <= 1800;
 }
 
 int treeWarps(int nLeaves, int maxRow, bool fp32) {

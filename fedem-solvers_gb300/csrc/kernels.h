@@ -313,10 +313,13 @@ void launchLargeBackward(const DevData& d, const PersistentPlan& p, bool fp32, i
 int largeBlocks(bool fp32, int sms);
 // values of L a block of the large-front solves stages for a front shared by G blocks
 int64_t largeSolveStage(int nr, int np, int G, size_t elemBytes);
-// the height from which a batch's small fronts go to the trees on thread blocks:
-// 0 (all of them), more (the cascades below it), or -1 (none), by its leaf fronts,
-// the largest height and the number of subtrees' lowest fronts from a height on
-int treeFromHeight(int nLeaves, int maxHeight, const std::function<long long(int)>& lowest);
+// The trees on thread blocks take all small fronts of a batch of at most kTreeAllLeaves
+// leaf fronts, or the levels from a height on (treeTopHeight, -1: none; lowest: the number
+// of subtrees' lowest fronts from a height on) of one of at most kTreeTopLeaves, where
+// the cut into chunks pays; else the cascades do.
+constexpr int kTreeAllLeaves = 8192, kTreeTopLeaves = 32768;
+int treeTopHeight(int maxHeight, const std::function<long long(int)>& lowest);
+bool treesPay(int nChunks, long long nFronts, int warps, int fromHeight);
 // their warps per block (and fronts per chunk) for nLeaves leaf fronts (0: the upper
 // levels of a larger batch) and fronts of at most maxRow rows; 0: too few fit
 int treeWarps(int nLeaves, int maxRow, bool fp32);
