@@ -1003,6 +1003,13 @@ int fgpu_batch_probe_root_wait_timeout(fgpu_batch* b, long long spins, int* flag
   return rc ? fail(rc, "root wait probe failed") : 0;
 }
 
+int fgpu_batch_probe_front_wait_timeout(fgpu_batch* b, int which, long long spins, int* flag) {
+  if (!b || spins < 1) return fail(-1, "bad argument");
+  OnDevice onDev(b->engine.device());
+  int rc = b->engine.probeFrontWaitTimeout(which, spins, flag);
+  return rc ? fail(rc, "front wait probe failed") : 0;
+}
+
 int fgpu_probe_refuse_launch(int n) {
   const int left = t_refuseLaunch;
   t_refuseLaunch = n;

@@ -2371,6 +2371,66 @@ int Engine::probeRootWaitTimeout(long long spins, int* flag) {
   return 0;
 }
 
+namespace {
+void readBack(void* dst, const void* src, size_t n) { cudaMemcpy(dst, src, n, cudaMemcpyDeviceToHost); }
+}  // namespace
+
+// The waits of the trees on thread blocks (0 an empty queue slot, 1 a root that nothing
+// releases) and of the large fronts (2 large children that nothing signals, 3 the second
+// block of a front), on counters and queues of the probe's own.
+int Engine::probeFrontWaitTimeout(int which, long long spins, int* flag) {
+  const bool tree = which < 2;
+  if (which < 0 || which > 3 || (tree ? pplan_.tree.warps : pplan_.nLarge) <= 0) return -957;
+  const int nL = pplan_.nLarge, nC = pplan_.tree.nChunks;
+  LargeTask task{-1, 0, 0, which == 3 ? 2 : 1};
+  int root = -1;
+  if (tree) {
+    std::vector<TreeChunk> chunks(nC);
+    readBack(chunks.data(), pplan_.tree.chunks, sizeof(TreeChunk) * nC);
+    for (int c = 0; c < nC && root < 0; ++c)
+      if (chunks[c].parent < 0 && chunks[c].model == 0) root = c;
+    if (root < 0) return -957;
+  } else {
+    const LargePlan& lp = pplan_.large[4];
+    std::vector<LargeTask> tasks((size_t)lp.nWaves * lp.grid);
+    std::vector<int> expect(nL), parent(nL), fmodel(d_.nfrontTot);
+    readBack(tasks.data(), lp.tasks, sizeof(LargeTask) * tasks.size());
+    readBack(expect.data(), lp.expect, sizeof(int) * nL);
+    readBack(parent.data(), lp.parent, sizeof(int) * nL);
+    readBack(fmodel.data(), d_.fModel, sizeof(int) * fmodel.size());
+    for (const LargeTask& t : tasks)
+      if (task.f < 0 && t.f >= 0 && fmodel[t.f] == 0 && (which == 2 ? expect[t.li] > 0 : parent[t.li] < 0)) {
+        task.f = t.f;
+        task.li = t.li;
+      }
+    if (task.f < 0) return -957;
+  }
+  // queue slot, {take 0, fill 1, total 1}; counters; the task
+  const size_t ints = 8 + (tree ? (size_t)nC + 1 : 2 * (size_t)nL), bytes = sizeof(int) * ints + sizeof(LargeTask);
+  int* q = nullptr;
+  if (cudaMalloc(&q, bytes) != cudaSuccess) return -955;
+  const int init[8] = {which == 1 ? root : -1, 0, 0, 0, 0, 1, 1, 0};
+  LargeTask* dTask = reinterpret_cast<LargeTask*>(q + ints);
+  int fl0 = 0, f = 0;
+  cudaMemsetAsync(q, 0, bytes, stream_);
+  cudaMemcpyAsync(q, init, sizeof(init), cudaMemcpyHostToDevice, stream_);
+  cudaMemcpyAsync(dTask, &task, sizeof(task), cudaMemcpyHostToDevice, stream_);
+  cudaMemcpyAsync(&fl0, d_.m.flags, sizeof(int), cudaMemcpyDeviceToHost, stream_);
+  cudaStreamSynchronize(stream_);
+  const int act = fl0 | FL_ACTIVE;  // model 0, marked active for the probe
+  cudaMemcpyAsync(d_.m.flags, &act, sizeof(int), cudaMemcpyHostToDevice, stream_);
+  takeLaunchError();
+  if (tree) launchTreeWaitProbe(d_, pplan_, opt_.fp32Factor, q, q + 4, q + 8, which == 1, spins, stream_);
+  else launchLargeWaitProbe(d_, pplan_, opt_.fp32Factor, dTask, q + 8, q + 8 + nL, which == 3, spins, stream_);
+  cudaMemcpyAsync(d_.m.flags, &fl0, sizeof(int), cudaMemcpyHostToDevice, stream_);
+  cudaMemcpyAsync(&f, pplan_.errFlag, sizeof(int), cudaMemcpyDeviceToHost, stream_);
+  const cudaError_t e = cudaStreamSynchronize(stream_);
+  cudaFree(q);
+  if (e != cudaSuccess || takeLaunchError() != cudaSuccess) return -956;
+  if (flag) *flag = f;
+  return 0;
+}
+
 void Engine::dropGraphs() {
   for (int k = 0; k < 2; ++k) {
     if (graphExec_[k]) cudaGraphExecDestroy(graphExec_[k]);

@@ -148,6 +148,7 @@ class Engine {
   int probeWaitTimeout(long long spins, int* flag);
   // the same for the fused back substitution's wait for a root's elimination
   int probeRootWaitTimeout(long long spins, int* flag);
+  int probeFrontWaitTimeout(int which, long long spins, int* flag);
 
   // fronts, large fronts, blocks of the large fronts' launches, chunks and warps per
   // block of the trees on thread blocks (0: none)

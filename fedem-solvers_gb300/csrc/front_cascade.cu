@@ -1394,4 +1394,18 @@ void launchRootWaitProbe(const DevData& d, const PersistentPlan& p, int* queue, 
             (const double*)d.asmVal64, d.L64, d.U64, 1.0e-12, (const double*)d.del, d.x64, d.w64, cnt, fb);
 }
 
+void launchTreeWaitProbe(const DevData& d, const PersistentPlan& p, bool fp32, int* queue, int* ctr, int* cnt,
+                         bool root, long long spins, cudaStream_t s) {
+  // one block of the trees without a chunk to eliminate takes queue slot 0: it is empty,
+  // or holds a root whose elimination nothing releases (cnt is zero); the wait gives up
+  // before any front is touched
+  PersistentPlan one = p;
+  one.tree.nStart = 0;
+  FusedBackward fb = backwardOf(p, fp32, 0, true, true);
+  fb.queue = queue;
+  fb.ctr = ctr;
+  fb.spinLimit = spins;
+  treeLaunch(d, one, fp32, d.del, cnt, fb, root, false, s);
+}
+
 }  // namespace fgpu

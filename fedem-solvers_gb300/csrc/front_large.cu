@@ -993,4 +993,30 @@ void launchLargeBackward(const DevData& d, const PersistentPlan& p, bool fp32, i
                fin);
 }
 
+void launchLargeWaitProbe(const DevData& d, const PersistentPlan& p, bool fp32, const LargeTask* task, int* done,
+                          int* bar, bool backward, long long spins, cudaStream_t s) {
+  // one block with one front: the forward elimination waits for children that nothing
+  // signals, the back substitution of a root for the second block of the front; each goes
+  // on to its end on what is there (the solve vectors and update vectors, which the next
+  // solve rewrites)
+  LargePlan lp = p.large[4];
+  lp.spinLimit = spins;
+  lp.tasks = task;
+  lp.nWaves = lp.grid = 1;
+  lp.done = done;
+  lp.bar = bar;
+  if (backward) {
+    if (fp32)
+      coopLaunch(kLargeBackward<float>, 1, solveShared<float>(lp), s, d, lp, (const float*)d.L32, d.x32, 1, 0);
+    else
+      coopLaunch(kLargeBackward<double>, 1, solveShared<double>(lp), s, d, lp, (const double*)d.L64, d.x64, 0, 0);
+  } else if (fp32) {
+    coopLaunch(kLargeForward<float>, 1, solveShared<float>(lp), s, d, lp, (const float*)d.L32, (const double*)d.del,
+               d.x32, d.w32);
+  } else {
+    coopLaunch(kLargeForward<double>, 1, solveShared<double>(lp), s, d, lp, (const double*)d.L64,
+               (const double*)d.del, d.x64, d.w64);
+  }
+}
+
 }  // namespace fgpu

@@ -403,4 +403,12 @@ void launchRefineResidual(const DevData& d, cudaStream_t s);
 // batch's device (made current for the launch).
 int normsNoAlloc(const DevData& d, int m, int c0, int nc, int dev, cudaStream_t s, double* out18, std::string& err);
 
+// One block of the trees, or of a large-front solve, that waits at most `spins` polls for
+// what nothing gives: an empty queue slot 0 or (root) the elimination of the root in it;
+// the large children of a task's front or (backward) the second of its blocks.
+void launchTreeWaitProbe(const DevData& d, const PersistentPlan& p, bool fp32, int* queue, int* ctr, int* cnt,
+                         bool root, long long spins, cudaStream_t s);
+void launchLargeWaitProbe(const DevData& d, const PersistentPlan& p, bool fp32, const LargeTask* task, int* done,
+                          int* bar, bool backward, long long spins, cudaStream_t s);
+
 }  // namespace fgpu

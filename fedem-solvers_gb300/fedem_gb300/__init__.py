@@ -101,6 +101,7 @@ def load_library(path=None):
         "fgpu_batch_probe_wait_timeout": (c_int, [vp, c_ll, P(c_int)]),
         "fgpu_batch_probe_root_wait_timeout": (c_int, [vp, c_ll, P(c_int)]),
         "fgpu_batch_front_plan": (c_int, [vp, P(c_ll)]),
+        "fgpu_batch_probe_front_wait_timeout": (c_int, [vp, c_int, c_ll, P(c_int)]),
         "fgpu_probe_refuse_launch": (c_int, [c_int]),
         "fgpu_measure_fp64_peak": (c_int, [P(c_dbl), P(c_dbl)]),
         "fgpu_measure_tf32_mma_peak": (c_int, [P(c_dbl), P(c_dbl)]),

@@ -207,6 +207,14 @@ int fgpu_batch_probe_wait_timeout(fgpu_batch* b, long long spins, int* flag);
  * polls and sets the wait-error flag (*flag = 1).  No front is touched; the
  * running models then fail with status 16 as above. */
 int fgpu_batch_probe_root_wait_timeout(fgpu_batch* b, long long spins, int* flag);
+/* The same for the waits of the other front kernels: which = 0 a block of the
+ * small-front trees waits for an empty queue slot, 1 for the elimination of a
+ * root that nothing releases, 2 a large front's forward elimination for large
+ * children that nothing signals, 3 a root's back substitution for the second
+ * of its blocks.  Counters and queues are the probe's own; 2 and 3 go on to
+ * their end and overwrite solve vectors that the next solve rewrites.  Fails
+ * (-957) where the batch has no such front. */
+int fgpu_batch_probe_front_wait_timeout(fgpu_batch* b, int which, long long spins, int* flag);
 /* Test hook of the failure path of a launch: the n-th kernel launch that the
  * calling host thread makes from now asks for more shared memory than any
  * device has, which the runtime refuses on the host (n = 0: off).  The call
