@@ -155,6 +155,22 @@ def shard(cases, rank, world):
     return sorted(mine)
 
 
+# the keys of the result line; every other one is printed before it, on a line of its own
+RESULT_KEYS = ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
+               "vs_baseline", "dtype", "data", "config", "e2e", "gpu_launches", "clocks", "roofline", "cpu_baseline",
+               "time_steps_per_s", "kernels_per_batched_iteration", "batched_iterations", "models_failed",
+               "speedup_mixed_vs_batched_fp64", "max_rel_disp_err_mixed_vs_fp64", "speedup_vs_plain")
+
+
+def print_result(line):
+    """The result as the one JSON line, short enough to be kept whole by whoever captures the
+    output; the legs and details before it as `leg <key>: <json>`."""
+    for key in line:
+        if key not in RESULT_KEYS:
+            print(f"leg {key}: {json.dumps(line[key])}")
+    print(json.dumps({k: line[k] for k in line if k in RESULT_KEYS}), flush=True)
+
+
 def workload_config(args, cases):
     """The `config` of both arms: the same workload and the same timing boundary."""
     n_el = sum(c[2] for c in cases)
@@ -881,7 +897,7 @@ def main():
                 "value_definition": "Newton iterations of all models / device time of the batched mixed run, "
                                     "state resident in HBM (restored device-to-device between steps)"}
         line.update(extras)
-        print(json.dumps(line), flush=True)
+        print_result(line)
     if dist:
         dist.destroy_process_group()
 
