@@ -1300,14 +1300,35 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
       FG_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
       // (FGPU_LARGE_SMS set at batch creation: as on a partition of so many SMs)
       if (const char* e = std::getenv("FGPU_LARGE_SMS")) sms = std::max(1, std::min(sms, std::atoi(e)));
-      sms = largeBlocks(opt_.fp32Factor, sms);
-      if (sms < 1) { err = "large-front kernels do not fit on the device"; return -905; }
+      const int perFactor = largeBlocksPerSm(opt_.fp32Factor, false, false, 0);
+      const int perSolve = largeBlocksPerSm(opt_.fp32Factor, true, false, kMaxDynamicShared);
+      if (perFactor < 1 || perSolve < 1) { err = "large-front kernels do not fit on the device"; return -905; }
       const int levels = 1 + *std::max_element(level.begin(), level.end());
       std::vector<std::vector<int>> byLevel(levels);
       for (int li = 0; li < nL; ++li) byLevel[level[li]].push_back(li);
+      // Where at least half of the levels have more fronts than there are SMs, those
+      // levels take several blocks per SM, so that one front's waits hide behind another's
+      // work; the solves only where the blocks of an SM can stage every front's L whole.
+      // (Milliseconds for 5 steps of 256 chains of 16 reduced parts, FP64 and mixed, one
+      // block per SM against several: 19.7, 21.5 / 15.9, 16.2; of 256 frames of 3 x 2:
+      // 6.1, 5.6 / 5.3, 4.3.)  The kernels for it have fewer registers, which costs fronts
+      // shared by many blocks more than it gives: 16 towers, two of whose 14 levels are so
+      // wide, 17.3, 9.8 / 23.8, 10.0; 128 frames of 3 x 2, two of six, 4.2, 3.7 / 4.5, 3.5.
+      int64_t stageWhole = 0;
+      for (int li = 0; li < nL; ++li)
+        stageWhole = std::max(stageWhole, largeSolveStage(nrow[lf[li]], npiv[lf[li]], 1, elemB));
+      const int wideFactor = largeBlocksPerSm(opt_.fp32Factor, false, true, 0);
+      const int wideSolve =
+          largeBlocksPerSm(opt_.fp32Factor, true, true, largeSolveShared(base.maxRow, stageWhole, elemB));
+      int wideLevels = 0;
+      for (const auto& level : byLevel) wideLevels += (int)level.size() > sms;
+      const bool many = 2 * wideLevels >= levels;
       for (int shape = 0; shape < 5; ++shape) {
         const bool solve = shape == 4;
         const int cap = std::max(1, solve ? sms : sms * (2 << shape) / 16);
+        // (shares of the GPU stay shares)
+        const int capWide = cap * std::max(1, !many ? 1 : solve ? wideSolve : shape == 3 ? wideFactor : 1);
+        bool wide = false;
         // blocks a front can use: factorisation, four trailing blocks of the first
         // panel per thread block (one per sub-core); solves, 64 rows below the
         // pivots or 8 pivots (a warp each) per thread block, at most 16
@@ -1324,8 +1345,10 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
         for (int l = 0; l < levels; ++l) {
           std::vector<int> order = byLevel[l];
           std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return wanted(a) > wanted(b); });
-          for (size_t i0 = 0; i0 < order.size(); i0 += (size_t)cap) {
-            const size_t i1 = std::min(order.size(), i0 + (size_t)cap);
+          const int cw = (int)order.size() > cap ? capWide : cap;
+          wide |= cw > cap;
+          for (size_t i0 = 0; i0 < order.size(); i0 += (size_t)cw) {
+            const size_t i1 = std::min(order.size(), i0 + (size_t)cw);
             long long sum = 0;
             for (size_t i = i0; i < i1; ++i) sum += wanted(order[i]);
             std::vector<std::pair<int, int>> w;
@@ -1333,8 +1356,8 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
             for (size_t i = i0; i < i1; ++i) {
               // every front gets a block; the rest in proportion to what it can use
               long long g = wanted(order[i]);
-              const int rest = cap - used - (int)(i1 - i - 1);
-              if (sum > cap) g = std::max<long long>(1, g * cap / sum);
+              const int rest = cw - used - (int)(i1 - i - 1);
+              if (sum > cw) g = std::max<long long>(1, g * cw / sum);
               g = std::min<long long>(g, rest);
               w.push_back({order[i], (int)g});
               used += (int)g;
@@ -1345,7 +1368,7 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
         }
         // the solves take the blocks in turn from wave to wave: a block that waits
         // for its next front has the waves between to load that front's L
-        if (solve) width = cap;
+        if (solve) width = wide ? capWide : cap;
         tasks.assign(waves.size() * (size_t)width, LargeTask{-1, 0, 0, 1});
         int next = 0;
         for (size_t w = 0; w < waves.size(); ++w) {
@@ -1370,6 +1393,7 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
         pplan_.large[shape].expect = de;
         pplan_.large[shape].nWaves = (int)waves.size();
         pplan_.large[shape].grid = width;
+        pplan_.large[shape].wide = wide;
         pplan_.large[shape].stageCap = stageCap;
       }
     }

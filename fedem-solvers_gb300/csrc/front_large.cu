@@ -484,8 +484,8 @@ __device__ inline void scanWaves(const DevData& d, const LargePlan& lp, int base
   __syncthreads();
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kLT, 1) kLargeFactor(DevData d, LargePlan lp, const T* asmVal, T* Lbase, T* Ubase,
+template <typename T, int PER_SM>
+__global__ void __launch_bounds__(kLT, PER_SM) kLargeFactor(DevData d, LargePlan lp, const T* asmVal, T* Lbase, T* Ubase,
                                                      double tolFact) {
   pdlEntry();
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -742,8 +742,8 @@ __device__ void forwardLarge(const DevData& d, const LargePlan& lp, const LargeT
   }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kLT, 1) kLargeForward(DevData d, LargePlan lp, const T* Lbase, const double* rhs, T* X,
+template <typename T, int PER_SM>
+__global__ void __launch_bounds__(kLT, PER_SM) kLargeForward(DevData d, LargePlan lp, const T* Lbase, const double* rhs, T* X,
                                                       T* W) {
   pdlEntry();
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -879,8 +879,8 @@ __device__ void backwardLarge(const DevData& d, const LargePlan& lp, const Large
   }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kLT, 1) kLargeBackward(DevData d, LargePlan lp, const T* Lbase, T* X, int acc,
+template <typename T, int PER_SM>
+__global__ void __launch_bounds__(kLT, PER_SM) kLargeBackward(DevData d, LargePlan lp, const T* Lbase, T* X, int acc,
                                                        int finalize) {
   pdlEntry();
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -910,40 +910,69 @@ void coopLaunch(void (*kernel)(KArgs...), int grid, size_t smem, cudaStream_t s,
   launchWith(attr, 1, kernel, dim3(grid), dim3(kLT), smem, s, args...);
 }
 
+// blocks per SM of the kernels for plans with levels of more fronts than SMs
+// (registers: 80 and 64 a thread, the factorisation's with 50 to 110 bytes spilled)
+constexpr int kWideFactor = 3, kWideSolve = 4;
+
 template <typename T>
 size_t solveShared(const LargePlan& lp) {
-  return (size_t)(lp.maxRow + kLT + lp.stageCap) * sizeof(T);
+  return largeSolveShared(lp.maxRow, lp.stageCap, sizeof(T));
 }
 
 }  // namespace
 
-// Blocks of a cooperative launch must all be resident: at most as many as the device
-// (or the partition of it that this process has) holds of each kernel at once, and one
-// per SM.  The solves are asked with the most shared memory they can take.
-int largeBlocks(bool fp32, int sms) {
-  auto resident = [&](auto kernel, size_t smem) {
-    int perSm = 0;
+// Blocks of a cooperative launch must all be resident: as many per SM as the device holds
+// of each kernel at once, one, or (wide: batches of many fronts, see Engine::upload) up to
+// kWideFactor and kWideSolve.
+int largeBlocksPerSm(bool fp32, bool solve, bool wide, size_t smem) {
+  auto resident = [&](auto kernel, size_t bytes, int most) {
+    int n = 0;
     if (allowBigShared(kernel) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, kLT, smem) != cudaSuccess) {
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kLT, bytes) != cudaSuccess) {
       cudaGetLastError();
       return 0;
     }
-    return perSm * sms;
+    return std::min(n, most);
   };
-  if (fp32)
-    return std::min({sms, resident(kLargeFactor<float>, sizeof(FactorShared<float>)),
-                     resident(kLargeForward<float>, kMaxDynamicShared),
-                     resident(kLargeBackward<float>, kMaxDynamicShared)});
-  return std::min({sms, resident(kLargeFactor<double>, sizeof(FactorShared<double>)),
-                   resident(kLargeForward<double>, kMaxDynamicShared),
-                   resident(kLargeBackward<double>, kMaxDynamicShared)});
+  auto of = [&](auto zero) {
+    using T = decltype(zero);
+    const size_t fs = sizeof(FactorShared<T>);
+    if (!solve)
+      return wide ? resident(kLargeFactor<T, kWideFactor>, fs, kWideFactor) : resident(kLargeFactor<T, 1>, fs, 1);
+    return wide ? std::min(resident(kLargeForward<T, kWideSolve>, smem, kWideSolve),
+                           resident(kLargeBackward<T, kWideSolve>, smem, kWideSolve))
+                : std::min(resident(kLargeForward<T, 1>, smem, 1), resident(kLargeBackward<T, 1>, smem, 1));
+  };
+  return fp32 ? of(0.0f) : of(0.0);
 }
+
+size_t largeSolveShared(int maxRow, int64_t stage, size_t elemBytes) { return (maxRow + kLT + stage) * elemBytes; }
 
 // at most about 200 KB of staged L per block
 int64_t largeSolveStage(int nr, int np, int G, size_t elemBytes) {
   const int64_t want = std::max(forwardStage(nr, np, G), backwardStage(nr, np, G));
   return std::min<int64_t>(want, (int64_t)(200 * 1024 / elemBytes));
 }
+
+namespace {
+template <typename T>
+void factorLaunch(const DevData& d, const LargePlan& lp, const T* asmVal, T* L, T* U, cudaStream_t s) {
+  coopLaunch(lp.wide ? kLargeFactor<T, kWideFactor> : kLargeFactor<T, 1>, lp.grid, sizeof(FactorShared<T>), s, d, lp,
+             asmVal, L, U, 1.0e-12);
+  // the inverses of the pivot blocks, for the solves
+  pdlLaunch(kLargeInverse<T>, lp.nInvBlk, 128, 0, s, d, lp, (const T*)L);
+}
+template <typename T>
+void forwardLaunch(const DevData& d, const LargePlan& lp, const T* L, const double* rhs, T* X, T* W, cudaStream_t s) {
+  coopLaunch(lp.wide ? kLargeForward<T, kWideSolve> : kLargeForward<T, 1>, lp.grid, solveShared<T>(lp), s, d, lp, L,
+             rhs, X, W);
+}
+template <typename T>
+void backwardLaunch(const DevData& d, const LargePlan& lp, const T* L, T* X, int acc, int fin, cudaStream_t s) {
+  coopLaunch(lp.wide ? kLargeBackward<T, kWideSolve> : kLargeBackward<T, 1>, lp.grid, solveShared<T>(lp), s, d, lp, L,
+             X, acc, fin);
+}
+}  // namespace
 
 void launchLargeFactor(const DevData& d, const PersistentPlan& p, bool fp32, cudaStream_t s) {
   if (p.nLarge <= 0) return;
@@ -954,15 +983,8 @@ void launchLargeFactor(const DevData& d, const PersistentPlan& p, bool fp32, cud
   lp.spinLimit = p.spinLimit;
   lp.done = p.cntLarge;
   lp.bar = p.cntLarge + p.nLarge;
-  if (fp32)
-    coopLaunch(kLargeFactor<float>, lp.grid, sizeof(FactorShared<float>), s, d, lp, (const float*)d.asmVal32, d.L32,
-               d.U32, 1.0e-12);
-  else
-    coopLaunch(kLargeFactor<double>, lp.grid, sizeof(FactorShared<double>), s, d, lp, (const double*)d.asmVal64, d.L64,
-               d.U64, 1.0e-12);
-  // the inverses of the pivot blocks, for the solves
-  if (fp32) pdlLaunch(kLargeInverse<float>, lp.nInvBlk, 128, 0, s, d, lp, (const float*)d.L32);
-  else pdlLaunch(kLargeInverse<double>, lp.nInvBlk, 128, 0, s, d, lp, (const double*)d.L64);
+  if (fp32) factorLaunch<float>(d, lp, d.asmVal32, d.L32, d.U32, s);
+  else factorLaunch<double>(d, lp, d.asmVal64, d.L64, d.U64, s);
 }
 
 void launchLargeForward(const DevData& d, const PersistentPlan& p, bool fp32, const double* rhs, int sweep,
@@ -971,11 +993,8 @@ void launchLargeForward(const DevData& d, const PersistentPlan& p, bool fp32, co
   LargePlan lp = p.large[4];
   lp.spinLimit = p.spinLimit;
   lp.done = p.cntLarge + (size_t)(2 + 3 * sweep) * p.nLarge;
-  if (fp32)
-    coopLaunch(kLargeForward<float>, lp.grid, solveShared<float>(lp), s, d, lp, (const float*)d.L32, rhs, d.x32, d.w32);
-  else
-    coopLaunch(kLargeForward<double>, lp.grid, solveShared<double>(lp), s, d, lp, (const double*)d.L64, rhs, d.x64,
-               d.w64);
+  if (fp32) forwardLaunch<float>(d, lp, d.L32, rhs, d.x32, d.w32, s);
+  else forwardLaunch<double>(d, lp, d.L64, rhs, d.x64, d.w64, s);
 }
 
 void launchLargeBackward(const DevData& d, const PersistentPlan& p, bool fp32, int sweep, bool last, cudaStream_t s) {
@@ -986,11 +1005,8 @@ void launchLargeBackward(const DevData& d, const PersistentPlan& p, bool fp32, i
   lp.spinLimit = p.spinLimit;
   lp.done = p.cntLarge + (size_t)(3 + 3 * sweep) * p.nLarge;
   lp.bar = p.cntLarge + (size_t)(4 + 3 * sweep) * p.nLarge;
-  if (fp32)
-    coopLaunch(kLargeBackward<float>, lp.grid, solveShared<float>(lp), s, d, lp, (const float*)d.L32, d.x32, acc, fin);
-  else
-    coopLaunch(kLargeBackward<double>, lp.grid, solveShared<double>(lp), s, d, lp, (const double*)d.L64, d.x64, acc,
-               fin);
+  if (fp32) backwardLaunch<float>(d, lp, d.L32, d.x32, acc, fin, s);
+  else backwardLaunch<double>(d, lp, d.L64, d.x64, acc, fin, s);
 }
 
 void launchLargeWaitProbe(const DevData& d, const PersistentPlan& p, bool fp32, const LargeTask* task, int* done,
@@ -1006,16 +1022,12 @@ void launchLargeWaitProbe(const DevData& d, const PersistentPlan& p, bool fp32, 
   lp.done = done;
   lp.bar = bar;
   if (backward) {
-    if (fp32)
-      coopLaunch(kLargeBackward<float>, 1, solveShared<float>(lp), s, d, lp, (const float*)d.L32, d.x32, 1, 0);
-    else
-      coopLaunch(kLargeBackward<double>, 1, solveShared<double>(lp), s, d, lp, (const double*)d.L64, d.x64, 0, 0);
+    if (fp32) backwardLaunch<float>(d, lp, d.L32, d.x32, 1, 0, s);
+    else backwardLaunch<double>(d, lp, d.L64, d.x64, 0, 0, s);
   } else if (fp32) {
-    coopLaunch(kLargeForward<float>, 1, solveShared<float>(lp), s, d, lp, (const float*)d.L32, (const double*)d.del,
-               d.x32, d.w32);
+    forwardLaunch<float>(d, lp, d.L32, d.del, d.x32, d.w32, s);
   } else {
-    coopLaunch(kLargeForward<double>, 1, solveShared<double>(lp), s, d, lp, (const double*)d.L64,
-               (const double*)d.del, d.x64, d.w64);
+    forwardLaunch<double>(d, lp, d.L64, d.del, d.x64, d.w64, s);
   }
 }
 

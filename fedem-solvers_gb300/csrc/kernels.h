@@ -202,6 +202,7 @@ struct LargeTask {
 struct LargePlan {
   const LargeTask* tasks = nullptr;
   int nWaves = 0, grid = 0;
+  bool wide = false;             // some level has more fronts than SMs: several blocks per SM
   const int* expect = nullptr;   // per large front: signals of its large children's blocks
   const int* parent = nullptr;   // per large front: its (large) parent's ordinal, or -1
   // inverse row maps: inv[invOff[li] + c * nrow + i] = update row of child c at row i, or -1
@@ -309,8 +310,10 @@ void launchLargeFactor(const DevData& d, const PersistentPlan& p, bool fp32, cud
 void launchLargeForward(const DevData& d, const PersistentPlan& p, bool fp32, const double* rhs, int sweep,
                         cudaStream_t s);
 void launchLargeBackward(const DevData& d, const PersistentPlan& p, bool fp32, int sweep, bool last, cudaStream_t s);
-// blocks the large-front launches may have on a device of `sms` SMs (0: they do not fit)
-int largeBlocks(bool fp32, int sms);
+// blocks per SM of the large fronts' factorisation, or of their solves with so many bytes
+// of shared memory a block (0: not one fits); wide: more than one, see LargePlan
+int largeBlocksPerSm(bool fp32, bool solve, bool wide, size_t smem);
+size_t largeSolveShared(int maxRow, int64_t stage, size_t elemBytes);
 // values of L a block of the large-front solves stages for a front shared by G blocks
 int64_t largeSolveStage(int nr, int np, int G, size_t elemBytes);
 // The trees on thread blocks take all small fronts of a batch of at most kTreeAllLeaves
