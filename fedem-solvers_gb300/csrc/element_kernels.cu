@@ -117,7 +117,9 @@ __device__ inline void seedBackward(const BackwardSeed& b, int i, int lane, int 
 // other they were most of the launch).
 // With more than kSeedWarpRoots roots in a model's queues (a chain of 33,333 beams has
 // 1,500 in each of two), sixteen warps per model, the books by the first: one warp's
-// rounds of stores took 28.6 us, these 10.5.
+// rounds of stores took 28.6 us, these 10.5.  (Mixed iterations, one warp / sixteen: 1,536
+// roots 468 / 448 us, 576 496 / 489, 384 567 / 560, 160 467.6 / 465.6; 256 models of 2
+// roots 355 / 358.)
 constexpr int kSeedWarpRoots = 256, kSeedWarps = 16;
 template <int WARPS>
 __global__ void __launch_bounds__(WARPS > 1 ? 32 * WARPS : 128) kBeginStep(DevModels m, int* activeCount, long long* activeEl, BackwardSeed bs) {
@@ -880,7 +882,7 @@ __global__ void kResidual(DevData d) {
       v1 = b[1];
       v2 = b[2];
       v3 = b[3];
-        return;
+      return;
     }
     const bool el = s < blk;
     const double* b = el ? d.Fel + s : d.FelA + (s - blk);
@@ -1366,9 +1368,11 @@ __device__ inline bool isBad(double v) { return !(fabs(v) <= 1.0e300); }
 constexpr int NPART = 21;
 constexpr int CHUNK_TPB = 256;
 constexpr int kNormWarps = CHUNK_TPB / 32;
-// at most so many chunks as clusters of one-warp blocks (a chain of 3,827 beams, 12
-// chunks: 15.9 us a launch with 8-warp blocks; with 98 chunks, 784 warps for 608
-// sub-cores, the pass and its neighbours lost 6 us)
+// at most so many chunks as clusters of one-warp blocks (an iteration in microseconds with
+// them / with 8-warp blocks, FP64: a chain of 2,700 beams, 8 chunks, 139.5 / 143.5; of
+// 5,500, 17 chunks, 207.3 / 206.1; of 16,400, 49 chunks, 356.4 / 357.1; 32 chains of 100
+// 133.7 / 134.6, 48 145.7 / 144.9, 96 182.7 / 180.9: level between 17 and 48 chunks, 1 %
+// slower from there)
 constexpr int kWideNormChunks = 48;
 
 // the larger pattern, by 32-bit subtractions with borrow

@@ -300,8 +300,13 @@ struct PersistentPlan {
 // blocks each (front_large.cu); smaller ones by one warp each in shared memory.
 // 8 steps of the space-frame tower with the line at 96 / 64 / 48 rows: FP64 16.1 /
 // 15.6 / 13.8 ms, mixed 14.7 / 14.1 / 13.0; 20 steps of 16 reduced parts, FP64 (80
-// row leaf fronts): 24.4 / 19.9 / 19.0 ms.  Fronts of beam chains (up to 36 rows)
-// stay below it: there the trees' parallelism suffices.
+// row leaf fronts): 24.4 / 19.9 / 19.0 ms.  Batches, an iteration in microseconds at
+// 96 / 64 / 48, FP64 (mixed): 4 such towers 1168 / 1008 / 1005 (767 / 773 / 660), 16
+// frames of 6 x 3 737 / 672 / 662 (606 / 506 / 565), 128 of 3 x 2 713 / 560 / 529 (601 /
+// 493 / 467), 16 chains of 16 parts 371 / 287 / 287 (303 / 291 / 291).  Chains of 8 parts
+// of 32 DOFs, whose largest fronts have 60 rows, are better off at 64: 64 of them 205 / 204
+// / 220 (197 / 197 / 273).  Fronts of beam chains (up to 30 rows) stay below it: there the
+// trees' parallelism suffices.
 constexpr int kLargeFrontRows = 48;
 // the large-front kernels: factorisation (tangent models), forward elimination
 // of rhs and back substitution (active models; before the warp queue's small
