@@ -1321,7 +1321,7 @@ int Engine::upload(const std::vector<const HostModel*>& models, const EngineOpti
       const int wideSolve =
           largeBlocksPerSm(opt_.fp32Factor, true, true, largeSolveShared(base.maxRow, stageWhole, elemB));
       int wideLevels = 0;
-      for (const auto& level : byLevel) wideLevels += (int)level.size() > sms;
+      for (const auto& fronts : byLevel) wideLevels += (int)fronts.size() > sms;
       const bool many = 2 * wideLevels >= levels;
       for (int shape = 0; shape < 5; ++shape) {
         const bool solve = shape == 4;
